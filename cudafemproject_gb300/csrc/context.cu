@@ -43,8 +43,7 @@ MvParams<T> base_mv_t(cfem_ctx *c) {
 
 template <typename T>
 void launch_mv_t(cfem_ctx *c, int mode, const MvParams<T> &P) {
-  if (c->n_inst && !P.patch_inst)
-    throw Fail{CFEM_ERR_UNSUPPORTED, "a context of batched meshes supports cfem_batch_static_solve only"};
+  if (!P.patch_inst) single_mesh_only(c);
   // FP32: patch blocks streamed by bulk copies. FP64 keeps the plain fan
   // kernel below: it is bound by the FP64 pipe, and its twice-as-large blocks
   // would leave one CTA per SM.
@@ -368,32 +367,7 @@ void to_internal_f(cfem_ctx *c, const double *src, float *dst, double scale) { t
 void to_caller_d(cfem_ctx *c, const double *src, double *dst) { to_caller_t<double>(c, src, dst); }
 void to_caller_f(cfem_ctx *c, const float *src, double *dst) { to_caller_t<float>(c, src, dst); }
 
-// FP64 true residual r = f - K' x (f, x internal FP64; x == nullptr stands
-// for x = 0), ||r||^2 and ||f||^2 into the device doubles out2[0], out2[1];
-// queued on the context's stream.
-void true_residual_async(cfem_ctx *c, const double *f, const double *x, double *r, float *r32, double *out2) {
-  c->tmp64.zero(c->stream);
-  if (x) {  // (x == nullptr: x = 0, K' x = 0)
-    MvParams<double> mv = base_mv<double>(c);
-    mv.diagA = c->diagK.p;
-    mv.x = x;
-    mv.y = c->tmp64.p;
-    launch_mv<double>(c, MV_PLAIN, mv);
-  }
-  ResParams P{};
-  P.nvec = c->nvec;
-  P.f = f;
-  P.u = c->tmp64.p;
-  P.r = r;
-  P.r32 = r32;
-  P.out = out2;
-  P.partials = c->partials.p;
-  P.count = c->counters.p;
-  k_residual<<<c->grid_vec, kThreads, 0, c->stream>>>(P);
-  CKL();
-}
-
-// The same, waited for: returns ||r||^2, ||f||^2.
+// The true residual (true_residual_async), waited for: returns ||r||^2, ||f||^2.
 void true_residual(cfem_ctx *c, const double *f, const double *x, double *r, float *r32, double &rr, double &ff) {
   true_residual_async(c, f, x, r, r32, c->rr.p);
   CK(cudaMemcpyAsync(c->h_rr, c->rr.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -415,6 +389,7 @@ void set_diag_vectors(cfem_ctx *c, const double *diagA64) {
 // Static-type solve of K' x = f (f internal FP64 in c->v64.f). Result in c->v64.x.
 cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve_info *info) {
   cfem_solve_info inf{};
+  single_mesh_only(c);
   c->launches = 0;
   set_diag_vectors(c, c->diagK.p);
   CK(cudaEventRecord(c->ev0, c->stream));
@@ -875,7 +850,8 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
                                                      smem_max));
     c->grid_geo = (int)std::min<int64_t>(P.n_patches, (int64_t)c->n_sm * std::max(og, 1));
   }
-  int maxgrid = std::max({c->grid_mv, c->grid_vec, c->grid_fan, c->grid_ft32, c->grid_geo});
+  c->grid_rows = c->n_sm * 16;
+  int maxgrid = std::max({c->grid_mv, c->grid_vec, c->grid_fan, c->grid_ft32, c->grid_geo, c->grid_rows});
   c->partials.alloc((size_t)maxgrid * 4);
   c->partials_up.alloc((size_t)std::max(c->grid_upd, c->grid_vec) * 2);
   c->partials_up.zero(s);
@@ -997,6 +973,7 @@ void rebuild_operator(cfem_ctx *c) {
   CK(cudaMemcpyAsync(&herr, c->err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   if (herr) throw Fail{CFEM_ERR_MESH, "an element has zero or non-finite volume"};
+  build_rows(c);
 }
 
 void enter(cfem_ctx *c) {
@@ -1262,14 +1239,10 @@ cfem_status cfem_matvec(cfem_ctx *ctx, int32_t precision, const void *x, void *y
     check_ctx(ctx);
     enter(ctx);
     if (!x || !y) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "null vector"};
+    single_mesh_only(ctx);
     if (precision == CFEM_FP64) {
       to_internal<double>(ctx, (const double *)x, ctx->v64.z.p);
-      MvParams<double> mv = base_mv<double>(ctx);
-      mv.diagA = ctx->diagK.p;
-      mv.x = ctx->v64.z.p;
-      mv.y = ctx->tmp64.p;
-      ctx->tmp64.zero(ctx->stream);
-      launch_mv<double>(ctx, MV_PLAIN, mv);
+      rows_apply(ctx, ctx->v64.z.p, ctx->tmp64.p);
       to_caller<double>(ctx, ctx->tmp64.p, (double *)y);
     } else if (precision == CFEM_FP32) {
       // float in/out: stage through FP64 conversion buffers
@@ -1340,6 +1313,7 @@ cfem_status cfem_profile_matvec(cfem_ctx *ctx, int32_t precision, int32_t n_laun
   return run_guarded([&]() -> cfem_status {
     check_ctx(ctx);
     if (n_launches <= 0) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "n_launches must be positive"};
+    single_mesh_only(ctx);
     // scalars that make the kernel take its full path: an update has run
     // (u_iter 0) whose partials give r.z = 1 against gamma_prev = 1, so
     // beta = 1, and no stopping rule fires

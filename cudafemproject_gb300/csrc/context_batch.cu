@@ -132,17 +132,6 @@ void run_batch_pcg(cfem_ctx *c, BatchBufs &B, double tol, int rule, int maxit, s
   CK(cudaMemcpy(out.data(), B.isc.p, sizeof(Scalars) * c->n_inst, cudaMemcpyDeviceToHost));
 }
 
-// tmp64 = K64 x64 (all instances, FP64 operator with per-patch materials)
-void batch_kx(cfem_ctx *c, BatchBufs &B) {
-  MvParams<double> mv = base_mv<double>(c);
-  mv.diagA = c->diagK.p;
-  batch_mv<double>(c, B, mv);
-  mv.x = c->v64.x.p;
-  mv.y = c->tmp64.p;
-  c->tmp64.zero(c->stream);
-  launch_mv<double>(c, MV_PLAIN, mv);
-}
-
 // r64 = f64 - tmp64 per instance; f32 = r64 on active instances, 0 elsewhere;
 // rr/ff per instance.
 void batch_residual(cfem_ctx *c, BatchBufs &B, const std::vector<int> &active, std::vector<double> &rr,
@@ -352,7 +341,7 @@ extern "C" cfem_status cfem_batch_static_solve(cfem_ctx *ctx, const cfem_solve_p
         }
         k_accumulate<<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->v32.x.p, c->v64.x.p, c->vw);
         CKL();
-        batch_kx(c, B);
+        rows_apply(c, c->v64.x.p, c->tmp64.p);
         batch_residual(c, B, none, rr, ff);
       }
     }
@@ -361,7 +350,7 @@ extern "C" cfem_status cfem_batch_static_solve(cfem_ctx *ctx, const cfem_solve_p
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
     if (p.precision == CFEM_FP32) {
-      batch_kx(c, B);
+      rows_apply(c, c->v64.x.p, c->tmp64.p);
       batch_residual(c, B, none, rr, ff);
     }
     to_caller<double>(c, c->v64.x.p, u);

@@ -105,6 +105,7 @@ void launch_dyn_correct(cfem_ctx *c, const DynParams<T> &P) {
 template <typename T>
 cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet *w, double *u_out, cfem_dyn_info *info,
                     const int32_t *elems_caller) {
+  single_mesh_only(c);
   const double beta1 = prm->beta1, beta2 = prm->beta2, dt = prm->dt;
   const bool expl = beta2 == 0.0;
   const float dtf = (float)prm->dt, endf = (float)prm->endtime;
@@ -317,6 +318,7 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
 cfem_status run_dyn_adjoint(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet *w, int n_rec,
                             const int32_t *rec_nodes, const double *obs, double *loss, double *dLdE,
                             cfem_dyn_info *info) {
+  single_mesh_only(c);
   if (prm->beta2 != 0.0) throw Fail{CFEM_ERR_UNSUPPORTED, "the dynamics adjoint covers the explicit scheme (beta2 = 0)"};
   if (c->semantics != CFEM_CONSISTENT)
     throw Fail{CFEM_ERR_UNSUPPORTED, "the dynamics adjoint needs consistent semantics (no per-step re-sorted masses)"};
@@ -450,11 +452,7 @@ cfem_status run_dyn_adjoint(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_
         k_grad_young<2><<<nblk(c->ne), kThreads, 0, c->stream>>>(c->ne, c->G64.p, c->gstride, c->conn.p, c->bits.p,
                                                                  c->lam, c->mu, wb.p, dn, young, c->elem_new2old.p,
                                                                  gE.p, 1);
-      MvParams<double> m2 = base_mv<double>(c);
-      m2.diagA = c->diagK.p;
-      m2.x = wb.p;
-      m2.y = y.p;
-      launch_mv<double>(c, MV_PLAIN, m2);
+      rows_apply(c, wb.p, y.p);
       k_adj_post<<<nblk(nv), kThreads, 0, c->stream>>>(nv, dt, c2, y.p, db.p, vb.p, ab.p);
       CKL();
     }

@@ -95,6 +95,20 @@ struct GraphCache {
   }
 };
 
+// FP64 operator as assembled node rows (kernels_rows.cuh): structure, and the
+// values of one combination of stiffness and mass.
+struct RowsValues {
+  DBuf<double> val, D;
+  DBuf<uint8_t> flag;
+};
+struct RowsData {
+  DBuf<int32_t> inc_off, inc;  // elements of every node
+  DBuf<int32_t> row, col;
+  DBuf<int64_t> off;
+  int64_t n_slices = 0, steps = 0;
+  RowsValues K;
+};
+
 inline unsigned nblk(int64_t n, int t = kThreads) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace detail
@@ -152,6 +166,8 @@ struct cfem_ctx {
   size_t smem_geo = 0;
   int grid_geo = 0;
   int np_slots = 0;               // node slots per patch in shared memory
+  RowsData rows;                  // FP64 operator
+  int grid_rows = 0;              // CTAs of a grid-stride kernel over its slices
   DBuf<uint8_t> bits;
   DBuf<double> coords, escale, young_d;
   // operator
@@ -248,6 +264,11 @@ void true_residual_async(cfem_ctx *c, const double *f, const double *x, double *
 void make_rhs(cfem_ctx *c, double a, double b, double *dst);
 cfem_status run_guarded(const std::function<cfem_status()> &fn);
 void check_ctx(const cfem_ctx *c);
+// Calls that take one mesh refuse a context of batched meshes.
+inline void single_mesh_only(const cfem_ctx *c) {
+  if (c->n_inst)
+    throw Fail{CFEM_ERR_UNSUPPORTED, "a context of batched meshes supports cfem_batch_static_solve only"};
+}
 // Throws if a bulk-copy wait of the edge-fan matvec timed out (synchronises the stream).
 // Launch with programmatic stream serialization: the kernel may start while
 // the previous kernel in the stream runs (it calls griddep_wait before reading
@@ -276,6 +297,9 @@ void enter(cfem_ctx *c);
 cfem_solve_params default_params();
 cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve_info *info);
 void rebuild_operator(cfem_ctx *c);
+void build_rows(cfem_ctx *c);
+// y = K' x in FP64 (internal node vectors; y is overwritten)
+void rows_apply(cfem_ctx *c, const double *x, double *y);
 void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, const cfem_options *opt);
 void attach_stream(cfem_ctx *c, cudaStream_t s);
 

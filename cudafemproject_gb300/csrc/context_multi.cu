@@ -440,6 +440,7 @@ extern "C" cfem_status cfem_pcg_multi(cfem_ctx *ctx, const cfem_solve_params *pr
     check_ctx(ctx);
     enter(ctx);
     if (k <= 0 || !F || !U) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "bad multi-RHS arguments"};
+    single_mesh_only(ctx);
     cfem_solve_params p = prm ? *prm : default_params();
     cfem_status worst = CFEM_OK;
     const bool batched = ctx->fans && ctx->fan_tma && k > 1 &&

@@ -1,0 +1,133 @@
+// Host side of the FP64 row operator (kernels_rows.cuh): construction when a
+// context is created or its moduli change, applications, true residuals.
+#include "context_internal.cuh"
+#include "kernels_aux.cuh"
+#include "kernels_rows.cuh"
+
+namespace cfem {
+namespace detail {
+
+namespace {
+
+template <int DIM>
+RowsAssembly<DIM> assembly(cfem_ctx *c, double cK, double cM, const double *diag) {
+  RowsAssembly<DIM> P{};
+  P.conn = c->conn.p;
+  P.inc_off = c->rows.inc_off.p;
+  P.inc = c->rows.inc.p;
+  P.G64 = c->G64.p;
+  P.gstride = c->gstride;
+  P.lam = c->lam;
+  P.mu = c->mu;
+  P.cK = cK;
+  P.cM = cM;
+  P.lam_e = c->lam_e.p;
+  P.mu_e = c->mu_e.p;
+  P.mc = c->mc64.p;
+  P.bits = c->bits.p;
+  P.diag = diag;
+  return P;
+}
+
+// Node-element incidences, neighbour lists, row order and slices; the
+// neighbour lists stay in `nbr` for the first assembly.
+template <int NV>
+void build_structure(cfem_ctx *c, DBuf<int32_t> &nbr, DBuf<int32_t> &deg) {
+  RowsData &R = c->rows;
+  cudaStream_t s = c->stream;
+  const int64_t nn = c->nn, n_inc = c->ne * NV;
+  DBuf<int32_t> cnt, steps;
+  cnt.alloc(nn);
+  cnt.zero(s);
+  k_rows_count<<<nblk(n_inc), kThreads, 0, s>>>(n_inc, c->conn.p, cnt.p);
+  R.inc_off.alloc(nn + 1);
+  k_rows_scan<int32_t><<<1, 1024, 0, s>>>(nn, cnt.p, R.inc_off.p);
+  cnt.zero(s);
+  R.inc.alloc(n_inc);
+  k_rows_fill<<<nblk(n_inc), kThreads, 0, s>>>(n_inc, NV, c->conn.p, R.inc_off.p, cnt.p, R.inc.p);
+  nbr.alloc((size_t)(NV - 1) * n_inc);
+  deg.alloc(nn);
+  k_rows_neighbours<NV><<<nblk(nn), kThreads, 0, s>>>(nn, c->conn.p, R.inc_off.p, R.inc.p, nbr.p, deg.p);
+  const int64_t windows = (nn + kRowWindow - 1) / kRowWindow;
+  R.row.alloc((size_t)windows * kRowWindow);
+  steps.alloc((size_t)windows * (kRowWindow / kSliceRows));
+  k_rows_order<<<(unsigned)windows, kRowWindow, 0, s>>>(nn, deg.p, R.row.p, steps.p);
+  R.n_slices = (nn + kSliceRows - 1) / kSliceRows;  // (the padding sorts last)
+  R.off.alloc(R.n_slices + 1);
+  k_rows_scan<int64_t><<<1, 1024, 0, s>>>(R.n_slices, steps.p, R.off.p);
+  CKL();
+  CK(cudaMemcpyAsync(&R.steps, R.off.p + R.n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));  // (cnt and steps are freed here, too)
+  R.col.alloc((size_t)R.steps * 32);
+}
+
+template <int DIM>
+void assemble_dim(cfem_ctx *c, const int32_t *nbr, const int32_t *deg, double cK, double cM, const double *diag,
+                  RowsValues &V) {
+  RowsData &R = c->rows;
+  cudaStream_t s = c->stream;
+  if (!V.val.p) {
+    V.val.alloc((size_t)R.steps * 32 * DIM * DIM);
+    V.D.alloc((size_t)c->nn * DIM * DIM);
+    V.flag.alloc(R.n_slices);
+  }
+  V.flag.zero(s);
+  const RowsAssembly<DIM> P = assembly<DIM>(c, cK, cM, diag);
+  k_rows_assemble<DIM><<<nblk(R.n_slices, 4), 128, 0, s>>>(P, R.n_slices, R.off.p, R.row.p, nbr, deg, R.col.p,
+                                                            V.val.p);
+  k_rows_corrections<DIM><<<nblk(R.n_slices * kSliceRows), kThreads, 0, s>>>(P, R.n_slices * kSliceRows, R.off.p,
+                                                                             R.row.p, R.col.p, V.D.p, V.flag.p);
+  CKL();
+}
+
+void assemble(cfem_ctx *c, const int32_t *nbr, const int32_t *deg, double cK, double cM, const double *diag,
+              RowsValues &V) {
+  if (c->dim == 3) assemble_dim<3>(c, nbr, deg, cK, cM, diag, V);
+  else assemble_dim<2>(c, nbr, deg, cK, cM, diag, V);
+}
+
+RowOp op_of(cfem_ctx *c, const RowsValues &V) {
+  const RowsData &R = c->rows;
+  return RowOp{R.n_slices, R.off.p, R.row.p, R.col.p, V.val.p, V.flag.p, V.D.p, c->bits.p};
+}
+
+unsigned rows_grid(const cfem_ctx *c) { return nblk(c->rows.n_slices, kRowsThreads / 32); }
+
+}  // namespace
+
+void build_rows(cfem_ctx *c) {
+  if (!c->rows.col.p) {
+    DBuf<int32_t> nbr, deg;
+    if (c->dim == 3) build_structure<4>(c, nbr, deg);
+    else build_structure<3>(c, nbr, deg);
+    assemble(c, nbr.p, deg.p, 1.0, 0.0, c->diagK.p, c->rows.K);
+    CK(cudaStreamSynchronize(c->stream));  // (before nbr and deg are freed)
+  } else {
+    assemble(c, nullptr, nullptr, 1.0, 0.0, c->diagK.p, c->rows.K);
+  }
+}
+
+void rows_apply(cfem_ctx *c, const double *x, double *y) {
+  const RowOp A = op_of(c, c->rows.K);
+  if (c->dim == 3) k_rows_apply<3, false><<<rows_grid(c), kRowsThreads, 0, c->stream>>>(A, x, y, nullptr);
+  else k_rows_apply<2, false><<<rows_grid(c), kRowsThreads, 0, c->stream>>>(A, x, y, nullptr);
+  CKL();
+  c->launches += 1;
+}
+
+// FP64 true residual r = f - K' x (f, x internal FP64; x == nullptr stands
+// for x = 0), ||r||^2 and ||f||^2 into the device doubles out2[0], out2[1];
+// queued on the context's stream.
+void true_residual_async(cfem_ctx *c, const double *f, const double *x, double *r, float *r32, double *out2) {
+  const RowOp A = op_of(c, c->rows.K);
+  RowsResidual P{c->nn, f, x, r, r32, out2, c->partials.p, c->counters.p};
+  // (grid-stride over the slices: the partial sums are one pair per block)
+  const unsigned g = std::min<unsigned>(rows_grid(c), c->grid_rows);
+  if (c->dim == 3) k_rows_residual<3><<<g, kRowsThreads, 0, c->stream>>>(A, P);
+  else k_rows_residual<2><<<g, kRowsThreads, 0, c->stream>>>(A, P);
+  CKL();
+  c->launches += 1;
+}
+
+}  // namespace detail
+}  // namespace cfem

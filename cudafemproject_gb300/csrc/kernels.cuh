@@ -48,7 +48,8 @@ struct Scalars {
   // update's block partials, 0 before the first direction): every CTA derives
   // them identically, so no thread divides differently
   double alpha, beta;
-  int loop_ok, pad2;  // device-side loop: the body count is within the cap (k_pcg_update)
+  int loop_ok;  // device-side loop: the body count is within the cap (k_pcg_update)
+  int stalled;  // one-kernel runs: a CTA did not arrive at a grid-wide sum in time
 };
 
 struct DynState {

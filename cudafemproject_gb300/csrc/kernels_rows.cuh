@@ -1,0 +1,749 @@
+// FP64 operator as assembled node rows.
+//
+// GB300's FP64 pipe is narrow (about 2 lanes per SM and cycle), and the FP64
+// element kernels were bound by it: 97 FP64 operations per tetrahedron, 580 per
+// node of a hex-derived mesh. Summed per node pair, the same operator costs 12
+// per neighbour, 168 per node (14 neighbours): y_i = sum_j K_ij (x_j - x_i).
+// The difference form needs no diagonal block (the rows of a stiffness sum to
+// zero) and rounds relative to the displacement differences, like the element
+// form; K_ij x_j with the diagonal block would be 135 operations, but its
+// rounding is relative to the displacements themselves, which raises the floor
+// of the true residual by the ratio of the two (about the number of elements
+// along the body).
+//
+// Constraints: K' = P K P + (I - P) diag(K). Stored blocks are P_i K_ij P_j;
+// what the difference form misses next to constrained DOFs, and the diagonal
+// of the constrained DOFs themselves, is a small block D_i per node, read only
+// by the row slices that need it (a flag per slice).
+//
+// Layout: rows are sorted by their neighbour count within windows of kRowWindow
+// nodes and cut into slices of 16 rows, one warp per slice, two lanes per row:
+// lane = 16 * half + r holds neighbours half, half + 2, ... of row r. Step k of
+// a slice is 32 column ids and, per block component, 32 doubles: every load of
+// the operator is one contiguous 256-byte line per warp. Unused entries repeat
+// the row itself (difference zero).
+#pragma once
+
+#include "grid_sync.cuh"
+#include "kernels.cuh"
+
+namespace cfem {
+
+constexpr int kRowWindow = 512;  // nodes among which rows are sorted by neighbour count
+constexpr int kSliceRows = 16;
+
+struct RowOp {
+  int64_t n_slices;
+  const int64_t *off;   // [n_slices + 1] first step of each slice
+  const int32_t *row;   // [n_slices][16] node, or -1
+  const int32_t *col;   // [steps][32]
+  const double *val;    // [steps][DIM * DIM][32]
+  const uint8_t *flag;  // [n_slices] rows with a D block
+  const double *D;      // [n_nodes][DIM * DIM]
+  const uint8_t *bits;  // [n_nodes] constrained DOFs
+};
+
+template <int DIM, bool MASKED>
+__device__ __forceinline__ void rows_sum(const RowOp &A, int64_t k0, int n, const double *x, const double (&xi)[DIM],
+                                         double (&y)[DIM]) {
+  constexpr int VW = DIM == 3 ? 4 : 2, NC = DIM * DIM;
+  const int32_t *col = A.col + k0 * 32 + (threadIdx.x & 31);
+  const double *val = A.val + k0 * (32 * NC) + (threadIdx.x & 31);
+#pragma unroll 2
+  for (int k = 0; k < n; ++k) {
+    double K[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) K[c] = __ldcs(val + (k * NC + c) * 32);
+    const int32_t j = col[k * 32];
+    NodeV<double, VW> v = ldv<double, VW>(x, j);
+    if (MASKED) {  // values at constrained DOFs have no influence, whatever they are
+      const unsigned b = A.bits[j];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d)
+        if ((b >> d) & 1u) v.v[d] = 0;
+    }
+    double du[DIM];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) du[d] = v.v[d] - xi[d];
+#pragma unroll
+    for (int p = 0; p < DIM; ++p)
+#pragma unroll
+      for (int q = 0; q < DIM; ++q) y[p] = fma(K[p * DIM + q], du[q], y[p]);
+  }
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) y[d] += __shfl_xor_sync(0xffffffffu, y[d], 16);
+}
+
+// y = A x for the rows of slice s, given the rows (-1: padding) and their own
+// x; both lanes of a row get the sum. x is read with plain loads: callers may
+// have other CTAs' writes made visible by a grid barrier.
+template <int DIM>
+__device__ __forceinline__ void rows_product(const RowOp &A, int64_t s, int row, const double *x,
+                                             const double (&xi)[DIM], double (&y)[DIM]) {
+  constexpr int NC = DIM * DIM;
+  const int64_t k0 = A.off[s];
+  const int n = (int)(A.off[s + 1] - k0);
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) y[d] = 0;
+  if (!A.flag[s]) {
+    rows_sum<DIM, false>(A, k0, n, x, xi, y);
+    return;
+  }
+  const int i = row < 0 ? 0 : row;
+  const unsigned b = A.bits[i];
+  double xm[DIM];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) xm[d] = (b >> d) & 1u ? 0.0 : xi[d];
+  rows_sum<DIM, true>(A, k0, n, x, xm, y);
+  const double *D = A.D + (int64_t)i * NC;
+#pragma unroll
+  for (int p = 0; p < DIM; ++p) {
+    if ((b >> p) & 1u) {
+      y[p] = D[p * DIM + p] * xi[p];
+    } else {
+#pragma unroll
+      for (int q = 0; q < DIM; ++q) y[p] = fma(D[p * DIM + q], xm[q], y[p]);
+    }
+  }
+}
+
+// row of this lane in slice s and its own x
+template <int DIM>
+__device__ __forceinline__ int rows_own(const RowOp &A, int64_t s, const double *x, double (&xi)[DIM]) {
+  constexpr int VW = DIM == 3 ? 4 : 2;
+  const int row = A.row[s * kSliceRows + (threadIdx.x & 15)];
+  const NodeV<double, VW> own = ldv<double, VW>(x, row < 0 ? 0 : row);
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) xi[d] = own.v[d];
+  return row;
+}
+
+// ------------------------------------------------------------------ applications
+// Two slices per CTA: the FP64 pipe of an SM is what a slice takes its time on,
+// so a small mesh's slices are spread over as many SMs as there are (2601
+// nodes: 82 CTAs, against 21 with eight slices each).
+constexpr int kRowsThreads = 64;
+
+// y = A x, node vectors in the internal layout (XOUT false) or y in the
+// caller's order [n_nodes][DIM] (XOUT true).
+template <int DIM, bool XOUT>
+__global__ void __launch_bounds__(kRowsThreads) k_rows_apply(RowOp A, const double *x, double *y, const int32_t *new2old) {
+  constexpr int VW = DIM == 3 ? 4 : 2;
+  const int64_t W = (int64_t)gridDim.x * (kRowsThreads / 32);
+  for (int64_t s = blockIdx.x * (int64_t)(kRowsThreads / 32) + (threadIdx.x >> 5); s < A.n_slices; s += W) {
+    double v[DIM], xi[DIM];
+    const int row = rows_own<DIM>(A, s, x, xi);
+    rows_product<DIM>(A, s, row, x, xi, v);
+    if (row < 0 || (threadIdx.x & 16)) continue;
+    if constexpr (XOUT) {
+      const int64_t o = new2old[row];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) y[o * DIM + d] = v[d];
+    } else {
+      NodeV<double, VW> o;
+#pragma unroll
+      for (int d = 0; d < VW; ++d) o.v[d] = d < DIM ? v[d < DIM ? d : 0] : 0.0;
+      stv<double, VW>(y, row, o);
+    }
+  }
+}
+
+// r = f - A x (x == nullptr: r = f), its FP32 copy, ||r||^2 and ||f||^2 into
+// out[0], out[1] (partials: [grid][2], block order).
+struct RowsResidual {
+  int64_t nn;
+  const double *f, *x;
+  double *r;
+  float *r32;  // or nullptr
+  double *out, *partials;
+  unsigned int *count;
+};
+template <int DIM>
+__global__ void __launch_bounds__(kRowsThreads) k_rows_residual(RowOp A, RowsResidual P) {
+  constexpr int VW = DIM == 3 ? 4 : 2;
+  double acc[2] = {0, 0};
+  const int64_t W = (int64_t)gridDim.x * (kRowsThreads / 32);
+  for (int64_t s = blockIdx.x * (int64_t)(kRowsThreads / 32) + (threadIdx.x >> 5); s < A.n_slices; s += W) {
+    double v[DIM], xi[DIM];
+    int row;
+    if (P.x) {
+      row = rows_own<DIM>(A, s, P.x, xi);
+      rows_product<DIM>(A, s, row, P.x, xi, v);
+    } else {
+      row = A.row[s * kSliceRows + (threadIdx.x & 15)];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) v[d] = 0;
+    }
+    if (row < 0 || (threadIdx.x & 16)) continue;
+    const NodeV<double, VW> f = ldv<double, VW>(P.f, row);
+    NodeV<double, VW> r;
+    NodeV<float, VW> r32;
+#pragma unroll
+    for (int d = 0; d < VW; ++d) {
+      r.v[d] = d < DIM ? f.v[d] - v[d < DIM ? d : 0] : 0.0;
+      r32.v[d] = (float)r.v[d];
+    }
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      acc[0] += r.v[d] * r.v[d];
+      acc[1] += f.v[d] * f.v[d];
+    }
+    stv<double, VW>(P.r, row, r);
+    if (P.r32) stv<float, VW>(P.r32, row, r32);
+  }
+  if (grid_sum_last<2>(acc, P.partials, P.count)) {
+    P.out[0] = acc[0];
+    P.out[1] = acc[1];
+  }
+}
+
+// ------------------------------------------------------------------ Jacobi PCG
+// A whole FP64 PCG run in one cooperative kernel: the rows' products and the
+// vector updates alternate with grid-wide sums (grid_sync.cuh) instead of
+// kernel boundaries, and the run ends in the iteration that meets the stopping
+// rule. Three exchanges per iteration: p.Ap; r.z and r.r; the new direction
+// written before anyone reads it.
+// RESIDENT: every warp has at most one slice, whose rows' x, r, p and M^-1
+// stay in registers for the whole run; only p goes through memory, for the
+// neighbours. Otherwise the rows of A p and the vectors go through memory.
+struct RowsPcg {
+  RowOp A;
+  int64_t nn;
+  const double *f, *dinv;
+  double *x, *r, *z, *p, *u;  // RESIDENT: x and p only
+  Scalars *sc;                // tol, rule, maxit in; the run's scalars out
+  unsigned long long *slots;
+  long long wait_limit;
+  int warm;                   // start from x
+};
+constexpr int kRowsPcgThreads = 512;
+constexpr int kRowsPcgWarps = kRowsPcgThreads / 32;
+
+template <int DIM, bool RESIDENT>
+__global__ void __launch_bounds__(kRowsPcgThreads, 1) k_rows_pcg(RowsPcg P) {
+  constexpr int VW = DIM == 3 ? 4 : 2;
+  __shared__ GridShared sh;
+  GridSync G{P.slots, P.wait_limit, 0u};
+  const RowOp &A = P.A;
+  const int wid = threadIdx.x >> 5;
+  const bool upper = (threadIdx.x & 16) != 0;
+  // the CTA's slices, neighbours in node order
+  const int64_t s0 = A.n_slices * blockIdx.x / gridDim.x, s1 = A.n_slices * (blockIdx.x + 1) / gridDim.x;
+  const int64_t tid = blockIdx.x * (int64_t)kRowsPcgThreads + threadIdx.x, nthr = (int64_t)gridDim.x * kRowsPcgThreads;
+  auto stalled = [&]() {
+    if (threadIdx.x == 0) atomicExch(&P.sc->stalled, 1);
+  };
+  const double tol = P.sc->tol;
+  const int rule = P.sc->rule, maxit = P.sc->maxit;
+  // RESIDENT state of this lane's row (both lanes of a row hold it)
+  const int64_t s = s0 + wid;
+  const bool mine = RESIDENT && s < s1;
+  int row = -1;
+  double x[DIM], r[DIM], p[DIM], m[DIM], y[DIM];
+  double sums[3] = {0, 0, 0};  // r.z, r.r, f.f
+  if constexpr (RESIDENT) {
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) x[d] = r[d] = p[d] = m[d] = y[d] = 0;
+    if (mine) {
+      row = rows_own<DIM>(A, s, P.x, x);
+      if (P.warm) rows_product<DIM>(A, s, row, P.x, x, y);
+      if (row >= 0) {
+        const NodeV<double, VW> f = ldv<double, VW>(P.f, row), di = ldv<double, VW>(P.dinv, row);
+        NodeV<double, VW> pv;
+#pragma unroll
+        for (int d = 0; d < VW; ++d) pv.v[d] = 0;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+          if (!P.warm) x[d] = 0;
+          m[d] = di.v[d];
+          r[d] = P.warm ? f.v[d] - y[d] : f.v[d];
+          p[d] = r[d] * m[d];
+          pv.v[d] = p[d];
+          if (!upper) {
+            sums[0] += r[d] * p[d];
+            sums[1] += r[d] * r[d];
+            sums[2] += f.v[d] * f.v[d];
+          }
+        }
+        if (!upper) stv<double, VW>(P.p, row, pv);
+      }
+    }
+  } else {
+    if (P.warm) {
+      for (int64_t q = s0 + wid; q < s1; q += kRowsPcgWarps) {
+        double xi[DIM], v[DIM];
+        const int i = rows_own<DIM>(A, q, P.x, xi);
+        rows_product<DIM>(A, q, i, P.x, xi, v);
+        if (i >= 0 && !upper) {
+          NodeV<double, VW> o;
+#pragma unroll
+          for (int d = 0; d < VW; ++d) o.v[d] = d < DIM ? v[d < DIM ? d : 0] : 0.0;
+          stv<double, VW>(P.u, i, o);
+        }
+      }
+      double none[1] = {0};
+      if (!grid_sums<1>(G, none, sh)) return stalled();
+    }
+    for (int64_t n = tid; n < P.nn; n += nthr) {
+      const NodeV<double, VW> f = ldv<double, VW>(P.f, n), di = ldv<double, VW>(P.dinv, n);
+      NodeV<double, VW> u, rv, pv, zero;
+#pragma unroll
+      for (int d = 0; d < VW; ++d) zero.v[d] = u.v[d] = rv.v[d] = pv.v[d] = 0;
+      if (P.warm) u = ldv<double, VW>(P.u, n);
+      else stv<double, VW>(P.x, n, zero);
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        rv.v[d] = P.warm ? f.v[d] - u.v[d] : f.v[d];
+        pv.v[d] = rv.v[d] * di.v[d];
+        sums[0] += rv.v[d] * pv.v[d];
+        sums[1] += rv.v[d] * rv.v[d];
+        sums[2] += f.v[d] * f.v[d];
+      }
+      stv<double, VW>(P.r, n, rv);
+      stv<double, VW>(P.p, n, pv);
+    }
+  }
+  if (!grid_sums<3>(G, sums, sh)) return stalled();
+  const double gamma0 = sums[0], ff = sums[2];
+  double gamma = gamma0, gamma_prev = gamma0, rr = sums[1], sigma = 0, alpha = 0, beta = 0;
+  int it = 0, done = 0;
+  if (gamma0 == 0.0) done = 1;
+  if (rule == 1 && sqrt(rr) <= tol * sqrt(ff)) done = 1;
+  if (!isfinite(gamma0)) done = 2;
+  while (!done) {
+    double e[1] = {0};
+    if constexpr (RESIDENT) {
+      if (mine) {
+        rows_product<DIM>(A, s, row, P.p, p, y);
+        if (row >= 0 && !upper)
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) e[0] += p[d] * y[d];
+      }
+    } else {
+      for (int64_t q = s0 + wid; q < s1; q += kRowsPcgWarps) {
+        double pi[DIM], v[DIM];
+        const int i = rows_own<DIM>(A, q, P.p, pi);
+        rows_product<DIM>(A, q, i, P.p, pi, v);
+        if (i >= 0 && !upper) {
+          NodeV<double, VW> o;
+#pragma unroll
+          for (int d = 0; d < VW; ++d) o.v[d] = d < DIM ? v[d < DIM ? d : 0] : 0.0;
+          stv<double, VW>(P.u, i, o);
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) e[0] += pi[d] * v[d];
+        }
+      }
+    }
+    if (!grid_sums<1>(G, e, sh)) return stalled();
+    sigma = e[0];
+    alpha = gamma / sigma;
+    double g[2] = {0, 0};
+    if constexpr (RESIDENT) {
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        x[d] += alpha * p[d];
+        r[d] -= alpha * y[d];
+        const double z = r[d] * m[d];
+        if (row >= 0 && !upper) {
+          g[0] += r[d] * z;
+          g[1] += r[d] * r[d];
+        }
+      }
+    } else {
+      for (int64_t n = tid; n < P.nn; n += nthr) {
+        NodeV<double, VW> rv = ldv<double, VW>(P.r, n), zv;
+        const NodeV<double, VW> u = ldv<double, VW>(P.u, n), di = ldv<double, VW>(P.dinv, n);
+#pragma unroll
+        for (int d = 0; d < VW; ++d) zv.v[d] = 0;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+          rv.v[d] -= alpha * u.v[d];
+          zv.v[d] = rv.v[d] * di.v[d];
+          g[0] += rv.v[d] * zv.v[d];
+          g[1] += rv.v[d] * rv.v[d];
+        }
+        stv<double, VW>(P.r, n, rv);
+        stv<double, VW>(P.z, n, zv);
+      }
+    }
+    if (!grid_sums<2>(G, g, sh)) return stalled();
+    gamma_prev = gamma;
+    gamma = g[0];
+    rr = g[1];
+    ++it;
+    if (!isfinite(gamma) || !isfinite(alpha)) done = 2;
+    else if (rule == 0 && gamma < tol * gamma0) done = 1;
+    else if (rule == 1 && sqrt(rr) <= tol * sqrt(ff)) done = 1;
+    else if (it >= maxit) done = 3;
+    beta = gamma / gamma_prev;
+    if constexpr (RESIDENT) {
+      if (done) break;
+      NodeV<double, VW> pv;
+#pragma unroll
+      for (int d = 0; d < VW; ++d) pv.v[d] = 0;
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        p[d] = r[d] * m[d] + beta * p[d];
+        pv.v[d] = p[d];
+      }
+      if (row >= 0 && !upper) stv<double, VW>(P.p, row, pv);
+    } else {
+      for (int64_t n = tid; n < P.nn; n += nthr) {  // (the last pass too: x of the step just taken)
+        NodeV<double, VW> xv = ldv<double, VW>(P.x, n), pv = ldv<double, VW>(P.p, n);
+        const NodeV<double, VW> zv = ldv<double, VW>(P.z, n);
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+          xv.v[d] += alpha * pv.v[d];
+          pv.v[d] = zv.v[d] + beta * pv.v[d];
+        }
+        stv<double, VW>(P.x, n, xv);
+        if (!done) stv<double, VW>(P.p, n, pv);
+      }
+      if (done) break;
+    }
+    double none[1] = {0};
+    if (!grid_sums<1>(G, none, sh)) return stalled();
+  }
+  if constexpr (RESIDENT) {
+    if (row >= 0 && !upper) {
+      NodeV<double, VW> xv;
+#pragma unroll
+      for (int d = 0; d < VW; ++d) xv.v[d] = d < DIM ? x[d < DIM ? d : 0] : 0.0;
+      stv<double, VW>(P.x, row, xv);
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    Scalars *o = P.sc;
+    o->gamma0 = gamma0;
+    o->gamma = gamma;
+    o->gamma_prev = gamma_prev;
+    o->rr = rr;
+    o->ff = ff;
+    o->sigma = sigma;
+    o->alpha = alpha;
+    o->beta = beta;
+    o->iter = it;
+    o->done = done;
+  }
+}
+
+// ------------------------------------------------------------------ construction
+// Elements of every node (sorted), neighbour lists, slices, blocks.
+static __global__ void k_rows_count(int64_t n, const int32_t *conn, int32_t *cnt) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) atomicAdd(cnt + conn[i], 1);
+}
+
+// out[0] = 0, out[i + 1] = in[0] + .. + in[i], one block of 1024 threads.
+template <typename TO>
+__global__ void __launch_bounds__(1024) k_rows_scan(int64_t n, const int32_t *in, TO *out) {
+  __shared__ long long warp_sum[32];
+  __shared__ long long carry_s;
+  if (threadIdx.x == 0) {
+    carry_s = 0;
+    out[0] = 0;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int64_t base = 0; base < n; base += 4096) {
+    long long v[4], t = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int64_t i = base + threadIdx.x * 4 + q;
+      t += i < n ? in[i] : 0;
+      v[q] = t;
+    }
+    long long inc = t;
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    if (lane == 31) warp_sum[wid] = inc;
+    __syncthreads();
+    if (wid == 0) {
+      long long w = warp_sum[lane];
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long u = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += u;
+      }
+      warp_sum[lane] = w;
+    }
+    __syncthreads();
+    const long long before = carry_s + (wid ? warp_sum[wid - 1] : 0) + inc - t;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int64_t i = base + threadIdx.x * 4 + q;
+      if (i < n) out[i + 1] = (TO)(before + v[q]);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) carry_s += warp_sum[31];
+    __syncthreads();
+  }
+}
+
+static __global__ void k_rows_fill(int64_t n, int nv, const int32_t *conn, const int32_t *inc_off, int32_t *cursor,
+                                   int32_t *inc) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int32_t v = conn[i];
+  inc[inc_off[v] + atomicAdd(cursor + v, 1)] = (int32_t)(i / nv);
+}
+
+// ascending in-place sort of one thread's list: insertion while short, heap sort beyond
+__device__ __forceinline__ void sort_list(int32_t *a, int n) {
+  if (n <= 96) {
+    for (int i = 1; i < n; ++i) {
+      const int32_t v = a[i];
+      int j = i;
+      for (; j > 0 && a[j - 1] > v; --j) a[j] = a[j - 1];
+      a[j] = v;
+    }
+    return;
+  }
+  for (int start = n / 2 - 1, end = n; end > 1;) {
+    int root;
+    if (start >= 0) {
+      root = start--;
+    } else {
+      --end;
+      const int32_t t = a[end];
+      a[end] = a[0];
+      a[0] = t;
+      root = 0;
+    }
+    for (int child; (child = 2 * root + 1) < end; root = child) {
+      if (child + 1 < end && a[child + 1] > a[child]) ++child;
+      if (a[root] >= a[child]) break;
+      const int32_t t = a[root];
+      a[root] = a[child];
+      a[child] = t;
+    }
+  }
+}
+
+// One thread per node: its elements sorted, its neighbours sorted and unique
+// in nbr[(NV - 1) * inc_off[n] ..], their number in deg.
+template <int NV>
+__global__ void k_rows_neighbours(int64_t nn, const int32_t *conn, const int32_t *inc_off, int32_t *inc, int32_t *nbr,
+                                  int32_t *deg) {
+  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (n >= nn) return;
+  const int32_t i0 = inc_off[n], m = inc_off[n + 1] - i0;
+  sort_list(inc + i0, m);
+  int32_t *list = nbr + (int64_t)(NV - 1) * i0;
+  int c = 0;
+  if ((NV - 1) * m <= 96) {  // insert, skipping what is there
+    for (int q = 0; q < m; ++q)
+#pragma unroll
+      for (int a = 0; a < NV; ++a) {
+        const int32_t v = conn[(int64_t)inc[i0 + q] * NV + a];
+        if (v == n) continue;
+        int j = c;
+        for (; j > 0 && list[j - 1] > v; --j) {}
+        if (j > 0 && list[j - 1] == v) continue;
+        for (int t = c; t > j; --t) list[t] = list[t - 1];
+        list[j] = v;
+        ++c;
+      }
+  } else {
+    for (int q = 0; q < m; ++q)
+      for (int a = 0; a < NV; ++a) {
+        const int32_t v = conn[(int64_t)inc[i0 + q] * NV + a];
+        if (v != n) list[c++] = v;
+      }
+    sort_list(list, c);
+    int u = 0;
+    for (int t = 0; t < c; ++t)
+      if (t == 0 || list[t] != list[t - 1]) list[u++] = list[t];
+    c = u;
+  }
+  deg[n] = c;
+}
+
+// Rows of each window by descending neighbour count (ties by node), and the
+// steps of each slice. One block per window.
+static __global__ void __launch_bounds__(kRowWindow) k_rows_order(int64_t nn, const int32_t *deg, int32_t *row,
+                                                                  int32_t *steps) {
+  __shared__ int32_t d[kRowWindow];
+  const int64_t base = (int64_t)blockIdx.x * kRowWindow;
+  const int t = threadIdx.x, n = (int)min((int64_t)kRowWindow, nn - base);
+  d[t] = t < n ? deg[base + t] : -1;
+  __syncthreads();
+  const int mine = d[t];
+  int rank = 0;
+  for (int j = 0; j < kRowWindow; ++j) rank += d[j] > mine || (d[j] == mine && j < t);
+  row[base + rank] = t < n ? (int32_t)(base + t) : -1;
+  if (rank % kSliceRows == 0) steps[(base + rank) / kSliceRows] = mine < 0 ? 0 : (mine + 1) / 2;
+}
+
+// P_i K_ij P_j of the pair from the elements that hold both (in element order,
+// so K_ij and K_ji are the same numbers), plus the consistent mass if cM != 0.
+template <int DIM>
+struct RowsAssembly {
+  const int32_t *conn, *inc_off, *inc;
+  const double *G64;
+  int64_t gstride;
+  double lam, mu, cK, cM;
+  const double *lam_e, *mu_e;  // per-element material (new order) or nullptr
+  const double *mc;            // per-element consistent-mass coefficient (cM != 0)
+  const uint8_t *bits;
+  const double *diag;          // node vector: diagonal of the constrained DOFs
+};
+
+template <int DIM>
+__device__ __forceinline__ void vertex_gradient(const RowsAssembly<DIM> &P, int64_t e, int a, double (&g)[DIM]) {
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) g[d] = 0;
+  if (a > 0) {
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) g[d] = P.G64[(size_t)((a - 1) * DIM + d) * P.gstride + e];
+  } else {
+#pragma unroll
+    for (int b = 0; b < DIM; ++b)
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) g[d] -= P.G64[(size_t)(b * DIM + d) * P.gstride + e];
+  }
+}
+
+// the unmasked block of the pair (i, j)
+template <int DIM>
+__device__ __forceinline__ void pair_block(const RowsAssembly<DIM> &P, int32_t i, int32_t j, double (&K)[DIM * DIM],
+                                           double &mass) {
+  constexpr int NV = DIM + 1;
+#pragma unroll
+  for (int c = 0; c < DIM * DIM; ++c) K[c] = 0;
+  mass = 0;
+  const int32_t q1 = P.inc_off[i + 1];
+  for (int32_t q = P.inc_off[i]; q < q1;) {
+    // elements holding j are collected first: the FP64 part then runs with
+    // full warps
+    int32_t hit[8];
+    uint8_t at[8];
+    int n = 0;
+    for (; q < q1 && n < 8; ++q) {
+      const int32_t e = P.inc[q];
+      int ai = -1, aj = -1;
+#pragma unroll
+      for (int a = 0; a < NV; ++a) {
+        const int32_t v = P.conn[(int64_t)e * NV + a];
+        if (v == i) ai = a;
+        if (v == j) aj = a;
+      }
+      if (aj >= 0) {
+        hit[n] = e;
+        at[n] = (uint8_t)(ai * 4 + aj);
+        ++n;
+      }
+    }
+    for (int t = 0; t < n; ++t) {
+      const int64_t e = hit[t];
+      double gi[DIM], gj[DIM], dot = 0;
+      vertex_gradient<DIM>(P, e, at[t] >> 2, gi);
+      vertex_gradient<DIM>(P, e, at[t] & 3, gj);
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) dot += gi[d] * gj[d];
+      const double lam = P.lam_e ? P.lam_e[e] : P.lam, mu = P.mu_e ? P.mu_e[e] : P.mu;
+#pragma unroll
+      for (int p = 0; p < DIM; ++p)
+#pragma unroll
+        for (int r = 0; r < DIM; ++r)
+          K[p * DIM + r] += lam * (gi[p] * gj[r]) + mu * (gi[r] * gj[p]) + (p == r ? mu * dot : 0.0);
+      if (P.cM != 0) mass += P.mc[e];
+    }
+  }
+}
+
+// Columns (fill_cols) and blocks of every slice, one warp per slice.
+template <int DIM>
+__global__ void __launch_bounds__(128) k_rows_assemble(RowsAssembly<DIM> P, int64_t n_slices, const int64_t *off,
+                                                       const int32_t *row, const int32_t *nbr, const int32_t *deg,
+                                                       int32_t *col, double *val) {
+  constexpr int NC = DIM * DIM, NV = DIM + 1;
+  const int64_t s = blockIdx.x * (int64_t)4 + (threadIdx.x >> 5);
+  if (s >= n_slices) return;
+  const int lane = threadIdx.x & 31, half = lane >> 4;
+  const int32_t i = row[s * kSliceRows + (lane & 15)];
+  const int64_t k0 = off[s];
+  const int n = (int)(off[s + 1] - k0);
+  const unsigned bi = i < 0 ? 0u : P.bits[i];
+  for (int k = 0; k < n; ++k) {
+    const int64_t at = (k0 + k) * 32 + lane;
+    int32_t j;
+    if (nbr) {  // first assembly: the columns from the neighbour lists
+      j = i < 0 ? 0 : i;
+      if (i >= 0 && 2 * k + half < deg[i]) j = nbr[(int64_t)(NV - 1) * P.inc_off[i] + 2 * k + half];
+      col[at] = j;
+    } else {
+      j = col[at];
+    }
+    double K[NC], m = 0;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) K[c] = 0;
+    if (i >= 0 && j != i) pair_block<DIM>(P, i, j, K, m);
+    const unsigned bj = i < 0 ? 0u : P.bits[j];
+    double *v = val + (k0 + k) * (32 * NC) + lane;
+#pragma unroll
+    for (int p = 0; p < DIM; ++p)
+#pragma unroll
+      for (int q = 0; q < DIM; ++q) {
+        double t = P.cK * K[p * DIM + q];
+        if (p == q && P.cM != 0) t += P.cM * m;
+        v[(p * DIM + q) * 32] = ((bi >> p) & 1u) || ((bj >> q) & 1u) ? 0.0 : t;
+      }
+  }
+}
+
+// D blocks: what the difference form misses (see the head of this file), one
+// thread per row; a slice with any is flagged.
+template <int DIM>
+__global__ void k_rows_corrections(RowsAssembly<DIM> P, int64_t n_rows, const int64_t *off, const int32_t *row,
+                                   const int32_t *col, double *D, uint8_t *flag) {
+  constexpr int NC = DIM * DIM;
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= n_rows) return;
+  const int32_t i = row[t];
+  if (i < 0) return;
+  const int64_t s = t / kSliceRows;
+  const unsigned bi = P.bits[i];
+  double B[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) B[c] = 0;
+  bool any = bi != 0 || P.cM != 0;
+  for (int64_t k = off[s]; k < off[s + 1]; ++k)
+    for (int half = 0; half < 2; ++half) {
+      const int32_t j = col[k * 32 + half * 16 + (t & 15)];
+      if (j == i) continue;
+      const unsigned bj = P.bits[j];
+      if (bj == bi && P.cM == 0) continue;
+      any = true;
+      double K[NC], m;
+      pair_block<DIM>(P, i, j, K, m);
+#pragma unroll
+      for (int p = 0; p < DIM; ++p)
+#pragma unroll
+        for (int q = 0; q < DIM; ++q) {
+          const int fj = !((bj >> q) & 1u), fi = !((bi >> q) & 1u);
+          B[p * DIM + q] += P.cK * K[p * DIM + q] * (double)(fj - fi);
+          // mass: M_ij x_j = M_ij (x_j - x_i) + M_ij x_i on free DOFs
+          if (p == q) B[p * DIM + q] += P.cM * m * (double)fj;
+        }
+    }
+  if (P.cM != 0) {  // M_ii = twice the element coefficients
+    double m = 0;
+    for (int32_t q = P.inc_off[i]; q < P.inc_off[i + 1]; ++q) m += P.mc[P.inc[q]];
+#pragma unroll
+    for (int p = 0; p < DIM; ++p) B[p * DIM + p] += P.cM * 2.0 * m;
+  }
+  constexpr int VW = DIM == 3 ? 4 : 2;
+#pragma unroll
+  for (int p = 0; p < DIM; ++p)
+    if ((bi >> p) & 1u) {
+#pragma unroll
+      for (int q = 0; q < DIM; ++q) B[p * DIM + q] = p == q ? P.diag[(int64_t)i * VW + p] : 0.0;
+    }
+#pragma unroll
+  for (int c = 0; c < NC; ++c) D[(int64_t)i * NC + c] = B[c];
+  if (any) flag[s] = 1;
+}
+
+}  // namespace cfem

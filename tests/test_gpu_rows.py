@@ -1,0 +1,80 @@
+"""The FP64 operator as assembled node rows (csrc/kernels_rows.cuh) against the
+FP64 oracle: meshes whose node count falls on, before and after a slice (16
+rows) or a window (512 rows), a node with more neighbours than a list sorted by
+insertion, partly constrained nodes, per-element moduli.
+
+Tolerances: a row sums at most a few hundred products, each rounded relative to
+|K_ij| |x_j - x_i|, and K_ij is a sum over the elements of one edge: 1e-13 of
+the result's norm leaves two orders of magnitude.
+"""
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import rel
+from cudafemproject_gb300 import meshgen
+from cudafemproject_gb300.meshio import Problem
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(dim, nodes, elems, cons, young=None):
+    z = np.zeros((0, dim))
+    return Problem(dim=dim, nodes=np.asarray(nodes, np.float32).astype(np.float64), elems=np.asarray(elems, np.int32),
+                   cons=np.asarray(cons, np.int32).reshape(-1, 2), load_node=np.zeros(0, np.int32), load_vec=z,
+                   face_nodes=np.zeros((0, dim + 1), np.int32), face_elem=np.zeros(0, np.int32), face_normal=z,
+                   face_pressure=np.zeros(0), E=2e7, nu=0.25, rho=2000.0, elem_E=young)
+
+
+def _strip(n_nodes):
+    """A strip of triangles with exactly n_nodes nodes."""
+    i = np.arange(n_nodes)
+    nodes = np.stack([0.5 * i, (i % 2) * 0.8 + 0.01 * np.sin(i)], axis=1)
+    return _problem(2, nodes, np.stack([i[:-2], i[1:-1], i[2:]], axis=1), [[0, 3], [1, 1], [n_nodes - 1, 2]])
+
+
+def _hub(n_rim):
+    """A double cone of tetrahedra around one axis: two nodes with n_rim + 1 neighbours."""
+    t = 2 * np.pi * np.arange(n_rim) / n_rim
+    nodes = np.concatenate([[[0, 0, -1], [0, 0, 1]], np.stack([np.cos(t), np.sin(t), 0.1 * np.cos(3 * t)], axis=1)])
+    i = np.arange(n_rim)
+    elems = np.stack([np.zeros_like(i), np.ones_like(i), 2 + i, 2 + (i + 1) % n_rim], axis=1)
+    return _problem(3, nodes, elems, [[2, 7], [5, 1], [9, 2]], 2e7 * (1 + 0.5 * np.sin(i)))
+
+
+MESHES = {
+    "tet": lambda: _problem(3, [[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]], [[0, 1, 2, 3]], [[0, 7], [1, 2]]),
+    "strip15": lambda: _strip(15),
+    "strip16": lambda: _strip(16),
+    "strip17": lambda: _strip(17),
+    "strip511": lambda: _strip(511),
+    "strip512": lambda: _strip(512),
+    "strip513": lambda: _strip(513),
+    "hub20": lambda: _hub(20),
+    "hub300": lambda: _hub(300),
+    "delaunay": lambda: meshgen.random_tets(900, seed=11),
+    "box_code1": lambda: meshgen.box_3d(5, 4, 11, jitter=0.2, seed=1, clamp_code=1),
+    "box_code2": lambda: meshgen.box_3d(5, 4, 11, jitter=0.2, seed=1, clamp_code=2),
+}
+
+
+@pytest.mark.parametrize("name", MESHES)
+def test_fp64_rows_against_the_oracle(name):
+    from cudafemproject_gb300.solver import FemContext
+    p = MESHES[name]()
+    ctx, o = FemContext(p), O.Oracle(p)
+    x = np.random.default_rng(3).standard_normal(p.n_dof)
+    y, ref = ctx.matvec(x, "fp64"), o.matvec(x)
+    assert np.linalg.norm(y - ref) <= 1e-13 * np.linalg.norm(ref)
+    # values at constrained DOFs reach their own rows only, whatever they are
+    bc = ctx.bc_mask().astype(bool)
+    free = ~bc
+    for bad in (1e200, np.inf, np.nan):
+        xb = x.copy()
+        xb[bc] = bad
+        assert np.array_equal(ctx.matvec(xb, "fp64")[free], y[free])
+    # moduli changed in place: the rows are assembled again
+    young = 2e7 * np.exp(0.3 * np.random.default_rng(4).standard_normal(p.n_elems))
+    ctx.set_young(young)
+    p.elem_E = young
+    assert rel(ctx.matvec(x, "fp64"), O.Oracle(p).matvec(x)) <= 1e-13
