@@ -1,9 +1,10 @@
 // C-ABI implementation (include/cfem.h): context lifetime, static solvers.
 //
 // Host orchestration only; the arithmetic lives in kernels.cuh / kernels_aux.cuh.
-// PCG iterations are issued as captured CUDA graphs of 2*chunk kernels
+// FP32 PCG iterations are issued as captured CUDA graphs of 2*chunk kernels
 // (matvec with fused direction update, then the vector update), replayed until
-// the device-side stopping flag is set; all scalar recurrences stay on the GPU.
+// the device-side stopping flag is set; an FP64 run is one cooperative kernel
+// (context_rows.cu). All scalar recurrences stay on the GPU.
 #include <mutex>
 
 #include "context_internal.cuh"
@@ -167,7 +168,7 @@ void launch_update(cfem_ctx *c, const VecParams<T> &P) {
 template <typename T>
 PcgResult run_pcg_t(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int warm, double tol, int rule, int maxit,
                     const T *cont_p = nullptr, double cont_gamma_prev = 0) {
-  Scalars *sc = c->sc.p + (sizeof(T) == 8 ? 0 : 1);
+  Scalars *sc = c->sc.p + 1;
   Scalars h{};
   h.tol = tol;
   h.rule = rule;
@@ -196,7 +197,7 @@ PcgResult run_pcg_t(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int war
     CKL();
     c->launches += 1;
   }
-  GraphCache &gc = sizeof(T) == 8 ? c->graph64 : c->graph32;
+  GraphCache &gc = c->graph32;
   // directions alternate between pA and pB, A p between u and uB: the matvec
   // of iteration `it` accumulates into one u buffer and zeroes the other for
   // iteration it + 1 (the init kernel zeroes u for iteration 0; chunk is even)
@@ -354,10 +355,6 @@ MvParams<double> base_mv_d(cfem_ctx *c) { return base_mv_t<double>(c); }
 MvParams<float> base_mv_f(cfem_ctx *c) { return base_mv_t<float>(c); }
 void launch_mv_d(cfem_ctx *c, int mode, const MvParams<double> &P) { launch_mv_t<double>(c, mode, P); }
 void launch_mv_f(cfem_ctx *c, int mode, const MvParams<float> &P) { launch_mv_t<float>(c, mode, P); }
-PcgResult run_pcg_d(cfem_ctx *c, Vecs<double> &V, double cK, double cM, const double *mcoef, int warm, double tol,
-                    int rule, int maxit) {
-  return run_pcg_t<double>(c, V, cK, cM, mcoef, warm, tol, rule, maxit);
-}
 PcgResult run_pcg_f(cfem_ctx *c, Vecs<float> &V, float cK, float cM, const float *mcoef, int warm, double tol,
                     int rule, int maxit) {
   return run_pcg_t<float>(c, V, cK, cM, mcoef, warm, tol, rule, maxit);
@@ -1068,7 +1065,6 @@ cfem_status cfem_set_stream(cfem_ctx *ctx, void *stream) {
     check_ctx(ctx);
     CK(cudaStreamSynchronize(ctx->stream));
     attach_stream(ctx, (cudaStream_t)stream);
-    ctx->graph64.reset();
     ctx->graph32.reset();
     return CFEM_OK;
   });

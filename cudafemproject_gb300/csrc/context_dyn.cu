@@ -585,7 +585,6 @@ cfem_status cfem_set_young(cfem_ctx *ctx, const double *elem_young) {
     ctx->young = yv;
     rebuild_operator(ctx);
     // captured PCG iterations hold operator buffers that the rebuild may have replaced
-    ctx->graph64.reset();
     ctx->graph32.reset();
     return CFEM_OK;
   });

@@ -19,6 +19,7 @@
 #include "kernels_fan_tma.cuh"
 #include "kernels_multi.cuh"
 #include "kernels_batch.cuh"
+#include "grid_sync.cuh"
 #include "prep.hpp"
 
 namespace cfem {
@@ -106,7 +107,9 @@ struct RowsData {
   DBuf<int32_t> row, col;
   DBuf<int64_t> off;
   int64_t n_slices = 0, steps = 0;
-  RowsValues K;
+  RowsValues K;                 // stiffness
+  RowsValues KM;                // km_cK K + km_cM M of the last implicit FP64 run
+  double km_cK = -1, km_cM = -1;
 };
 
 inline unsigned nblk(int64_t n, int t = kThreads) { return (unsigned)((n + t - 1) / t); }
@@ -167,6 +170,7 @@ struct cfem_ctx {
   int grid_geo = 0;
   int np_slots = 0;               // node slots per patch in shared memory
   RowsData rows;                  // FP64 operator
+  DBuf<unsigned long long> grid_slots;  // grid-wide sums of the one-kernel PCG (grid_sync.cuh)
   int grid_rows = 0;              // CTAs of a grid-stride kernel over its slices
   DBuf<uint8_t> bits;
   DBuf<double> coords, escale, young_d;
@@ -205,7 +209,7 @@ struct cfem_ctx {
   DBuf<float> pmat32;
   DBuf<double> pmat64, lam_e, mu_e;
   int64_t launches = 0;  // kernels issued since the counter was last reset
-  GraphCache graph64, graph32;
+  GraphCache graph32;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // reference re-sorting quirk (compat dynamics)
   DBuf<int64_t> seg;
@@ -213,7 +217,6 @@ struct cfem_ctx {
   DBuf<double> slot_src, slot_tmp;
 
   ~cfem_ctx() {
-    graph64.reset();
     graph32.reset();
     if (h_sc) cudaFreeHost(h_sc);
     if (h_rr) cudaFreeHost(h_rr);

@@ -96,6 +96,7 @@ unsigned rows_grid(const cfem_ctx *c) { return nblk(c->rows.n_slices, kRowsThrea
 }  // namespace
 
 void build_rows(cfem_ctx *c) {
+  c->rows.km_cK = c->rows.km_cM = -1;  // (combined values of an earlier operator are stale)
   if (!c->rows.col.p) {
     DBuf<int32_t> nbr, deg;
     if (c->dim == 3) build_structure<4>(c, nbr, deg);
@@ -127,6 +128,74 @@ void true_residual_async(cfem_ctx *c, const double *f, const double *x, double *
   else k_rows_residual<2><<<g, kRowsThreads, 0, c->stream>>>(A, P);
   CKL();
   c->launches += 1;
+}
+
+// FP64 Jacobi PCG on A x = V.f, A = cM M + cK K' (has_mass) or K', as one
+// cooperative kernel (k_rows_pcg). V.dinv is the preconditioner; warm: V.x is
+// the start. diag_op: the operator's diagonal (combined operators).
+PcgResult run_pcg_d(cfem_ctx *c, Vecs<double> &V, double cK, double cM, const double *mcoef, int warm, double tol,
+                    int rule, int maxit) {
+  RowsData &R = c->rows;
+  const RowsValues *values = &R.K;
+  if (mcoef || cK != 1.0) {  // implicit dynamics: stiffness and mass in the same blocks, assembled once per run
+    if (!R.KM.val.p || R.km_cK != cK || R.km_cM != cM) {
+      assemble(c, nullptr, nullptr, cK, mcoef ? cM : 0.0, V.diagA.p, R.KM);
+      R.km_cK = cK;
+      R.km_cM = cM;
+    }
+    values = &R.KM;
+  }
+  Scalars *sc = c->sc.p;
+  Scalars h{};
+  h.tol = tol;
+  h.rule = rule;
+  h.maxit = maxit > 0 ? maxit : 1000000;
+  CK(cudaMemcpyAsync(sc, &h, sizeof(Scalars), cudaMemcpyHostToDevice, c->stream));
+  const size_t n_slots = grid_slots_count(kRowsPcgSets, c->n_sm);
+  if (!c->grid_slots.p) c->grid_slots.alloc(n_slots + 1);  // (the barrier's counter follows the slots)
+  CK(cudaMemsetAsync(c->grid_slots.p, 0xFF, n_slots * sizeof(unsigned long long), c->stream));
+  CK(cudaMemsetAsync(c->grid_slots.p + n_slots, 0, sizeof(unsigned long long), c->stream));
+  RowsPcg P{};
+  P.A = op_of(c, *values);
+  P.f = V.f.p;
+  P.dinv = V.dinv.p;
+  P.x = V.x.p;
+  P.r = V.r.p;
+  P.z = V.z.p;
+  P.p = V.pA.p;
+  P.u = V.u.p;
+  P.sc = sc;
+  P.sync = GridSync{c->grid_slots.p, reinterpret_cast<unsigned *>(c->grid_slots.p + n_slots), kWaitCycles};
+  P.warm = warm;
+  // One CTA per SM, and fewer while a CTA has a quarter of an SM for each of
+  // its slices: an exchange among 76 CTAs takes 0.4 us less than among 152, and
+  // a slice runs no faster alone on an SM.
+  const int grid = (int)std::min<int64_t>(c->n_sm, (R.n_slices + 3) / 4);
+  const bool small = R.n_slices <= (int64_t)grid * (kRowsPcgSmall / 32);
+  const bool resident = R.n_slices <= (int64_t)grid * (kRowsPcgThreads / 32);
+  auto pick = [&](auto k3, auto k2) { return c->dim == 3 ? (const void *)k3 : (const void *)k2; };
+  const void *k = small      ? pick(k_rows_pcg<3, true, kRowsPcgSmall>, k_rows_pcg<2, true, kRowsPcgSmall>)
+                  : resident ? pick(k_rows_pcg<3, true, kRowsPcgThreads>, k_rows_pcg<2, true, kRowsPcgThreads>)
+                             : pick(k_rows_pcg<3, false, kRowsPcgThreads>, k_rows_pcg<2, false, kRowsPcgThreads>);
+  void *args[] = {&P};
+  CK(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(small ? kRowsPcgSmall : kRowsPcgThreads), args, 0, c->stream));
+  c->launches += 1;
+  CK(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  if (c->h_sc->stalled) throw Fail{CFEM_ERR_CUDA, "a CTA of the FP64 PCG kernel did not arrive at a grid-wide sum in time"};
+  if (!c->h_sc->done) throw Fail{CFEM_ERR_CUDA, "PCG recurrence stopped advancing on the device"};
+  if (c->verbose)
+    std::printf("iteration %d gamma %.6e gamma0 %.6e\n", c->h_sc->iter, c->h_sc->gamma, c->h_sc->gamma0);
+  PcgResult res;
+  res.iters = c->h_sc->iter;
+  res.gamma0 = c->h_sc->gamma0;
+  res.gamma = c->h_sc->gamma;
+  res.rr = c->h_sc->rr;
+  res.ff = c->h_sc->ff;
+  res.gamma_prev = c->h_sc->gamma_prev;
+  const int d = c->h_sc->done;
+  res.status = d == 1 ? CFEM_OK : d == 2 ? CFEM_ERR_DIVERGED : CFEM_ERR_NOT_CONVERGED;
+  return res;
 }
 
 }  // namespace detail

@@ -201,90 +201,127 @@ __global__ void __launch_bounds__(kRowsThreads) k_rows_residual(RowOp A, RowsRes
 // A whole FP64 PCG run in one cooperative kernel: the rows' products and the
 // vector updates alternate with grid-wide sums (grid_sync.cuh) instead of
 // kernel boundaries, and the run ends in the iteration that meets the stopping
-// rule. Three exchanges per iteration: p.Ap; r.z and r.r; the new direction
-// written before anyone reads it.
+// rule. Per iteration: the sum p.Ap; the sums r.z and r.r; a barrier behind
+// which the new direction can be read.
 // RESIDENT: every warp has at most one slice, whose rows' x, r, p and M^-1
 // stay in registers for the whole run; only p goes through memory, for the
-// neighbours. Otherwise the rows of A p and the vectors go through memory.
+// neighbours. The two lanes of a row share its components (kOwn of them each:
+// 0 and 1 in the lower half, 2 in the upper; in 2D one each), because an FP64
+// instruction costs the same whatever lanes are active. Otherwise the rows of
+// A p and the vectors go through memory.
 struct RowsPcg {
   RowOp A;
-  int64_t nn;
   const double *f, *dinv;
   double *x, *r, *z, *p, *u;  // RESIDENT: x and p only
   Scalars *sc;                // tol, rule, maxit in; the run's scalars out
-  unsigned long long *slots;
-  long long wait_limit;
+  GridSync sync;              // two sets of slots for the loop, one for the start
   int warm;                   // start from x
 };
-constexpr int kRowsPcgThreads = 512;
-constexpr int kRowsPcgWarps = kRowsPcgThreads / 32;
+// Threads: 512 fill the FP64 pipe and hide the loads; 128, where no CTA has
+// more than four slices, shorten every sum by three FP64 additions.
+constexpr int kRowsPcgThreads = 512, kRowsPcgSmall = 128;
+constexpr int kRowsPcgSets = 5;  // start; p.Ap and r.z of even, of odd iterations
 
-template <int DIM, bool RESIDENT>
-__global__ void __launch_bounds__(kRowsPcgThreads, 1) k_rows_pcg(RowsPcg P) {
+template <int DIM, bool RESIDENT, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) k_rows_pcg(RowsPcg P) {
+  constexpr int WARPS = THREADS / 32;
   constexpr int VW = DIM == 3 ? 4 : 2;
-  __shared__ GridShared sh;
-  GridSync G{P.slots, P.wait_limit, 0u};
+  constexpr int OWN = DIM == 3 ? 2 : 1;
+  __shared__ GridShared<THREADS> sh;
+  const GridSync &G = P.sync;
   const RowOp &A = P.A;
-  const int wid = threadIdx.x >> 5;
-  const bool upper = (threadIdx.x & 16) != 0;
+  const int wid = threadIdx.x >> 5, half = (threadIdx.x >> 4) & 1;
   // the CTA's slices, neighbours in node order
   const int64_t s0 = A.n_slices * blockIdx.x / gridDim.x, s1 = A.n_slices * (blockIdx.x + 1) / gridDim.x;
-  const int64_t tid = blockIdx.x * (int64_t)kRowsPcgThreads + threadIdx.x, nthr = (int64_t)gridDim.x * kRowsPcgThreads;
+  // not RESIDENT: the nodes of the same slices, so that every vector but p
+  // stays with one CTA
+  auto each_node = [&](auto &&body) {
+    for (int64_t t = s0 * kSliceRows + threadIdx.x; t < s1 * kSliceRows; t += THREADS) {
+      const int n = A.row[t];
+      if (n >= 0) body(n);
+    }
+  };
+  unsigned epoch = 0;
   auto stalled = [&]() {
     if (threadIdx.x == 0) atomicExch(&P.sc->stalled, 1);
   };
   const double tol = P.sc->tol;
   const int rule = P.sc->rule, maxit = P.sc->maxit;
-  // RESIDENT state of this lane's row (both lanes of a row hold it)
+  // RESIDENT state: the whole p of the lane's row, the components c0 + k of the others
   const int64_t s = s0 + wid;
   const bool mine = RESIDENT && s < s1;
+  const int c0 = half * OWN;  // (3D: component 3 of the upper half is a zero)
   int row = -1;
-  double x[DIM], r[DIM], p[DIM], m[DIM], y[DIM];
+  double x[OWN], r[OWN], m[OWN], p[DIM], y[DIM], yo[OWN];
+  auto own_of = [&](const double (&v)[DIM], double (&o)[OWN]) {
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+      o[k] = half ? (OWN + k < DIM ? v[OWN + k < DIM ? OWN + k : 0] : 0.0) : v[k];
+    }
+  };
+  // the whole direction of the row from both lanes' components
+  auto share_p = [&](const double (&o)[OWN]) {
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+      const double other = __shfl_xor_sync(0xffffffffu, o[k], 16);
+      p[k] = half ? other : o[k];
+      if (OWN + k < DIM) p[OWN + k < DIM ? OWN + k : 0] = half ? o[k] : other;
+    }
+  };
+  auto store_p = [&]() {
+    if (row < 0 || half) return;
+    NodeV<double, VW> pv;
+#pragma unroll
+    for (int d = 0; d < VW; ++d) pv.v[d] = d < DIM ? p[d < DIM ? d : 0] : 0.0;
+    stv<double, VW>(P.p, row, pv);
+  };
   double sums[3] = {0, 0, 0};  // r.z, r.r, f.f
   if constexpr (RESIDENT) {
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) x[d] = r[d] = p[d] = m[d] = y[d] = 0;
+    for (int k = 0; k < OWN; ++k) x[k] = r[k] = m[k] = 0;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) p[d] = y[d] = 0;
     if (mine) {
-      row = rows_own<DIM>(A, s, P.x, x);
-      if (P.warm) rows_product<DIM>(A, s, row, P.x, x, y);
-      if (row >= 0) {
-        const NodeV<double, VW> f = ldv<double, VW>(P.f, row), di = ldv<double, VW>(P.dinv, row);
-        NodeV<double, VW> pv;
+      row = rows_own<DIM>(A, s, P.x, p);
+      if (P.warm) rows_product<DIM>(A, s, row, P.x, p, y);
+      own_of(p, x);
+      own_of(y, yo);
+      NodeV<double, VW> f = ldv<double, VW>(P.f, row < 0 ? 0 : row), di = ldv<double, VW>(P.dinv, row < 0 ? 0 : row);
+      double fa[DIM], fo[OWN], po[OWN];
 #pragma unroll
-        for (int d = 0; d < VW; ++d) pv.v[d] = 0;
+      for (int d = 0; d < DIM; ++d) fa[d] = row < 0 ? 0.0 : f.v[d];
+      own_of(fa, fo);
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-          if (!P.warm) x[d] = 0;
-          m[d] = di.v[d];
-          r[d] = P.warm ? f.v[d] - y[d] : f.v[d];
-          p[d] = r[d] * m[d];
-          pv.v[d] = p[d];
-          if (!upper) {
-            sums[0] += r[d] * p[d];
-            sums[1] += r[d] * r[d];
-            sums[2] += f.v[d] * f.v[d];
-          }
-        }
-        if (!upper) stv<double, VW>(P.p, row, pv);
+      for (int d = 0; d < DIM; ++d) fa[d] = row < 0 ? 0.0 : di.v[d];
+      own_of(fa, m);
+#pragma unroll
+      for (int k = 0; k < OWN; ++k) {
+        if (!P.warm || row < 0) x[k] = 0;
+        r[k] = P.warm && row >= 0 ? fo[k] - yo[k] : fo[k];
+        po[k] = r[k] * m[k];
+        sums[0] += r[k] * po[k];
+        sums[1] += r[k] * r[k];
+        sums[2] += fo[k] * fo[k];
       }
+      share_p(po);
+      store_p();
     }
   } else {
     if (P.warm) {
-      for (int64_t q = s0 + wid; q < s1; q += kRowsPcgWarps) {
+      for (int64_t q = s0 + wid; q < s1; q += WARPS) {
         double xi[DIM], v[DIM];
         const int i = rows_own<DIM>(A, q, P.x, xi);
         rows_product<DIM>(A, q, i, P.x, xi, v);
-        if (i >= 0 && !upper) {
+        if (i >= 0 && !half) {
           NodeV<double, VW> o;
 #pragma unroll
           for (int d = 0; d < VW; ++d) o.v[d] = d < DIM ? v[d < DIM ? d : 0] : 0.0;
           stv<double, VW>(P.u, i, o);
         }
       }
-      double none[1] = {0};
-      if (!grid_sums<1>(G, none, sh)) return stalled();
+      __syncthreads();
     }
-    for (int64_t n = tid; n < P.nn; n += nthr) {
+    each_node([&](int n) {
       const NodeV<double, VW> f = ldv<double, VW>(P.f, n), di = ldv<double, VW>(P.dinv, n);
       NodeV<double, VW> u, rv, pv, zero;
 #pragma unroll
@@ -301,30 +338,40 @@ __global__ void __launch_bounds__(kRowsPcgThreads, 1) k_rows_pcg(RowsPcg P) {
       }
       stv<double, VW>(P.r, n, rv);
       stv<double, VW>(P.p, n, pv);
-    }
+    });
   }
-  if (!grid_sums<3>(G, sums, sh)) return stalled();
-  const double gamma0 = sums[0], ff = sums[2];
+  // sqrt(rr) <= tol sqrt(ff) is tested as rr <= (tol sqrt(ff))^2
+  if (!grid_sums<3>(G, 0, sums, sh, [&](const double (&t)[3]) {
+        const double lim = tol * sqrt(t[2]);
+        sh.total[kMaxGridSums] = lim * lim;
+      }))
+    return stalled();
+  const double gamma0 = sums[0], ff = sums[2], rr_stop = sh.total[kMaxGridSums], gamma_stop = tol * gamma0;
   double gamma = gamma0, gamma_prev = gamma0, rr = sums[1], sigma = 0, alpha = 0, beta = 0;
   int it = 0, done = 0;
   if (gamma0 == 0.0) done = 1;
-  if (rule == 1 && sqrt(rr) <= tol * sqrt(ff)) done = 1;
+  if (rule == 1 && rr <= rr_stop) done = 1;
   if (!isfinite(gamma0)) done = 2;
+  if (!grid_barrier(G, ++epoch, sh)) return stalled();
   while (!done) {
+    const int set = 1 + 2 * (it & 1);
     double e[1] = {0};
     if constexpr (RESIDENT) {
       if (mine) {
         rows_product<DIM>(A, s, row, P.p, p, y);
-        if (row >= 0 && !upper)
+        double po[OWN];
+        own_of(y, yo);
+        own_of(p, po);
+        if (row >= 0)
 #pragma unroll
-          for (int d = 0; d < DIM; ++d) e[0] += p[d] * y[d];
+          for (int k = 0; k < OWN; ++k) e[0] += po[k] * yo[k];
       }
     } else {
-      for (int64_t q = s0 + wid; q < s1; q += kRowsPcgWarps) {
+      for (int64_t q = s0 + wid; q < s1; q += WARPS) {
         double pi[DIM], v[DIM];
         const int i = rows_own<DIM>(A, q, P.p, pi);
         rows_product<DIM>(A, q, i, P.p, pi, v);
-        if (i >= 0 && !upper) {
+        if (i >= 0 && !half) {
           NodeV<double, VW> o;
 #pragma unroll
           for (int d = 0; d < VW; ++d) o.v[d] = d < DIM ? v[d < DIM ? d : 0] : 0.0;
@@ -334,23 +381,26 @@ __global__ void __launch_bounds__(kRowsPcgThreads, 1) k_rows_pcg(RowsPcg P) {
         }
       }
     }
-    if (!grid_sums<1>(G, e, sh)) return stalled();
+    if (!grid_sums<1>(G, set, e, sh, [&](const double (&t)[1]) { sh.total[kMaxGridSums] = gamma / t[0]; }))
+      return stalled();
     sigma = e[0];
-    alpha = gamma / sigma;
+    alpha = sh.total[kMaxGridSums];
+    grid_reset<1>(G, 4 - set);  // (the sets of the next iteration)
+    grid_reset<2>(G, 5 - set);
     double g[2] = {0, 0};
     if constexpr (RESIDENT) {
+      if (mine) {
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) {
-        x[d] += alpha * p[d];
-        r[d] -= alpha * y[d];
-        const double z = r[d] * m[d];
-        if (row >= 0 && !upper) {
-          g[0] += r[d] * z;
-          g[1] += r[d] * r[d];
+        for (int k = 0; k < OWN; ++k) {
+          r[k] -= alpha * yo[k];
+          const double z = r[k] * m[k];
+          g[0] += r[k] * z;
+          g[1] += r[k] * r[k];
         }
+        if (row < 0) g[0] = g[1] = 0;
       }
     } else {
-      for (int64_t n = tid; n < P.nn; n += nthr) {
+      each_node([&](int n) {
         NodeV<double, VW> rv = ldv<double, VW>(P.r, n), zv;
         const NodeV<double, VW> u = ldv<double, VW>(P.u, n), di = ldv<double, VW>(P.dinv, n);
 #pragma unroll
@@ -364,31 +414,33 @@ __global__ void __launch_bounds__(kRowsPcgThreads, 1) k_rows_pcg(RowsPcg P) {
         }
         stv<double, VW>(P.r, n, rv);
         stv<double, VW>(P.z, n, zv);
-      }
+      });
     }
-    if (!grid_sums<2>(G, g, sh)) return stalled();
+    if (!grid_sums<2>(G, set + 1, g, sh, [&](const double (&t)[2]) { sh.total[kMaxGridSums] = t[0] / gamma; }))
+      return stalled();
     gamma_prev = gamma;
     gamma = g[0];
     rr = g[1];
+    beta = sh.total[kMaxGridSums];
     ++it;
     if (!isfinite(gamma) || !isfinite(alpha)) done = 2;
-    else if (rule == 0 && gamma < tol * gamma0) done = 1;
-    else if (rule == 1 && sqrt(rr) <= tol * sqrt(ff)) done = 1;
+    else if (rule == 0 && gamma < gamma_stop) done = 1;
+    else if (rule == 1 && rr <= rr_stop) done = 1;
     else if (it >= maxit) done = 3;
-    beta = gamma / gamma_prev;
     if constexpr (RESIDENT) {
-      if (done) break;
-      NodeV<double, VW> pv;
+      if (mine) {
+        double po[OWN];
+        own_of(p, po);
 #pragma unroll
-      for (int d = 0; d < VW; ++d) pv.v[d] = 0;
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) {
-        p[d] = r[d] * m[d] + beta * p[d];
-        pv.v[d] = p[d];
+        for (int k = 0; k < OWN; ++k) {
+          x[k] += alpha * po[k];
+          po[k] = r[k] * m[k] + beta * po[k];
+        }
+        share_p(po);
+        if (!done) store_p();
       }
-      if (row >= 0 && !upper) stv<double, VW>(P.p, row, pv);
     } else {
-      for (int64_t n = tid; n < P.nn; n += nthr) {  // (the last pass too: x of the step just taken)
+      each_node([&](int n) {  // (the last pass too: x of the step just taken)
         NodeV<double, VW> xv = ldv<double, VW>(P.x, n), pv = ldv<double, VW>(P.p, n);
         const NodeV<double, VW> zv = ldv<double, VW>(P.z, n);
 #pragma unroll
@@ -398,19 +450,16 @@ __global__ void __launch_bounds__(kRowsPcgThreads, 1) k_rows_pcg(RowsPcg P) {
         }
         stv<double, VW>(P.x, n, xv);
         if (!done) stv<double, VW>(P.p, n, pv);
-      }
-      if (done) break;
+      });
     }
-    double none[1] = {0};
-    if (!grid_sums<1>(G, none, sh)) return stalled();
+    if (done) break;
+    if (!grid_barrier(G, ++epoch, sh)) return stalled();
   }
   if constexpr (RESIDENT) {
-    if (row >= 0 && !upper) {
-      NodeV<double, VW> xv;
+    if (mine && row >= 0)
 #pragma unroll
-      for (int d = 0; d < VW; ++d) xv.v[d] = d < DIM ? x[d < DIM ? d : 0] : 0.0;
-      stv<double, VW>(P.x, row, xv);
-    }
+      for (int k = 0; k < OWN; ++k)
+        if (c0 + k < DIM) P.x[(int64_t)row * VW + c0 + k] = x[k];
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     Scalars *o = P.sc;

@@ -78,3 +78,25 @@ def test_fp64_rows_against_the_oracle(name):
     ctx.set_young(young)
     p.elem_E = young
     assert rel(ctx.matvec(x, "fp64"), O.Oracle(p).matvec(x)) <= 1e-13
+
+
+@pytest.mark.parametrize("n", [7, 98, 99, 196, 198])
+def test_fp64_pcg_shapes_against_the_oracle(n):
+    """The one-kernel PCG in its three shapes (four slices per CTA, one per warp,
+    many per warp; 98/99 and 196/198 quads a side lie on either side of the
+    limits of a 152-SM GPU): the first two iterates (two recurrences that differ
+    in the order of their sums: 1e-12) and the converged solution (1e-10, the
+    bar of every FP64 solve)."""
+    from cudafemproject_gb300.solver import FemContext
+    p = meshgen.square_2d(n)
+    f = np.zeros((p.n_nodes, 2))
+    f[p.nodes[:, 0] > 1 - 1e-9] = (0.7, -0.2)
+    f = f.ravel()
+    ctx, o = FemContext(p), O.Oracle(p)
+    for iters in (1, 2):
+        x, it = o.pcg(f, tol=1e-30, rule=1, maxit=iters, allow_maxit=True)
+        u, info = ctx.pcg(f, "fp64", tol=1e-30, stop_rule="residual", max_iter=iters, allow_not_converged=True)
+        assert info["iterations"] == it == iters
+        assert rel(u, x) <= 1e-12
+    u, _ = ctx.pcg(f, "fp64", tol=1e-13, stop_rule="residual")
+    assert rel(u, o.pcg(f, tol=1e-13, rule=1)[0]) <= 1e-10
