@@ -545,7 +545,6 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
   if (!err.empty()) throw Fail{CFEM_ERR_MESH, err};
   err = build_rhs(*m, c->prep, c->semantics, c->rhs);
   if (!err.empty()) throw Fail{CFEM_ERR_MESH, err};
-  c->elems_caller.assign(m->elems, m->elems + c->ne * c->nv);
   if (m->elem_young) {
     c->young.assign(m->elem_young, m->elem_young + c->ne);
     for (double y : c->young)

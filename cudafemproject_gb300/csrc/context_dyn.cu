@@ -2,6 +2,8 @@
 // femfunc.cpp:130-381), multi-RHS PCG, adjoint sensitivities, material update.
 #include "context_internal.cuh"
 #include "kernels_aux.cuh"
+#include "kernels_steps.cuh"
+#include "rows_op.cuh"
 
 namespace cfem {
 namespace detail {
@@ -43,32 +45,80 @@ __global__ void k_slot_mass(int64_t ne, int w, const double *vol, double c, cons
   for (int j = 0; j < w; ++j) out[eo * w + j] = m;
 }
 
-// Stable sort of the DOF keys of all element slots (counting sort == the
-// multimap order of cpu_matrix.cpp:189-223), in the caller's numbering.
-void build_slot_perm(cfem_ctx *c, const int32_t *elems_caller) {
-  if (c->perm.p) return;
-  const int64_t nloc = c->ne * c->w, nd = c->nd;
-  std::vector<int64_t> cnt(nd + 1, 0);
-  std::vector<int32_t> mask(nloc);
-  for (int64_t e = 0; e < c->ne; ++e)
-    for (int a = 0; a < c->nv; ++a)
-      for (int d = 0; d < c->dim; ++d) mask[e * c->w + c->dim * a + d] = elems_caller[e * c->nv + a] * c->dim + d;
-  for (int64_t i = 0; i < nloc; ++i) cnt[mask[i] + 1]++;
-  for (int64_t k = 0; k < nd; ++k) cnt[k + 1] += cnt[k];
-  std::vector<int64_t> pos(cnt.begin(), cnt.end());
-  std::vector<int32_t> perm(nloc);
-  for (int64_t i = 0; i < nloc; ++i) perm[pos[mask[i]]++] = (int32_t)i;
-  c->perm.upload(perm.data(), perm.size(), c->stream);
-  c->seg.upload(cnt.data(), cnt.size(), c->stream);
-  c->slot_src.alloc(nloc);
-  c->slot_tmp.alloc(nloc);
+// Elements at every caller node (in caller node order).
+__global__ void k_slot_counts(int64_t nn, const int32_t *old2new, const int32_t *inc_off, int32_t *cnt) {
+  const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (o >= nn) return;
+  const int32_t n = old2new[o];
+  cnt[o] = inc_off[n + 1] - inc_off[n];
 }
 
-// assembled node vector (FP64) of the slot source, then the in-place re-sort
-void slot_assemble_and_resort(cfem_ctx *c, double *out64) {
-  k_assemble_slots<<<nblk(c->nd), kThreads, 0, c->stream>>>(c->nd, c->dim, c->vw, c->seg.p, c->perm.p, c->slot_src.p,
-                                                            c->node_old2new.p, out64, 0, nullptr);
-  k_permute<<<nblk(c->ne * c->w), kThreads, 0, c->stream>>>(c->ne * c->w, c->perm.p, c->slot_src.p, c->slot_tmp.p);
+// Slots of every DOF of a caller node, by caller element (one thread per
+// node): DOF dim o + d has slots seg[dim o + d] .. of which slot t belongs to
+// the t-th element at the node.
+template <int DIM>
+__global__ void k_slot_perm(int64_t nn, const int32_t *old2new, const int32_t *inc_off, const int32_t *inc,
+                            const int32_t *conn, const int32_t *elem_new2old, const int32_t *caller_off, int64_t *seg,
+                            int32_t *perm) {
+  constexpr int NV = DIM + 1, W = 6 * (DIM - 1);
+  const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (o >= nn) return;
+  const int32_t n = old2new[o], i0 = inc_off[n], m = inc_off[n + 1] - i0;
+  const int64_t at = (int64_t)DIM * caller_off[o];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) seg[DIM * o + d] = at + (int64_t)d * m;
+  if (o == nn - 1) seg[DIM * nn] = at + (int64_t)DIM * m;
+  int32_t *code = perm + at;  // caller element * NV + vertex, sorted
+  for (int t = 0; t < m; ++t) {
+    const int32_t e = inc[i0 + t];
+    int v = 0;
+#pragma unroll
+    for (int q = 1; q < NV; ++q)
+      if (conn[(int64_t)e * NV + q] == n) v = q;
+    code[t] = elem_new2old[e] * NV + v;
+  }
+  sort_list(code, m);
+  for (int t = 0; t < m; ++t) {  // (DOF 0 overwrites the codes last)
+    const int32_t e = code[t] / NV, v = code[t] % NV;
+    for (int d = DIM - 1; d >= 0; --d) code[(int64_t)d * m + t] = e * W + DIM * v + d;
+  }
+}
+
+// Stable sort of the DOF keys of all element slots (the multimap order of
+// cpu_matrix.cpp:189-223), in the caller's numbering.
+void build_slot_perm(cfem_ctx *c) {
+  if (c->perm.p) return;
+  const int64_t nloc = c->ne * c->w;
+  const RowsData &R = c->rows;
+  DBuf<int32_t> cnt, off;
+  cnt.alloc(c->nn);
+  off.alloc(c->nn + 1);
+  k_slot_counts<<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, c->node_old2new.p, R.inc_off.p, cnt.p);
+  k_rows_scan<int32_t><<<1, 1024, 0, c->stream>>>(c->nn, cnt.p, off.p);
+  c->seg.alloc(c->nd + 1);
+  c->slot_src.alloc(nloc);
+  c->slot_tmp.alloc(nloc);
+  c->perm.alloc(nloc);
+  if (c->dim == 3)
+    k_slot_perm<3><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, c->node_old2new.p, R.inc_off.p, R.inc.p, c->conn.p,
+                                                           c->elem_new2old.p, off.p, c->seg.p, c->perm.p);
+  else
+    k_slot_perm<2><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, c->node_old2new.p, R.inc_off.p, R.inc.p, c->conn.p,
+                                                           c->elem_new2old.p, off.p, c->seg.p, c->perm.p);
+  CKL();
+  CK(cudaStreamSynchronize(c->stream));  // (before cnt and off are freed)
+}
+
+Resort resort_of(cfem_ctx *c) {
+  return Resort{c->nd, c->dim, c->vw, c->seg.p, c->perm.p, c->node_old2new.p};
+}
+
+// One assembly of the slot source: node vector of its sums (or their
+// inverses), and the re-sorted source of the next assembly in its place.
+template <typename T>
+void slot_assemble_and_resort(cfem_ctx *c, T *out, int invert) {
+  k_resort<T><<<nblk(c->nd, 32 * (kThreads / 32)), kThreads, 0, c->stream>>>(resort_of(c), c->slot_src.p, c->slot_tmp.p,
+                                                                            out, invert);
   CKL();
   std::swap(c->slot_src.p, c->slot_tmp.p);
 }
@@ -85,8 +135,8 @@ void set_pcg_vectors(cfem_ctx *c, const double *diag_op, const double *diag_pre)
 // counter through DynState::pstep, P.parity and P.dto set by the caller).
 template <typename T>
 void launch_dyn_explicit_step(cfem_ctx *c, const DynParams<T> &P) {
-  if (c->dim == 3) launch_pdl(k_dyn_explicit<T, 3, true>, dim3(c->grid_vec), dim3(kThreads), 0, c->stream, P);
-  else k_dyn_explicit<T, 2, true><<<c->grid_vec, kThreads, 0, c->stream>>>(P);
+  if (c->dim == 3) launch_pdl(k_dyn_explicit<T, 3>, dim3(c->grid_vec), dim3(kThreads), 0, c->stream, P);
+  else k_dyn_explicit<T, 2><<<c->grid_vec, kThreads, 0, c->stream>>>(P);
   CKL();
 }
 template <typename T>
@@ -102,9 +152,82 @@ void launch_dyn_correct(cfem_ctx *c, const DynParams<T> &P) {
   CKL();
 }
 
+// Cooperative launch of a step kernel: one CTA per SM, fewer while every slice
+// has a quarter of an SM to itself (k_rows_pcg's rule; re-sorting masses takes
+// every SM's loads). pick(resident) chooses the instance.
+template <typename P, typename F>
+void launch_rows_loop(cfem_ctx *c, P &prm, bool all_sms, size_t smem, F pick) {
+  const RowsData &R = c->rows;
+  prm.A = op_of(c, R.K);
+  prm.stalled = c->steps.stalled.p;
+  prm.sync = start_grid_sync(c, 0);
+  const int grid = (int)std::min<int64_t>(c->n_sm, all_sms ? c->n_sm : (R.n_slices + 3) / 4);
+  const void *k = pick(R.n_slices <= (int64_t)grid * kStepWarps);
+  CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  void *args[] = {&prm};
+  CK(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kStepThreads), args, smem, c->stream));
+  c->launches += 1;
+}
+
+void launch_steps(cfem_ctx *c, RowsSteps &P) {
+  launch_rows_loop(c, P, P.resort != 0, P.resort ? sizeof(double) * kStepWarps * kResortTile : 0, [&](bool resident) {
+    return c->dim == 3 ? (resident ? (const void *)k_rows_steps<3, true> : (const void *)k_rows_steps<3, false>)
+                       : (resident ? (const void *)k_rows_steps<2, true> : (const void *)k_rows_steps<2, false>);
+  });
+}
+
+void launch_reverse(cfem_ctx *c, RowsReverse &P) {
+  launch_rows_loop(c, P, false, 0, [&](bool resident) {
+    return c->dim == 3 ? (resident ? (const void *)k_rows_reverse<3, true> : (const void *)k_rows_reverse<3, false>)
+                       : (resident ? (const void *)k_rows_reverse<2, true> : (const void *)k_rows_reverse<2, false>);
+  });
+}
+
+// Before the first step kernel of a call.
+void begin_steps(cfem_ctx *c) {
+  c->steps.stalled.ensure(1);
+  c->steps.stalled.zero(c->stream);
+}
+
+// Reports a step kernel whose CTAs lost one another (synchronises the stream).
+void check_steps(cfem_ctx *c) {
+  int h = 0;
+  CK(cudaMemcpyAsync(&h, c->steps.stalled.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  if (h) throw Fail{CFEM_ERR_CUDA, "a CTA of a time-stepping kernel did not arrive at a grid barrier in time"};
+}
+
+void launch_grad_pairs(cfem_ctx *c, const double *u, const double *w, int64_t stride, int count, const double *young,
+                       double *g, int accumulate) {
+  auto go = [&](auto kern, unsigned blocks) {
+    kern<<<blocks, 128, 0, c->stream>>>(c->ne, c->G64.p, c->gstride, c->conn.p, c->bits.p, c->lam, c->mu, u, w, stride,
+                                        count, young, c->elem_new2old.p, g, accumulate);
+  };
+  if (count >= 4) {
+    if (c->dim == 3) go(k_grad_pairs<3, 4>, nblk(c->ne, 32));
+    else go(k_grad_pairs<2, 4>, nblk(c->ne, 32));
+  } else {
+    if (c->dim == 3) go(k_grad_pairs<3, 1>, nblk(c->ne, 128));
+    else go(k_grad_pairs<2, 1>, nblk(c->ne, 128));
+  }
+  CKL();
+}
+
+// Per-element moduli on the device (the material's where none were given).
+const double *young_on_device(cfem_ctx *c) {
+  if (c->young_d.p) return c->young_d.p;
+  DBuf<double> &y = c->steps.young;
+  if (!y.p) {
+    std::vector<double> h(c->ne, c->E);
+    y.alloc(c->ne);
+    CK(cudaMemcpyAsync(y.p, h.data(), sizeof(double) * c->ne, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+  }
+  return y.p;
+}
+
 template <typename T>
-cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet *w, double *u_out, cfem_dyn_info *info,
-                    const int32_t *elems_caller) {
+cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet *w, double *u_out, cfem_dyn_info *info) {
   single_mesh_only(c);
   const double beta1 = prm->beta1, beta2 = prm->beta2, dt = prm->dt;
   const bool expl = beta2 == 0.0;
@@ -121,22 +244,27 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
   std::vector<double> coef(2 * (size_t)(nsteps + 1));
   sch.eval(0.f, coef[0], coef[1]);
   for (int s = 1; s <= nsteps; ++s) sch.eval((float)s * dtf, coef[2 * s], coef[2 * s + 1]);
-  DBuf<double> dcoef;
-  dcoef.upload(coef.data(), coef.size(), c->stream);
+  StepWork &W = c->steps;
+  StepVecs<T> &S = [&]() -> StepVecs<T> & {
+    if constexpr (sizeof(T) == 8) return W.f64; else return W.f32;
+  }();
   Vecs<T> &V = [&]() -> Vecs<T> & {
     if constexpr (sizeof(T) == 8) return c->v64; else return c->v32;
   }();
-  DBuf<T> d0, d1, vel, acc, y, minv;
-  for (auto *b : {&d0, &d1, &vel, &acc, &y}) { b->alloc(c->nvec); b->zero(c->stream); }
-  DBuf<DynState> st;
-  st.alloc(1);
+  W.coef.ensure(coef.size());
+  CK(cudaMemcpyAsync(W.coef.p, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice, c->stream));
+  S.d.ensure(2 * (size_t)c->nvec);
+  for (auto *b : {&S.v, &S.a, &S.y}) b->ensure(c->nvec);
+  S.minv.ensure(2 * (size_t)c->nvec);
+  for (auto *b : {&S.d, &S.v, &S.a, &S.y}) b->zero(c->stream);
+  T *const d0 = S.d.p, *const d1 = S.d.p + c->nvec;
+  W.st.ensure(1);
   DynState hs{};
   hs.step = 1;
   hs.pstep[0] = 1;  // explicit: the first step has parity 0
-  CK(cudaMemcpyAsync(st.p, &hs, sizeof(hs), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(W.st.p, &hs, sizeof(hs), cudaMemcpyHostToDevice, c->stream));
   const int nrec = prm->n_receivers > 0 && prm->receiver_nodes && prm->receiver_trace ? prm->n_receivers : 0;
-  DBuf<int32_t> recv;
-  DBuf<double> trace;
+  const size_t n_trace = (size_t)nsteps * nrec * c->dim;
   if (nrec) {
     std::vector<int32_t> rn(nrec);
     for (int i = 0; i < nrec; ++i) {
@@ -144,23 +272,24 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
       if (o < 0 || o >= c->nn) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "receiver node out of range"};
       rn[i] = c->prep.node_old2new[o];
     }
-    recv.upload(rn.data(), rn.size(), c->stream);
-    trace.alloc((size_t)nsteps * nrec * c->dim);
+    W.recv.ensure(nrec);
+    CK(cudaMemcpyAsync(W.recv.p, rn.data(), sizeof(int32_t) * nrec, cudaMemcpyHostToDevice, c->stream));
+    W.trace.ensure(n_trace);
   }
   const T *FA, *FB;
   if constexpr (sizeof(T) == 8) { FA = c->FA.p; FB = c->FB.p; } else { FA = c->FA32.p; FB = c->FB32.p; }
   DynParams<T> dp{};
   dp.n_nodes = c->nn;
-  dp.v = vel.p;
-  dp.a = acc.p;
-  dp.y = y.p;
+  dp.v = S.v.p;
+  dp.a = S.a.p;
+  dp.y = S.y.p;
   dp.FA = FA;
   dp.FB = FB;
-  dp.coef = dcoef.p;
-  dp.st = st.p;
-  dp.recv = recv.p;
+  dp.coef = W.coef.p;
+  dp.st = W.st.p;
+  dp.recv = W.recv.p;
   dp.n_recv = nrec;
-  dp.trace = trace.p;
+  dp.trace = W.trace.p;
   dp.dim = c->dim;
   dp.c_old = (T)((1 - beta1) * dt);
   dp.c_new = (T)(beta1 * dt);
@@ -169,19 +298,22 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
   if constexpr (sizeof(T) == 8) mv.diagA = c->diagK.p; else mv.diagA = c->diagK32.p;  // r = F - K' d
   mv.c1 = (T)dt;
   mv.c2 = (T)(0.5 * (1 - beta2) * dt * dt);
-  mv.x2 = vel.p;
-  mv.x3 = acc.p;
-  mv.y = y.p;
-  DBuf<double> diag_pre, diag_op;
-  diag_pre.alloc(c->nvec);
-  diag_op.alloc(c->nvec);
+  mv.x2 = S.v.p;
+  mv.x3 = S.a.p;
+  mv.y = S.y.p;
+  DBuf<double> &diag_pre = W.diag_pre, &diag_op = W.diag_op;
+  if (!expl) {
+    diag_pre.ensure(c->nvec);
+    diag_pre.zero(c->stream);
+    diag_op.ensure(c->nvec);
+  }
   bool resort = false;
   const double cK = 0.5 * beta2 * dt * dt;
   // operator / mass factors per semantics (cpu_fem_utils.cpp:598-734)
   const double lump_c = c->dim == 2 ? 1.0 / 3 : (compat ? 1.0 / 12 : 1.0 / 4);
   const double mdiag_c = c->dim == 2 ? 1.0 / 6 : (compat ? 1.0 / 24 : 1.0 / 10);
   if (compat) {
-    build_slot_perm(c, elems_caller);
+    build_slot_perm(c);
     if (expl) {
       k_slot_mass<<<nblk(c->ne), kThreads, 0, c->stream>>>(c->ne, c->w, c->vol.p, lump_c * c->rho, c->elem_new2old.p,
                                                            c->slot_src.p);
@@ -197,12 +329,9 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
     resort = true;
   }
   if (expl) {
-    minv.alloc(c->nvec);
-    if (!compat) {
-      k_invert<T><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->mlump.p, minv.p);
-      CKL();
-    }
-    set_pcg_vectors(c, c->diagK.p, c->diagK.p);  // diagA: constrained term of K'
+    if (compat) S.minv.zero(c->stream);  // (the pad lanes)
+    else k_invert<T><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->mlump.p, S.minv.p);
+    CKL();
   } else {
     if (compat) {
       CK(cudaMemcpyAsync(diag_op.p, c->diagK.p, sizeof(double) * c->nvec, cudaMemcpyDeviceToDevice, c->stream));
@@ -214,7 +343,7 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
       set_pcg_vectors(c, diag_op.p, diag_op.p);
     }
   }
-  dp.minv = minv.p;
+  dp.minv = S.minv.p;
   const T *mc = nullptr;
   if constexpr (sizeof(T) == 8) mc = c->mc64.p; else mc = c->mc32.p;
   const T opK = compat ? T(1) : (T)cK, opM = compat ? T(0) : T(1);
@@ -226,62 +355,98 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
   CK(cudaEventRecord(c->ev0, c->stream));
   int64_t pcg_total = 0;
   int status = CFEM_OK;
-  T *dcur = d0.p, *dnext = d1.p;
+  T *dcur = d0, *dnext = d1;
   V.x.zero(c->stream);  // acceleration warm start / PCG solution
-  auto one_step = [&](T *from, T *to, int parity) {
-    mv.x = from;
-    mv.xout = to;
-    launch_mv<T>(c, MV_DYN, mv);
-    if (expl) {
+  if (expl && sizeof(T) == 8) {
+    if constexpr (sizeof(T) == 8) {
+      begin_steps(c);
+      RowsSteps P{};
+      P.first = 1;
+      P.last = nsteps;
+      P.v = S.v.p;
+      P.a = S.a.p;
+      P.d = S.d.p;  // d_n at parity n & 1
+      P.mask = 1;
+      P.stride = c->nvec;
+      P.FA = c->FA.p;
+      P.FB = c->FB.p;
+      P.coef = W.coef.p;
+      P.minv = S.minv.p;
+      P.dt = dt;
+      P.c2 = 0.5 * (1 - beta2) * dt * dt;
+      P.c_old = (1 - beta1) * dt;
+      P.c_new = beta1 * dt;
+      P.n_recv = nrec;
+      P.dim = c->dim;
+      P.recv = W.recv.p;
+      P.trace = W.trace.p;
       if (resort) {
-        slot_assemble_and_resort(c, diag_pre.p);
-        k_invert<T><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, diag_pre.p, minv.p);
-        CKL();
+        P.resort = 1;
+        P.R = resort_of(c);
+        P.src[0] = c->slot_src.p;
+        P.src[1] = c->slot_tmp.p;
+        P.minv2[0] = S.minv.p;
+        P.minv2[1] = S.minv.p + c->nvec;
       }
-      DynParams<T> de = dp;
-      de.dto = to;
-      de.parity = parity;
-      launch_dyn_explicit_step<T>(c, de);
+      launch_steps(c, P);
+      dcur = (nsteps & 1) ? d1 : d0;
     }
-  };
-  if (expl) {
-    // two steps per captured graph (the displacement buffers alternate)
-    cudaGraphExec_t exec = nullptr;
-    int pairs = nsteps / 2;
-    if (pairs > 0) {
-      cudaGraph_t g;
-      CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-      try {
-        one_step(d0.p, d1.p, 0);
-        one_step(d1.p, d0.p, 1);
-      } catch (...) {
-        cudaGraph_t broken = nullptr;
-        cudaStreamEndCapture(c->stream, &broken);
-        if (broken) cudaGraphDestroy(broken);
-        (void)cudaGetLastError();
-        throw;
+  } else if (expl) {
+    if constexpr (sizeof(T) == 4) {
+      auto one_step = [&](T *from, T *to, int parity) {
+        mv.x = from;
+        mv.xout = to;
+        launch_mv<T>(c, MV_DYN, mv);
+        if (resort) slot_assemble_and_resort<T>(c, S.minv.p, 1);
+        DynParams<T> de = dp;
+        de.dto = to;
+        de.parity = parity;
+        launch_dyn_explicit_step<T>(c, de);
+      };
+      // two steps per captured graph (the displacement buffers alternate)
+      cudaGraphExec_t exec = nullptr;
+      int pairs = nsteps / 2;
+      if (pairs > 0) {
+        cudaGraph_t g;
+        CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+        try {
+          one_step(d0, d1, 0);
+          one_step(d1, d0, 1);
+        } catch (...) {
+          cudaGraph_t broken = nullptr;
+          cudaStreamEndCapture(c->stream, &broken);
+          if (broken) cudaGraphDestroy(broken);
+          (void)cudaGetLastError();
+          throw;
+        }
+        CK(cudaStreamEndCapture(c->stream, &g));
+        CK(cudaGraphInstantiate(&exec, g, 0));
+        cudaGraphDestroy(g);
+        for (int i = 0; i < pairs; ++i) CK(cudaGraphLaunch(exec, c->stream));
+        cudaGraphExecDestroy(exec);
+        // the resort swaps are captured: after an even number of steps slot_src is back in place
       }
-      CK(cudaStreamEndCapture(c->stream, &g));
-      CK(cudaGraphInstantiate(&exec, g, 0));
-      cudaGraphDestroy(g);
-      for (int i = 0; i < pairs; ++i) CK(cudaGraphLaunch(exec, c->stream));
-      cudaGraphExecDestroy(exec);
-      // the resort swaps are captured: after an even number of steps slot_src is back in place
-    }
-    dcur = d0.p;
-    if (nsteps & 1) {  // (after the pairs the next step's counter is pstep[0])
-      one_step(d0.p, d1.p, 0);
-      dcur = d1.p;
+      dcur = d0;
+      if (nsteps & 1) {  // (after the pairs the next step's counter is pstep[0])
+        one_step(d0, d1, 0);
+        dcur = d1;
+      }
     }
   } else {
     for (int s = 1; s <= nsteps; ++s) {
-      mv.x = dcur;
-      mv.xout = dnext;
-      launch_mv<T>(c, MV_DYN, mv);
+      if constexpr (sizeof(T) == 8) {
+        k_dyn_predict<<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, dcur, S.v.p, S.a.p, mv.c1, mv.c2, dnext);
+        CKL();
+        rows_apply(c, dnext, S.y.p);
+      } else {
+        mv.x = dcur;
+        mv.xout = dnext;
+        launch_mv<T>(c, MV_DYN, mv);
+      }
       dp.rhs = V.f.p;
       launch_dyn_rhs<T>(c, dp);
       if (compat) {
-        slot_assemble_and_resort(c, diag_pre.p);
+        slot_assemble_and_resort<double>(c, diag_pre.p, 0);
         set_pcg_vectors(c, diag_op.p, diag_pre.p);
       }
       const double tol = compat ? 1e-4 : (prm->pcg_tol > 0 ? prm->pcg_tol : 1e-10);
@@ -303,8 +468,9 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
   float ms = 0;
   CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   to_caller<T>(c, dcur, u_out);
-  if (nrec) CK(cudaMemcpyAsync(prm->receiver_trace, trace.p, sizeof(double) * trace.n, cudaMemcpyDefault, c->stream));
-  check_copy_error(c);
+  if (nrec) CK(cudaMemcpyAsync(prm->receiver_trace, W.trace.p, sizeof(double) * n_trace, cudaMemcpyDefault, c->stream));
+  if (expl && sizeof(T) == 8) check_steps(c);
+  else check_copy_error(c);
   if (info) {
     info->status = status;
     info->steps = nsteps;
@@ -314,7 +480,15 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
   return (cfem_status)status;
 }
 
-// Explicit GN22 receiver-misfit adjoint with sqrt(N) checkpointing (FP64).
+// States of the dynamics adjoint (displacements and adjoint accelerations of
+// every step) that are held at once; longer or larger runs go by segments.
+// CFEM_DYN_STATES_MB overrides the limit.
+double step_states_bytes() {
+  const char *e = std::getenv("CFEM_DYN_STATES_MB");
+  return (e ? std::max(0.0, std::atof(e)) : 1024.0) * 1024 * 1024;
+}
+
+// Explicit GN22 receiver-misfit adjoint (FP64); checkpoints as described there.
 cfem_status run_dyn_adjoint(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet *w, int n_rec,
                             const int32_t *rec_nodes, const double *obs, double *loss, double *dLdE,
                             cfem_dyn_info *info) {
@@ -328,8 +502,15 @@ cfem_status run_dyn_adjoint(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_
   if (!(dtf > 0)) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "dt must be positive"};
   int N = endf < 0 ? 1 : (int)(endf / dtf);
   if (N < 1) N = 1;
-  const int C = (int)std::ceil(std::sqrt((double)N));
   const int64_t nv = c->nvec;
+  // The reverse sweep needs d_n of every step and leaves w_n for the gradient.
+  // Segments of C steps: all of them where both sequences fit in
+  // step_states_bytes(), else ceil(sqrt(N)) with the states at the start of every
+  // segment kept and its steps taken again (the last segment's are still there).
+  const double limit = step_states_bytes();
+  const bool whole = 2.0 * (N + 1) * nv * sizeof(double) <= limit;
+  const int C = whole ? N : (int)std::ceil(std::sqrt((double)N));
+  const int n_seg = (N + C - 1) / C;
   const double h_old = (1 - beta1) * dt, h_new = beta1 * dt, c2 = 0.5 * dt * dt;
   RhsSchedule sch;
   sch.semantics = c->semantics;
@@ -338,131 +519,139 @@ cfem_status run_dyn_adjoint(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_
   std::vector<double> coef(2 * (size_t)(N + 1));
   sch.eval(0.f, coef[0], coef[1]);
   for (int s = 1; s <= N; ++s) sch.eval((float)s * dtf, coef[2 * s], coef[2 * s + 1]);
-  DBuf<double> dcoef, minv, vel, acc, y, dA, dB, trace, obs_d, gE;
-  DBuf<int32_t> recv;
-  dcoef.upload(coef.data(), coef.size(), c->stream);
-  for (auto *b : {&minv, &vel, &acc, &y, &dA, &dB}) { b->alloc(nv); b->zero(c->stream); }
-  k_invert<double><<<nblk(nv), kThreads, 0, c->stream>>>(nv, c->mlump.p, minv.p);
-  std::vector<int32_t> rn(n_rec);
-  for (int i = 0; i < n_rec; ++i) {
+  // receivers of every node, in the caller's order
+  std::vector<int32_t> rn(n_rec), head(c->nn, -1), next(n_rec, -1);
+  for (int i = n_rec - 1; i >= 0; --i) {
     if (rec_nodes[i] < 0 || rec_nodes[i] >= c->nn) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "receiver node out of range"};
     rn[i] = c->prep.node_old2new[rec_nodes[i]];
+    next[i] = head[rn[i]];
+    head[rn[i]] = i;
   }
-  recv.upload(rn.data(), rn.size(), c->stream);
-  trace.alloc((size_t)N * n_rec * c->dim);
-  obs_d.alloc((size_t)N * n_rec * c->dim);
-  CK(cudaMemcpyAsync(obs_d.p, obs, sizeof(double) * obs_d.n, cudaMemcpyDefault, c->stream));
-  gE.alloc(c->ne);
-  gE.zero(c->stream);
-  DBuf<DynState> st;
-  st.alloc(1);
-  // checkpoints of (d, v, a) after steps 0, C, 2C, ... and one segment of displacements
-  const int ncp = N / C + 1;
-  DBuf<double> cps, seg;
-  cps.alloc((size_t)ncp * 3 * nv);
-  seg.alloc((size_t)(C + 1) * nv);
-  const double *young = c->young_d.p;
-  DBuf<double> yd;
-  if (!young) {
-    std::vector<double> yv(c->ne, c->E);
-    yd.upload(yv.data(), yv.size(), c->stream);
-    young = yd.p;
-  }
-  DynParams<double> dp{};
-  dp.n_nodes = c->nn;
-  dp.v = vel.p;
-  dp.a = acc.p;
-  dp.y = y.p;
-  dp.FA = c->FA.p;
-  dp.FB = c->FB.p;
-  dp.coef = dcoef.p;
-  dp.st = st.p;
-  dp.dim = c->dim;
-  dp.minv = minv.p;
-  dp.c_old = h_old;
-  dp.c_new = h_new;
-  MvParams<double> mv = base_mv<double>(c);
-  mv.diagA = c->diagK.p;
-  mv.c1 = dt;
-  mv.c2 = c2;
-  mv.x2 = vel.p;
-  mv.x3 = acc.p;
-  mv.y = y.p;
-  auto set_step = [&](int step) {
-    DynState hs{};
-    hs.step = step;
-    CK(cudaMemcpyAsync(st.p, &hs, sizeof(hs), cudaMemcpyHostToDevice, c->stream));
+  StepWork &W = c->steps;
+  StepVecs<double> &S = W.f64;
+  cudaStream_t st = c->stream;
+  auto up = [&](auto &buf, const auto &h) {
+    buf.ensure(h.size());
+    CK(cudaMemcpyAsync(buf.p, h.data(), sizeof(h[0]) * h.size(), cudaMemcpyHostToDevice, st));
   };
-  auto step = [&](const double *from, double *to, bool record) {
-    mv.x = from;
-    mv.xout = to;
-    launch_mv<double>(c, MV_DYN, mv);
-    if (c->dim == 3) k_dyn_explicit<double, 3><<<c->grid_vec, kThreads, 0, c->stream>>>(dp);
-    else k_dyn_explicit<double, 2><<<c->grid_vec, kThreads, 0, c->stream>>>(dp);
-    DynParams<double> de = dp;
-    if (record) { de.recv = recv.p; de.n_recv = n_rec; de.trace = trace.p; } else { de.n_recv = 0; }
-    k_dyn_end_step<double><<<1, kThreads, 0, c->stream>>>(de, to, c->vw);
-    CKL();
+  up(W.coef, coef);
+  up(W.recv, rn);
+  up(W.rec_head, head);
+  up(W.rec_next, next);
+  const size_t n_obs = (size_t)N * n_rec * c->dim;
+  W.trace.ensure(n_obs);
+  W.obs.ensure(n_obs);
+  CK(cudaMemcpyAsync(W.obs.p, obs, sizeof(double) * n_obs, cudaMemcpyDefault, st));
+  W.grad.ensure(c->ne);
+  for (auto *b : {&S.v, &S.a}) { b->ensure(nv); b->zero(st); }
+  S.d.ensure(2 * (size_t)nv);
+  S.d.zero(st);
+  S.minv.ensure(2 * (size_t)nv);
+  k_invert<double><<<nblk(nv), kThreads, 0, st>>>(nv, c->mlump.p, S.minv.p);
+  // d of a segment [C + 1], w of a segment [C + 1], db, vb, ab, then the states at segment starts
+  W.states.ensure(((size_t)2 * (C + 1) + 3 + (whole ? 0 : (size_t)n_seg * 3)) * nv);
+  double *seg = W.states.p, *wseg = seg + (size_t)(C + 1) * nv, *adj = wseg + (size_t)(C + 1) * nv, *cps = adj + 3 * nv;
+  struct Release {  // more than the limit is not kept
+    DBuf<double> &b;
+    double limit;
+    ~Release() {
+      if ((double)b.n * sizeof(double) > limit + 4.0 * 1024 * 1024) b.release();
+    }
+  } release{W.states, limit};
+  const double *young = young_on_device(c);
+  RowsSteps P{};
+  P.v = S.v.p;
+  P.a = S.a.p;
+  P.stride = nv;
+  P.FA = c->FA.p;
+  P.FB = c->FB.p;
+  P.coef = W.coef.p;
+  P.minv = S.minv.p;
+  P.dt = dt;
+  P.c2 = c2;
+  P.c_old = h_old;
+  P.c_new = h_new;
+  P.dim = c->dim;
+  P.recv = W.recv.p;
+  P.trace = W.trace.p;
+  auto copy = [&](double *to, const double *from) {
+    CK(cudaMemcpyAsync(to, from, sizeof(double) * nv, cudaMemcpyDeviceToDevice, st));
   };
-  auto save_cp = [&](int k, const double *d) {
-    double *base = cps.p + (size_t)k * 3 * nv;
-    CK(cudaMemcpyAsync(base, d, sizeof(double) * nv, cudaMemcpyDeviceToDevice, c->stream));
-    CK(cudaMemcpyAsync(base + nv, vel.p, sizeof(double) * nv, cudaMemcpyDeviceToDevice, c->stream));
-    CK(cudaMemcpyAsync(base + 2 * nv, acc.p, sizeof(double) * nv, cudaMemcpyDeviceToDevice, c->stream));
+  // steps k0 + 1 .. k1 with d_n at seg + (n - k0) nv, from the states at hand
+  auto into_segment = [&](int k0, int k1, int n_recv) {
+    P.first = k0 + 1;
+    P.last = k1;
+    P.d = seg;
+    P.n0 = k0;
+    P.mask = ~0;
+    P.n_recv = n_recv;
+    launch_steps(c, P);
   };
-  CK(cudaEventRecord(c->ev0, c->stream));
-  // forward with checkpoints
-  set_step(1);
-  double *cur = dA.p, *nxt = dB.p;
-  save_cp(0, cur);
-  for (int n = 1; n <= N; ++n) {
-    step(cur, nxt, true);
-    std::swap(cur, nxt);
-    if (n % C == 0 && n / C < ncp) save_cp(n / C, cur);
-  }
-  std::vector<double> htrace(trace.n);
-  CK(cudaMemcpyAsync(htrace.data(), trace.p, sizeof(double) * trace.n, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  std::vector<double> hobs(obs_d.n);
-  CK(cudaMemcpy(hobs.data(), obs_d.p, sizeof(double) * obs_d.n, cudaMemcpyDeviceToHost));
-  double L = 0;
-  for (size_t i = 0; i < htrace.size(); ++i) L += 0.5 * (htrace[i] - hobs[i]) * (htrace[i] - hobs[i]);
-  // reverse sweep
-  DBuf<double> db, vb, ab, wb;
-  for (auto *b : {&db, &vb, &ab, &wb}) { b->alloc(nv); b->zero(c->stream); }
-  for (int s = (N - 1) / C; s >= 0; --s) {
+  begin_steps(c);
+  CK(cudaEventRecord(c->ev0, st));
+  // forward, keeping the states at the start of every segment
+  for (int s = 0; s < n_seg; ++s) {
     const int k0 = s * C, k1 = std::min(N, k0 + C);
-    // restore the checkpoint after step k0 and recompute steps k0+1..k1
-    const double *base = cps.p + (size_t)s * 3 * nv;
-    CK(cudaMemcpyAsync(seg.p, base, sizeof(double) * nv, cudaMemcpyDeviceToDevice, c->stream));
-    CK(cudaMemcpyAsync(vel.p, base + nv, sizeof(double) * nv, cudaMemcpyDeviceToDevice, c->stream));
-    CK(cudaMemcpyAsync(acc.p, base + 2 * nv, sizeof(double) * nv, cudaMemcpyDeviceToDevice, c->stream));
-    set_step(k0 + 1);
-    for (int n = k0 + 1; n <= k1; ++n) step(seg.p + (size_t)(n - 1 - k0) * nv, seg.p + (size_t)(n - k0) * nv, false);
-    for (int n = k1; n > k0; --n) {
-      const double *dn = seg.p + (size_t)(n - k0) * nv;
-      k_adj_receivers<<<nblk(n_rec * c->dim), kThreads, 0, c->stream>>>(n_rec, c->dim, c->vw, recv.p, dn,
-                                                                       obs_d.p + (size_t)(n - 1) * n_rec * c->dim, db.p);
-      k_adj_pre<<<nblk(nv), kThreads, 0, c->stream>>>(nv, h_old, h_new, minv.p, vb.p, ab.p, wb.p);
-      if (c->dim == 3)
-        k_grad_young<3><<<nblk(c->ne), kThreads, 0, c->stream>>>(c->ne, c->G64.p, c->gstride, c->conn.p, c->bits.p,
-                                                                 c->lam, c->mu, wb.p, dn, young, c->elem_new2old.p,
-                                                                 gE.p, 1);
-      else
-        k_grad_young<2><<<nblk(c->ne), kThreads, 0, c->stream>>>(c->ne, c->G64.p, c->gstride, c->conn.p, c->bits.p,
-                                                                 c->lam, c->mu, wb.p, dn, young, c->elem_new2old.p,
-                                                                 gE.p, 1);
-      rows_apply(c, wb.p, y.p);
-      k_adj_post<<<nblk(nv), kThreads, 0, c->stream>>>(nv, dt, c2, y.p, db.p, vb.p, ab.p);
-      CKL();
+    const double *d_k0 = S.d.p + (size_t)(k0 & 1) * nv;
+    if (!whole) {
+      copy(cps + (size_t)3 * s * nv, d_k0);
+      copy(cps + (size_t)(3 * s + 1) * nv, S.v.p);
+      copy(cps + (size_t)(3 * s + 2) * nv, S.a.p);
+    }
+    if (s == n_seg - 1) {
+      copy(seg, d_k0);
+      into_segment(k0, k1, n_rec);
+    } else {
+      P.first = k0 + 1;
+      P.last = k1;
+      P.d = S.d.p;
+      P.n0 = 0;
+      P.mask = 1;
+      P.n_recv = n_rec;
+      launch_steps(c, P);
     }
   }
-  CK(cudaEventRecord(c->ev1, c->stream));
-  CK(cudaEventSynchronize(c->ev1));
+  CK(cudaMemsetAsync(adj, 0, sizeof(double) * 3 * nv, st));
+  for (int s = n_seg - 1; s >= 0; --s) {
+    const int k0 = s * C, k1 = std::min(N, k0 + C);
+    if (s < n_seg - 1) {
+      copy(seg, cps + (size_t)3 * s * nv);
+      copy(S.v.p, cps + (size_t)(3 * s + 1) * nv);
+      copy(S.a.p, cps + (size_t)(3 * s + 2) * nv);
+      into_segment(k0, k1, 0);
+    }
+    RowsReverse Q{};
+    Q.first = k0 + 1;
+    Q.last = k1;
+    Q.db = adj;
+    Q.vb = adj + nv;
+    Q.ab = adj + 2 * nv;
+    Q.d = seg;
+    Q.w = wseg;
+    Q.n0 = k0;
+    Q.stride = nv;
+    Q.minv = S.minv.p;
+    Q.dt = dt;
+    Q.c2 = c2;
+    Q.h_old = h_old;
+    Q.h_new = h_new;
+    Q.rec_head = W.rec_head.p;
+    Q.rec_next = W.rec_next.p;
+    Q.n_rec = n_rec;
+    Q.obs = W.obs.p;
+    launch_reverse(c, Q);
+    launch_grad_pairs(c, seg + nv, wseg + nv, nv, k1 - k0, young, W.grad.p, s < n_seg - 1);
+  }
+  CK(cudaEventRecord(c->ev1, st));
+  std::vector<double> htrace(n_obs), hobs(n_obs);
+  CK(cudaMemcpyAsync(htrace.data(), W.trace.p, sizeof(double) * n_obs, cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(hobs.data(), W.obs.p, sizeof(double) * n_obs, cudaMemcpyDeviceToHost, st));
+  if (dLdE) CK(cudaMemcpyAsync(dLdE, W.grad.p, sizeof(double) * c->ne, cudaMemcpyDefault, st));
+  check_steps(c);
   float ms = 0;
   CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-  if (dLdE) CK(cudaMemcpyAsync(dLdE, gE.p, sizeof(double) * c->ne, cudaMemcpyDefault, c->stream));
-  check_copy_error(c);
+  double L = 0;
+  for (size_t i = 0; i < n_obs; ++i) L += 0.5 * (htrace[i] - hobs[i]) * (htrace[i] - hobs[i]);
   if (loss) *loss = L;
   if (info) {
     info->status = CFEM_OK;
@@ -495,8 +684,8 @@ cfem_status cfem_dyn(cfem_ctx *ctx, const cfem_dyn_params *prm, const cfem_wavel
     check_ctx(ctx);
     enter(ctx);
     if (!prm || !u) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "null argument"};
-    if (prm->precision == CFEM_FP64) return run_dyn<double>(ctx, prm, w, u, info, ctx->elems_caller.data());
-    if (prm->precision == CFEM_FP32) return run_dyn<float>(ctx, prm, w, u, info, ctx->elems_caller.data());
+    if (prm->precision == CFEM_FP64) return run_dyn<double>(ctx, prm, w, u, info);
+    if (prm->precision == CFEM_FP32) return run_dyn<float>(ctx, prm, w, u, info);
     throw Fail{CFEM_ERR_INVALID_ARGUMENT, "dynamics precision must be CFEM_FP64 or CFEM_FP32"};
   });
 }
@@ -513,26 +702,10 @@ cfem_status cfem_adjoint(cfem_ctx *ctx, const cfem_solve_params *prm, const doub
     cfem_status st = solve_internal(ctx, &p, info);
     if (dLdf) to_caller<double>(ctx, ctx->v64.x.p, dLdf);
     if (dLdE) {
-      DBuf<double> uin, g, yd;
-      uin.alloc(ctx->nvec);
-      g.alloc(ctx->ne);
-      to_internal<double>(ctx, u, uin.p);
-      const double *young = ctx->young_d.p;
-      if (!young) {
-        std::vector<double> yv(ctx->ne, ctx->E);
-        yd.upload(yv.data(), yv.size(), ctx->stream);
-        young = yd.p;
-      }
-      if (ctx->dim == 3)
-        k_grad_young<3><<<nblk(ctx->ne), kThreads, 0, ctx->stream>>>(ctx->ne, ctx->G64.p, ctx->gstride, ctx->conn.p, ctx->bits.p,
-                                                                    ctx->lam, ctx->mu, ctx->v64.x.p, uin.p, young,
-                                                                    ctx->elem_new2old.p, g.p);
-      else
-        k_grad_young<2><<<nblk(ctx->ne), kThreads, 0, ctx->stream>>>(ctx->ne, ctx->G64.p, ctx->gstride, ctx->conn.p, ctx->bits.p,
-                                                                    ctx->lam, ctx->mu, ctx->v64.x.p, uin.p, young,
-                                                                    ctx->elem_new2old.p, g.p);
-      CKL();
-      CK(cudaMemcpyAsync(dLdE, g.p, sizeof(double) * ctx->ne, cudaMemcpyDefault, ctx->stream));
+      to_internal<double>(ctx, u, ctx->tmp64.p);
+      ctx->steps.grad.ensure(ctx->ne);
+      launch_grad_pairs(ctx, ctx->tmp64.p, ctx->v64.x.p, 0, 1, young_on_device(ctx), ctx->steps.grad.p, 0);
+      CK(cudaMemcpyAsync(dLdE, ctx->steps.grad.p, sizeof(double) * ctx->ne, cudaMemcpyDefault, ctx->stream));
     }
     CK(cudaStreamSynchronize(ctx->stream));
     return st;

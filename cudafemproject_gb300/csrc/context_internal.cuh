@@ -64,6 +64,9 @@ struct DBuf {
     CK(cudaMalloc(&p, count * sizeof(T)));
     n = count;
   }
+  void ensure(size_t count) {  // at least count elements, contents undefined when it grows
+    if (n < count) alloc(count);
+  }
   void zero(cudaStream_t s) {
     if (p) CK(cudaMemsetAsync(p, 0, n * sizeof(T), s));
   }
@@ -112,6 +115,20 @@ struct RowsData {
   double km_cK = -1, km_cM = -1;
 };
 
+// Work buffers of the time-stepping calls, kept with the context.
+template <typename T>
+struct StepVecs {
+  DBuf<T> d, v, a, y, minv;  // d: two node vectors; minv: two when re-sorted
+};
+struct StepWork {
+  StepVecs<double> f64;
+  StepVecs<float> f32;
+  DBuf<double> coef, diag_pre, diag_op, trace, obs, grad, young, states;
+  DBuf<int32_t> recv, rec_head, rec_next;
+  DBuf<DynState> st;
+  DBuf<int> stalled;
+};
+
 inline unsigned nblk(int64_t n, int t = kThreads) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace detail
@@ -134,7 +151,6 @@ struct cfem_ctx {
   Prep prep;
   RhsParts rhs;
   std::vector<double> young;  // per-element Young's modulus (caller order), empty if uniform
-  std::vector<int32_t> elems_caller;  // caller connectivity (reference slot order for the re-sorting quirk)
   double lump_c = 0, cons_c = 0;
   // mesh on device
   DBuf<int32_t> elem_off, node_off, nodes, own, node_new2old, elem_new2old, elem_old2new, conn;
@@ -170,6 +186,7 @@ struct cfem_ctx {
   int grid_geo = 0;
   int np_slots = 0;               // node slots per patch in shared memory
   RowsData rows;                  // FP64 operator
+  StepWork steps;
   DBuf<unsigned long long> grid_slots;  // grid-wide sums of the one-kernel PCG (grid_sync.cuh)
   int grid_rows = 0;              // CTAs of a grid-stride kernel over its slices
   DBuf<uint8_t> bits;
@@ -301,6 +318,8 @@ cfem_solve_params default_params();
 cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve_info *info);
 void rebuild_operator(cfem_ctx *c);
 void build_rows(cfem_ctx *c);
+// Slots and counter of a cooperative kernel's exchanges, emptied on the stream.
+GridSync start_grid_sync(cfem_ctx *c, int sets);
 // y = K' x in FP64 (internal node vectors; y is overwritten)
 void rows_apply(cfem_ctx *c, const double *x, double *y);
 void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, const cfem_options *opt);

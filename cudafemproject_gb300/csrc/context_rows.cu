@@ -2,7 +2,7 @@
 // context is created or its moduli change, applications, true residuals.
 #include "context_internal.cuh"
 #include "kernels_aux.cuh"
-#include "kernels_rows.cuh"
+#include "rows_op.cuh"
 
 namespace cfem {
 namespace detail {
@@ -86,14 +86,22 @@ void assemble(cfem_ctx *c, const int32_t *nbr, const int32_t *deg, double cK, do
   else assemble_dim<2>(c, nbr, deg, cK, cM, diag, V);
 }
 
+unsigned rows_grid(const cfem_ctx *c) { return nblk(c->rows.n_slices, kRowsThreads / 32); }
+
+}  // namespace
+
 RowOp op_of(cfem_ctx *c, const RowsValues &V) {
   const RowsData &R = c->rows;
   return RowOp{R.n_slices, R.off.p, R.row.p, R.col.p, V.val.p, V.flag.p, V.D.p, c->bits.p};
 }
 
-unsigned rows_grid(const cfem_ctx *c) { return nblk(c->rows.n_slices, kRowsThreads / 32); }
-
-}  // namespace
+GridSync start_grid_sync(cfem_ctx *c, int sets) {
+  const size_t n = grid_slots_count(kRowsPcgSets, c->n_sm);
+  if (!c->grid_slots.p) c->grid_slots.alloc(n + 1);  // (the barrier's counter follows the slots)
+  if (sets) CK(cudaMemsetAsync(c->grid_slots.p, 0xFF, n * sizeof(unsigned long long), c->stream));
+  CK(cudaMemsetAsync(c->grid_slots.p + n, 0, sizeof(unsigned long long), c->stream));
+  return GridSync{c->grid_slots.p, reinterpret_cast<unsigned *>(c->grid_slots.p + n), kWaitCycles};
+}
 
 void build_rows(cfem_ctx *c) {
   c->rows.km_cK = c->rows.km_cM = -1;  // (combined values of an earlier operator are stale)
@@ -151,10 +159,6 @@ PcgResult run_pcg_d(cfem_ctx *c, Vecs<double> &V, double cK, double cM, const do
   h.rule = rule;
   h.maxit = maxit > 0 ? maxit : 1000000;
   CK(cudaMemcpyAsync(sc, &h, sizeof(Scalars), cudaMemcpyHostToDevice, c->stream));
-  const size_t n_slots = grid_slots_count(kRowsPcgSets, c->n_sm);
-  if (!c->grid_slots.p) c->grid_slots.alloc(n_slots + 1);  // (the barrier's counter follows the slots)
-  CK(cudaMemsetAsync(c->grid_slots.p, 0xFF, n_slots * sizeof(unsigned long long), c->stream));
-  CK(cudaMemsetAsync(c->grid_slots.p + n_slots, 0, sizeof(unsigned long long), c->stream));
   RowsPcg P{};
   P.A = op_of(c, *values);
   P.f = V.f.p;
@@ -165,7 +169,7 @@ PcgResult run_pcg_d(cfem_ctx *c, Vecs<double> &V, double cK, double cM, const do
   P.p = V.pA.p;
   P.u = V.u.p;
   P.sc = sc;
-  P.sync = GridSync{c->grid_slots.p, reinterpret_cast<unsigned *>(c->grid_slots.p + n_slots), kWaitCycles};
+  P.sync = start_grid_sync(c, kRowsPcgSets);
   P.warm = warm;
   // One CTA per SM, and fewer while a CTA has a quarter of an SM for each of
   // its slices: an exchange among 76 CTAs takes 0.4 us less than among 152, and

@@ -233,27 +233,26 @@ struct DynParams {
 };
 
 // explicit: a_new = (F(t) - K d) / M ; v += (1-beta1) dt a_old + beta1 dt a_new.
-// END_STEP: the step also ends here (receivers of P.dto recorded by CTA 0, the
-// step counter advanced through the parity pair of DynState) instead of in
-// k_dyn_end_step.
-template <typename T, int DIM, bool END_STEP = false>
+// The step also ends here: receivers of P.dto recorded by CTA 0, the step
+// counter advanced through the parity pair of DynState.
+template <typename T, int DIM>
 __global__ void k_dyn_explicit(DynParams<T> P) {
   constexpr int VW = DIM == 3 ? 4 : 2;
   griddep_wait();               // y (and the new displacements) from the step's matvec
-  griddep_launch_dependents();  // (the end-of-step kernel or the next matvec)
+  griddep_launch_dependents();  // (the next matvec)
   // thread 0 reads the step and its load factors once per CTA (every thread
   // reading the same line would queue at one L2 slice)
   __shared__ T s_coef[2];
   __shared__ int s_step;
   if (threadIdx.x == 0) {
-    const int step = END_STEP ? P.st->pstep[P.parity] : P.st->step;
+    const int step = P.st->pstep[P.parity];
     s_step = step;
     s_coef[0] = (T)P.coef[2 * step];
     s_coef[1] = (T)P.coef[2 * step + 1];
   }
   __syncthreads();
   const T ca = s_coef[0], cb = s_coef[1];
-  if (END_STEP && blockIdx.x == 0)
+  if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < P.n_recv * P.dim; i += blockDim.x) {
       const int r = i / P.dim, k = i % P.dim;
       P.trace[((int64_t)(s_step - 1) * P.n_recv + r) * P.dim + k] = (double)P.dto[(int64_t)P.recv[r] * VW + k];
@@ -273,7 +272,7 @@ __global__ void k_dyn_explicit(DynParams<T> P) {
     stv<T, VW>(P.v, n, v);
     stv<T, VW>(P.y, n, zero);
   }
-  if (END_STEP && blockIdx.x == 0 && threadIdx.x == 0) P.st->pstep[P.parity ^ 1] = s_step + 1;
+  if (blockIdx.x == 0 && threadIdx.x == 0) P.st->pstep[P.parity ^ 1] = s_step + 1;
 }
 
 // implicit: rhs = F(t) - K d ; y = 0
@@ -331,34 +330,11 @@ __global__ void k_dyn_end_step(DynParams<T> P, const T *d, int VW) {
   if (threadIdx.x == 0) P.st->step = step + 1;
 }
 
-static __global__ void k_dyn_advance(DynState *st) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) st->step += 1;
-}
-
-// ------------------------------------------------------------------ reference re-sorting quirk
-// The reference assembles an element-local vector by sorting it by DOF key in
-// place (cpu_fem_utils.cpp:437-445): after each assembly the source holds its
-// values in key order. For sources that are assembled repeatedly (lumped mass
-// in explicit dynamics, preconditioner diagonal in implicit dynamics) the next
-// assembly then mixes values of different elements. These kernels reproduce
-// it: out[dof] = sum of the DOF's slots in element order, then src = src[perm].
-static __global__ void k_assemble_slots(int64_t ndof, int dim, int vw, const int64_t *seg, const int32_t *perm,
-                                 const double *src, const int32_t *old2new, double *out_node_vec, int invert,
-                                 float *out32) {
-  int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (k >= ndof) return;
-  double acc = 0;
-  for (int64_t j = seg[k]; j < seg[k + 1]; ++j) acc += src[perm[j]];
-  int64_t node = k / dim, d = k % dim;
-  int64_t idx = (int64_t)old2new[node] * vw + d;
-  double v = invert ? (acc != 0 ? 1.0 / acc : 0.0) : acc;
-  out_node_vec[idx] = v;
-  if (out32) out32[idx] = (float)v;
-}
-
-static __global__ void k_permute(int64_t n, const int32_t *perm, const double *src, double *dst) {
-  int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (j < n) dst[j] = src[perm[j]];
+// FP64 implicit predictor: d_new = d + c1 v + c2 a
+static __global__ void k_dyn_predict(int64_t n, const double *d, const double *v, const double *a, double c1, double c2,
+                                     double *to) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) to[i] = d[i] + (c1 * v[i] + c2 * a[i]);
 }
 
 // ------------------------------------------------------------------ element matrices (checks)
@@ -397,89 +373,6 @@ __global__ void k_element_matrices(int64_t first, int64_t count, const int32_t *
           if (r != c && (cr || cc)) v = 0;
           K[r * W + c] = v;
         }
-}
-
-// dL/dE_e = -(1/E_e) lambda_e^T K'_e u_e (gradient form; constrained slots keep K_e's diagonal)
-template <int DIM>
-__global__ void k_grad_young(int64_t ne, const double *G64, int64_t gstride, const int32_t *conn, const uint8_t *bits,
-                             double lam, double mu, const double *lamv, const double *uv, const double *young,
-                             const int32_t *elem_new2old, double *g_out, int accumulate = 0) {
-  constexpr int NV = DIM + 1, VW = DIM == 3 ? 4 : 2;
-  int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  double G[DIM * DIM], u[NV][DIM], l[NV][DIM], f[NV][DIM];
-  for (int k = 0; k < DIM * DIM; ++k) G[k] = G64[(size_t)k * gstride + e];
-  double diag_terms = 0;
-  for (int a = 0; a < NV; ++a) {
-    int n = conn[e * NV + a];
-    unsigned b = bits[n];
-    for (int d = 0; d < DIM; ++d) {
-      bool c = b >> d & 1u;
-      u[a][d] = c ? 0.0 : uv[(int64_t)n * VW + d];
-      l[a][d] = c ? 0.0 : lamv[(int64_t)n * VW + d];
-    }
-  }
-  element_force<double, DIM>(u, G, lam, mu, 1.0, 0.0, f);
-  double acc = 0;
-  for (int a = 0; a < NV; ++a)
-    for (int d = 0; d < DIM; ++d) acc += l[a][d] * f[a][d];
-  // constrained slots: K_e diagonal term
-  double g0[DIM];
-  for (int d = 0; d < DIM; ++d) {
-    g0[d] = 0;
-    for (int a = 1; a < NV; ++a) g0[d] -= G[(a - 1) * DIM + d];
-  }
-  for (int a = 0; a < NV; ++a) {
-    int n = conn[e * NV + a];
-    unsigned b = bits[n];
-    if (!b) continue;
-    double sq[DIM], tot = 0;
-    for (int d = 0; d < DIM; ++d) {
-      double gd = a == 0 ? g0[d] : G[(a - 1) * DIM + d];
-      sq[d] = gd * gd;
-      tot += sq[d];
-    }
-    for (int d = 0; d < DIM; ++d)
-      if (b >> d & 1u) {
-        double kd = (lam + 2 * mu) * sq[d] + mu * (tot - sq[d]);
-        diag_terms += lamv[(int64_t)n * VW + d] * kd * uv[(int64_t)n * VW + d];
-      }
-  }
-  int64_t eo = elem_new2old[e];
-  const double v = -(acc + diag_terms) / young[eo];
-  g_out[eo] = accumulate ? g_out[eo] + v : v;
-}
-
-// ---- explicit GN22 adjoint (reverse of one step; see cfem_dyn_adjoint) ----
-// receiver misfit: db[node_r] += d_n[node_r] - obs_n[r]
-static __global__ void k_adj_receivers(int n_rec, int dim, int vw, const int32_t *recv, const double *d,
-                                       const double *obs_n, double *db) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_rec * dim) return;
-  int r = i / dim, q = i % dim;
-  int64_t k = (int64_t)recv[r] * vw + q;
-  db[k] += d[k] - obs_n[i];
-}
-
-// w = (a_bar + h_new v_bar) / M ; a_bar = h_old v_bar
-static __global__ void k_adj_pre(int64_t n, double h_old, double h_new, const double *minv, const double *vb,
-                                 double *ab, double *wb) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double an = ab[i] + h_new * vb[i];
-  wb[i] = an * minv[i];
-  ab[i] = h_old * vb[i];
-}
-
-// d_tot = d_bar - K w ; d_bar = d_tot ; v_bar += dt d_tot ; a_bar += c2 d_tot ; y = 0
-static __global__ void k_adj_post(int64_t n, double dt, double c2, double *y, double *db, double *vb, double *ab) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double t = db[i] - y[i];
-  y[i] = 0;
-  db[i] = t;
-  vb[i] += dt * t;
-  ab[i] += c2 * t;
 }
 
 // Element strain / stress recovery (deprecated/femfunc/femfunc.cpp:42-106:

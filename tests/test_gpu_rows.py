@@ -100,3 +100,52 @@ def test_fp64_pcg_shapes_against_the_oracle(n):
         assert rel(u, x) <= 1e-12
     u, _ = ctx.pcg(f, "fp64", tol=1e-13, stop_rule="residual")
     assert rel(u, o.pcg(f, tol=1e-13, rule=1)[0]) <= 1e-10
+
+
+def _column(nx, ny, nz):
+    return meshgen.box_3d(nx, ny, nz, lz=4.0, jitter=0.2, seed=5, rho=2000.0, traction=None,
+                          point_load=("top_centre", (0.4, -0.3, -1.0)))
+
+
+@pytest.mark.parametrize("semantics", ["consistent", "compat"])
+@pytest.mark.parametrize("mesh,steps", [("tet", 1), ("tet", 2), ("hub300", 5), ("strip513", 6), ("column", 7), ("plate198", 3)])
+def test_fp64_explicit_steps_against_the_oracle(semantics, mesh, steps):
+    """One-kernel explicit steps, rows in registers (the small meshes) and in
+    memory (39,601 nodes: more slices than warps), constant and re-sorted lumped
+    masses (segments longer than a staging tile: the hub's 301 elements). The
+    recurrence is the oracle's with other summation orders: a few steps stay
+    within 1e-11."""
+    from cudafemproject_gb300.solver import FemContext
+    p = {"column": lambda: _column(4, 3, 17), "plate198": lambda: meshgen.square_2d(198)}.get(mesh, MESHES.get(mesh))()
+    if not len(p.face_elem) and not len(p.load_node):
+        p.load_node, p.load_vec = np.array([p.n_nodes - 1], np.int32), np.full((1, p.dim), 0.5)
+    dt, T = 1e-6, steps * 1e-6 * 1.0000001
+    rec = np.array([p.n_nodes - 1, 0, p.n_nodes // 2, p.n_nodes - 1], np.int32)
+    ug, st, _ = O.Oracle(p, consistent=semantics == "consistent").dyn(0.5, 0.0, dt, T)
+    u, info, trace = FemContext(p, semantics=semantics).dyn(0.5, 0.0, dt, T, precision="fp64", receivers=rec)
+    assert info["steps"] == st == steps
+    assert rel(u, ug) <= 1e-11
+    assert np.array_equal(trace[-1], u[rec])
+
+
+@pytest.mark.parametrize("states_mb", [None, "0"])
+@pytest.mark.parametrize("mesh,steps", [("column", 1), ("column", 16), ("column", 17), ("strip513", 9)])
+def test_dyn_adjoint_whole_and_by_segments(monkeypatch, states_mb, mesh, steps):
+    """The reverse sweep with every state held and with checkpoints (one segment,
+    full ones, a short last one), a receiver listed twice."""
+    from cudafemproject_gb300.solver import FemContext
+    if states_mb is None:
+        monkeypatch.delenv("CFEM_DYN_STATES_MB", raising=False)
+    else:
+        monkeypatch.setenv("CFEM_DYN_STATES_MB", states_mb)
+    p = _column(4, 3, 17) if mesh == "column" else _strip(513)
+    if not len(p.load_node):
+        p.load_node, p.load_vec = np.array([400], np.int32), np.full((1, 2), 0.5)
+    dt, T = 1e-5, steps * 1e-5 * 1.0000001
+    rec = np.array([p.n_nodes - 3, p.n_nodes // 2, p.n_nodes - 3], np.int32)
+    obs = 1e-9 * np.random.default_rng(1).standard_normal((steps, 3, p.dim))
+    L, g, info = FemContext(p, semantics="consistent").dyn_adjoint(0.5, dt, T, rec, obs)
+    Lo, go = O.Oracle(p, consistent=True).dyn_adjoint(0.5, dt, T, rec, obs)
+    assert info["steps"] == steps
+    assert abs(L - Lo) <= 1e-11 * abs(Lo)
+    assert rel(g, go) <= 1e-11
