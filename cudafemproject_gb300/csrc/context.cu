@@ -42,79 +42,59 @@ MvParams<T> base_mv_t(cfem_ctx *c) {
   return P;
 }
 
-template <typename T>
-void launch_mv_t(cfem_ctx *c, int mode, const MvParams<T> &P) {
+void launch_mv_f(cfem_ctx *c, int mode, const MvParams<float> &P) {
   if (!P.patch_inst) single_mesh_only(c);
-  // FP32: patch blocks streamed by bulk copies. FP64 keeps the plain fan
-  // kernel below: it is bound by the FP64 pipe, and its twice-as-large blocks
-  // would leave one CTA per SM.
-  if constexpr (sizeof(T) == 4) {
-    if (c->fans && c->fan_tma) {
-      FanTmaParams F{};
-      F.blocks = c->blk32.p;
-      F.L = c->L32;
-      F.fan_off = c->fan_off.p;
-      F.fan_elem_off = c->fan_elem_off.p;
-      F.err = c->tma_err.p;
-      F.skip_patch_plus1 = c->selftest_skip_plus1;
-      F.wait_limit = c->selftest_wait_limit;
-      const double l2_half = 0.5 * c->l2_bytes;
-      F.evict_first = (double)c->L32.bytes * c->prep.n_patches > l2_half;
-      if (c->geo && !P.patch_inst) {
-        F.blocks = c->blkg.p;
-        F.L = c->Lg;
-        F.evict_first = (double)c->Lg.bytes * c->prep.n_patches > l2_half;
-        dim3 g(c->grid_geo), b(kHfanThreads);
-        if (P.mcoef && mode == MV_PLAIN)
-          k_matvec_fan_tma<float, MV_PLAIN, true, true><<<g, b, c->smem_geo, c->stream>>>(P, F);
-        else if (P.mcoef && mode == MV_PCG)
-          launch_pdl(k_matvec_fan_tma<float, MV_PCG, true, true>, g, b, c->smem_geo, c->stream, P, F);
-        else if (mode == MV_PLAIN) k_matvec_fan_tma<float, MV_PLAIN, true><<<g, b, c->smem_geo, c->stream>>>(P, F);
-        else if (mode == MV_PCG) launch_pdl(k_matvec_fan_tma<float, MV_PCG, true>, g, b, c->smem_geo, c->stream, P, F);
-        else launch_pdl(k_matvec_fan_tma<float, MV_DYN, true>, g, b, c->smem_geo, c->stream, P, F);
-        CKL();
-        c->launches += 1;
-        return;
-      }
-      dim3 g(c->grid_ft32), b(kHfanThreads);
-      if (P.patch_inst) {
-        if (mode != MV_PCG || P.mcoef) throw Fail{CFEM_ERR_UNSUPPORTED, "batched meshes: PCG-form static matvec only"};
-        launch_pdl(k_matvec_fan_tma<float, MV_PCG, false, false, true>, g, b, c->smem_ft32, c->stream, P, F);
-      } else if (P.mcoef && mode == MV_PLAIN)
-        k_matvec_fan_tma<float, MV_PLAIN, false, true><<<g, b, c->smem_ft32, c->stream>>>(P, F);
+  if (c->fans) {  // patch blocks streamed by bulk copies
+    FanTmaParams F{};
+    F.blocks = c->blk32.p;
+    F.L = c->L32;
+    F.fan_off = c->fan_off.p;
+    F.fan_elem_off = c->fan_elem_off.p;
+    F.err = c->tma_err.p;
+    F.skip_patch_plus1 = c->selftest_skip_plus1;
+    F.wait_limit = c->selftest_wait_limit;
+    const double l2_half = 0.5 * c->l2_bytes;
+    F.evict_first = (double)c->L32.bytes * c->prep.n_patches > l2_half;
+    if (c->geo && !P.patch_inst) {
+      F.blocks = c->blkg.p;
+      F.L = c->Lg;
+      F.evict_first = (double)c->Lg.bytes * c->prep.n_patches > l2_half;
+      dim3 g(c->grid_geo), b(kHfanThreads);
+      if (P.mcoef && mode == MV_PLAIN)
+        k_matvec_fan_tma<float, MV_PLAIN, true, true><<<g, b, c->smem_geo, c->stream>>>(P, F);
       else if (P.mcoef && mode == MV_PCG)
-        launch_pdl(k_matvec_fan_tma<float, MV_PCG, false, true>, g, b, c->smem_ft32, c->stream, P, F);
-      else if (mode == MV_PLAIN) k_matvec_fan_tma<float, MV_PLAIN><<<g, b, c->smem_ft32, c->stream>>>(P, F);
-      else if (mode == MV_PCG) launch_pdl(k_matvec_fan_tma<float, MV_PCG>, g, b, c->smem_ft32, c->stream, P, F);
-      else launch_pdl(k_matvec_fan_tma<float, MV_DYN>, g, b, c->smem_ft32, c->stream, P, F);
+        launch_pdl(k_matvec_fan_tma<float, MV_PCG, true, true>, g, b, c->smem_geo, c->stream, P, F);
+      else if (mode == MV_PLAIN) k_matvec_fan_tma<float, MV_PLAIN, true><<<g, b, c->smem_geo, c->stream>>>(P, F);
+      else if (mode == MV_PCG) launch_pdl(k_matvec_fan_tma<float, MV_PCG, true>, g, b, c->smem_geo, c->stream, P, F);
+      else launch_pdl(k_matvec_fan_tma<float, MV_DYN, true>, g, b, c->smem_geo, c->stream, P, F);
       CKL();
       c->launches += 1;
       return;
     }
-  }
-  if (c->fans && c->dim == 3) {
-    FanParams F{c->fan_off.p, c->fan_elem_off.p, c->fan_slot.p, c->finc.p, c->finc_start.p, c->fstride};
-    const T *Gf;
-    if constexpr (sizeof(T) == 8) Gf = c->Gf64.p; else Gf = c->Gf32.p;
-    const size_t smem = sizeof(T) == 8 ? c->smem_fan64 : c->smem_fan32;
-    dim3 g(c->grid_fan), b(kFanThreads);
-    if (mode == MV_PLAIN) k_matvec_fan<T, MV_PLAIN><<<g, b, smem, c->stream>>>(P, F, Gf);
-    else if (mode == MV_PCG) k_matvec_fan<T, MV_PCG><<<g, b, smem, c->stream>>>(P, F, Gf);
-    else k_matvec_fan<T, MV_DYN><<<g, b, smem, c->stream>>>(P, F, Gf);
-    CKL();
+    dim3 g(c->grid_ft32), b(kHfanThreads);
+    if (P.patch_inst) {
+      if (mode != MV_PCG || P.mcoef) throw Fail{CFEM_ERR_UNSUPPORTED, "batched meshes: PCG-form static matvec only"};
+      launch_pdl(k_matvec_fan_tma<float, MV_PCG, false, false, true>, g, b, c->smem_ft32, c->stream, P, F);
+    } else if (P.mcoef && mode == MV_PLAIN)
+      k_matvec_fan_tma<float, MV_PLAIN, false, true><<<g, b, c->smem_ft32, c->stream>>>(P, F);
+    else if (P.mcoef && mode == MV_PCG)
+      launch_pdl(k_matvec_fan_tma<float, MV_PCG, false, true>, g, b, c->smem_ft32, c->stream, P, F);
+    else if (mode == MV_PLAIN) k_matvec_fan_tma<float, MV_PLAIN><<<g, b, c->smem_ft32, c->stream>>>(P, F);
+    else if (mode == MV_PCG) launch_pdl(k_matvec_fan_tma<float, MV_PCG>, g, b, c->smem_ft32, c->stream, P, F);
+    else launch_pdl(k_matvec_fan_tma<float, MV_DYN>, g, b, c->smem_ft32, c->stream, P, F);
+  CKL();
     c->launches += 1;
     return;
   }
-  size_t smem = sizeof(T) == 8 ? c->smem64 : c->smem32;
   dim3 g(c->grid_mv), b(kThreads);
   if (c->dim == 3) {
-    if (mode == MV_PLAIN) k_matvec<T, 3, MV_PLAIN><<<g, b, smem, c->stream>>>(P);
-    else if (mode == MV_PCG) k_matvec<T, 3, MV_PCG><<<g, b, smem, c->stream>>>(P);
-    else k_matvec<T, 3, MV_DYN><<<g, b, smem, c->stream>>>(P);
+    if (mode == MV_PLAIN) k_matvec<float, 3, MV_PLAIN><<<g, b, c->smem32, c->stream>>>(P);
+    else if (mode == MV_PCG) k_matvec<float, 3, MV_PCG><<<g, b, c->smem32, c->stream>>>(P);
+    else k_matvec<float, 3, MV_DYN><<<g, b, c->smem32, c->stream>>>(P);
   } else {
-    if (mode == MV_PLAIN) k_matvec<T, 2, MV_PLAIN><<<g, b, smem, c->stream>>>(P);
-    else if (mode == MV_PCG) k_matvec<T, 2, MV_PCG><<<g, b, smem, c->stream>>>(P);
-    else k_matvec<T, 2, MV_DYN><<<g, b, smem, c->stream>>>(P);
+    if (mode == MV_PLAIN) k_matvec<float, 2, MV_PLAIN><<<g, b, c->smem32, c->stream>>>(P);
+    else if (mode == MV_PCG) k_matvec<float, 2, MV_PCG><<<g, b, c->smem32, c->stream>>>(P);
+    else k_matvec<float, 2, MV_DYN><<<g, b, c->smem32, c->stream>>>(P);
   }
   CKL();
   c->launches += 1;
@@ -125,8 +105,7 @@ void launch_mv_t(cfem_ctx *c, int mode, const MvParams<T> &P) {
 template <typename T>
 int pcg_mv_grid(const cfem_ctx *c) {
   if constexpr (sizeof(T) == 4)
-    if (c->fans && c->fan_tma) return c->geo ? c->grid_geo : c->grid_ft32;
-  if (c->fans && c->dim == 3) return c->grid_fan;
+    if (c->fans) return c->geo ? c->grid_geo : c->grid_ft32;
   return c->grid_mv;
 }
 
@@ -184,7 +163,7 @@ PcgResult run_pcg_t(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int war
     mv.x = V.x.p;
     mv.y = V.u.p;
     V.u.zero(c->stream);
-    launch_mv<T>(c, MV_PLAIN, mv);
+    launch_mv_f(c, MV_PLAIN, mv);
   }
   launch_init<T>(c, vec_params<T>(c, V, V.pA.p, sc), warm);
   if (cont_p && cont_gamma_prev > 0) {
@@ -212,7 +191,7 @@ PcgResult run_pcg_t(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int war
       m.xout = pnew;
       m.y = ucur;
       m.yzero = (it & 1) ? V.u.p : V.uB.p;
-      launch_mv<T>(c, MV_PCG, m);
+      launch_mv_f(c, MV_PCG, m);
       VecParams<T> up = vec_params<T>(c, V, pnew, sc);
       up.u = ucur;
       up.cond = cond;
@@ -353,8 +332,6 @@ void to_caller_t(cfem_ctx *c, const T *src, double *dst) {
 
 MvParams<double> base_mv_d(cfem_ctx *c) { return base_mv_t<double>(c); }
 MvParams<float> base_mv_f(cfem_ctx *c) { return base_mv_t<float>(c); }
-void launch_mv_d(cfem_ctx *c, int mode, const MvParams<double> &P) { launch_mv_t<double>(c, mode, P); }
-void launch_mv_f(cfem_ctx *c, int mode, const MvParams<float> &P) { launch_mv_t<float>(c, mode, P); }
 PcgResult run_pcg_f(cfem_ctx *c, Vecs<float> &V, float cK, float cM, const float *mcoef, int warm, double tol,
                     int rule, int maxit) {
   return run_pcg_t<float>(c, V, cK, cM, mcoef, warm, tol, rule, maxit);
@@ -566,15 +543,8 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
     c->inc_start.upload(P.inc_start.data(), P.inc_start.size(), s);
   }
   if (c->fans) {
-    c->fstride = (P.n_fans + 31) / 32 * 32;
-    std::vector<uint16_t> slot((size_t)kFanSlots * c->fstride, 0);
-    for (int64_t f = 0; f < P.n_fans; ++f)
-      for (int k = 0; k < kFanSlots; ++k) slot[(size_t)k * c->fstride + f] = P.fan_slot[f * kFanSlots + k];
-    c->fan_slot.upload(slot.data(), slot.size(), s);
     c->fan_off.upload(P.p_fan_off.data(), P.p_fan_off.size(), s);
     c->fan_elem_off.upload(P.fan_elem_off.data(), P.fan_elem_off.size(), s);
-    c->finc.upload(P.finc.data(), P.finc.size(), s);
-    c->finc_start.upload(P.finc_start.data(), P.finc_start.size(), s);
     std::vector<int32_t> pos(c->ne);
     for (int64_t f = 0; f < P.n_fans; ++f)
       for (int32_t e = P.fan_elem_off[f]; e < P.fan_elem_off[f + 1]; ++e) pos[e] = (int32_t)(f * 8 + (e - P.fan_elem_off[f]));
@@ -690,7 +660,7 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
     // instance tables: patch -> instance, instance patch ranges, owned node ranges, materials
     std::vector<int32_t> pinst(P.n_patches), ipo(c->n_inst + 1, 0), ofirst(P.n_patches + 1);
     std::vector<float> pm32(2 * (size_t)P.n_patches);
-    std::vector<double> pm64(2 * (size_t)P.n_patches), le(c->ne), me(c->ne);
+    std::vector<double> le(c->ne), me(c->ne);
     int64_t running = 0;
     for (int p = 0; p < P.n_patches; ++p) {
       pinst[p] = c->elem_group[P.elem_new2old[P.p_elem_off[p]]];
@@ -702,8 +672,6 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
       running += n - own;
       pm32[2 * p] = (float)c->inst_lam[pinst[p]];
       pm32[2 * p + 1] = (float)c->inst_mu[pinst[p]];
-      pm64[2 * p] = c->inst_lam[pinst[p]];
-      pm64[2 * p + 1] = c->inst_mu[pinst[p]];
     }
     ofirst[P.n_patches] = (int32_t)running;
     if (running != c->nn) throw Fail{CFEM_ERR_MESH, "internal error: owned node count"};
@@ -717,7 +685,6 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
     c->inst_patch_off.upload(ipo.data(), ipo.size(), s);
     c->own_first.upload(ofirst.data(), ofirst.size(), s);
     c->pmat32.upload(pm32.data(), pm32.size(), s);
-    c->pmat64.upload(pm64.data(), pm64.size(), s);
     c->lam_e.upload(le.data(), le.size(), s);
     c->mu_e.upload(me.data(), me.size(), s);
     CK(cudaStreamSynchronize(s));
@@ -780,17 +747,11 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
   };
   int occ = 1;
   if (c->dim == 3) {
-    set_smem((const void *)k_matvec<double, 3, MV_PLAIN>, c->smem64);
-    set_smem((const void *)k_matvec<double, 3, MV_PCG>, c->smem64);
-    set_smem((const void *)k_matvec<double, 3, MV_DYN>, c->smem64);
     set_smem((const void *)k_matvec<float, 3, MV_PLAIN>, c->smem32);
     set_smem((const void *)k_matvec<float, 3, MV_PCG>, c->smem32);
     set_smem((const void *)k_matvec<float, 3, MV_DYN>, c->smem32);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_matvec<float, 3, MV_PCG>, kThreads, c->smem32));
   } else {
-    set_smem((const void *)k_matvec<double, 2, MV_PLAIN>, c->smem64);
-    set_smem((const void *)k_matvec<double, 2, MV_PCG>, c->smem64);
-    set_smem((const void *)k_matvec<double, 2, MV_DYN>, c->smem64);
     set_smem((const void *)k_matvec<float, 2, MV_PLAIN>, c->smem32);
     set_smem((const void *)k_matvec<float, 2, MV_PCG>, c->smem32);
     set_smem((const void *)k_matvec<float, 2, MV_DYN>, c->smem32);
@@ -799,31 +760,16 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
   occ = std::max(occ, 1);
   c->grid_mv = (int)std::min<int64_t>(P.n_patches, (int64_t)c->n_sm * occ);
   if (c->fans) {
-    c->smem_fan64 = fan_smem_bytes(sizeof(double), c->np_slots);
-    c->smem_fan32 = fan_smem_bytes(sizeof(float), c->np_slots);
-    if (c->smem_fan64 + 8192 > (size_t)smem_optin)
-      throw Fail{CFEM_ERR_INVALID_ARGUMENT, "fan patch too large for shared memory: lower patch_elems"};
-    for (const void *k : {(const void *)k_matvec_fan<double, MV_PLAIN>, (const void *)k_matvec_fan<double, MV_PCG>,
-                          (const void *)k_matvec_fan<double, MV_DYN>, (const void *)k_matvec_fan<float, MV_PLAIN>,
-                          (const void *)k_matvec_fan<float, MV_PCG>, (const void *)k_matvec_fan<float, MV_DYN>})
-      CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 8192));
-    int occf = 1;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occf, k_matvec_fan<float, MV_PCG>, kFanThreads, c->smem_fan32));
-    c->grid_fan = (int)std::min<int64_t>(P.n_patches, (int64_t)c->n_sm * std::max(occf, 1));
     c->smem_ft32 = fan_tma_smem_bytes(c->L32, sizeof(float));
-    if (c->smem_ft32 + 8192 > (size_t)smem_optin) c->fan_tma = false;
-    if (c->fan_tma) {
-      for (const void *k : {(const void *)k_matvec_fan_tma<float, MV_PLAIN>, (const void *)k_matvec_fan_tma<float, MV_PCG>,
-                            (const void *)k_matvec_fan_tma<float, MV_DYN>,
-                            (const void *)k_matvec_fan_tma<float, MV_PLAIN, false, true>,
-                            (const void *)k_matvec_fan_tma<float, MV_PCG, false, true>,
-                            (const void *)k_matvec_fan_tma<float, MV_PCG, false, false, true>})
-        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 8192));
-      int o32 = 1;
-      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o32, k_matvec_fan_tma<float, MV_PCG>, kHfanThreads, c->smem_ft32));
-      c->grid_ft32 = (int)std::min<int64_t>(P.n_patches, (int64_t)c->n_sm * std::max(o32, 1));
-    }
-    if (c->geo && !c->fan_tma) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "fan patch too large for shared memory: lower patch_elems"};
+    for (const void *k : {(const void *)k_matvec_fan_tma<float, MV_PLAIN>, (const void *)k_matvec_fan_tma<float, MV_PCG>,
+                          (const void *)k_matvec_fan_tma<float, MV_DYN>,
+                          (const void *)k_matvec_fan_tma<float, MV_PLAIN, false, true>,
+                          (const void *)k_matvec_fan_tma<float, MV_PCG, false, true>,
+                          (const void *)k_matvec_fan_tma<float, MV_PCG, false, false, true>})
+      CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 8192));
+    int o32 = 1;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o32, k_matvec_fan_tma<float, MV_PCG>, kHfanThreads, c->smem_ft32));
+    c->grid_ft32 = (int)std::min<int64_t>(P.n_patches, (int64_t)c->n_sm * std::max(o32, 1));
     if (c->geo) {
       // the largest layout (with scale rows) bounds the shared memory of every later rebuild
       const size_t smem_max = fan_tma_smem_bytes(fan_geo_block_layout(P.np_max, true), sizeof(float));
@@ -847,7 +793,7 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
     c->grid_geo = (int)std::min<int64_t>(P.n_patches, (int64_t)c->n_sm * std::max(og, 1));
   }
   c->grid_rows = c->n_sm * 16;
-  int maxgrid = std::max({c->grid_mv, c->grid_vec, c->grid_fan, c->grid_ft32, c->grid_geo, c->grid_rows});
+  int maxgrid = std::max({c->grid_mv, c->grid_vec, c->grid_ft32, c->grid_geo, c->grid_rows});
   c->partials.alloc((size_t)maxgrid * 4);
   c->partials_up.alloc((size_t)std::max(c->grid_upd, c->grid_vec) * 2);
   c->partials_up.zero(s);
@@ -945,15 +891,6 @@ void rebuild_operator(cfem_ctx *c) {
   else k_geometry<2><<<nblk(c->ne), kThreads, 0, s>>>(gp);
   CKL();
   if (c->fans) {
-    if (!c->Gf64.p) {
-      c->Gf64.alloc((size_t)kFanMax * 9 * c->fstride);
-      c->Gf32.alloc((size_t)kFanMax * 9 * c->fstride);
-    }
-    c->Gf64.zero(s);
-    c->Gf32.zero(s);
-    k_fan_gradients<<<nblk(c->ne), kThreads, 0, s>>>(c->ne, c->G64.p, c->gstride, c->fan_pos.p, c->fan_perm.p, c->Gf64.p,
-                                                     c->Gf32.p, c->fstride);
-    CKL();
     k_fan_block_gradients<<<nblk(c->ne), kThreads, 0, s>>>(c->ne, c->G64.p, c->gstride, c->fan_pos.p, c->fan_perm.p,
                                                            c->fan_patch.p, c->fan_off.p, c->blk32.p, c->L32);
     CKL();
@@ -1196,7 +1133,7 @@ cfem_status cfem_rhs(cfem_ctx *ctx, const cfem_wavelet *w, double t, double *f) 
 cfem_status cfem_selftest_copy_timeout(cfem_ctx *ctx) {
   return run_guarded([&]() -> cfem_status {
     check_ctx(ctx);
-    if (!(ctx->fans && ctx->fan_tma) || ctx->n_inst)
+    if (!ctx->fans || ctx->n_inst)
       throw Fail{CFEM_ERR_UNSUPPORTED, "the copy-timeout self-test needs a single-mesh 3D edge-fan context"};
     enter(ctx);
     // one FP32 matvec whose first block of patch 0 is never requested, with
@@ -1211,7 +1148,7 @@ cfem_status cfem_selftest_copy_timeout(cfem_ctx *ctx) {
     ctx->selftest_skip_plus1 = 1;
     ctx->selftest_wait_limit = 2000000;
     try {
-      launch_mv<float>(ctx, MV_PLAIN, mv);
+      launch_mv_f(ctx, MV_PLAIN, mv);
     } catch (...) {
       ctx->selftest_skip_plus1 = 0;
       ctx->selftest_wait_limit = 0;
@@ -1255,7 +1192,7 @@ cfem_status cfem_matvec(cfem_ctx *ctx, int32_t precision, const void *x, void *y
       mv.x = ctx->v32.z.p;
       mv.y = ctx->v32.u.p;
       ctx->v32.u.zero(ctx->stream);
-      launch_mv<float>(ctx, MV_PLAIN, mv);
+      launch_mv_f(ctx, MV_PLAIN, mv);
       to_caller<float>(ctx, ctx->v32.u.p, xin.p);
       k_convert<double, float><<<nblk(ctx->nd), kThreads, 0, ctx->stream>>>(ctx->nd, xin.p, xf.p);
       CKL();
@@ -1323,30 +1260,21 @@ cfem_status cfem_profile_matvec(cfem_ctx *ctx, int32_t precision, int32_t n_laun
     ctx->partials_up.zero(ctx->stream);
     static const double one[2] = {1.0, 1.0};
     CK(cudaMemcpyAsync(ctx->partials_up.p, one, sizeof(one), cudaMemcpyHostToDevice, ctx->stream));
-    const size_t ts = precision == CFEM_FP64 ? 8 : 4;
     auto run = [&](int n) {
       for (int i = 0; i < n; ++i) {
         if (precision == CFEM_FP64) {
-          MvParams<double> mv = base_mv<double>(ctx);
-          mv.diagA = ctx->v64.diagA.p;
-          mv.sc = sc;
-          mv.x = ctx->v64.z.p;
-          mv.x2 = (i & 1) ? ctx->v64.pB.p : ctx->v64.pA.p;
-          mv.xout = (i & 1) ? ctx->v64.pA.p : ctx->v64.pB.p;
-          mv.y = (i & 1) ? ctx->v64.uB.p : ctx->v64.u.p;
-          mv.yzero = (i & 1) ? ctx->v64.u.p : ctx->v64.uB.p;
-          launch_mv<double>(ctx, MV_PCG, mv);
-        } else {
-          MvParams<float> mv = base_mv<float>(ctx);
-          mv.diagA = ctx->v32.diagA.p;
-          mv.sc = sc;
-          mv.x = ctx->v32.z.p;
-          mv.x2 = (i & 1) ? ctx->v32.pB.p : ctx->v32.pA.p;
-          mv.xout = (i & 1) ? ctx->v32.pA.p : ctx->v32.pB.p;
-          mv.y = (i & 1) ? ctx->v32.uB.p : ctx->v32.u.p;
-          mv.yzero = (i & 1) ? ctx->v32.u.p : ctx->v32.uB.p;
-          launch_mv<float>(ctx, MV_PCG, mv);
+          rows_apply(ctx, ctx->v64.z.p, ctx->tmp64.p);
+          continue;
         }
+        MvParams<float> mv = base_mv<float>(ctx);
+        mv.diagA = ctx->v32.diagA.p;
+        mv.sc = sc;
+        mv.x = ctx->v32.z.p;
+        mv.x2 = (i & 1) ? ctx->v32.pB.p : ctx->v32.pA.p;
+        mv.xout = (i & 1) ? ctx->v32.pA.p : ctx->v32.pB.p;
+        mv.y = (i & 1) ? ctx->v32.uB.p : ctx->v32.u.p;
+        mv.yzero = (i & 1) ? ctx->v32.u.p : ctx->v32.uB.p;
+        launch_mv_f(ctx, MV_PCG, mv);
       }
     };
     run(3);  // warm-up
@@ -1357,23 +1285,21 @@ cfem_status cfem_profile_matvec(cfem_ctx *ctx, int32_t precision, int32_t n_laun
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
     if (ms_per_launch) *ms_per_launch = ms / n_launches;
-    // algorithmic bytes: the operator (stored gradients + 8 bytes of connectivity
-    // per element; geometry form: the streamed patch blocks, which hold the
-    // connectivity, scatter tables and coordinates) and five node-vector
-    // streams (z and p_old read, p and A p written, the next A p zeroed)
-    if (bytes_per_launch)
-      *bytes_per_launch = (ctx->geo && precision == CFEM_FP32
-                               ? (double)ctx->prep.n_patches * ctx->Lg.bytes
-                               : (double)ctx->ne * (ctx->ncomp * ts + 8)) +
-                          (double)ctx->nn * ctx->vw * ts * 5;
-    // leave the work vectors clean for the next solve
-    if (precision == CFEM_FP64) {
-      ctx->v64.u.zero(ctx->stream);
-      ctx->v64.uB.zero(ctx->stream);
-    } else {
-      ctx->v32.u.zero(ctx->stream);
-      ctx->v32.uB.zero(ctx->stream);
+    // algorithmic bytes, FP32: the operator (stored gradients + 8 bytes of
+    // connectivity per element; geometry form: the streamed patch blocks, which
+    // hold the connectivity, scatter tables and coordinates) and five node-vector
+    // streams (z and p_old read, p and A p written, the next A p zeroed); FP64:
+    // the row blocks and their columns, x read and y written
+    if (bytes_per_launch) {
+      if (precision == CFEM_FP64)
+        *bytes_per_launch = (double)ctx->rows.steps * 32 * (ctx->ncomp * 8 + 4) + (double)ctx->nn * ctx->vw * 8 * 2;
+      else
+        *bytes_per_launch = (ctx->geo ? (double)ctx->prep.n_patches * ctx->Lg.bytes : (double)ctx->ne * (ctx->ncomp * 4 + 8)) +
+                            (double)ctx->nn * ctx->vw * 4 * 5;
     }
+    // leave the work vectors clean for the next solve
+    ctx->v32.u.zero(ctx->stream);
+    ctx->v32.uB.zero(ctx->stream);
     check_copy_error(ctx);
     return CFEM_OK;
   });

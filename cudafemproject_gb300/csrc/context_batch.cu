@@ -39,10 +39,9 @@ BatchVecParams<T> vec_params_batch(cfem_ctx *c, BatchBufs &B, int k_active) {
   return P;
 }
 
-template <typename T>
-void batch_mv(cfem_ctx *c, BatchBufs &B, MvParams<T> &mv) {
+void batch_mv(cfem_ctx *c, BatchBufs &B, MvParams<float> &mv) {
   mv.patch_inst = c->patch_inst.p;
-  if constexpr (sizeof(T) == 8) mv.pmat = c->pmat64.p; else mv.pmat = c->pmat32.p;
+  mv.pmat = c->pmat32.p;
   mv.isc = B.isc.p;
   mv.bctl = B.ctl.p;
   mv.patch_energy = B.pe.p;
@@ -77,7 +76,7 @@ void run_batch_pcg(cfem_ctx *c, BatchBufs &B, double tol, int rule, int maxit, s
   c->launches += 1;
   MvParams<float> mv = base_mv<float>(c);
   mv.diagA = V.diagA.p;
-  batch_mv<float>(c, B, mv);
+  batch_mv(c, B, mv);
   cudaGraph_t graph;
   cudaGraphExec_t exec = nullptr;
   const int64_t before = c->launches;
@@ -91,7 +90,7 @@ void run_batch_pcg(cfem_ctx *c, BatchBufs &B, double tol, int rule, int maxit, s
       m.x2 = pold;
       m.xout = pnew;
       m.y = V.u.p;
-      launch_mv<float>(c, MV_PCG, m);
+      launch_mv_f(c, MV_PCG, m);
       k_batch_vec_flat<float><<<gv, kThreads, sv, c->stream>>>(vp, V.x.p, V.r.p, V.z.p, pnew, V.u.p, V.f.p, V.dinv.p, 0);
       CKL();
     }
@@ -258,7 +257,6 @@ extern "C" cfem_status cfem_batch_static_solve(cfem_ctx *ctx, const cfem_solve_p
     check_ctx(ctx);
     if (!ctx->n_inst) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "not a context of batched meshes"};
     if (!u) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "null output"};
-    if (!ctx->fan_tma) throw Fail{CFEM_ERR_UNSUPPORTED, "batched solve needs the FP32 edge-fan matvec"};
     enter(ctx);
     cfem_solve_params p = prm ? *prm : default_params();
     if (p.precision != CFEM_FP32 && p.precision != CFEM_FP32_REFINE)

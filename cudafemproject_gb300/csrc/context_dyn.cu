@@ -396,7 +396,7 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
       auto one_step = [&](T *from, T *to, int parity) {
         mv.x = from;
         mv.xout = to;
-        launch_mv<T>(c, MV_DYN, mv);
+        launch_mv_f(c, MV_DYN, mv);
         if (resort) slot_assemble_and_resort<T>(c, S.minv.p, 1);
         DynParams<T> de = dp;
         de.dto = to;
@@ -441,7 +441,7 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
       } else {
         mv.x = dcur;
         mv.xout = dnext;
-        launch_mv<T>(c, MV_DYN, mv);
+        launch_mv_f(c, MV_DYN, mv);
       }
       dp.rhs = V.f.p;
       launch_dyn_rhs<T>(c, dp);

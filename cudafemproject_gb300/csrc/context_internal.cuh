@@ -15,7 +15,6 @@
 
 #include "../../include/cfem.h"
 #include "kernels.cuh"
-#include "kernels_fan.cuh"
 #include "kernels_fan_tma.cuh"
 #include "kernels_multi.cuh"
 #include "kernels_batch.cuh"
@@ -158,16 +157,9 @@ struct cfem_ctx {
   DBuf<uint16_t> inc, inc_start;  // per-patch incidence lists
   // edge-fan form (3D): fan tables, gradients in fan vertex order
   bool fans = false;
-  int64_t fstride = 0;
   DBuf<int32_t> fan_off, fan_elem_off, fan_pos;
-  DBuf<uint16_t> fan_slot, finc, finc_start;
   DBuf<uint8_t> fan_perm;
-  DBuf<double> Gf64;
-  DBuf<float> Gf32;
-  size_t smem_fan64 = 0, smem_fan32 = 0;
-  int grid_fan = 0;
   // edge-fan form, FP32, with bulk-copied patch blocks (kernels_fan_tma.cuh)
-  bool fan_tma = true;
   FanBlockLayout L32{};
   DBuf<unsigned char> blk32;
   DBuf<int32_t> fan_patch;
@@ -224,7 +216,7 @@ struct cfem_ctx {
   std::vector<int64_t> inst_node_off, inst_elem_off;  // caller order
   DBuf<int32_t> patch_inst, inst_patch_off, own_first;
   DBuf<float> pmat32;
-  DBuf<double> pmat64, lam_e, mu_e;
+  DBuf<double> lam_e, mu_e;
   int64_t launches = 0;  // kernels issued since the counter was last reset
   GraphCache graph32;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -268,7 +260,6 @@ struct PcgResult {
 
 MvParams<double> base_mv_d(cfem_ctx *c);
 MvParams<float> base_mv_f(cfem_ctx *c);
-void launch_mv_d(cfem_ctx *c, int mode, const MvParams<double> &P);
 void launch_mv_f(cfem_ctx *c, int mode, const MvParams<float> &P);
 PcgResult run_pcg_d(cfem_ctx *c, Vecs<double> &V, double cK, double cM, const double *mcoef, int warm, double tol,
                     int rule, int maxit);
@@ -328,10 +319,6 @@ void attach_stream(cfem_ctx *c, cudaStream_t s);
 template <typename T>
 inline MvParams<T> base_mv(cfem_ctx *c) {
   if constexpr (sizeof(T) == 8) return base_mv_d(c); else return base_mv_f(c);
-}
-template <typename T>
-inline void launch_mv(cfem_ctx *c, int mode, const MvParams<T> &P) {
-  if constexpr (sizeof(T) == 8) launch_mv_d(c, mode, P); else launch_mv_f(c, mode, P);
 }
 template <typename T>
 inline PcgResult run_pcg(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int warm, double tol, int rule, int maxit) {

@@ -443,7 +443,7 @@ extern "C" cfem_status cfem_pcg_multi(cfem_ctx *ctx, const cfem_solve_params *pr
     single_mesh_only(ctx);
     cfem_solve_params p = prm ? *prm : default_params();
     cfem_status worst = CFEM_OK;
-    const bool batched = ctx->fans && ctx->fan_tma && k > 1 &&
+    const bool batched = ctx->fans && k > 1 &&
                          (p.precision == CFEM_FP32 || p.precision == CFEM_FP32_REFINE);
     if (batched) {
       for (int b0 = 0; b0 < k; b0 += kMaxCases) {

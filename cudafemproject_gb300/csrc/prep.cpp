@@ -323,30 +323,6 @@ std::string build_prep(const cfem_mesh &m, int patch_elems, bool use_fans, Prep 
         for (int a = 0; a < nv; ++a) P.inc[e0 * 4 + pos[P.lconn[ei * 4 + a]]++] = (uint16_t)((ei - e0) * 4 + a);
     }
   }
-  // ---- fan incidence lists: codes fl*16 + slot (slot 0 = P, 1 = Q, 2 + k = R_k) ----
-  if (P.fans) {
-    P.finc.assign(P.n_fans * kFanSlots, 0);
-    P.finc_start.assign(P.p_nodes.size() + P.n_patches, 0);
-    std::vector<int32_t> pos;
-    for (int p = 0; p < P.n_patches; ++p) {
-      const int64_t f0 = P.p_fan_off[p], f1 = P.p_fan_off[p + 1];
-      const int n = P.p_node_off[p + 1] - P.p_node_off[p];
-      pos.assign(n + 1, 0);
-      for (int64_t f = f0; f < f1; ++f) {
-        const int len = P.fan_slot[f * kFanSlots + kFanSlots - 1];
-        for (int k = 0; k < len + 3; ++k) ++pos[P.fan_slot[f * kFanSlots + k] + 1];
-      }
-      for (int i = 0; i < n; ++i) pos[i + 1] += pos[i];
-      uint16_t *st = P.finc_start.data() + P.p_node_off[p] + p;
-      for (int i = 0; i <= n; ++i) st[i] = (uint16_t)pos[i];
-      for (int64_t f = f0; f < f1; ++f) {
-        const int len = P.fan_slot[f * kFanSlots + kFanSlots - 1];
-        for (int k = 0; k < len + 3; ++k)
-          P.finc[f0 * kFanSlots + pos[P.fan_slot[f * kFanSlots + k]]++] = (uint16_t)((f - f0) * 16 + k);
-      }
-    }
-  }
-
   // ---- constraints (datakeeper.cpp:139-171) ----
   P.dof_bc.assign(nn * dim, 0);
   P.ctype.assign(nn, 0);

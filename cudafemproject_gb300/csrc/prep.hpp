@@ -47,14 +47,12 @@ struct Prep {
   // node indices of P, Q, R_0..R_kFanMax (unused tail repeats the last ring
   // vertex) and fan_slot[f][kFanSlots-1] the fan length. fan_perm[e] packs,
   // two bits per fan vertex b, which vertex of the element's own connectivity
-  // it is. finc / finc_start: per patch the incidence lists of the fan slots
-  // (codes fl*16 + slot, fl the patch-local fan), laid out like inc / inc_start
-  // with patch p's codes starting at kFanSlots*p_fan_off[p].
+  // it is.
   bool fans = false;
   int64_t n_fans = 0;
   std::vector<int32_t> fan_elem_off, p_fan_off, fan_ring;
   std::vector<uint8_t> fan_perm;
-  std::vector<uint16_t> fan_slot, finc, finc_start;
+  std::vector<uint16_t> fan_slot;
   std::vector<uint8_t> node_bits;  // [nn] new order: bit d set if DOF d is constrained
   std::vector<uint8_t> dof_bc;     // [nn*dim] original order
   std::vector<int32_t> ctype;      // [nn] original order: last Constraint::Type code or 0

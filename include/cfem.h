@@ -71,6 +71,9 @@ typedef enum cfem_stop_rule {
   CFEM_STOP_RESIDUAL = 1   /* ||r||_2 <= tol * ||f||_2 */
 } cfem_stop_rule;
 
+/* How the FP32 matvec applies the operator. In FP64 every form sums the same
+ * elements into 3x3 (2x2) node blocks once, when the operator is built: GB300's
+ * FP64 pipe makes operations, not bytes, the cost there. */
 typedef enum cfem_matvec_form {
   CFEM_FORM_AUTO = 0,      /* edge fans in 3D, per element in 2D */
   CFEM_FORM_GRADIENT = 1,  /* stored scaled shape gradients: K_e p = G^T D G p, one thread per element */
@@ -273,11 +276,13 @@ CFEM_API cfem_status cfem_batch_info(const cfem_ctx *ctx, int32_t *n, int64_t *n
  * instances); info: NULL or [n]. */
 CFEM_API cfem_status cfem_batch_static_solve(cfem_ctx *ctx, const cfem_solve_params *prm, double *u,
                                              cfem_solve_info *info);
-/* Measurement: n back-to-back launches of the PCG-form matvec kernel (direction
- * update + element operator + scatter + p.Ap reduction) on the context's stream,
- * timed with CUDA events. Returns the mean device time per launch and the
- * algorithmic DRAM bytes of one launch: per element the stored operator and
- * local connectivity, per node z and p read, p written, y accumulated. */
+/* Measurement: n back-to-back launches of the FP32 PCG-form matvec kernel
+ * (direction update + element operator + scatter + p.Ap reduction) or of the
+ * FP64 node-row product on the context's stream, timed with CUDA events.
+ * Returns the mean device time per launch and the algorithmic DRAM bytes of one
+ * launch (FP32: per element the stored operator and local connectivity, per
+ * node z and p read, p written, y accumulated; FP64: the node blocks and their
+ * columns, x read, y written). */
 CFEM_API cfem_status cfem_profile_matvec(cfem_ctx *ctx, int32_t precision, int32_t n_launches, double *ms_per_launch,
                                          double *bytes_per_launch);
 /* Autotuner for the elements per CTA patch (no counterpart in the reference):
