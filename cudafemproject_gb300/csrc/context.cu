@@ -1253,7 +1253,7 @@ cfem_status cfem_profile_matvec(cfem_ctx *ctx, int32_t precision, int32_t n_laun
     h.iter = 1;
     h.u_iter = 0;
     h.gamma = h.gamma_prev = h.gamma0 = 1.0;
-    h.alpha = h.beta = 1.0;
+    h.alpha = h.beta = h.inv_gamma_prev = 1.0;
     h.maxit = 1 << 30;
     Scalars *sc = ctx->sc.p + 2;
     CK(cudaMemcpyAsync(sc, &h, sizeof(Scalars), cudaMemcpyHostToDevice, ctx->stream));

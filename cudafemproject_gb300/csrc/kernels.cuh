@@ -50,6 +50,8 @@ struct Scalars {
   double alpha, beta;
   int loop_ok;  // device-side loop: the body count is within the cap (k_pcg_update)
   int stalled;  // one-kernel runs: a CTA did not arrive at a grid-wide sum in time
+  // stopping limits (init kernel: tol gamma0; (tol ||f||)^2) and 1 / gamma_prev (update kernel)
+  double gamma_stop, rr_stop, inv_gamma_prev;
 };
 
 struct DynState {
@@ -119,60 +121,89 @@ __device__ __forceinline__ void atomic_addv(T *p, int64_t node, const NodeV<T, V
   }
 }
 
+// FP64 sums. One FP64 instruction of a warp holds its quarter of an SM for 64
+// cycles on GB300 whatever lanes are active, and a serial chain of additions
+// pays 64 cycles each, so block and grid totals are formed by few warps in few
+// steps: eight warp totals by a three-step tree of eight lanes (a chain in one
+// thread took 540 cycles), block partials by four warps, one per quarter (in
+// every warp of a 256-thread block the same tree took twice as long).
+
+// Warp 0 (all lanes): totals of N groups of warp sums red[k * 8 + warp],
+// k < N <= 4; lanes 8k .. 8k + 7 get sum k.
+template <int N>
+__device__ __forceinline__ double warp_totals(const double *red) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  double v = lane < 8 * N && (lane & 7) < nw ? red[lane] : 0.0;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // Sum N doubles over the block; result valid in thread 0.
 template <int N>
 __device__ __forceinline__ void block_sum(double (&v)[N]) {
-  __shared__ double red[N][kThreads / 32];
+  static_assert(N <= 4, "");
+  __shared__ double red[N * 8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-  for (int k = 0; k < N; ++k) {
-    double x = v[k];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) red[k][wid] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-      double s = 0;
-      for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += red[k][i];
-      v[k] = s;
-    }
+    for (int k = 0; k < N; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < N; ++k) red[k * 8 + wid] = v[k];
+  __syncthreads();
+  if (wid == 0) {
+    const double t = warp_totals<N>(red);
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = __shfl_sync(0xffffffffu, t, 8 * k);
   }
   __syncthreads();
 }
 
-// Sum of the per-block partials in the last block: strided per-thread sums,
-// a shuffle tree per warp and the warp totals in warp order, so the result is
-// a fixed function of the partials. Result valid in thread 0.
+// Fixed-order sums of per-block partials part[b * N + k], b < nblocks, by the
+// first four warps of the block: kPartWarps<N> warps per sum, five loads in
+// flight per lane, a tree per warp; warp sums at red[k * 4 + warp of the sum].
+// After a barrier, partials_total() adds those. (All threads may call.)
 template <int N>
-__device__ __forceinline__ void last_block_total(double (&v)[N], const double *partials) {
-  __shared__ double red2[N][kThreads / 32];
+constexpr int kPartWarps = N == 1 ? 4 : N == 2 ? 2 : 1;
+template <int N>
+__device__ __forceinline__ void partials_warp_sums(const double *part, int nblocks, double *red) {
+  constexpr int PW = kPartWarps<N>;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int k = wid / PW, w = wid % PW;
+  if (k >= N) return;
+  double s = 0;
+  for (int b0 = w * 32 + lane; b0 < nblocks; b0 += 5 * 32 * PW) {
+    double v[5];
 #pragma unroll
-  for (int k = 0; k < N; ++k) {
-    double s = 0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s += __ldcg(partials + (size_t)b * N + k);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) red2[k][wid] = s;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-      double t = 0;
-      for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red2[k][i];
-      v[k] = t;
+    for (int q = 0; q < 5; ++q) {
+      const int b = b0 + q * 32 * PW;
+      v[q] = b < nblocks ? __ldcg(part + (size_t)b * N + k) : 0.0;
     }
+    s += ((v[0] + v[1]) + (v[2] + v[3])) + v[4];
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) red[k * 4 + w] = s;
+}
+template <int N>
+__device__ __forceinline__ double partials_total(const double *red, int k) {
+  const double *r = red + k * 4;
+  if (kPartWarps<N> == 4) return (r[0] + r[1]) + (r[2] + r[3]);
+  if (kPartWarps<N> == 2) return r[0] + r[1];
+  return r[0];
 }
 
 // Publishes this block's partial sums (thread 0 holds them after block_sum);
 // returns true in thread 0 of the last block to finish, which then holds the
-// grid totals. The ticket counter is reset for the next launch.
+// grid totals (a fixed function of the partials). The ticket counter is reset
+// for the next launch. Blocks of 128 threads or more.
 template <int N>
 __device__ __forceinline__ bool publish_and_total(double (&v)[N], double *partials, unsigned int *count) {
+  static_assert(N <= 3, "");
   __shared__ bool last;
+  __shared__ double red2[N * 4];
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int k = 0; k < N; ++k) partials[(size_t)blockIdx.x * N + k] = v[k];
@@ -183,12 +214,17 @@ __device__ __forceinline__ bool publish_and_total(double (&v)[N], double *partia
   __syncthreads();
   if (!last) return false;
   __threadfence();
-  last_block_total<N>(v, partials);
-  if (threadIdx.x == 0) *count = 0;
-  return threadIdx.x == 0;
+  partials_warp_sums<N>(partials, gridDim.x, red2);
+  __syncthreads();
+  if (threadIdx.x != 0) return false;
+#pragma unroll
+  for (int k = 0; k < N; ++k) v[k] = partials_total<N>(red2, k);
+  *count = 0;
+  return true;
 }
 
 // Grid sum of N doubles per thread (block order, scheduling-independent).
+// Blocks of 128 threads or more.
 template <int N>
 __device__ __forceinline__ bool grid_sum_last(double (&v)[N], double *partials, unsigned int *count) {
   block_sum<N>(v);
@@ -245,9 +281,7 @@ __device__ __forceinline__ double block_total(const DotAcc<T> &a) {
   }
   if (lane == 0) red_bt[wid] = w;
   __syncthreads();
-  double t = 0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red_bt[i];
+  const double t = wid == 0 ? warp_totals<1>(red_bt) : 0.0;
   __syncthreads();
   return t;
 }
@@ -261,7 +295,7 @@ __device__ __forceinline__ bool grid_sum_acc(DotAcc<T> (&a)[N], double (&v)[N], 
     for (int k = 0; k < N; ++k) v[k] = a[k].s;
     return grid_sum_last<N>(v, partials, count);
   } else {
-    __shared__ double red[N][kThreads / 32];
+    __shared__ double red[N * 8];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < N; ++k) {
@@ -270,16 +304,13 @@ __device__ __forceinline__ bool grid_sum_acc(DotAcc<T> (&a)[N], double (&v)[N], 
         const float h2 = __shfl_down_sync(0xffffffffu, c.hi, o), l2 = __shfl_down_sync(0xffffffffu, c.lo, o);
         c.merge(h2, l2);
       }
-      if (lane == 0) red[k][wid] = (double)c.hi + (double)c.lo;
+      if (lane == 0) red[k * 8 + wid] = (double)c.hi + (double)c.lo;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (wid == 0) {
+      const double t = warp_totals<N>(red);
 #pragma unroll
-      for (int k = 0; k < N; ++k) {
-        double s = 0;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += red[k][i];
-        v[k] = s;
-      }
+      for (int k = 0; k < N; ++k) v[k] = __shfl_sync(0xffffffffu, t, 8 * k);
     }
     __syncthreads();
     return publish_and_total<N>(v, partials, count);
@@ -295,10 +326,10 @@ __device__ __forceinline__ bool grid_sum_acc(DotAcc<T> (&a)[N], double (&v)[N], 
 // same order in every CTA, so all CTAs derive bit-identical scalars. CTA 0
 // then publishes them for the kernel after it and for the host. A kernel
 // reads only Scalars fields that the kernel before it wrote:
-//   matvec reads  u_iter, gamma_prev, alpha (update) and the constants,
+//   matvec reads  u_iter, inv_gamma_prev, alpha (update) and the constants,
 //          writes gamma, rr, iter, beta, done;
 //   update reads  gamma, iter, done (matvec),
-//          writes alpha, sigma, gamma_prev, u_iter.
+//          writes alpha, sigma, gamma_prev, inv_gamma_prev, u_iter.
 // u_iter < 0 (init kernel): no update yet; the matvec takes the init kernel's
 // scalars and beta = 0.
 
@@ -324,105 +355,73 @@ __device__ __forceinline__ void store_block_partials(const DotAcc<T> (&a)[N], do
     if (lane == 0) red[k * 8 + wid] = w;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-      double t = 0;
-      for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red[k * 8 + i];
-      part[(size_t)blockIdx.x * N + k] = t;
-    }
+  if (wid == 0) {
+    const double t = warp_totals<N>(red);
+    if ((lane & 7) == 0 && lane < 8 * N) part[(size_t)blockIdx.x * N + (lane >> 3)] = t;
   }
 }
 
-// First half of a fixed-order sum of per-block partials: thread t adds
-// part[b * N + k] for b = t, t + blockDim, ... in turn (two loads in flight),
-// a shuffle tree per warp, lane 0 stores the warp sum at red[k * 8 + warp].
-// After a barrier, partials_total() adds the warp sums in warp order. Blocks
-// of at most 256 threads.
-template <int N>
-__device__ __forceinline__ void partials_warp_sums(const double *part, int nblocks, double *red) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int B = blockDim.x;
-  double sum[N];
-#pragma unroll
-  for (int k = 0; k < N; ++k) sum[k] = 0;
-  for (int b0 = threadIdx.x; b0 < nblocks; b0 += 2 * B) {
-    double v[2][N];
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-#pragma unroll
-      for (int k = 0; k < N; ++k) v[q][k] = b0 + q * B < nblocks ? __ldcg(part + (size_t)(b0 + q * B) * N + k) : 0.0;
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-#pragma unroll
-      for (int k = 0; k < N; ++k)
-        if (b0 + q * B < nblocks) sum[k] += v[q][k];
-  }
-#pragma unroll
-  for (int k = 0; k < N; ++k) {
-    double x = sum[k];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) red[k * 8 + wid] = x;
-  }
-}
-__device__ __forceinline__ double partials_total(const double *red, int k) {
-  double t = 0;
-  for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red[k * 8 + i];
-  return t;
+__device__ __forceinline__ bool finite_bits(double v) {  // (no FP64 instruction)
+  return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000;
 }
 
 // Start of a single-mesh PCG-form matvec (all threads, after the dependency
 // wait): r.z and r.r of the update before it, beta and the stopping test
 // (reference rule gamma < tol gamma0, residual rule ||r|| <= tol ||f||, the
-// iteration cap). Returns true once the solve has stopped (uniform). Thread 0
-// alone reads the scalars, in the same round trip as every thread's partial
-// loads, and shares the result through red (24 doubles of shared scratch):
-// the CTAs of a grid reading the same line thread by thread would queue at
-// one L2 slice.
+// iteration cap). Returns true once the solve has stopped (uniform). Warp 0
+// alone reads the scalars, in the same round trip as the partial loads, and
+// shares the result through red (24 doubles of shared scratch): the CTAs of a
+// grid reading the same line thread by thread would queue at one L2 slice.
+// What it divides by and compares with was formed before: 1 / gamma_prev by
+// the update kernel, the limits by the init kernel (a division and two square
+// roots here held up every CTA by 1900 cycles).
 template <typename T>
 __device__ __forceinline__ bool pcg_matvec_scalars(Scalars *s, const double *up_part, int n_up, T &beta,
                                                    double *red) {
   int ui = 0, done0 = 0, rule = 0, maxit = 0;
-  double alpha = 0, tol = 0, g0 = 0, ff = 0, gp = 1;
+  double alpha = 0, limit = 0, inv = 1;
   if (threadIdx.x == 0) {
     ui = s->u_iter;
     done0 = s->done;
     alpha = s->alpha;
-    tol = s->tol;
-    g0 = s->gamma0;
-    ff = s->ff;
-    gp = s->gamma_prev;
     rule = s->rule;
+    limit = rule == 0 ? s->gamma_stop : s->rr_stop;
+    inv = s->inv_gamma_prev;
     maxit = s->maxit;
   }
   partials_warp_sums<2>(up_part, n_up, red);  // (ignored before the first update)
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double b = 0;
-    int done = done0;
-    if (ui >= 0) {
-      const double g = partials_total(red, 0), rr = partials_total(red, 1);
-      const int it = ui + 1;
-      done = 0;
-      if (!isfinite(g) || !isfinite(alpha)) done = 2;
-      else if (rule == 0 && g < tol * g0) done = 1;
-      else if (rule == 1 && sqrt(rr) <= tol * sqrt(ff)) done = 1;
-      else if (it >= maxit) done = 3;
-      b = g / gp;
-      if (blockIdx.x == 0) {
-        s->gamma = g;
-        s->rr = rr;
-        s->iter = it;
-        s->beta = b;
-        s->done = done;
+  if (threadIdx.x < 32) {
+    // lane 0: r.z, lane 1: r.r
+    const double sum = threadIdx.x < 2 ? partials_total<2>(red, threadIdx.x) : 0.0;
+    const double rr = __shfl_sync(0xffffffffu, sum, 1);
+    if (threadIdx.x == 0) {
+      double b = 0;
+      int done = done0;
+      if (ui >= 0) {
+        const double g = sum;
+        const int it = ui + 1;
+        const double v = rule == 0 ? g : rr;
+        done = 0;
+        if (!finite_bits(g) || !finite_bits(alpha)) done = 2;
+        else if (rule == 0 ? v < limit : rule == 1 && v <= limit) done = 1;
+        else if (it >= maxit) done = 3;
+        b = g * inv;
+        if (blockIdx.x == 0) {
+          s->gamma = g;
+          s->rr = rr;
+          s->iter = it;
+          s->beta = b;
+          s->done = done;
+        }
       }
+      red[18] = b;
+      reinterpret_cast<int *>(red + 19)[0] = done;
     }
-    red[18] = b;
-    red[19] = (double)done;
   }
   __syncthreads();
   beta = T(red[18]);
-  const bool stop = red[19] != 0.0;
+  const bool stop = reinterpret_cast<const int *>(red + 19)[0] != 0;
   __syncthreads();  // (red may be reused)
   return stop;
 }
@@ -807,9 +806,12 @@ __global__ void __launch_bounds__(kThreads) k_pcg_init(VecParams<T> P, int warm)
     s->sigma = 0;
     s->alpha = 0;
     s->beta = 0;
+    const double lim = s->tol * sqrt(acc[2]);
+    s->gamma_stop = s->tol * acc[0];
+    s->rr_stop = lim < 0 ? -1.0 : lim * lim;  // (a negative tol stops nothing)
     int done = 0;
     if (acc[0] == 0.0) done = 1;
-    if (s->rule == 1 && sqrt(acc[1]) <= s->tol * sqrt(acc[2])) done = 1;
+    if (s->rule == 1 && acc[1] <= s->rr_stop) done = 1;
     if (!isfinite(acc[0])) done = 2;
     s->done = done;
   }
@@ -890,9 +892,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_pcg_update(VecParams<T> P) {
   partials_warp_sums<1>(P.mv_part, P.n_mv, red_pcg);
   __syncthreads();
   if (threadIdx.x == 0) {
-    const double sig = partials_total(red_pcg, 0), a = gamma / sig;
+    const double sig = partials_total<1>(red_pcg, 0), a = gamma / sig;
     red_pcg[18] = a;
-    red_pcg[19] = (double)done0;
+    reinterpret_cast<int *>(red_pcg + 19)[0] = done0;
     if (blockIdx.x == 0 && !done0) {
       s->sigma = sig;
       s->alpha = a;
@@ -901,9 +903,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_pcg_update(VecParams<T> P) {
     }
   }
   __syncthreads();
-  if (red_pcg[19] != 0.0) return;
-  const double alpha_d = red_pcg[18];
-  const T alpha = (T)alpha_d;
+  if (reinterpret_cast<const int *>(red_pcg + 19)[0] != 0) return;
+  const T alpha = (T)red_pcg[18];
+  if (blockIdx.x == 0 && threadIdx.x == kThreads - 1) s->inv_gamma_prev = 1.0 / s->gamma;  // (for the next matvec)
   DotAcc<T> acc[2];
   for (bool first = true; base < P.n_nodes; base += U * nthr, first = false) {
     if (!first) {

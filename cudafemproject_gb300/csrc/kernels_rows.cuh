@@ -119,10 +119,9 @@ __device__ __forceinline__ int rows_own(const RowOp &A, int64_t s, const double 
 }
 
 // ------------------------------------------------------------------ applications
-// Two slices per CTA: the FP64 pipe of an SM is what a slice takes its time on,
-// so a small mesh's slices are spread over as many SMs as there are (2601
-// nodes: 82 CTAs, against 21 with eight slices each).
-constexpr int kRowsThreads = 64;
+// Four slices per CTA, one for the FP64 pipe of each SM quarter; more would
+// leave SMs of a small mesh without any (2601 nodes: 41 CTAs).
+constexpr int kRowsThreads = 128;
 
 // y = A x, node vectors in the internal layout (XOUT false) or y in the
 // caller's order [n_nodes][DIM] (XOUT true).
@@ -343,7 +342,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_rows_pcg(RowsPcg P) {
   // sqrt(rr) <= tol sqrt(ff) is tested as rr <= (tol sqrt(ff))^2
   if (!grid_sums<3>(G, 0, sums, sh, [&](const double (&t)[3]) {
         const double lim = tol * sqrt(t[2]);
-        sh.total[kMaxGridSums] = lim * lim;
+        sh.total[kMaxGridSums] = lim < 0 ? -1.0 : lim * lim;  // (a negative tol stops nothing)
       }))
     return stalled();
   const double gamma0 = sums[0], ff = sums[2], rr_stop = sh.total[kMaxGridSums], gamma_stop = tol * gamma0;
