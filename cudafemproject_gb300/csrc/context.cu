@@ -50,7 +50,7 @@ void launch_mv_f(cfem_ctx *c, int mode, const MvParams<float> &P) {
     F.L = c->L32;
     F.fan_off = c->fan_off.p;
     F.fan_elem_off = c->fan_elem_off.p;
-    F.err = c->tma_err.p;
+    F.err = c->h_tma_err;
     F.skip_patch_plus1 = c->selftest_skip_plus1;
     F.wait_limit = c->selftest_wait_limit;
     const double l2_half = 0.5 * c->l2_bytes;
@@ -143,10 +143,12 @@ void launch_update(cfem_ctx *c, const VecParams<T> &P) {
 }
 
 // Jacobi PCG on A x = V.f with A = cM*M + cK*K' (mcoef selects the mass term).
-// V.x holds the warm start when warm != 0. Returns after the device flag says done.
+// V.x holds the warm start when warm != 0. Returns after the device flag says
+// done and what `then` has queued behind the run is complete.
 template <typename T>
 PcgResult run_pcg_t(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int warm, double tol, int rule, int maxit,
-                    const T *cont_p = nullptr, double cont_gamma_prev = 0) {
+                    const T *cont_p = nullptr, double cont_gamma_prev = 0,
+                    const std::function<void()> &then = nullptr) {
   Scalars *sc = c->sc.p + 1;
   Scalars h{};
   h.tol = tol;
@@ -270,6 +272,7 @@ PcgResult run_pcg_t(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int war
   PcgResult res;
   if (gc.device_loop) {
     CK(cudaGraphLaunch(gc.exec, c->stream));
+    if (then) then();
     CK(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     c->launches += (int64_t)2 * c->chunk * c->h_sc->loops;
@@ -277,7 +280,7 @@ PcgResult run_pcg_t(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int war
       std::printf("iteration %d gamma %.6e gamma0 %.6e (%d loops)\n", c->h_sc->iter, c->h_sc->gamma, c->h_sc->gamma0,
                   c->h_sc->loops);
     if (!c->h_sc->done) {
-      check_copy_error(c);
+      check_copy_flag(c);
       throw Fail{CFEM_ERR_CUDA, "PCG recurrence stopped advancing on the device"};
     }
   } else {
@@ -300,8 +303,12 @@ PcgResult run_pcg_t(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int war
       stalled = c->h_sc->iter == last_iter ? stalled + 1 : 0;
       last_iter = c->h_sc->iter;
     }
+    if (then) {
+      then();
+      CK(cudaStreamSynchronize(c->stream));
+    }
   }
-  check_copy_error(c);
+  check_copy_flag(c);
   res.iters = c->h_sc->iter;
   res.gamma0 = c->h_sc->gamma0;
   res.gamma = c->h_sc->gamma;
@@ -313,21 +320,28 @@ PcgResult run_pcg_t(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int war
   return res;
 }
 
-// caller-order FP64 array (host or device) -> internal node vector of type T
-template <typename T>
-void to_internal_t(cfem_ctx *c, const double *src, T *dst, double scale) {
-  CK(cudaMemcpyAsync(c->io.p, src, sizeof(double) * c->nd, cudaMemcpyDefault, c->stream));
-  if (c->dim == 3) k_to_internal<T, 3><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, c->io.p, c->node_new2old.p, dst, scale);
-  else k_to_internal<T, 2><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, c->io.p, c->node_new2old.p, dst, scale);
+// caller-order array (host or device) -> internal node vector of type T; a
+// device array is read in place, anything else through c->io
+template <typename T, typename S>
+void to_internal_t(cfem_ctx *c, const S *src, T *dst, T *zero = nullptr) {
+  if (!direct_access(c, src, sizeof(S))) {
+    S *io = reinterpret_cast<S *>(c->io.p);
+    CK(cudaMemcpyAsync(io, src, sizeof(S) * c->nd, cudaMemcpyDefault, c->stream));
+    src = io;
+  }
+  if (c->dim == 3) k_to_internal<T, 3, S><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, src, c->node_new2old.p, dst, zero);
+  else k_to_internal<T, 2, S><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, src, c->node_new2old.p, dst, zero);
   CKL();
 }
 
-template <typename T>
-void to_caller_t(cfem_ctx *c, const T *src, double *dst) {
-  if (c->dim == 3) k_to_caller<T, 3><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, src, c->node_new2old.p, c->io.p);
-  else k_to_caller<T, 2><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, src, c->node_new2old.p, c->io.p);
+template <typename T, typename S>
+void to_caller_t(cfem_ctx *c, const T *src, S *dst) {
+  const bool direct = direct_access(c, dst, sizeof(S));
+  S *to = direct ? dst : reinterpret_cast<S *>(c->io.p);
+  if (c->dim == 3) k_to_caller<T, 3, S><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, src, c->node_new2old.p, to);
+  else k_to_caller<T, 2, S><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, src, c->node_new2old.p, to);
   CKL();
-  CK(cudaMemcpyAsync(dst, c->io.p, sizeof(double) * c->nd, cudaMemcpyDefault, c->stream));
+  if (!direct) CK(cudaMemcpyAsync(dst, to, sizeof(S) * c->nd, cudaMemcpyDefault, c->stream));
 }
 
 MvParams<double> base_mv_d(cfem_ctx *c) { return base_mv_t<double>(c); }
@@ -336,28 +350,30 @@ PcgResult run_pcg_f(cfem_ctx *c, Vecs<float> &V, float cK, float cM, const float
                     int rule, int maxit) {
   return run_pcg_t<float>(c, V, cK, cM, mcoef, warm, tol, rule, maxit);
 }
-void to_internal_d(cfem_ctx *c, const double *src, double *dst, double scale) { to_internal_t<double>(c, src, dst, scale); }
-void to_internal_f(cfem_ctx *c, const double *src, float *dst, double scale) { to_internal_t<float>(c, src, dst, scale); }
-void to_caller_d(cfem_ctx *c, const double *src, double *dst) { to_caller_t<double>(c, src, dst); }
-void to_caller_f(cfem_ctx *c, const float *src, double *dst) { to_caller_t<float>(c, src, dst); }
+void to_internal_d(cfem_ctx *c, const double *src, double *dst) { to_internal_t<double, double>(c, src, dst); }
+void to_caller_d(cfem_ctx *c, const double *src, double *dst) { to_caller_t<double, double>(c, src, dst); }
+void to_caller_f(cfem_ctx *c, const float *src, double *dst) { to_caller_t<float, double>(c, src, dst); }
 
-// The true residual (true_residual_async), waited for: returns ||r||^2, ||f||^2.
+// The true residual (true_residual_async), waited for: ||r||^2, ||f||^2
+// (written to pinned memory by the kernel).
 void true_residual(cfem_ctx *c, const double *f, const double *x, double *r, float *r32, double &rr, double &ff) {
-  true_residual_async(c, f, x, r, r32, c->rr.p);
-  CK(cudaMemcpyAsync(c->h_rr, c->rr.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  true_residual_async(c, f, x, r, r32, c->h_rr);
   CK(cudaStreamSynchronize(c->stream));
-  rr = c->h_rr[0];
-  ff = c->h_rr[1];
-  check_copy_error(c);
+  rr = ((volatile double *)c->h_rr)[0];
+  ff = ((volatile double *)c->h_rr)[1];
+  check_copy_flag(c);
 }
 
-void set_diag_vectors(cfem_ctx *c, const double *diagA64) {
-  // dinv and diagA for both precisions from one FP64 diagonal (internal layout)
-  k_invert<double><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, diagA64, c->v64.dinv.p);
-  k_invert<float><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, diagA64, c->v32.dinv.p);
-  CK(cudaMemcpyAsync(c->v64.diagA.p, diagA64, sizeof(double) * c->nvec, cudaMemcpyDeviceToDevice, c->stream));
-  k_convert<double, float><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, diagA64, c->v32.diagA.p);
+// dinv and diagA for both precisions from diag(K) (kept until another diagonal
+// takes their place or the operator is rebuilt)
+void set_diag_vectors(cfem_ctx *c) {
+  if (c->diag_is_K) return;
+  k_invert<double><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->diagK.p, c->v64.dinv.p);
+  k_invert<float><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->diagK.p, c->v32.dinv.p);
+  CK(cudaMemcpyAsync(c->v64.diagA.p, c->diagK.p, sizeof(double) * c->nvec, cudaMemcpyDeviceToDevice, c->stream));
+  k_convert<double, float><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->diagK.p, c->v32.diagA.p);
   CKL();
+  c->diag_is_K = true;
 }
 
 // Static-type solve of K' x = f (f internal FP64 in c->v64.f). Result in c->v64.x.
@@ -365,10 +381,11 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
   cfem_solve_info inf{};
   single_mesh_only(c);
   c->launches = 0;
-  set_diag_vectors(c, c->diagK.p);
+  set_diag_vectors(c);
   CK(cudaEventRecord(c->ev0, c->stream));
   const int prec = prm->precision;
   int status = CFEM_OK;
+  double rr_end = -1, ff_end = 0;
   if (prec == CFEM_FP64) {
     PcgResult r = run_pcg<double>(c, c->v64, 1.0, 0.0, nullptr, 0, prm->tol, prm->stop_rule, prm->max_iter);
     status = r.status;
@@ -418,21 +435,30 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
       // Replaced seldom, the recursive residual drifts too far from the true
       // one for the old direction to stay conjugate, so tighter inner
       // tolerances restart.
+      // behind the run, without waiting for it: x64 += d and the true residual
+      // (its norms arrive with the run's scalars)
+      auto then = [&]() {
+        k_accumulate<<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->v32.x.p, c->v64.x.p, c->vw, c->sc.p + 1);
+        CKL();
+        true_residual_async(c, c->v64.f.p, c->v64.x.p, c->v64.r.p, c->v32.f.p, c->h_rr);
+      };
       PcgResult r = cont_iters > 0 && prm->tol >= kContinueTol
                         ? run_pcg_t<float>(c, c->v32, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, prm->max_iter,
-                                           ((cont_iters - 1) & 1) ? c->v32.pA.p : c->v32.pB.p, cont_gprev)
-                        : run_pcg<float>(c, c->v32, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, prm->max_iter);
+                                           ((cont_iters - 1) & 1) ? c->v32.pA.p : c->v32.pB.p, cont_gprev, then)
+                        : run_pcg_t<float>(c, c->v32, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, prm->max_iter,
+                                           nullptr, 0, then);
       cont_iters = r.status == CFEM_OK || r.status == CFEM_ERR_NOT_CONVERGED ? r.iters : 0;
       cont_gprev = r.gamma_prev;
       total += r.iters;
       if (outer == 0) inf.gamma0 = r.gamma0;
       inf.gamma = r.gamma;
       if (r.status == CFEM_ERR_DIVERGED) { status = CFEM_ERR_DIVERGED; break; }
-      k_accumulate<<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->v32.x.p, c->v64.x.p, c->vw);
-      CKL();
       ++outer;
-      true_residual(c, c->v64.f.p, c->v64.x.p, c->v64.r.p, c->v32.f.p, rr, ff);
+      rr = ((volatile double *)c->h_rr)[0];
+      ff = ((volatile double *)c->h_rr)[1];
     }
+    rr_end = rr;
+    ff_end = ff;
     if (status != CFEM_OK && std::sqrt(rr) <= outer_tol * std::sqrt(ff)) status = CFEM_OK;
     inf.iterations = total;
     inf.outer_iterations = outer;
@@ -445,8 +471,8 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
   CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   inf.solve_ms = ms;
   inf.kernel_launches = c->launches;
-  double rr = 0, ff = 0;
-  true_residual(c, c->v64.f.p, c->v64.x.p, c->tmp64b.p, nullptr, rr, ff);
+  double rr = rr_end, ff = ff_end;  // (the refinement knows the residual of its last iterate)
+  if (rr < 0) true_residual(c, c->v64.f.p, c->v64.x.p, c->tmp64b.p, nullptr, rr, ff);
   inf.rel_residual = ff > 0 ? std::sqrt(rr / ff) : std::sqrt(rr);
   inf.status = status;
   if (info) *info = inf;
@@ -523,9 +549,11 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
   err = build_rhs(*m, c->prep, c->semantics, c->rhs);
   if (!err.empty()) throw Fail{CFEM_ERR_MESH, err};
   if (m->elem_young) {
-    c->young.assign(m->elem_young, m->elem_young + c->ne);
-    for (double y : c->young)
-      if (!(y > 0)) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "per-element Young's modulus must be positive"};
+    for (int64_t e = 0; e < c->ne; ++e)
+      if (!(m->elem_young[e] > 0))
+        throw Fail{CFEM_ERR_INVALID_ARGUMENT, "per-element Young's modulus must be positive"};
+    c->young_d.upload(m->elem_young, c->ne, c->stream);
+    c->has_young = true;
   }
   const Prep &P = c->prep;
   cudaStream_t s = c->stream;
@@ -652,9 +680,8 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
     c->blk32.zero(s);
     CK(cudaMemcpy2DAsync(c->blk32.p, c->L32.bytes, hb.data(), pre, pre, P.n_patches, cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));  // hb is pageable and goes out of scope
-    c->tma_err.alloc(1);
-    c->tma_err.zero(s);
     CK(cudaMallocHost(&c->h_tma_err, sizeof(int)));
+    *c->h_tma_err = 0;
   }
   if (c->n_inst) {
     // instance tables: patch -> instance, instance patch ranges, owned node ranges, materials
@@ -799,7 +826,6 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
   c->partials_up.zero(s);
   c->counters.alloc(4);
   c->counters.zero(s);
-  c->rr.alloc(4);
   c->sc.alloc(3);
   c->sc.zero(s);
   CK(cudaMallocHost(&c->h_sc, sizeof(Scalars)));
@@ -814,7 +840,7 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
 static void build_geo_blocks(cfem_ctx *c) {
   cudaStream_t s = c->stream;
   const Prep &P = c->prep;
-  const bool with_scale = !c->young.empty();
+  const bool with_scale = c->has_young;
   const FanBlockLayout L = fan_geo_block_layout(P.np_max, with_scale);
   if (!c->blkg.p || L.bytes != c->Lg.bytes || L.c_off != c->Lg.c_off) c->blkg.alloc((size_t)L.bytes * P.n_patches);
   c->Lg = L;
@@ -837,28 +863,34 @@ void rebuild_operator(cfem_ctx *c) {
   cudaStream_t s = c->stream;
   const Prep &P = c->prep;
   (void)P;
-  if (!c->young.empty()) {
-    std::vector<double> sc(c->ne);
-    for (int64_t e = 0; e < c->ne; ++e) sc[e] = c->young[c->prep.elem_new2old[e]] / c->E;
-    c->escale.upload(sc.data(), sc.size(), s);
-    c->young_d.upload(c->young.data(), c->young.size(), s);
+  c->diag_is_K = false;
+  if (c->has_young) {
+    c->escale.ensure(c->ne);
+    k_young_scale<<<nblk(c->ne), kThreads, 0, s>>>(c->ne, c->young_d.p, c->elem_new2old.p, c->E, c->escale.p);
+    CKL();
   }
-  c->gstride = (c->ne + 31) / 32 * 32;
-  c->G64.alloc((size_t)c->ncomp * c->gstride);
-  c->G32.alloc((size_t)c->ncomp * c->gstride);
-  c->vol.alloc(c->ne);
-  c->mc64.alloc(c->ne);
-  c->mc32.alloc(c->ne);
-  c->diagK.alloc(c->nvec);
-  c->mlump.alloc(c->nvec);
-  c->mcdiag.alloc(c->nvec);
+  const bool first = !c->G64.p;  // (buffers keep their place when the moduli change)
+  if (first) {
+    c->gstride = (c->ne + 31) / 32 * 32;
+    c->G64.alloc((size_t)c->ncomp * c->gstride);
+    c->G32.alloc((size_t)c->ncomp * c->gstride);
+    c->vol.alloc(c->ne);
+    c->mc64.alloc(c->ne);
+    c->mc32.alloc(c->ne);
+    c->diagK.alloc(c->nvec);
+    c->mlump.alloc(c->nvec);
+    c->mcdiag.alloc(c->nvec);
+    c->diagK32.alloc(c->nvec);
+    c->err.alloc(1);
+  }
   c->diagK.zero(s);
   c->mlump.zero(s);
   c->mcdiag.zero(s);
-  if (!c->err.p) c->err.alloc(1);
   c->err.zero(s);
-  c->G64.zero(s);
-  c->G32.zero(s);
+  if (first) {  // (the padding)
+    c->G64.zero(s);
+    c->G32.zero(s);
+  }
   // mass factors: lumped per DOF and consistent coefficient (M_ab = c (1 + delta_ab) rho V)
   double &lump_c = c->lump_c, &cons_c = c->cons_c;
   if (c->dim == 2) { lump_c = 1.0 / 3; cons_c = 1.0 / 12; }
@@ -900,7 +932,6 @@ void rebuild_operator(cfem_ctx *c) {
   k_axpby64<<<nblk(c->nvec), kThreads, 0, s>>>(c->nvec, 2 * cons_c / lump_c, c->mlump.p, 0.0, c->mcdiag.p);
   CKL();
   int herr = 0;
-  c->diagK32.alloc(c->nvec);
   k_convert<double, float><<<nblk(c->nvec), kThreads, 0, s>>>(c->nvec, c->diagK.p, c->diagK32.p);
   CKL();
   CK(cudaMemcpyAsync(&herr, c->err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -936,14 +967,25 @@ void attach_stream(cfem_ctx *c, cudaStream_t s) {
   }
 }
 
+void check_copy_flag(cfem_ctx *c) {
+  if (!c->h_tma_err || !*(volatile int *)c->h_tma_err) return;
+  *c->h_tma_err = 0;
+  throw Fail{CFEM_ERR_CUDA, "a bulk copy of the edge-fan matvec did not complete in time"};
+}
+
 void check_copy_error(cfem_ctx *c) {
-  if (!c->h_tma_err) return;
-  CK(cudaMemcpyAsync(c->h_tma_err, c->tma_err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  if (*c->h_tma_err) {
-    c->tma_err.zero(c->stream);
-    throw Fail{CFEM_ERR_CUDA, "a bulk copy of the edge-fan matvec did not complete in time"};
+  check_copy_flag(c);
+}
+
+bool direct_access(const cfem_ctx *c, const void *p, size_t elem) {
+  cudaPointerAttributes at{};
+  if (reinterpret_cast<uintptr_t>(p) % elem) return false;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
   }
+  return at.type == cudaMemoryTypeDevice && at.device == c->device;
 }
 
 void check_ctx(const cfem_ctx *c) {
@@ -1173,31 +1215,24 @@ cfem_status cfem_matvec(cfem_ctx *ctx, int32_t precision, const void *x, void *y
     if (!x || !y) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "null vector"};
     single_mesh_only(ctx);
     if (precision == CFEM_FP64) {
-      to_internal<double>(ctx, (const double *)x, ctx->v64.z.p);
-      rows_apply(ctx, ctx->v64.z.p, ctx->tmp64.p);
-      to_caller<double>(ctx, ctx->tmp64.p, (double *)y);
+      const size_t bytes = sizeof(double) * ctx->nd;
+      const uintptr_t px = reinterpret_cast<uintptr_t>(x), py = reinterpret_cast<uintptr_t>(y);
+      if ((px + bytes <= py || py + bytes <= px) && direct_access(ctx, x, sizeof(double)) &&
+          direct_access(ctx, y, sizeof(double))) {
+        rows_apply(ctx, (const double *)x, (double *)y, true);
+      } else {
+        to_internal<double>(ctx, (const double *)x, ctx->v64.z.p);
+        rows_apply(ctx, ctx->v64.z.p, ctx->tmp64.p);
+        to_caller<double>(ctx, ctx->tmp64.p, (double *)y);
+      }
     } else if (precision == CFEM_FP32) {
-      // float in/out: stage through FP64 conversion buffers
-      DBuf<double> xin;
-      xin.alloc(ctx->nd);
-      DBuf<float> xf;
-      xf.alloc(ctx->nd);
-      CK(cudaMemcpyAsync(xf.p, x, sizeof(float) * ctx->nd, cudaMemcpyDefault, ctx->stream));
-      k_convert<float, double><<<nblk(ctx->nd), kThreads, 0, ctx->stream>>>(ctx->nd, xf.p, xin.p);
-      CKL();
-      to_internal<float>(ctx, xin.p, ctx->v32.z.p);
-      k_convert<double, float><<<nblk(ctx->nvec), kThreads, 0, ctx->stream>>>(ctx->nvec, ctx->diagK.p, ctx->v32.diagA.p);
+      to_internal_t<float, float>(ctx, (const float *)x, ctx->v32.z.p, ctx->v32.u.p);
       MvParams<float> mv = base_mv<float>(ctx);
-      mv.diagA = ctx->v32.diagA.p;
+      mv.diagA = ctx->diagK32.p;
       mv.x = ctx->v32.z.p;
       mv.y = ctx->v32.u.p;
-      ctx->v32.u.zero(ctx->stream);
       launch_mv_f(ctx, MV_PLAIN, mv);
-      to_caller<float>(ctx, ctx->v32.u.p, xin.p);
-      k_convert<double, float><<<nblk(ctx->nd), kThreads, 0, ctx->stream>>>(ctx->nd, xin.p, xf.p);
-      CKL();
-      CK(cudaMemcpyAsync(y, xf.p, sizeof(float) * ctx->nd, cudaMemcpyDefault, ctx->stream));
-      ctx->v32.u.zero(ctx->stream);
+      to_caller_t<float, float>(ctx, ctx->v32.u.p, (float *)y);
     } else {
       throw Fail{CFEM_ERR_INVALID_ARGUMENT, "matvec precision must be CFEM_FP64 or CFEM_FP32"};
     }

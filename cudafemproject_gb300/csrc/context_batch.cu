@@ -276,7 +276,7 @@ extern "C" cfem_status cfem_batch_static_solve(cfem_ctx *ctx, const cfem_solve_p
     B.rrff.alloc((size_t)n * 2);
     B.active.alloc(n);
     c->launches = 0;
-    set_diag_vectors(c, c->diagK.p);
+    set_diag_vectors(c);
     RhsSchedule sch;
     sch.semantics = c->semantics;
     sch.has_loads = c->rhs.has_loads;
@@ -337,7 +337,7 @@ extern "C" cfem_status cfem_batch_static_solve(cfem_ctx *ctx, const cfem_solve_p
           if (res[i].done == 2) status[i] = CFEM_ERR_DIVERGED;
           rr_prev[i] = rr[i];
         }
-        k_accumulate<<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->v32.x.p, c->v64.x.p, c->vw);
+        k_accumulate<<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->v32.x.p, c->v64.x.p, c->vw, nullptr);
         CKL();
         rows_apply(c, c->v64.x.p, c->tmp64.p);
         batch_residual(c, B, none, rr, ff);

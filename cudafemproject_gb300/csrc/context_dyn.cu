@@ -123,7 +123,13 @@ void slot_assemble_and_resort(cfem_ctx *c, T *out, int invert) {
   std::swap(c->slot_src.p, c->slot_tmp.p);
 }
 
+__global__ void k_fill(int64_t n, double v, double *p) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) p[i] = v;
+}
+
 void set_pcg_vectors(cfem_ctx *c, const double *diag_op, const double *diag_pre) {
+  c->diag_is_K = false;
   k_invert<double><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, diag_pre, c->v64.dinv.p);
   k_invert<float><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, diag_pre, c->v32.dinv.p);
   CK(cudaMemcpyAsync(c->v64.diagA.p, diag_op, sizeof(double) * c->nvec, cudaMemcpyDeviceToDevice, c->stream));
@@ -215,15 +221,13 @@ void launch_grad_pairs(cfem_ctx *c, const double *u, const double *w, int64_t st
 
 // Per-element moduli on the device (the material's where none were given).
 const double *young_on_device(cfem_ctx *c) {
-  if (c->young_d.p) return c->young_d.p;
-  DBuf<double> &y = c->steps.young;
-  if (!y.p) {
-    std::vector<double> h(c->ne, c->E);
-    y.alloc(c->ne);
-    CK(cudaMemcpyAsync(y.p, h.data(), sizeof(double) * c->ne, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+  if (c->has_young) return c->young_d.p;
+  if (!c->young_d.p) {
+    c->young_d.alloc(c->ne);
+    k_fill<<<nblk(c->ne), kThreads, 0, c->stream>>>(c->ne, c->E, c->young_d.p);
+    CKL();
   }
-  return y.p;
+  return c->young_d.p;
 }
 
 template <typename T>
@@ -719,25 +723,24 @@ cfem_status cfem_element_stress(cfem_ctx *ctx, const double *u, double *strain, 
     if (!u) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "null displacement"};
     enter(ctx);
     const int S = 3 * (ctx->dim - 1);
-    DBuf<double> uin, de, ds, dm;
-    uin.alloc(ctx->nvec);
-    uin.zero(ctx->stream);
-    to_internal<double>(ctx, u, uin.p);
-    if (strain) de.alloc((size_t)ctx->ne * S);
-    if (stress) ds.alloc((size_t)ctx->ne * S);
-    if (mises) dm.alloc(ctx->ne);
+    // strain, stress, von Mises in one buffer kept with the context
+    DBuf<double> &out = ctx->steps.stress;
+    out.ensure((size_t)ctx->ne * (2 * S + 1));
+    double *de = strain ? out.p : nullptr, *ds = stress ? out.p + (size_t)ctx->ne * S : nullptr,
+           *dm = mises ? out.p + (size_t)ctx->ne * 2 * S : nullptr;
+    to_internal<double>(ctx, u, ctx->tmp64.p);
     if (ctx->dim == 3)
       k_element_stress<3><<<nblk(ctx->ne), kThreads, 0, ctx->stream>>>(ctx->ne, ctx->G64.p, ctx->gstride, ctx->vol.p, ctx->escale.p,
-                                                                        ctx->conn.p, uin.p, ctx->lam, ctx->mu, ctx->elem_new2old.p,
-                                                                        de.p, ds.p, dm.p);
+                                                                        ctx->conn.p, ctx->tmp64.p, ctx->lam, ctx->mu, ctx->elem_new2old.p,
+                                                                        de, ds, dm);
     else
       k_element_stress<2><<<nblk(ctx->ne), kThreads, 0, ctx->stream>>>(ctx->ne, ctx->G64.p, ctx->gstride, ctx->vol.p, ctx->escale.p,
-                                                                        ctx->conn.p, uin.p, ctx->lam, ctx->mu, ctx->elem_new2old.p,
-                                                                        de.p, ds.p, dm.p);
+                                                                        ctx->conn.p, ctx->tmp64.p, ctx->lam, ctx->mu, ctx->elem_new2old.p,
+                                                                        de, ds, dm);
     CKL();
-    if (strain) CK(cudaMemcpyAsync(strain, de.p, sizeof(double) * de.n, cudaMemcpyDefault, ctx->stream));
-    if (stress) CK(cudaMemcpyAsync(stress, ds.p, sizeof(double) * ds.n, cudaMemcpyDefault, ctx->stream));
-    if (mises) CK(cudaMemcpyAsync(mises, dm.p, sizeof(double) * dm.n, cudaMemcpyDefault, ctx->stream));
+    if (strain) CK(cudaMemcpyAsync(strain, de, sizeof(double) * ctx->ne * S, cudaMemcpyDefault, ctx->stream));
+    if (stress) CK(cudaMemcpyAsync(stress, ds, sizeof(double) * ctx->ne * S, cudaMemcpyDefault, ctx->stream));
+    if (mises) CK(cudaMemcpyAsync(mises, dm, sizeof(double) * ctx->ne, cudaMemcpyDefault, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return CFEM_OK;
   });
@@ -749,16 +752,24 @@ cfem_status cfem_set_young(cfem_ctx *ctx, const double *elem_young) {
     if (ctx->n_inst) throw Fail{CFEM_ERR_UNSUPPORTED, "not available for a context of batched meshes"};
     enter(ctx);
     if (!elem_young) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "null array"};
-    std::vector<double> yv(ctx->ne);
-    // on the context's stream, which enter() ordered after the caller's
-    CK(cudaMemcpyAsync(yv.data(), elem_young, sizeof(double) * ctx->ne, cudaMemcpyDefault, ctx->stream));
+    // the new moduli are looked over before anything changes
+    DBuf<double> &in = ctx->steps.young;
+    in.ensure(ctx->ne);
+    CK(cudaMemcpyAsync(in.p, elem_young, sizeof(double) * ctx->ne, cudaMemcpyDefault, ctx->stream));
+    int *bad = reinterpret_cast<int *>(ctx->h_rr);
+    *bad = 0;
+    k_young_check<<<nblk(ctx->ne), kThreads, 0, ctx->stream>>>(ctx->ne, in.p, bad);
+    CKL();
     CK(cudaStreamSynchronize(ctx->stream));
-    for (double y : yv)
-      if (!(y > 0)) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "per-element Young's modulus must be positive"};
-    ctx->young = yv;
+    if (*(volatile int *)bad) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "per-element Young's modulus must be positive"};
+    std::swap(in.p, ctx->young_d.p);
+    std::swap(in.n, ctx->young_d.n);
+    ctx->has_young = true;
+    const int bytes = ctx->Lg.bytes;
     rebuild_operator(ctx);
-    // captured PCG iterations hold operator buffers that the rebuild may have replaced
-    ctx->graph32.reset();
+    // captured PCG iterations hold the place and layout of the geometry blocks,
+    // which grow when the first moduli are given
+    if (ctx->geo && bytes != ctx->Lg.bytes) ctx->graph32.reset();
     return CFEM_OK;
   });
 }

@@ -122,7 +122,7 @@ struct StepVecs {
 struct StepWork {
   StepVecs<double> f64;
   StepVecs<float> f32;
-  DBuf<double> coef, diag_pre, diag_op, trace, obs, grad, young, states;
+  DBuf<double> coef, stress, diag_pre, diag_op, trace, obs, grad, young, states;
   DBuf<int32_t> recv, rec_head, rec_next;
   DBuf<DynState> st;
   DBuf<int> stalled;
@@ -149,7 +149,7 @@ struct cfem_ctx {
   double E = 0, nu = 0, rho = 0, lam = 0, mu = 0;
   Prep prep;
   RhsParts rhs;
-  std::vector<double> young;  // per-element Young's modulus (caller order), empty if uniform
+  bool has_young = false;  // per-element moduli in young_d (caller order)
   double lump_c = 0, cons_c = 0;
   // mesh on device
   DBuf<int32_t> elem_off, node_off, nodes, own, node_new2old, elem_new2old, elem_old2new, conn;
@@ -163,8 +163,7 @@ struct cfem_ctx {
   FanBlockLayout L32{};
   DBuf<unsigned char> blk32;
   DBuf<int32_t> fan_patch;
-  DBuf<int> tma_err;
-  int *h_tma_err = nullptr;
+  int *h_tma_err = nullptr;  // pinned; written by a kernel whose copy wait ran out
   int selftest_skip_plus1 = 0;       // FanTmaParams::skip_patch_plus1 (cfem_selftest_copy_timeout only)
   long long selftest_wait_limit = 0;  // FanTmaParams::wait_limit (likewise)
   size_t smem_ft32 = 0;
@@ -192,7 +191,7 @@ struct cfem_ctx {
   // work
   Vecs<double> v64;
   Vecs<float> v32;
-  DBuf<double> io, tmp64, tmp64b, rr;
+  DBuf<double> io, tmp64, tmp64b;
   DBuf<Scalars> sc;  // [0] FP64 solve, [1] FP32 solve, [2] misc counters
   DBuf<double> partials;     // grid-sum scratch; the PCG-form matvec's p.Ap partials
   DBuf<double> partials_up;  // r.z, r.r partials of the PCG update kernel [grid][2]
@@ -219,6 +218,7 @@ struct cfem_ctx {
   DBuf<double> lam_e, mu_e;
   int64_t launches = 0;  // kernels issued since the counter was last reset
   GraphCache graph32;
+  bool diag_is_K = false;  // dinv and diagA of v64 and v32 belong to diagK
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // reference re-sorting quirk (compat dynamics)
   DBuf<int64_t> seg;
@@ -265,11 +265,10 @@ PcgResult run_pcg_d(cfem_ctx *c, Vecs<double> &V, double cK, double cM, const do
                     int rule, int maxit);
 PcgResult run_pcg_f(cfem_ctx *c, Vecs<float> &V, float cK, float cM, const float *mcoef, int warm, double tol,
                     int rule, int maxit);
-void to_internal_d(cfem_ctx *c, const double *src, double *dst, double scale = 1.0);
-void to_internal_f(cfem_ctx *c, const double *src, float *dst, double scale = 1.0);
+void to_internal_d(cfem_ctx *c, const double *src, double *dst);
 void to_caller_d(cfem_ctx *c, const double *src, double *dst);
 void to_caller_f(cfem_ctx *c, const float *src, double *dst);
-void set_diag_vectors(cfem_ctx *c, const double *diagA64);
+void set_diag_vectors(cfem_ctx *c);
 void true_residual(cfem_ctx *c, const double *f, const double *x, double *r, float *r32, double &rr, double &ff);
 void true_residual_async(cfem_ctx *c, const double *f, const double *x, double *r, float *r32, double *out2);
 void make_rhs(cfem_ctx *c, double a, double b, double *dst);
@@ -302,7 +301,12 @@ inline void launch_pdl(void (*kern)(KArgs...), dim3 g, dim3 b, size_t smem, cuda
   CK(cudaLaunchKernelEx(&cfg, kern, args...));
 }
 
+// The same after the stream has been waited for.
+void check_copy_flag(cfem_ctx *c);
 void check_copy_error(cfem_ctx *c);
+// Whether the kernels may work on a caller's array in place: device memory of
+// the context's GPU, aligned to its elements.
+bool direct_access(const cfem_ctx *c, const void *p, size_t elem);
 // Orders the context's stream after the caller's stream (device inputs written there).
 void enter(cfem_ctx *c);
 cfem_solve_params default_params();
@@ -311,8 +315,8 @@ void rebuild_operator(cfem_ctx *c);
 void build_rows(cfem_ctx *c);
 // Slots and counter of a cooperative kernel's exchanges, emptied on the stream.
 GridSync start_grid_sync(cfem_ctx *c, int sets);
-// y = K' x in FP64 (internal node vectors; y is overwritten)
-void rows_apply(cfem_ctx *c, const double *x, double *y);
+// y = K' x in FP64 (node vectors, or the caller's arrays; y is overwritten)
+void rows_apply(cfem_ctx *c, const double *x, double *y, bool caller_order = false);
 void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, const cfem_options *opt);
 void attach_stream(cfem_ctx *c, cudaStream_t s);
 
@@ -326,8 +330,9 @@ inline PcgResult run_pcg(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, in
   else return run_pcg_f(c, V, cK, cM, mcoef, warm, tol, rule, maxit);
 }
 template <typename T>
-inline void to_internal(cfem_ctx *c, const double *src, T *dst, double scale = 1.0) {
-  if constexpr (sizeof(T) == 8) to_internal_d(c, src, dst, scale); else to_internal_f(c, src, dst, scale);
+inline void to_internal(cfem_ctx *c, const double *src, T *dst) {
+  static_assert(sizeof(T) == 8, "");
+  to_internal_d(c, src, dst);
 }
 template <typename T>
 inline void to_caller(cfem_ctx *c, const T *src, double *dst) {

@@ -88,7 +88,7 @@ MultiParams<float> multi_params(cfem_ctx *c, MultiState &M) {
   P.F.L = c->L32;
   P.F.fan_off = c->fan_off.p;
   P.F.fan_elem_off = c->fan_elem_off.p;
-  P.F.err = c->tma_err.p;
+  P.F.err = c->h_tma_err;
   return P;
 }
 
@@ -297,7 +297,7 @@ cfem_status solve_batch(cfem_ctx *c, const cfem_solve_params &p, int kb, const d
   const int64_t nn = c->nn;
   const size_t nitems = (size_t)nn * K;
   c->launches = 0;
-  set_diag_vectors(c, c->diagK.p);
+  set_diag_vectors(c);
   CK(cudaMemcpyAsync(M.io.p, F, sizeof(double) * (size_t)kb * c->nd, cudaMemcpyDefault, c->stream));
   k_multi_to_internal<double><<<nblk(nitems), kThreads, 0, c->stream>>>(nn, K, kb, c->nd, M.io.p,
                                                                          c->node_new2old.p, M.f64.p);

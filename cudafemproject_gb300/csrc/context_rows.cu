@@ -10,7 +10,7 @@ namespace detail {
 namespace {
 
 template <int DIM>
-RowsAssembly<DIM> assembly(cfem_ctx *c, double cK, double cM, const double *diag) {
+RowsAssembly<DIM> assembly(cfem_ctx *c, double cK, double cM) {
   RowsAssembly<DIM> P{};
   P.conn = c->conn.p;
   P.inc_off = c->rows.inc_off.p;
@@ -25,7 +25,6 @@ RowsAssembly<DIM> assembly(cfem_ctx *c, double cK, double cM, const double *diag
   P.mu_e = c->mu_e.p;
   P.mc = c->mc64.p;
   P.bits = c->bits.p;
-  P.diag = diag;
   return P;
 }
 
@@ -62,8 +61,7 @@ void build_structure(cfem_ctx *c, DBuf<int32_t> &nbr, DBuf<int32_t> &deg) {
 }
 
 template <int DIM>
-void assemble_dim(cfem_ctx *c, const int32_t *nbr, const int32_t *deg, double cK, double cM, const double *diag,
-                  RowsValues &V) {
+void assemble_dim(cfem_ctx *c, const int32_t *nbr, const int32_t *deg, double cK, double cM, RowsValues &V) {
   RowsData &R = c->rows;
   cudaStream_t s = c->stream;
   if (!V.val.p) {
@@ -72,7 +70,7 @@ void assemble_dim(cfem_ctx *c, const int32_t *nbr, const int32_t *deg, double cK
     V.flag.alloc(R.n_slices);
   }
   V.flag.zero(s);
-  const RowsAssembly<DIM> P = assembly<DIM>(c, cK, cM, diag);
+  const RowsAssembly<DIM> P = assembly<DIM>(c, cK, cM);
   k_rows_assemble<DIM><<<nblk(R.n_slices, 4), 128, 0, s>>>(P, R.n_slices, R.off.p, R.row.p, nbr, deg, R.col.p,
                                                             V.val.p);
   k_rows_corrections<DIM><<<nblk(R.n_slices * kSliceRows), kThreads, 0, s>>>(P, R.n_slices * kSliceRows, R.off.p,
@@ -80,10 +78,9 @@ void assemble_dim(cfem_ctx *c, const int32_t *nbr, const int32_t *deg, double cK
   CKL();
 }
 
-void assemble(cfem_ctx *c, const int32_t *nbr, const int32_t *deg, double cK, double cM, const double *diag,
-              RowsValues &V) {
-  if (c->dim == 3) assemble_dim<3>(c, nbr, deg, cK, cM, diag, V);
-  else assemble_dim<2>(c, nbr, deg, cK, cM, diag, V);
+void assemble(cfem_ctx *c, const int32_t *nbr, const int32_t *deg, double cK, double cM, RowsValues &V) {
+  if (c->dim == 3) assemble_dim<3>(c, nbr, deg, cK, cM, V);
+  else assemble_dim<2>(c, nbr, deg, cK, cM, V);
 }
 
 unsigned rows_grid(const cfem_ctx *c) { return nblk(c->rows.n_slices, kRowsThreads / 32); }
@@ -109,17 +106,18 @@ void build_rows(cfem_ctx *c) {
     DBuf<int32_t> nbr, deg;
     if (c->dim == 3) build_structure<4>(c, nbr, deg);
     else build_structure<3>(c, nbr, deg);
-    assemble(c, nbr.p, deg.p, 1.0, 0.0, c->diagK.p, c->rows.K);
+    assemble(c, nbr.p, deg.p, 1.0, 0.0, c->rows.K);
     CK(cudaStreamSynchronize(c->stream));  // (before nbr and deg are freed)
   } else {
-    assemble(c, nullptr, nullptr, 1.0, 0.0, c->diagK.p, c->rows.K);
+    assemble(c, nullptr, nullptr, 1.0, 0.0, c->rows.K);
   }
 }
 
-void rows_apply(cfem_ctx *c, const double *x, double *y) {
+void rows_apply(cfem_ctx *c, const double *x, double *y, bool caller_order) {
   const RowOp A = op_of(c, c->rows.K);
-  if (c->dim == 3) k_rows_apply<3, false><<<rows_grid(c), kRowsThreads, 0, c->stream>>>(A, x, y, nullptr);
-  else k_rows_apply<2, false><<<rows_grid(c), kRowsThreads, 0, c->stream>>>(A, x, y, nullptr);
+  auto go = [&](auto k) { k<<<rows_grid(c), kRowsThreads, 0, c->stream>>>(A, x, y, c->node_new2old.p); };
+  if (c->dim == 3) caller_order ? go(k_rows_apply<3, true>) : go(k_rows_apply<3, false>);
+  else caller_order ? go(k_rows_apply<2, true>) : go(k_rows_apply<2, false>);
   CKL();
   c->launches += 1;
 }
@@ -140,14 +138,14 @@ void true_residual_async(cfem_ctx *c, const double *f, const double *x, double *
 
 // FP64 Jacobi PCG on A x = V.f, A = cM M + cK K' (has_mass) or K', as one
 // cooperative kernel (k_rows_pcg). V.dinv is the preconditioner; warm: V.x is
-// the start. diag_op: the operator's diagonal (combined operators).
+// the start.
 PcgResult run_pcg_d(cfem_ctx *c, Vecs<double> &V, double cK, double cM, const double *mcoef, int warm, double tol,
                     int rule, int maxit) {
   RowsData &R = c->rows;
   const RowsValues *values = &R.K;
   if (mcoef || cK != 1.0) {  // implicit dynamics: stiffness and mass in the same blocks, assembled once per run
     if (!R.KM.val.p || R.km_cK != cK || R.km_cM != cM) {
-      assemble(c, nullptr, nullptr, cK, mcoef ? cM : 0.0, V.diagA.p, R.KM);
+      assemble(c, nullptr, nullptr, cK, mcoef ? cM : 0.0, R.KM);
       R.km_cK = cK;
       R.km_cM = cM;
     }

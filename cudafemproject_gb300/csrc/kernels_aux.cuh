@@ -118,28 +118,30 @@ __global__ void k_geometry(GeomParams P) {
 }
 
 // ------------------------------------------------------------------ layout conversion
-// caller order [nn][dim] (FP64) -> node vectors [nn][VW] (T) in locality order
-template <typename T, int DIM>
-__global__ void k_to_internal(int64_t nn, const double *src, const int32_t *new2old, T *dst, double scale) {
+// caller order [nn][dim] -> node vectors [nn][VW] (T) in locality order; zero:
+// a node vector to clear on the way, or nullptr
+template <typename T, int DIM, typename S>
+__global__ void k_to_internal(int64_t nn, const S *src, const int32_t *new2old, T *dst, T *zero) {
   constexpr int VW = DIM == 3 ? 4 : 2;
   int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= nn) return;
   int64_t o = new2old[n];
   NodeV<T, VW> v;
 #pragma unroll
-  for (int d = 0; d < VW; ++d) v.v[d] = d < DIM ? (T)(src[o * DIM + d] * scale) : T(0);
+  for (int d = 0; d < VW; ++d) v.v[d] = d < DIM ? (T)src[o * DIM + d] : T(0);
   stv<T, VW>(dst, n, v);
+  if (zero) stv_zero<T, VW>(zero, n);
 }
 
-template <typename T, int DIM>
-__global__ void k_to_caller(int64_t nn, const T *src, const int32_t *new2old, double *dst) {
+template <typename T, int DIM, typename S>
+__global__ void k_to_caller(int64_t nn, const T *src, const int32_t *new2old, S *dst) {
   constexpr int VW = DIM == 3 ? 4 : 2;
   int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= nn) return;
   int64_t o = new2old[n];
   NodeV<T, VW> v = ldv<T, VW>(src, n);
 #pragma unroll
-  for (int d = 0; d < DIM; ++d) dst[o * DIM + d] = (double)v.v[d];
+  for (int d = 0; d < DIM; ++d) dst[o * DIM + d] = (S)v.v[d];
 }
 
 // dinv = 1 / diag (0 where diag == 0), in T
@@ -157,33 +159,20 @@ __global__ void k_convert(int64_t n, const TA *a, TB *b) {
   if (i < n) b[i] = (TB)a[i];
 }
 
+// *bad = 1 (pinned host memory) where a modulus is not positive
+static __global__ void k_young_check(int64_t n, const double *young, int *bad) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n && !(young[i] > 0)) *(volatile int *)bad = 1;
+}
+static __global__ void k_young_scale(int64_t n, const double *young, const int32_t *new2old, double E, double *escale) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) escale[i] = young[new2old[i]] / E;
+}
+
 // y = a*x + b*y over raw arrays
 static __global__ void k_axpby64(int64_t n, double a, const double *x, double b, double *y) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) y[i] = a * x[i] + b * y[i];
-}
-
-// Refinement: r64 = f - u64 (u64 = K x64), u64 = 0, r32 = (float) r64, ||r||^2 and ||f||^2.
-struct ResParams {
-  int64_t nvec;
-  const double *f;
-  double *u, *r;
-  float *r32;
-  double *out;       // [2]: ||r||^2, ||f||^2
-  double *partials;
-  unsigned int *count;
-};
-static __global__ void __launch_bounds__(kThreads) k_residual(ResParams P) {
-  double acc[2] = {0, 0};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < P.nvec; i += (int64_t)gridDim.x * blockDim.x) {
-    double r = P.f[i] - P.u[i];
-    P.u[i] = 0;
-    P.r[i] = r;
-    if (P.r32) P.r32[i] = (float)r;
-    acc[0] += r * r;
-    acc[1] += P.f[i] * P.f[i];
-  }
-  if (grid_sum_last<2>(acc, P.partials, P.count)) { P.out[0] = acc[0]; P.out[1] = acc[1]; }
 }
 
 // Continued PCG run: z += (gamma / gamma_prev) p_last on the DOF lanes (the
@@ -204,9 +193,10 @@ __global__ void k_fold_direction(int64_t nn, const Scalars *sc, double gamma_pre
 }
 
 // x64 += (double) x32 on the DOF lanes (vw 4: the fourth lane of x32 carries
-// M^-1, see k_pcg_init)
-static __global__ void k_accumulate(int64_t n, const float *x32, double *x64, int vw) {
+// M^-1, see k_pcg_init); nothing where the run that made x32 diverged (sc).
+static __global__ void k_accumulate(int64_t n, const float *x32, double *x64, int vw, const Scalars *sc) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (sc && sc->done == 2) return;
   if (i < n && !(vw == 4 && (i & 3) == 3)) x64[i] += (double)x32[i];
 }
 

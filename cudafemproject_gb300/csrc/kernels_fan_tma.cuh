@@ -186,7 +186,7 @@ struct FanTmaParams {
   FanBlockLayout L;
   const int32_t *fan_off;       // [n_patches + 1]
   const int32_t *fan_elem_off;  // [n_fans + 1] (consistent-mass coefficients)
-  int *err;                     // kErrTmaTimeout on a copy that never completed
+  int *err;                     // kErrTmaTimeout on a copy that never completed (pinned host memory)
   int evict_first;              // blocks larger than about half the L2: stream them with an
                                 // evict-first policy, so that the node vectors stay resident
   // Self-test of the copy-timeout path (cfem_selftest_copy_timeout), zero
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kHfanThreads, 3) k_matvec_fan_tma(MvParams<T> 
     auto copy_failed = [&]() {
       if (PREFETCH) cp_async_wait<0>();
       if (threadIdx.x == 0) {
-        atomicOr(F.err, kErrTmaTimeout);
+        *(volatile int *)F.err = kErrTmaTimeout;
         if (patch + step < P.n_patches && patch_live(patch + step))
           mbar_wait_bounded(&bar[b ^ 1], (phase >> (b ^ 1)) & 1u, lim);
       }

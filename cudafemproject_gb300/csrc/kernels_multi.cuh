@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kHfanThreads, C <= 2 ? 3 : 2) k_matvec_multi(M
       const bool ok = mbar_wait_bounded(&bar[0], nload & 1u);
       ++nload;
       if (__syncthreads_or(!ok)) {
-        if (threadIdx.x == 0) atomicOr(P.F.err, kErrTmaTimeout);
+        if (threadIdx.x == 0) *(volatile int *)P.F.err = kErrTmaTimeout;
         return;
       }
       cur = patch;

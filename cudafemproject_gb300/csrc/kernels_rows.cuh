@@ -43,8 +43,29 @@ struct RowOp {
   const uint8_t *bits;  // [n_nodes] constrained DOFs
 };
 
-template <int DIM, bool MASKED>
-__device__ __forceinline__ void rows_sum(const RowOp &A, int64_t k0, int n, const double *x, const double (&xi)[DIM],
+// Where a row product reads x: a node vector, or the caller's [n_nodes][DIM].
+template <int DIM>
+struct NodeX {
+  static constexpr int VW = DIM == 3 ? 4 : 2;
+  const double *x;
+  __device__ __forceinline__ NodeV<double, VW> operator()(int32_t j) const { return ldv<double, VW>(x, j); }
+};
+template <int DIM>
+struct CallerX {
+  static constexpr int VW = DIM == 3 ? 4 : 2;
+  const double *x;
+  const int32_t *new2old;
+  __device__ __forceinline__ NodeV<double, VW> operator()(int32_t j) const {
+    const double *p = x + (int64_t)new2old[j] * DIM;
+    NodeV<double, VW> v;
+#pragma unroll
+    for (int d = 0; d < VW; ++d) v.v[d] = d < DIM ? p[d < DIM ? d : 0] : 0.0;
+    return v;
+  }
+};
+
+template <int DIM, bool MASKED, typename X>
+__device__ __forceinline__ void rows_sum(const RowOp &A, int64_t k0, int n, const X &x, const double (&xi)[DIM],
                                          double (&y)[DIM]) {
   constexpr int VW = DIM == 3 ? 4 : 2, NC = DIM * DIM;
   const int32_t *col = A.col + k0 * 32 + (threadIdx.x & 31);
@@ -55,7 +76,7 @@ __device__ __forceinline__ void rows_sum(const RowOp &A, int64_t k0, int n, cons
 #pragma unroll
     for (int c = 0; c < NC; ++c) K[c] = __ldcs(val + (k * NC + c) * 32);
     const int32_t j = col[k * 32];
-    NodeV<double, VW> v = ldv<double, VW>(x, j);
+    NodeV<double, VW> v = x(j);
     if (MASKED) {  // values at constrained DOFs have no influence, whatever they are
       const unsigned b = A.bits[j];
 #pragma unroll
@@ -77,9 +98,9 @@ __device__ __forceinline__ void rows_sum(const RowOp &A, int64_t k0, int n, cons
 // y = A x for the rows of slice s, given the rows (-1: padding) and their own
 // x; both lanes of a row get the sum. x is read with plain loads: callers may
 // have other CTAs' writes made visible by a grid barrier.
-template <int DIM>
-__device__ __forceinline__ void rows_product(const RowOp &A, int64_t s, int row, const double *x,
-                                             const double (&xi)[DIM], double (&y)[DIM]) {
+template <int DIM, typename X>
+__device__ __forceinline__ void rows_product_of(const RowOp &A, int64_t s, int row, const X &x,
+                                                const double (&xi)[DIM], double (&y)[DIM]) {
   constexpr int NC = DIM * DIM;
   const int64_t k0 = A.off[s];
   const int n = (int)(A.off[s + 1] - k0);
@@ -107,6 +128,12 @@ __device__ __forceinline__ void rows_product(const RowOp &A, int64_t s, int row,
   }
 }
 
+template <int DIM>
+__device__ __forceinline__ void rows_product(const RowOp &A, int64_t s, int row, const double *x,
+                                             const double (&xi)[DIM], double (&y)[DIM]) {
+  rows_product_of<DIM>(A, s, row, NodeX<DIM>{x}, xi, y);
+}
+
 // row of this lane in slice s and its own x
 template <int DIM>
 __device__ __forceinline__ int rows_own(const RowOp &A, int64_t s, const double *x, double (&xi)[DIM]) {
@@ -123,27 +150,33 @@ __device__ __forceinline__ int rows_own(const RowOp &A, int64_t s, const double 
 // leave SMs of a small mesh without any (2601 nodes: 41 CTAs).
 constexpr int kRowsThreads = 128;
 
-// y = A x, node vectors in the internal layout (XOUT false) or y in the
-// caller's order [n_nodes][DIM] (XOUT true).
-template <int DIM, bool XOUT>
+// y = A x; CALLER: x and y are the caller's [n_nodes][DIM] arrays (not
+// overlapping), else node vectors.
+template <int DIM, bool CALLER>
 __global__ void __launch_bounds__(kRowsThreads) k_rows_apply(RowOp A, const double *x, double *y, const int32_t *new2old) {
   constexpr int VW = DIM == 3 ? 4 : 2;
-  const int64_t W = (int64_t)gridDim.x * (kRowsThreads / 32);
-  for (int64_t s = blockIdx.x * (int64_t)(kRowsThreads / 32) + (threadIdx.x >> 5); s < A.n_slices; s += W) {
-    double v[DIM], xi[DIM];
-    const int row = rows_own<DIM>(A, s, x, xi);
-    rows_product<DIM>(A, s, row, x, xi, v);
-    if (row < 0 || (threadIdx.x & 16)) continue;
-    if constexpr (XOUT) {
-      const int64_t o = new2old[row];
+  const int64_t s = blockIdx.x * (int64_t)(kRowsThreads / 32) + (threadIdx.x >> 5);
+  if (s >= A.n_slices) return;
+  double v[DIM], xi[DIM];
+  const int row = A.row[s * kSliceRows + (threadIdx.x & 15)];
+  auto product = [&](const auto &X) {
+    const NodeV<double, VW> own = X(row < 0 ? 0 : row);
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) y[o * DIM + d] = v[d];
-    } else {
-      NodeV<double, VW> o;
+    for (int d = 0; d < DIM; ++d) xi[d] = own.v[d];
+    rows_product_of<DIM>(A, s, row, X, xi, v);
+  };
+  if constexpr (CALLER) product(CallerX<DIM>{x, new2old});
+  else product(NodeX<DIM>{x});
+  if (row < 0 || (threadIdx.x & 16)) return;
+  if constexpr (CALLER) {
+    const int64_t o = new2old[row];
 #pragma unroll
-      for (int d = 0; d < VW; ++d) o.v[d] = d < DIM ? v[d < DIM ? d : 0] : 0.0;
-      stv<double, VW>(y, row, o);
-    }
+    for (int d = 0; d < DIM; ++d) y[o * DIM + d] = v[d];
+  } else {
+    NodeV<double, VW> o;
+#pragma unroll
+    for (int d = 0; d < VW; ++d) o.v[d] = d < DIM ? v[d < DIM ? d : 0] : 0.0;
+    stv<double, VW>(y, row, o);
   }
 }
 
@@ -635,7 +668,6 @@ struct RowsAssembly {
   const double *lam_e, *mu_e;  // per-element material (new order) or nullptr
   const double *mc;            // per-element consistent-mass coefficient (cM != 0)
   const uint8_t *bits;
-  const double *diag;          // node vector: diagonal of the constrained DOFs
 };
 
 template <int DIM>
@@ -782,13 +814,31 @@ __global__ void k_rows_corrections(RowsAssembly<DIM> P, int64_t n_rows, const in
 #pragma unroll
     for (int p = 0; p < DIM; ++p) B[p * DIM + p] += P.cM * 2.0 * m;
   }
-  constexpr int VW = DIM == 3 ? 4 : 2;
+  if (bi) {  // constrained DOFs: the diagonal of cK K + cM M, from the node's elements in order
+    double diag[DIM], m = 0;
 #pragma unroll
-  for (int p = 0; p < DIM; ++p)
-    if ((bi >> p) & 1u) {
+    for (int p = 0; p < DIM; ++p) diag[p] = 0;
+    for (int32_t t = P.inc_off[i]; t < P.inc_off[i + 1]; ++t) {
+      const int32_t e = P.inc[t];
+      int a = 0;
 #pragma unroll
-      for (int q = 0; q < DIM; ++q) B[p * DIM + q] = p == q ? P.diag[(int64_t)i * VW + p] : 0.0;
+      for (int v = 1; v <= DIM; ++v)
+        if (P.conn[(int64_t)e * (DIM + 1) + v] == i) a = v;
+      double g[DIM], tot = 0;
+      vertex_gradient<DIM>(P, e, a, g);
+      const double lam = P.lam_e ? P.lam_e[e] : P.lam, mu = P.mu_e ? P.mu_e[e] : P.mu;
+#pragma unroll
+      for (int p = 0; p < DIM; ++p) tot += g[p] * g[p];
+#pragma unroll
+      for (int p = 0; p < DIM; ++p) diag[p] += (lam + 2 * mu) * (g[p] * g[p]) + mu * (tot - g[p] * g[p]);
+      if (P.cM != 0) m += 2.0 * P.mc[e];
     }
+#pragma unroll
+    for (int p = 0; p < DIM; ++p)
+      if ((bi >> p) & 1u)
+#pragma unroll
+        for (int q = 0; q < DIM; ++q) B[p * DIM + q] = p == q ? P.cK * diag[p] + P.cM * m : 0.0;
+  }
 #pragma unroll
   for (int c = 0; c < NC; ++c) D[(int64_t)i * NC + c] = B[c];
   if (any) flag[s] = 1;

@@ -149,3 +149,55 @@ def test_dyn_adjoint_whole_and_by_segments(monkeypatch, states_mb, mesh, steps):
     assert info["steps"] == steps
     assert abs(L - Lo) <= 1e-11 * abs(Lo)
     assert rel(g, go) <= 1e-11
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_matvec_on_device_arrays(precision):
+    """Device arrays in place, overlapping (x is y), offset to odd elements, and
+    host arrays: the same product."""
+    import torch
+    from cudafemproject_gb300.solver import FemContext
+    p = MESHES["box_code1"]()
+    ctx = FemContext(p)
+    dt, tol = (torch.float64, 0.0) if precision == "fp64" else (torch.float32, 2e-6)
+    x = torch.tensor(np.random.default_rng(6).standard_normal(p.n_dof), dtype=dt)
+    ref = np.array(ctx.matvec(x.numpy().copy(), precision))
+    same = lambda y: np.linalg.norm(y.cpu().numpy() - ref) <= tol * np.linalg.norm(ref)  # FP32 sums are atomic
+    xd = x.cuda()
+    assert same(ctx.matvec(xd, precision))
+    buf = torch.zeros(2 * p.n_dof + 3, dtype=dt, device="cuda")
+    xo, yo = buf[1:1 + p.n_dof], buf[2 + p.n_dof:2 + 2 * p.n_dof]
+    xo.copy_(xd)
+    torch.cuda.synchronize()
+    assert same(ctx.matvec(xo, precision, out=yo))
+    assert torch.equal(xo, xd) and float(buf[0]) == 0.0 == float(buf[1 + p.n_dof])
+    assert same(ctx.matvec(xd, precision, out=xd))
+
+
+def test_set_young_on_device_and_refused_values():
+    """Moduli from a device array equal those from the host; a value that is not
+    positive is refused and leaves the operator as it was; the captured FP32
+    iterations follow the new moduli."""
+    import torch
+    from cudafemproject_gb300 import capi
+    from cudafemproject_gb300.solver import FemContext
+    p = meshgen.box_3d(5, 4, 11, jitter=0.2, seed=1)
+    young = 2e7 * np.exp(0.3 * np.random.default_rng(4).standard_normal(p.n_elems))
+    f = np.random.default_rng(5).standard_normal(p.n_dof)
+    kw = dict(precision="fp32_refine", tol=1e-3, stop_rule="residual", outer_tol=1e-10)
+    for form in ("auto", "geometry", "gradient"):
+        a, b = FemContext(p, matvec_form=form), FemContext(p, matvec_form=form)
+        a.pcg(f, **kw)
+        a.set_young(torch.tensor(young, device="cuda"))
+        b.set_young(young)
+        y = a.matvec(f, "fp64")
+        assert np.array_equal(y, b.matvec(f, "fp64"))
+        for bad in (0.0, -1.0, np.nan):
+            wrong = young.copy()
+            wrong[-1] = bad
+            with pytest.raises(capi.CfemError):
+                a.set_young(wrong)
+            assert np.array_equal(a.matvec(f, "fp64"), y)
+        p2 = meshgen.box_3d(5, 4, 11, jitter=0.2, seed=1)
+        p2.elem_E = young
+        assert rel(a.pcg(f, **kw)[0], O.Oracle(p2).pcg(f, tol=1e-13, rule=1)[0]) <= 1e-8
