@@ -34,7 +34,6 @@ MvParams<T> base_mv_t(cfem_ctx *c) {
   P.cM = 0;
   P.partials = c->partials.p;
   P.up_part = c->partials_up.p;
-  P.n_up = c->dim == 3 ? c->grid_upd : c->grid_vec;
   P.inc = c->inc.p;
   P.inc_start = c->inc_start.p;
   P.pe = c->prep.patch_elems;
@@ -43,10 +42,10 @@ MvParams<T> base_mv_t(cfem_ctx *c) {
 }
 
 void launch_mv_f(cfem_ctx *c, int mode, const MvParams<float> &P) {
-  if (!P.patch_inst) single_mesh_only(c);
+  if (!P.patch_inst && !P.instance) single_mesh_only(c);
   if (c->fans) {  // patch blocks streamed by bulk copies
     FanTmaParams F{};
-    F.blocks = c->blk32.p;
+    F.blocks = c->blk32.p + (size_t)P.first_patch * c->L32.bytes;
     F.L = c->L32;
     F.fan_off = c->fan_off.p;
     F.fan_elem_off = c->fan_elem_off.p;
@@ -55,7 +54,7 @@ void launch_mv_f(cfem_ctx *c, int mode, const MvParams<float> &P) {
     F.wait_limit = c->selftest_wait_limit;
     const double l2_half = 0.5 * c->l2_bytes;
     F.evict_first = (double)c->L32.bytes * c->prep.n_patches > l2_half;
-    if (c->geo && !P.patch_inst) {
+    if (c->geo && !c->n_inst) {
       F.blocks = c->blkg.p;
       F.L = c->Lg;
       F.evict_first = (double)c->Lg.bytes * c->prep.n_patches > l2_half;
@@ -71,7 +70,7 @@ void launch_mv_f(cfem_ctx *c, int mode, const MvParams<float> &P) {
       c->launches += 1;
       return;
     }
-    dim3 g(c->grid_ft32), b(kHfanThreads);
+    dim3 g(std::min(c->grid_ft32, P.n_patches)), b(kHfanThreads);
     if (P.patch_inst) {
       if (mode != MV_PCG || P.mcoef) throw Fail{CFEM_ERR_UNSUPPORTED, "batched meshes: PCG-form static matvec only"};
       launch_pdl(k_matvec_fan_tma<float, MV_PCG, false, false, true>, g, b, c->smem_ft32, c->stream, P, F);
@@ -100,108 +99,188 @@ void launch_mv_f(cfem_ctx *c, int mode, const MvParams<float> &P) {
   c->launches += 1;
 }
 
-// Grid of the PCG-form matvec that launch_mv_t runs for precision T (the
-// number of p.Ap partials the update kernel adds up).
-template <typename T>
-int pcg_mv_grid(const cfem_ctx *c) {
-  if constexpr (sizeof(T) == 4)
-    if (c->fans) return c->geo ? c->grid_geo : c->grid_ft32;
-  return c->grid_mv;
+// Grid of the PCG-form matvec that launch_mv_f runs on n patches (the number
+// of p.Ap partials the update kernel adds up).
+int pcg_mv_grid(const cfem_ctx *c, int n_patches) {
+  return std::min(n_patches, !c->fans ? c->grid_mv : c->geo && !c->n_inst ? c->grid_geo : c->grid_ft32);
 }
 
-template <typename T>
-VecParams<T> vec_params(cfem_ctx *c, Vecs<T> &V, T *p, Scalars *sc) {
-  VecParams<T> P{};
-  P.n_nodes = c->nn;
-  P.x = V.x.p; P.r = V.r.p; P.z = V.z.p; P.p = p; P.u = V.u.p;
-  P.dinv = V.dinv.p;
-  P.f = V.f.p;
-  P.sc = sc;
-  P.partials = c->partials.p;
-  P.mv_part = c->partials.p;
-  P.n_mv = pcg_mv_grid<T>(c);
-  P.up_part = c->partials_up.p;
+// Where a PCG run takes place: the whole context, or the patches and nodes of
+// one instance of a batch, with its own scalars and partial sums.
+PcgSite whole_mesh(cfem_ctx *c) {
+  PcgSite S{};
+  S.sc = c->sc.p + 1;
+  S.n_patches = c->prep.n_patches;
+  S.n_nodes = c->nn;
+  S.lam = (float)c->lam;
+  S.mu = (float)c->mu;
+  S.partials = c->partials.p;
+  S.partials_up = c->partials_up.p;
+  return S;
+}
+
+VecParams<float> vec_params(cfem_ctx *c, const PcgSite &S, float *p, float *u) {
+  Vecs<float> &V = c->v32;
+  const int64_t o = S.first_node * c->vw;
+  VecParams<float> P{};
+  P.n_nodes = S.n_nodes;
+  P.x = V.x.p + o; P.r = V.r.p + o; P.z = V.z.p + o; P.p = p + o; P.u = u + o;
+  P.dinv = V.dinv.p + o;
+  P.f = V.f.p + o;
+  P.sc = S.sc;
+  P.partials = S.partials;
+  P.mv_part = S.partials;
+  P.n_mv = pcg_mv_grid(c, S.n_patches);
+  P.up_part = S.partials_up;
   return P;
 }
 
-template <typename T>
-void launch_init(cfem_ctx *c, const VecParams<T> &P, int warm) {
-  if (c->dim == 3) k_pcg_init<T, 3><<<c->grid_vec, kThreads, 0, c->stream>>>(P, warm);
-  else k_pcg_init<T, 2><<<c->grid_vec, kThreads, 0, c->stream>>>(P, warm);
+int update_grid(const cfem_ctx *c, int64_t n_nodes) {
+  // 3D: two CTAs per SM keep enough loads in flight for the bandwidth and leave
+  // room for the next matvec's CTAs to start early (PDL)
+  return (int)std::min<int64_t>(std::max<int64_t>(1, nblk(n_nodes)), (int64_t)c->n_sm * (c->dim == 3 ? 2 : 4));
+}
+
+void launch_init(cfem_ctx *c, const VecParams<float> &P, int warm) {
+  const int g = (int)std::min<int64_t>(std::max<int64_t>(1, nblk(P.n_nodes)), (int64_t)c->n_sm * 4);
+  if (c->dim == 3 && P.cond) k_pcg_init<float, 3, true><<<g, kThreads, 0, c->stream>>>(P, warm);
+  else if (c->dim == 3) k_pcg_init<float, 3><<<g, kThreads, 0, c->stream>>>(P, warm);
+  else k_pcg_init<float, 2><<<g, kThreads, 0, c->stream>>>(P, warm);
   CKL();
   c->launches += 1;
 }
 
-template <typename T>
-void launch_update(cfem_ctx *c, const VecParams<T> &P) {
-  if (c->dim == 3 && P.cond) launch_pdl(k_pcg_update<T, 3, true>, dim3(c->grid_upd), dim3(kThreads), 0, c->stream, P);
-  else if (c->dim == 3) launch_pdl(k_pcg_update<T, 3>, dim3(c->grid_upd), dim3(kThreads), 0, c->stream, P);
-  else if (P.cond) k_pcg_update<T, 2, true><<<c->grid_vec, kThreads, 0, c->stream>>>(P);
-  else k_pcg_update<T, 2><<<c->grid_vec, kThreads, 0, c->stream>>>(P);
+void launch_update(cfem_ctx *c, const VecParams<float> &P) {
+  const int g = update_grid(c, P.n_nodes);
+  if (c->dim == 3 && P.cond) launch_pdl(k_pcg_update<float, 3, true>, dim3(g), dim3(kThreads), 0, c->stream, P);
+  else if (c->dim == 3) launch_pdl(k_pcg_update<float, 3>, dim3(g), dim3(kThreads), 0, c->stream, P);
+  else if (P.cond) k_pcg_update<float, 2, true><<<g, kThreads, 0, c->stream>>>(P);
+  else k_pcg_update<float, 2><<<g, kThreads, 0, c->stream>>>(P);
   CKL();
   c->launches += 1;
 }
 
-// Jacobi PCG on A x = V.f with A = cM*M + cK*K' (mcoef selects the mass term).
+MvParams<float> site_mv(cfem_ctx *c, const PcgSite &S, float cK, float cM, const float *mcoef) {
+  MvParams<float> mv = base_mv<float>(c);
+  mv.cK = cK;
+  mv.cM = cM;
+  mv.mcoef = mcoef;
+  mv.diagA = c->v32.diagA.p;
+  mv.sc = S.sc;
+  mv.instance = c->n_inst > 0;
+  mv.first_patch = S.first_patch;
+  mv.n_patches = S.n_patches;
+  mv.lam = S.lam;
+  mv.mu = S.mu;
+  mv.partials = S.partials;
+  mv.up_part = S.partials_up;
+  mv.n_up = update_grid(c, S.n_nodes);
+  return mv;
+}
+
+// `chunk` PCG iterations on c->stream (captured): directions alternate between
+// pA and pB, A p between u and uB: the matvec of iteration `it` accumulates
+// into one u buffer and zeroes the other for iteration it + 1 (the init kernel
+// zeroes u for iteration 0; chunk is even). cond: the graph's loop condition,
+// or 0.
+void capture_iterations(cfem_ctx *c, const PcgSite &S, const MvParams<float> &mv, int chunk, unsigned long long cond) {
+  Vecs<float> &V = c->v32;
+  for (int it = 0; it < chunk; ++it) {
+    float *pold = (it & 1) ? V.pB.p : V.pA.p;
+    float *pnew = (it & 1) ? V.pA.p : V.pB.p;
+    float *ucur = (it & 1) ? V.uB.p : V.u.p;
+    MvParams<float> m = mv;
+    m.x = V.z.p;
+    m.x2 = pold;
+    m.xout = pnew;
+    m.y = ucur;
+    m.yzero = (it & 1) ? V.u.p : V.uB.p;
+    launch_mv_f(c, MV_PCG, m);
+    VecParams<float> up = vec_params(c, S, pnew, ucur);
+    up.cond = cond;
+    up.cond_role = (it == 0 ? 1 : 0) | (it == chunk - 1 ? 2 : 0);
+    up.cond_chunk = chunk;
+    launch_update(c, up);
+  }
+}
+
+// A WHILE node in `graph` behind `before` (or first), its body captured from
+// c->stream by `capture`, which gets the loop condition; false where the
+// runtime does not build it.
+bool add_loop(cfem_ctx *c, cudaGraph_t graph, unsigned initial, const std::function<void(cudaGraphConditionalHandle)> &prologue,
+              const std::function<void(cudaGraphConditionalHandle)> &capture) {
+  cudaGraphConditionalHandle h = 0;
+  if (cudaGraphConditionalHandleCreate(&h, graph, initial, cudaGraphCondAssignDefault) != cudaSuccess) return false;
+  auto record = [&](cudaGraph_t into, const std::function<void(cudaGraphConditionalHandle)> &fn) {
+    if (cudaStreamBeginCaptureToGraph(c->stream, into, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) !=
+        cudaSuccess)
+      return false;
+    bool ok = true;
+    try {
+      fn(h);
+    } catch (...) {
+      ok = false;
+    }
+    cudaGraph_t captured = nullptr;
+    return cudaStreamEndCapture(c->stream, &captured) == cudaSuccess && ok;
+  };
+  auto nodes = [&](std::vector<cudaGraphNode_t> &v) {
+    size_t n = 0;
+    if (cudaGraphGetNodes(graph, nullptr, &n) != cudaSuccess) return false;
+    v.resize(n);
+    return n == 0 || cudaGraphGetNodes(graph, v.data(), &n) == cudaSuccess;
+  };
+  // the prologue is one kernel: the node it adds is the loop's dependency
+  cudaGraphNode_t dep{};
+  if (prologue) {
+    std::vector<cudaGraphNode_t> before, after;
+    if (!nodes(before) || !record(graph, prologue) || !nodes(after) || after.size() != before.size() + 1) return false;
+    for (cudaGraphNode_t v : after)
+      if (std::find(before.begin(), before.end(), v) == before.end()) dep = v;
+  }
+  cudaGraphNodeParams np{};
+  np.type = cudaGraphNodeTypeConditional;
+  np.conditional.handle = h;
+  np.conditional.type = cudaGraphCondTypeWhile;
+  np.conditional.size = 1;
+  cudaGraphNode_t node;
+  if (cudaGraphAddNode(&node, graph, prologue ? &dep : nullptr, nullptr, prologue ? 1 : 0, &np) != cudaSuccess) return false;
+  return record(np.conditional.phGraph_out[0], capture);
+}
+
+// FP32 Jacobi PCG on A x = V.f (V = c->v32) with A = cM*M + cK*K' (mcoef selects the mass term).
 // V.x holds the warm start when warm != 0. Returns after the device flag says
 // done and what `then` has queued behind the run is complete.
-template <typename T>
-PcgResult run_pcg_t(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int warm, double tol, int rule, int maxit,
-                    const T *cont_p = nullptr, double cont_gamma_prev = 0,
-                    const std::function<void()> &then = nullptr) {
-  Scalars *sc = c->sc.p + 1;
+PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
+                    const float *cont_p, double cont_gamma_prev, const std::function<void()> &then) {
+  Vecs<float> &V = c->v32;
+  const PcgSite S = whole_mesh(c);
+  Scalars *sc = S.sc;
   Scalars h{};
   h.tol = tol;
   h.rule = rule;
   h.maxit = maxit > 0 ? maxit : 1000000;
   CK(cudaMemcpyAsync(sc, &h, sizeof(Scalars), cudaMemcpyHostToDevice, c->stream));
-  MvParams<T> mv = base_mv<T>(c);
-  mv.cK = cK;
-  mv.cM = cM;
-  mv.mcoef = mcoef;
-  mv.diagA = V.diagA.p;
-  mv.sc = sc;
+  const MvParams<float> mv = site_mv(c, S, cK, cM, mcoef);
   if (warm) {
-    mv.x = V.x.p;
-    mv.y = V.u.p;
+    MvParams<float> m = mv;
+    m.x = V.x.p;
+    m.y = V.u.p;
     V.u.zero(c->stream);
-    launch_mv_f(c, MV_PLAIN, mv);
+    launch_mv_f(c, MV_PLAIN, m);
   }
-  launch_init<T>(c, vec_params<T>(c, V, V.pA.p, sc), warm);
+  launch_init(c, vec_params(c, S, V.pA.p, V.u.p), warm);
   if (cont_p && cont_gamma_prev > 0) {
     // Continuation of an earlier run on a new residual: its last direction
     // p_last stays, and the first direction becomes the conjugate-gradient
     // step from it, z + (gamma / gamma_prev) p_last, folded into z here (the
     // first matvec takes p = z).
-    if (c->dim == 3) k_fold_direction<T, 3><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, sc, cont_gamma_prev, cont_p, V.z.p);
-    else k_fold_direction<T, 2><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, sc, cont_gamma_prev, cont_p, V.z.p);
+    if (c->dim == 3) k_fold_direction<float, 3><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, sc, cont_gamma_prev, cont_p, V.z.p);
+    else k_fold_direction<float, 2><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, sc, cont_gamma_prev, cont_p, V.z.p);
     CKL();
     c->launches += 1;
   }
   GraphCache &gc = c->graph32;
-  // directions alternate between pA and pB, A p between u and uB: the matvec
-  // of iteration `it` accumulates into one u buffer and zeroes the other for
-  // iteration it + 1 (the init kernel zeroes u for iteration 0; chunk is even)
-  auto capture_iterations = [&](unsigned long long cond) {
-    for (int it = 0; it < c->chunk; ++it) {
-      T *pold = (it & 1) ? V.pB.p : V.pA.p;
-      T *pnew = (it & 1) ? V.pA.p : V.pB.p;
-      T *ucur = (it & 1) ? V.uB.p : V.u.p;
-      MvParams<T> m = mv;
-      m.x = V.z.p;
-      m.x2 = pold;
-      m.xout = pnew;
-      m.y = ucur;
-      m.yzero = (it & 1) ? V.u.p : V.uB.p;
-      launch_mv_f(c, MV_PCG, m);
-      VecParams<T> up = vec_params<T>(c, V, pnew, sc);
-      up.u = ucur;
-      up.cond = cond;
-      up.cond_role = (it == 0 ? 1 : 0) | (it == c->chunk - 1 ? 2 : 0);
-      up.cond_chunk = c->chunk;
-      launch_update<T>(c, up);
-    }
-  };
   if (!gc.exec || gc.key0 != (const void *)mcoef || gc.key1 != (double)cK || gc.key2 != (double)cM) {
     gc.reset();
     const int64_t launches_before_capture = c->launches;
@@ -212,31 +291,8 @@ PcgResult run_pcg_t(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int war
     if (!c->host_loop) {
       cudaGraph_t graph = nullptr;
       cudaGraphExec_t exec = nullptr;
-      cudaGraphConditionalHandle h = 0;
       bool ok = cudaGraphCreate(&graph, 0) == cudaSuccess &&
-                cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault) == cudaSuccess;
-      cudaGraph_t body = nullptr;
-      if (ok) {
-        cudaGraphNodeParams np{};
-        np.type = cudaGraphNodeTypeConditional;
-        np.conditional.handle = h;
-        np.conditional.type = cudaGraphCondTypeWhile;
-        np.conditional.size = 1;
-        cudaGraphNode_t node;
-        ok = cudaGraphAddNode(&node, graph, nullptr, nullptr, 0, &np) == cudaSuccess;
-        if (ok) body = np.conditional.phGraph_out[0];
-      }
-      if (ok) ok = cudaStreamBeginCaptureToGraph(c->stream, body, nullptr, nullptr, 0,
-                                                 cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-      if (ok) {
-        try {
-          capture_iterations(h);
-        } catch (...) {
-          ok = false;
-        }
-        cudaGraph_t captured = nullptr;
-        if (cudaStreamEndCapture(c->stream, &captured) != cudaSuccess) ok = false;
-      }
+                add_loop(c, graph, 1, nullptr, [&](cudaGraphConditionalHandle cond) { capture_iterations(c, S, mv, c->chunk, cond); });
       if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
       if (graph) cudaGraphDestroy(graph);
       (void)cudaGetLastError();
@@ -251,7 +307,7 @@ PcgResult run_pcg_t(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int war
       cudaGraph_t graph;
       CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
       try {
-        capture_iterations(0);
+        capture_iterations(c, S, mv, c->chunk, 0);
       } catch (...) {
         cudaGraph_t broken = nullptr;
         cudaStreamEndCapture(c->stream, &broken);
@@ -346,10 +402,6 @@ void to_caller_t(cfem_ctx *c, const T *src, S *dst) {
 
 MvParams<double> base_mv_d(cfem_ctx *c) { return base_mv_t<double>(c); }
 MvParams<float> base_mv_f(cfem_ctx *c) { return base_mv_t<float>(c); }
-PcgResult run_pcg_f(cfem_ctx *c, Vecs<float> &V, float cK, float cM, const float *mcoef, int warm, double tol,
-                    int rule, int maxit) {
-  return run_pcg_t<float>(c, V, cK, cM, mcoef, warm, tol, rule, maxit);
-}
 void to_internal_d(cfem_ctx *c, const double *src, double *dst) { to_internal_t<double, double>(c, src, dst); }
 void to_caller_d(cfem_ctx *c, const double *src, double *dst) { to_caller_t<double, double>(c, src, dst); }
 void to_caller_f(cfem_ctx *c, const float *src, double *dst) { to_caller_t<float, double>(c, src, dst); }
@@ -443,9 +495,9 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
         true_residual_async(c, c->v64.f.p, c->v64.x.p, c->v64.r.p, c->v32.f.p, c->h_rr);
       };
       PcgResult r = cont_iters > 0 && prm->tol >= kContinueTol
-                        ? run_pcg_t<float>(c, c->v32, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, prm->max_iter,
+                        ? run_pcg_f(c, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, prm->max_iter,
                                            ((cont_iters - 1) & 1) ? c->v32.pA.p : c->v32.pB.p, cont_gprev, then)
-                        : run_pcg_t<float>(c, c->v32, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, prm->max_iter,
+                        : run_pcg_f(c, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, prm->max_iter,
                                            nullptr, 0, then);
       cont_iters = r.status == CFEM_OK || r.status == CFEM_ERR_NOT_CONVERGED ? r.iters : 0;
       cont_gprev = r.gamma_prev;
@@ -711,6 +763,8 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
     c->patch_inst.upload(pinst.data(), pinst.size(), s);
     c->inst_patch_off.upload(ipo.data(), ipo.size(), s);
     c->own_first.upload(ofirst.data(), ofirst.size(), s);
+    c->h_inst_patch_off = ipo;
+    c->h_own_first = ofirst;
     c->pmat32.upload(pm32.data(), pm32.size(), s);
     c->lam_e.upload(le.data(), le.size(), s);
     c->mu_e.upload(me.data(), me.size(), s);
@@ -809,9 +863,6 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
     }
   }
   c->grid_vec = (int)std::min<int64_t>(std::max<int64_t>(1, nblk(c->nn)), (int64_t)c->n_sm * 4);
-  // PCG update: two CTAs per SM keep enough loads in flight for the bandwidth
-  // and leave room for the next matvec's CTAs to start early (PDL)
-  c->grid_upd = (int)std::min<int64_t>(std::max<int64_t>(1, nblk(c->nn)), (int64_t)c->n_sm * 2);
   if (c->geo) {  // the grid of the largest geometry layout fits every later one
     int og = 1;
     const size_t smem_max = fan_tma_smem_bytes(fan_geo_block_layout(P.np_max, true), sizeof(float));
@@ -822,7 +873,7 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
   c->grid_rows = c->n_sm * 16;
   int maxgrid = std::max({c->grid_mv, c->grid_vec, c->grid_ft32, c->grid_geo, c->grid_rows});
   c->partials.alloc((size_t)maxgrid * 4);
-  c->partials_up.alloc((size_t)std::max(c->grid_upd, c->grid_vec) * 2);
+  c->partials_up.alloc((size_t)c->n_sm * 4 * 2);
   c->partials_up.zero(s);
   c->counters.alloc(4);
   c->counters.zero(s);
@@ -1301,8 +1352,7 @@ cfem_status cfem_profile_matvec(cfem_ctx *ctx, int32_t precision, int32_t n_laun
           rows_apply(ctx, ctx->v64.z.p, ctx->tmp64.p);
           continue;
         }
-        MvParams<float> mv = base_mv<float>(ctx);
-        mv.diagA = ctx->v32.diagA.p;
+        MvParams<float> mv = site_mv(ctx, whole_mesh(ctx), 1.f, 0.f, nullptr);
         mv.sc = sc;
         mv.x = ctx->v32.z.p;
         mv.x2 = (i & 1) ? ctx->v32.pB.p : ctx->v32.pA.p;

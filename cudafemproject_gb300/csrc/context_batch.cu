@@ -4,17 +4,17 @@
 // and element arrays are concatenated (instance-major, caller order), the
 // locality renumbering keeps every instance's elements, fans, patches and
 // owned nodes contiguous, and each patch carries its instance's lambda and mu.
-// One solve runs all instances together: every matvec launch covers the
-// patches of all instances (persistent CTAs), every instance has its own PCG
-// scalars and stopping test, and a converged instance is masked out (its
-// patches and nodes are skipped). The iterations replay from a captured CUDA
-// graph; FP32_REFINE adds a per-instance FP64 iterative refinement.
+// One solve runs all instances together, each with its own PCG scalars and
+// stopping test: up to kMaxLoops of them as one graph with a loop of its own per
+// instance, more as launches that cover the patches of all instances
+// (persistent CTAs, a converged instance's patches and nodes skipped), replayed
+// from a captured graph. FP32_REFINE adds a per-instance FP64 iterative
+// refinement.
 #include "context_internal.cuh"
 #include "kernels_aux.cuh"
 
 namespace cfem {
 namespace detail {
-namespace {
 
 struct BatchBufs {
   DBuf<Scalars> isc;
@@ -22,6 +22,21 @@ struct BatchBufs {
   DBuf<double> pe, pp, scratch, rrff, seg;
   DBuf<int> active;
 };
+
+struct BatchState {  // kept with the context
+  BatchBufs bufs;
+  bool tried = false;              // to build the graph of instance loops
+  cudaGraphExec_t loops = nullptr;
+  DBuf<Scalars> sc;                // per instance
+  DBuf<double> part;
+  ~BatchState() {
+    if (loops) cudaGraphExecDestroy(loops);
+  }
+};
+
+void destroy_batch(BatchState *b) { delete b; }
+
+namespace {
 
 template <typename T>
 BatchVecParams<T> vec_params_batch(cfem_ctx *c, BatchBufs &B, int k_active) {
@@ -129,6 +144,85 @@ void run_batch_pcg(cfem_ctx *c, BatchBufs &B, double tol, int rule, int maxit, s
   check_copy_error(c);
   out.resize(c->n_inst);
   CK(cudaMemcpy(out.data(), B.isc.p, sizeof(Scalars) * c->n_inst, cudaMemcpyDeviceToHost));
+}
+
+// The same with every instance's PCG on its own: the kernels of a single mesh on
+// the instance's patches and nodes, each instance a loop of its own in one
+// graph, so that the GPU runs the instances side by side and each stops when it
+// is done. A launch of all instances together costs every iteration of the
+// slowest what the sum of them takes, in kernels that carry every instance's
+// scalars (12 boxes of 6 to 20 elements a side: 119 ms against 63).
+// Up to kMaxLoops instances; more would queue for the GPU's 128
+// concurrent kernels and cost more to build than the shared launches.
+constexpr int kMaxLoops = 64;
+
+PcgSite instance_site(cfem_ctx *c, BatchState &L, int i) {
+  PcgSite S{};
+  S.sc = L.sc.p + i;
+  S.first_patch = c->h_inst_patch_off[i];
+  S.n_patches = c->h_inst_patch_off[i + 1] - S.first_patch;
+  S.first_node = c->h_own_first[S.first_patch];
+  S.n_nodes = c->h_own_first[S.first_patch + S.n_patches] - S.first_node;
+  S.lam = (float)c->inst_lam[i];
+  S.mu = (float)c->inst_mu[i];
+  const size_t n = (size_t)c->n_sm * 4;  // the largest grid of a site's kernels
+  S.partials = L.part.p + (size_t)i * n * 5;
+  S.partials_up = S.partials + n * 3;
+  return S;
+}
+
+// Builds the graph once per context; false where the runtime does not.
+bool build_loops(cfem_ctx *c) {
+  BatchState &L = *c->batch;
+  if (L.tried) return L.loops != nullptr;
+  L.tried = true;
+  if (c->host_loop || c->n_inst > kMaxLoops) return false;
+  L.sc.alloc(c->n_inst);
+  L.part.alloc((size_t)c->n_inst * c->n_sm * 4 * 5);
+  L.part.zero(c->stream);
+  cudaGraph_t graph = nullptr;
+  const int64_t before = c->launches;
+  bool ok = cudaGraphCreate(&graph, 0) == cudaSuccess;
+  Vecs<float> &V = c->v32;
+  for (int i = 0; ok && i < c->n_inst; ++i) {
+    const PcgSite S = instance_site(c, L, i);
+    const MvParams<float> mv = site_mv(c, S, 1.f, 0.f, nullptr);
+    ok = add_loop(
+        c, graph, 0,
+        [&](cudaGraphConditionalHandle cond) {
+          VecParams<float> P = vec_params(c, S, V.pA.p, V.u.p);
+          P.cond = cond;
+          launch_init(c, P, 0);
+        },
+        [&](cudaGraphConditionalHandle cond) { capture_iterations(c, S, mv, c->chunk, cond); });
+  }
+  if (ok) ok = cudaGraphInstantiate(&L.loops, graph, 0) == cudaSuccess;
+  if (graph) cudaGraphDestroy(graph);
+  if (!ok) L.loops = nullptr;
+  (void)cudaGetLastError();
+  c->launches = before;
+  return ok;
+}
+
+void run_loops(cfem_ctx *c, double tol, int rule, int maxit, std::vector<Scalars> &out) {
+  BatchState &L = *c->batch;
+  std::vector<Scalars> h(c->n_inst);
+  for (auto &s : h) {
+    s = Scalars{};
+    s.tol = tol;
+    s.rule = rule;
+    s.maxit = maxit > 0 ? maxit : 1000000;
+  }
+  CK(cudaMemcpyAsync(L.sc.p, h.data(), sizeof(Scalars) * h.size(), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaGraphLaunch(L.loops, c->stream));
+  out.resize(c->n_inst);
+  CK(cudaMemcpyAsync(out.data(), L.sc.p, sizeof(Scalars) * c->n_inst, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  check_copy_flag(c);
+  for (const Scalars &s : out) {
+    c->launches += 1 + (int64_t)2 * c->chunk * s.loops;
+    if (!s.done) throw Fail{CFEM_ERR_CUDA, "batched PCG recurrence stopped advancing on the device"};
+  }
 }
 
 // r64 = f64 - tmp64 per instance; f32 = r64 on active instances, 0 elsewhere;
@@ -263,18 +357,19 @@ extern "C" cfem_status cfem_batch_static_solve(cfem_ctx *ctx, const cfem_solve_p
       throw Fail{CFEM_ERR_UNSUPPORTED, "batched solves run in CFEM_FP32 or CFEM_FP32_REFINE"};
     cfem_ctx *c = ctx;
     const int n = c->n_inst;
-    BatchBufs B;
-    B.isc.alloc(n);
-    B.ctl.alloc(1);
-    B.pe.alloc(c->prep.n_patches);
-    B.pp.alloc((size_t)c->prep.n_patches * 3);
-    B.seg.alloc((size_t)flat_grid(c) * n * 3);
+    if (!c->batch) c->batch = new BatchState();
+    BatchBufs &B = c->batch->bufs;
+    B.isc.ensure(n);
+    B.ctl.ensure(1);
+    B.pe.ensure(c->prep.n_patches);
+    B.pp.ensure((size_t)c->prep.n_patches * 3);
+    B.seg.ensure((size_t)flat_grid(c) * n * 3);
     if (flat_smem(c) > 48 * 1024)
       CK(cudaFuncSetAttribute((const void *)k_batch_vec_flat<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)flat_smem(c)));
-    B.scratch.alloc((size_t)n * 3);
-    B.rrff.alloc((size_t)n * 2);
-    B.active.alloc(n);
+    B.scratch.ensure((size_t)n * 3);
+    B.rrff.ensure((size_t)n * 2);
+    B.active.ensure(n);
     c->launches = 0;
     set_diag_vectors(c);
     RhsSchedule sch;
@@ -288,10 +383,15 @@ extern "C" cfem_status cfem_batch_static_solve(cfem_ctx *ctx, const cfem_solve_p
     std::vector<double> rr, ff, rr_prev(n, -1), g0(n, 0), g1(n, 0);
     std::vector<int> stalls(n, 0);
     std::vector<Scalars> res;
+    const bool loops = build_loops(c);
+    auto run_pcgs = [&](std::vector<Scalars> &r) {
+      if (loops) run_loops(c, p.tol, p.stop_rule, p.max_iter, r);
+      else run_batch_pcg(c, B, p.tol, p.stop_rule, p.max_iter, r);
+    };
     if (p.precision == CFEM_FP32) {
       k_convert<double, float><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->v64.f.p, c->v32.f.p);
       CKL();
-      run_batch_pcg(c, B, p.tol, p.stop_rule, p.max_iter, res);
+      run_pcgs(res);
       for (int i = 0; i < n; ++i) {
         iters[i] = res[i].iter;
         g0[i] = res[i].gamma0;
@@ -327,7 +427,7 @@ extern "C" cfem_status cfem_batch_static_solve(cfem_ctx *ctx, const cfem_solve_p
           std::vector<double> rr2, ff2;
           batch_residual(c, B, act, rr2, ff2);
         }
-        run_batch_pcg(c, B, p.tol, p.stop_rule, p.max_iter, res);
+        run_pcgs(res);
         for (int i = 0; i < n; ++i) {
           if (!act[i]) continue;
           iters[i] += res[i].iter;

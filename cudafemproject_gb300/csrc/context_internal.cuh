@@ -28,6 +28,8 @@ extern thread_local std::string g_last_error;
 
 struct MultiState;                    // multi-RHS work arrays (context_multi.cu)
 void destroy_multi(MultiState *m);
+struct BatchState;                    // batched solves (context_batch.cu)
+void destroy_batch(BatchState *b);
 
 struct Fail {
   cfem_status st;
@@ -142,7 +144,6 @@ struct cfem_ctx {
   bool own_stream = false;
   cudaEvent_t ev_in = nullptr;
   int device = 0, n_sm = 0, l2_bytes = 0;
-  int grid_upd = 0;  // PCG update kernel (3D)
   int dim = 0, nv = 0, w = 0, vw = 0, ncomp = 0;
   int64_t nn = 0, ne = 0, nd = 0, nvec = 0;
   int semantics = 0, form = CFEM_FORM_GRADIENT, verbose = 0;
@@ -208,12 +209,14 @@ struct cfem_ctx {
   // inside a graph WHILE node (CFEM_HOST_LOOP set in the environment)
   bool host_loop = std::getenv("CFEM_HOST_LOOP") != nullptr;
   MultiState *multi = nullptr;
+  BatchState *batch = nullptr;
   // batch of independent meshes (cfem_create_batch); n_inst == 0 for one mesh
   int n_inst = 0;
   std::vector<int32_t> elem_group;               // caller element -> instance
   std::vector<double> inst_lam, inst_mu;
   std::vector<int64_t> inst_node_off, inst_elem_off;  // caller order
   DBuf<int32_t> patch_inst, inst_patch_off, own_first;
+  std::vector<int32_t> h_inst_patch_off, h_own_first;
   DBuf<float> pmat32;
   DBuf<double> lam_e, mu_e;
   int64_t launches = 0;  // kernels issued since the counter was last reset
@@ -231,6 +234,7 @@ struct cfem_ctx {
     if (h_rr) cudaFreeHost(h_rr);
     if (h_tma_err) cudaFreeHost(h_tma_err);
     if (multi) destroy_multi(multi);
+    if (batch) destroy_batch(batch);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (ev_in) cudaEventDestroy(ev_in);
@@ -263,8 +267,23 @@ MvParams<float> base_mv_f(cfem_ctx *c);
 void launch_mv_f(cfem_ctx *c, int mode, const MvParams<float> &P);
 PcgResult run_pcg_d(cfem_ctx *c, Vecs<double> &V, double cK, double cM, const double *mcoef, int warm, double tol,
                     int rule, int maxit);
-PcgResult run_pcg_f(cfem_ctx *c, Vecs<float> &V, float cK, float cM, const float *mcoef, int warm, double tol,
-                    int rule, int maxit);
+PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
+                    const float *cont_p = nullptr, double cont_gamma_prev = 0,
+                    const std::function<void()> &then = nullptr);
+struct PcgSite {
+  Scalars *sc;
+  int first_patch, n_patches;
+  int64_t first_node, n_nodes;
+  float lam, mu;
+  double *partials, *partials_up;  // [matvec and init grid][3], [update grid][2]
+};
+VecParams<float> vec_params(cfem_ctx *c, const PcgSite &S, float *p, float *u);
+MvParams<float> site_mv(cfem_ctx *c, const PcgSite &S, float cK, float cM, const float *mcoef);
+void launch_init(cfem_ctx *c, const VecParams<float> &P, int warm);
+void capture_iterations(cfem_ctx *c, const PcgSite &S, const MvParams<float> &mv, int chunk, unsigned long long cond);
+bool add_loop(cfem_ctx *c, cudaGraph_t graph, unsigned initial,
+              const std::function<void(cudaGraphConditionalHandle)> &prologue,
+              const std::function<void(cudaGraphConditionalHandle)> &capture);
 void to_internal_d(cfem_ctx *c, const double *src, double *dst);
 void to_caller_d(cfem_ctx *c, const double *src, double *dst);
 void to_caller_f(cfem_ctx *c, const float *src, double *dst);
@@ -327,7 +346,7 @@ inline MvParams<T> base_mv(cfem_ctx *c) {
 template <typename T>
 inline PcgResult run_pcg(cfem_ctx *c, Vecs<T> &V, T cK, T cM, const T *mcoef, int warm, double tol, int rule, int maxit) {
   if constexpr (sizeof(T) == 8) return run_pcg_d(c, V, cK, cM, mcoef, warm, tol, rule, maxit);
-  else return run_pcg_f(c, V, cK, cM, mcoef, warm, tol, rule, maxit);
+  else return run_pcg_f(c, cK, cM, mcoef, warm, tol, rule, maxit);
 }
 template <typename T>
 inline void to_internal(cfem_ctx *c, const double *src, T *dst) {

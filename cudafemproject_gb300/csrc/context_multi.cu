@@ -199,7 +199,7 @@ struct MultiCont {
 // Multi-RHS FP32 PCG on M.f (cases >= k_active are padding). Returns after
 // every case has stopped; per-case results in M.h_sc. With `cont`, cases with
 // a previous run start from the conjugate-gradient step off its last direction
-// (z_c + gamma_c / gamma_prev_c p_last_c), as run_pcg_t does for one case.
+// (z_c + gamma_c / gamma_prev_c p_last_c), as run_pcg_f does for one case.
 void run_pcg_multi(cfem_ctx *c, MultiState &M, int k_active, double tol, int rule, int maxit,
                    const MultiCont *cont = nullptr) {
   MultiCtl h{};

@@ -515,6 +515,8 @@ struct BatchCtl {
 template <typename T>
 struct MvParams {
   int n_patches;
+  int instance;      // one instance of a batch: patches first_patch .. first_patch + n_patches - 1
+  int first_patch;   // of the context's patches (an instance of a batch; its blocks start there)
   const int32_t *elem_off, *node_off, *nodes, *own;
   const uint2 *lconn;
   const uint8_t *bits;
@@ -757,7 +759,8 @@ struct VecParams {
 // of the x DOF, r.w of the y DOF, z.w (and so p.w, which the matvec copies
 // from z) of the z DOF. Every kernel that reads these vectors for their
 // values uses only the first three lanes.
-template <typename T, int DIM>
+// LOOP: also sets the condition of the graph loop that follows it.
+template <typename T, int DIM, bool LOOP = false>
 __global__ void __launch_bounds__(kThreads) k_pcg_init(VecParams<T> P, int warm) {
   constexpr int VW = DIM == 3 ? 4 : 2;
   DotAcc<T> acc[3];  // r.z, r.r, f.f
@@ -814,6 +817,7 @@ __global__ void __launch_bounds__(kThreads) k_pcg_init(VecParams<T> P, int warm)
     if (s->rule == 1 && acc[1] <= s->rr_stop) done = 1;
     if (!isfinite(acc[0])) done = 2;
     s->done = done;
+    if constexpr (LOOP) cudaGraphSetConditional(P.cond, done == 0 ? 1u : 0u);
   }
 }
 

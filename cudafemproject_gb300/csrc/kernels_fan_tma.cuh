@@ -205,7 +205,9 @@ template <typename T, int MODE, bool GEO = false, bool MASS = false, bool BATCH 
 __global__ void __launch_bounds__(kHfanThreads, 3) k_matvec_fan_tma(MvParams<T> P, FanTmaParams F) {
   static_assert(sizeof(T) == 4, "patch blocks are FP32");
   constexpr int DIM = 3, VW = 4;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
+  // (16 bytes suffice for the bulk copies; 128 would pad the static part by 112
+  // bytes, which costs meshes with about 290 nodes per patch the third CTA per SM)
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const FanBlockLayout &L = F.L;
   unsigned char *buf0 = smem_raw, *buf1 = smem_raw + L.bytes;
   unsigned char *tail = smem_raw + 2 * (size_t)L.bytes;

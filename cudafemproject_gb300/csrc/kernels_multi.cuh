@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kHfanThreads, C <= 2 ? 3 : 2) k_matvec_multi(M
   constexpr int ROUNDS = kHfanThreads / (NW * HPW);
   constexpr int SU = C <= 2 ? 2 : 4;             // staging items in flight per thread
   static_assert(C == 2 || C == 4 || C == 8, "C: 2, 4 or 8 cases per item");
-  extern __shared__ __align__(128) unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const FanBlockLayout &L = P.F.L;
   const int K = P.K, NC = K / C;
   const MultiSmem S = multi_smem(L, C, K);

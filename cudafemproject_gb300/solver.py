@@ -307,7 +307,7 @@ class FemContext:
 
 class BatchContext:
     """Independent 3D meshes, each with its own material, solved together
-    (cfem_create_batch): one set of kernel launches for all instances, with a
+    (cfem_create_batch): all instances in the same graph launches, with a
     per-instance stopping test. ``problems`` is a list of Problem."""
 
     def __init__(self, problems, semantics: str = "consistent", stream=None, patch_elems: int = 0,

@@ -270,9 +270,10 @@ CFEM_API cfem_status cfem_create_batch(cfem_ctx **out, int32_t n, const cfem_mes
  * the concatenated caller order. */
 CFEM_API cfem_status cfem_batch_info(const cfem_ctx *ctx, int32_t *n, int64_t *node_off, int64_t *elem_off);
 /* Static solve of every instance under its own loads, all instances in the
- * same kernel launches with per-instance PCG scalars and stopping tests (a
- * converged instance is skipped). prm->precision CFEM_FP32 or CFEM_FP32_REFINE
- * (per-instance FP64 refinement). u: concatenated displacements (n_dof of all
+ * same graph launch (up to 64 side by side, each in a loop of its own; more in
+ * shared kernel launches) with per-instance PCG scalars and stopping tests (a
+ * converged instance takes no further part). prm->precision CFEM_FP32 or
+ * CFEM_FP32_REFINE (per-instance FP64 refinement). u: concatenated displacements (n_dof of all
  * instances); info: NULL or [n]. */
 CFEM_API cfem_status cfem_batch_static_solve(cfem_ctx *ctx, const cfem_solve_params *prm, double *u,
                                              cfem_solve_info *info);

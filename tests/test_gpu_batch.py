@@ -50,3 +50,24 @@ def test_batch_context_rejects_single_mesh_calls():
     assert st == capi.ERR_UNSUPPORTED
     with pytest.raises(capi.CfemError):
         b.static_solve("fp64")
+
+
+@pytest.mark.parametrize("side_by_side", [True, False])
+@pytest.mark.parametrize("boxes", [1, 4])
+def test_batch_loops_and_shared_launches(monkeypatch, side_by_side, boxes):
+    """Both ways of running the instances' PCG: a graph loop per instance, and
+    launches shared by all (where the graph is not built), twice on one context
+    (the graph is kept)."""
+    from cudafemproject_gb300.solver import BatchContext
+    if side_by_side:
+        monkeypatch.delenv("CFEM_HOST_LOOP", raising=False)
+    else:
+        monkeypatch.setenv("CFEM_HOST_LOOP", "1")
+    probs = [p for i, p in enumerate(_boxes()) if i != 2][:boxes]
+    b = BatchContext(probs)
+    for tol in (1e-4, 0.3):
+        us, infos = b.static_solve("fp32_refine", tol=tol, outer_tol=1e-11)
+        for i, p in enumerate(probs):
+            xo, _ = O.Oracle(p, consistent=True).static(tol=1e-14, rule=1)
+            assert infos[i]["status"] == 0
+            assert rel(us[i], xo) <= 1e-8, (i, tol)
