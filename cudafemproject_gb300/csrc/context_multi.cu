@@ -4,13 +4,14 @@
 // every matvec streams the patch blocks once for all cases of a batch (at most
 // kMaxCases), each case keeps its own scalars and stopping test, and FP32_REFINE
 // wraps it in an FP64 iterative refinement whose true residuals f_c - K x_c are
-// formed case by case with the FP64 operator. Other forms and FP64 solve the
+// formed for all cases in one kernel on the FP64 rows. Other forms and FP64 solve the
 // cases one after the other.
 #include <chrono>
 #include <cstdlib>
 
 #include "context_internal.cuh"
 #include "kernels_aux.cuh"
+#include "rows_op.cuh"
 
 namespace cfem {
 namespace detail {
@@ -19,11 +20,8 @@ struct MultiState {
   int K = 0, C = 0;  // cases per solve (power of two), cases per matvec item
   DBuf<float> x, r, z, pA, pB, u, f;  // [node][K][4]
   DBuf<double> x64, f64, r64, io;     // [node][K][4]; io: caller-order staging
-  DBuf<double> s_f, s_x, s_r;         // one case in the single-RHS layout
   DBuf<MultiScalars> sc;
   DBuf<MultiCtl> ctl;
-  DBuf<double> partials, gpart;
-  DBuf<unsigned> gcnt;  // group tickets: [0, n) matvec, [n, 2n) vector kernel
   DBuf<int> active;
   DBuf<double> res_norms;  // [K][2] ||r_c||^2, ||f_c||^2 of the FP64 true residuals
   DBuf<float> fold_beta;  // [K] continuation of the next run: z_c += beta_c p_last_c
@@ -33,6 +31,9 @@ struct MultiState {
   int grid_mv = 0, grid_vec = 0;
   size_t smem = 0;
   cudaGraphExec_t graph = nullptr;
+  bool device_loop = false;  // graph is a WHILE node around the iterations
+  // (a case's flags of the two parities differ only while it is running)
+  int done_of(int cs) const { return std::max(h_sc[cs].done[0], h_sc[cs].done[1]); }
   ~MultiState() {
     if (graph) cudaGraphExecDestroy(graph);
     if (h_ctl) cudaFreeHost(h_ctl);
@@ -80,10 +81,6 @@ MultiParams<float> multi_params(cfem_ctx *c, MultiState &M) {
   P.n_nodes = c->nn;
   P.sc = M.sc.p;
   P.ctl = M.ctl.p;
-  P.partials = M.partials.p;
-  P.gpart = M.gpart.p;
-  P.gcnt_mv = M.gcnt.p;
-  P.gcnt_up = M.gcnt.p + M.gcnt.n / 2;
   P.F.blocks = c->blk32.p;
   P.F.L = c->L32;
   P.F.fan_off = c->fan_off.p;
@@ -110,6 +107,7 @@ bool configure_c(cfem_ctx *c, MultiState &M, int C) {
   if (M.graph) {
     cudaGraphExecDestroy(M.graph);
     M.graph = nullptr;
+    M.device_loop = false;
   }
   return true;
 }
@@ -158,7 +156,6 @@ MultiState &multi_state(cfem_ctx *c, int K) {
   }
   for (auto *b : {&M->x64, &M->f64, &M->r64}) b->alloc(n);
   M->io.alloc((size_t)K * c->nd);
-  for (auto *b : {&M->s_f, &M->s_x, &M->s_r}) b->alloc(c->nvec);
   M->sc.alloc(K);
   M->sc.zero(c->stream);
   M->ctl.alloc(1);
@@ -172,19 +169,15 @@ MultiState &multi_state(cfem_ctx *c, int K) {
   // four items per thread per round: two CTAs per SM keep enough loads in flight
   M->grid_vec = (int)std::min<int64_t>(std::max<int64_t>(1, (int64_t)(((size_t)c->nn * K + kThreads - 1) / kThreads)),
                                        (int64_t)c->n_sm * 2);
-  const int max_mv_grid = c->n_sm * 8;
-  const int max_grid = std::max(max_mv_grid, M->grid_vec);
-  M->partials.alloc((size_t)max_grid * K * 3);
-  const int max_groups = (max_grid + kSumGroup - 1) / kSumGroup;
-  M->gpart.alloc((size_t)max_groups * K * 3);
-  M->gcnt.alloc((size_t)2 * max_groups);
-  M->gcnt.zero(c->stream);
   return *M;
 }
 
 void launch_vec(cfem_ctx *c, MultiState &M, const MultiParams<float> &P, const float *p, int init) {
-  k_pcg_multi_vec<float><<<M.grid_vec, kThreads, 0, c->stream>>>(P, M.x.p, M.r.p, M.z.p, p, M.u.p, M.f.p,
-                                                                  c->v32.dinv.p, init);
+  auto go = [&](auto k) {
+    k<<<M.grid_vec, kThreads, 0, c->stream>>>(P, M.x.p, M.r.p, M.z.p, p, M.u.p, M.f.p, c->v32.dinv.p, init);
+  };
+  if (P.cond) go(k_pcg_multi_vec<float, true>);
+  else go(k_pcg_multi_vec<float>);
   CKL();
   c->launches += 1;
 }
@@ -208,9 +201,11 @@ void run_pcg_multi(cfem_ctx *c, MultiState &M, int k_active, double tol, int rul
   h.maxit = maxit > 0 ? maxit : 1000000;
   h.k_active = k_active;
   CK(cudaMemcpyAsync(M.ctl.p, &h, sizeof(MultiCtl), cudaMemcpyHostToDevice, c->stream));
-  M.gcnt.zero(c->stream);  // (tickets of a launch that stopped early are not left behind)
+  M.sc.zero(c->stream);
   MultiParams<float> P = multi_params(c, M);
   launch_vec(c, M, P, nullptr, 1);
+  k_multi_start<<<1, kMaxCases, 0, c->stream>>>(M.sc.p, M.ctl.p, M.K);
+  CKL();
   if (cont) {
     CK(cudaMemcpyAsync(M.h_sc.data(), M.sc.p, sizeof(MultiScalars) * M.K, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -218,7 +213,7 @@ void run_pcg_multi(cfem_ctx *c, MultiState &M, int k_active, double tol, int rul
     std::vector<int> par(M.K, 0);
     bool any = false;
     for (int cs = 0; cs < M.K && cs < (int)cont->iters.size(); ++cs) {
-      if (M.h_sc[cs].done || cont->iters[cs] <= 0 || !(cont->gamma_prev[cs] > 0)) continue;
+      if (M.h_sc[cs].done[0] || cont->iters[cs] <= 0 || !(cont->gamma_prev[cs] > 0)) continue;
       beta[cs] = (float)(M.h_sc[cs].gamma / cont->gamma_prev[cs]);
       par[cs] = (cont->iters[cs] - 1) & 1;
       any = true;
@@ -234,27 +229,46 @@ void run_pcg_multi(cfem_ctx *c, MultiState &M, int k_active, double tol, int rul
     }
   }
   if (!M.graph) {
-    cudaGraph_t graph;
     const int64_t before = c->launches;
-    CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    try {
+    auto iterations = [&](unsigned long long cond) {
+      MultiParams<float> Q = P;
       for (int it = 0; it < c->chunk; ++it) {
         float *pold = (it & 1) ? M.pB.p : M.pA.p;
         float *pnew = (it & 1) ? M.pA.p : M.pB.p;
-        launch_mvm_c(c, M, MV_PCG, P, M.z.p, pold, pnew, M.u.p);
-        launch_vec(c, M, P, pnew, 0);
+        Q.parity = it & 1;
+        Q.cond = cond;
+        Q.cond_role = (it == 0 ? 1 : 0) | (it == c->chunk - 1 ? 2 : 0);
+        Q.cond_chunk = c->chunk;
+        launch_mvm_c(c, M, MV_PCG, Q, M.z.p, pold, pnew, M.u.p);
+        launch_vec(c, M, Q, pnew, 0);
       }
-    } catch (...) {
-      cudaGraph_t broken = nullptr;
-      cudaStreamEndCapture(c->stream, &broken);
-      if (broken) cudaGraphDestroy(broken);
+    };
+    if (!c->host_loop) {
+      cudaGraph_t graph = nullptr;
+      M.device_loop = cudaGraphCreate(&graph, 0) == cudaSuccess &&
+                      add_loop(c, graph, 1, nullptr, [&](cudaGraphConditionalHandle cond) { iterations(cond); }) &&
+                      cudaGraphInstantiate(&M.graph, graph, 0) == cudaSuccess;
+      if (graph) cudaGraphDestroy(graph);
+      if (!M.device_loop) M.graph = nullptr;
       (void)cudaGetLastError();
-      throw;
     }
-    CK(cudaStreamEndCapture(c->stream, &graph));
+    if (!M.graph) {
+      cudaGraph_t graph;
+      CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+      try {
+        iterations(0);
+      } catch (...) {
+        cudaGraph_t broken = nullptr;
+        cudaStreamEndCapture(c->stream, &broken);
+        if (broken) cudaGraphDestroy(broken);
+        (void)cudaGetLastError();
+        throw;
+      }
+      CK(cudaStreamEndCapture(c->stream, &graph));
+      CK(cudaGraphInstantiate(&M.graph, graph, 0));
+      cudaGraphDestroy(graph);
+    }
     c->launches = before;
-    CK(cudaGraphInstantiate(&M.graph, graph, 0));
-    cudaGraphDestroy(graph);
   }
   const int64_t max_launches = (int64_t)h.maxit / c->chunk + 16;
   int last_iter = -1, stalled = 0;
@@ -264,10 +278,14 @@ void run_pcg_multi(cfem_ctx *c, MultiState &M, int k_active, double tol, int rul
       throw Fail{CFEM_ERR_CUDA, "multi-RHS PCG recurrence stopped advancing on the device"};
     }
     CK(cudaGraphLaunch(M.graph, c->stream));
-    c->launches += 2 * c->chunk;
     CK(cudaMemcpyAsync(M.h_ctl, M.ctl.p, sizeof(MultiCtl), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    c->launches += (int64_t)2 * c->chunk * (M.device_loop ? M.h_ctl->loops : 1);
     if (M.h_ctl->all_done) break;
+    if (M.device_loop) {
+      check_copy_flag(c);
+      throw Fail{CFEM_ERR_CUDA, "multi-RHS PCG recurrence stopped advancing on the device"};
+    }
     stalled = M.h_ctl->iter == last_iter ? stalled + 1 : 0;
     last_iter = M.h_ctl->iter;
   }
@@ -314,20 +332,23 @@ cfem_status solve_batch(cfem_ctx *c, const cfem_solve_params &p, int kb, const d
   std::vector<double> norms(2 * (size_t)kb, 0.0);
   auto residuals = [&](bool all) {
     // r_c = f_c - K' x_c in FP64 with ||r_c||^2 and ||f_c||^2 for the cases
-    // still running (all: every case), all queued on the stream and read back once
+    // still running (all: every case), in one kernel
     auto wanted = [&](int cs) { return all || (status[cs] != CFEM_OK && status[cs] != CFEM_ERR_DIVERGED); };
-    int queued = 0;
-    for (int cs = 0; cs < kb; ++cs) {
-      if (!wanted(cs)) continue;
-      k_case_copy<double, double><<<nblk(nn), kThreads, 0, c->stream>>>(nn, K, cs, M.f64.p, M.s_f.p, 1);
-      k_case_copy<double, double><<<nblk(nn), kThreads, 0, c->stream>>>(nn, K, cs, M.x64.p, M.s_x.p, 1);
-      CKL();
-      true_residual_async(c, M.s_f.p, M.s_x.p, M.s_r.p, nullptr, M.res_norms.p + 2 * cs);
-      k_case_copy<double, double><<<nblk(nn), kThreads, 0, c->stream>>>(nn, K, cs, M.s_r.p, M.r64.p, 0);
-      CKL();
-      ++queued;
-    }
-    if (!queued) return;
+    std::vector<int> skip(K, 1);
+    bool any = false;
+    for (int cs = 0; cs < kb; ++cs)
+      if (wanted(cs)) {
+        skip[cs] = 0;
+        any = true;
+      }
+    if (!any) return;
+    CK(cudaMemcpyAsync(M.active.p, skip.data(), sizeof(int) * K, cudaMemcpyHostToDevice, c->stream));
+    M.res_norms.zero(c->stream);
+    RowsCases P{op_of(c, c->rows.K), K, M.f64.p, M.x64.p, M.r64.p, M.res_norms.p, M.active.p};
+    const int64_t items = P.A.n_slices * kSliceRows * K;
+    k_rows_cases_residual<<<(unsigned)std::min<int64_t>(nblk(items), (int64_t)c->n_sm * 4), kThreads, 0, c->stream>>>(P);
+    CKL();
+    c->launches += 1;
     CK(cudaMemcpyAsync(norms.data(), M.res_norms.p, sizeof(double) * 2 * kb, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     check_copy_error(c);
@@ -345,7 +366,7 @@ cfem_status solve_batch(cfem_ctx *c, const cfem_solve_params &p, int kb, const d
       iters[cs] = M.h_sc[cs].iters;
       gamma0[cs] = M.h_sc[cs].gamma0;
       gamma[cs] = M.h_sc[cs].gamma;
-      status[cs] = status_of(M.h_sc[cs].done);
+      status[cs] = status_of(M.done_of(cs));
     }
     k_convert<float, double><<<nblk(nitems * 4), kThreads, 0, c->stream>>>(nitems * 4, M.x.p, M.x64.p);
     CKL();
@@ -383,14 +404,14 @@ cfem_status solve_batch(cfem_ctx *c, const cfem_solve_params &p, int kb, const d
       run_pcg_multi(c, M, kb, p.tol, p.stop_rule, p.max_iter, continued ? &cont : nullptr);
       for (int cs = 0; cs < kb; ++cs) {
         if (!act[cs]) continue;
-        const int d = M.h_sc[cs].done;
+        const int d = M.done_of(cs);
         cont.iters[cs] = d == 1 || d == 3 ? M.h_sc[cs].iters : 0;
         cont.gamma_prev[cs] = M.h_sc[cs].gamma_prev;
         iters[cs] += M.h_sc[cs].iters;
         if (outer[cs] == 0) gamma0[cs] = M.h_sc[cs].gamma0;
         gamma[cs] = M.h_sc[cs].gamma;
         outer[cs] += 1;
-        if (M.h_sc[cs].done == 2) status[cs] = CFEM_ERR_DIVERGED;
+        if (M.done_of(cs) == 2) status[cs] = CFEM_ERR_DIVERGED;
         rr_prev[cs] = rr[cs];
       }
       k_multi_accumulate<<<nblk(nitems * 4), kThreads, 0, c->stream>>>(nitems * 4, M.x.p, M.x64.p);

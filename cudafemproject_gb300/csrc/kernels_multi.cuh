@@ -17,18 +17,31 @@
 namespace cfem {
 
 constexpr int kMaxCases = 256;
-constexpr int kSumGroup = 16;  // blocks per group of the first level of the per-case grid sums
 
-struct MultiScalars {  // per case
+// Scalars of a case. The two kernels of an iteration pass their per-case sums
+// on as FP64 atomic additions and every CTA of the kernel behind derives what
+// it needs from them (no last-block phase: its two levels of ticket, fences and
+// serial FP64 additions took most of an iteration of few cases). A kernel reads
+// only what the kernel before it wrote; CTA 0 publishes:
+//   matvec of iteration `it` (parity q = it & 1): reads sum_b[q ^ 1], alpha,
+//     inv_gamma, done[q ^ 1], ctl->iter; writes gamma, gamma_prev, beta, rr,
+//     iters, done[q], ctl->all_done; empties sum_b[q]; adds p.Ap to sum_a[q];
+//   vector kernel: reads sum_a[q], gamma, done[q], ctl->all_done; writes sigma,
+//     alpha, inv_gamma, ctl->iter; empties sum_a[q ^ 1]; adds r.z, r.r to sum_b[q].
+struct MultiScalars {
   double gamma, gamma_prev, gamma0, sigma, alpha, beta, rr, ff;
-  int done, iters;  // done: 0 running, 1 converged, 2 diverged, 3 iteration cap
+  double gamma_stop, rr_stop, inv_gamma;  // tol gamma0, (tol ||f||)^2, 1 / gamma
+  double sum_a[2], sum_b[2][2];
+  int done[2], iters;  // done: 0 running, 1 converged, 2 diverged, 3 iteration cap
+  int pad;
 };
 
 struct MultiCtl {  // shared by the cases of one solve
   double tol;
   int rule, maxit, iter, all_done;
   int k_active;     // cases 0..k_active-1 are real, the rest are padding
-  unsigned int count_mv, count_up;
+  int loops;        // graph loop: bodies started in this run
+  int loop_ok, pad;
 };
 
 template <typename T>
@@ -41,9 +54,9 @@ struct MultiParams {
   int64_t n_nodes;
   MultiScalars *sc;     // [K]
   MultiCtl *ctl;
-  double *partials;     // [grid][K] (matvec) / [grid][K][3] (vector kernels)
-  double *gpart;        // [grid / kSumGroup][K][3] group sums of the partials
-  unsigned *gcnt_mv, *gcnt_up;  // [grid / kSumGroup] group tickets of the matvec / vector kernel
+  int parity;           // of the iteration
+  unsigned long long cond;  // iterations inside a graph loop (0: host loop), see k_pcg_update
+  int cond_role, cond_chunk;
   FanTmaParams F;       // patch blocks (layout and fan offsets)
 };
 
@@ -66,59 +79,6 @@ __host__ __device__ inline MultiSmem multi_smem(const FanBlockLayout &L, int C, 
   m.done = off; off += K * 4;
   m.bytes = off;
   return m;
-}
-
-// Per-case grid sums in two fixed-order levels. Every block calls it (all
-// threads) once its partials part[(b * K + c) * NQ + k] are written. The last
-// block of each group of kSumGroup blocks adds the group's partials in block
-// order into gpart[(g * K + c) * NQ + k]; the last of those group finishers
-// adds the groups in group order into out[c * NQ + k] (shared memory) and
-// returns true there, false everywhere else (uniform per block). Each level
-// is one round of independent loads per sum instead of a chain over all blocks.
-// The tickets return to zero for the next launch.
-template <int NQ>
-__device__ __forceinline__ bool tree_case_sums(const double *part, double *gpart, unsigned *gcnt, unsigned *top, int K,
-                                               double *out) {
-  __shared__ bool s_last;
-  const int n = K * NQ;
-  const int g = blockIdx.x / kSumGroup, ng = (gridDim.x + kSumGroup - 1) / kSumGroup;
-  const int b0 = g * kSumGroup, nb = min(kSumGroup, (int)gridDim.x - b0);
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(&gcnt[g], 1u) == (unsigned)(nb - 1);
-  __syncthreads();
-  if (!s_last) return false;
-  __threadfence();
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    double v[kSumGroup];
-#pragma unroll
-    for (int q = 0; q < kSumGroup; ++q) v[q] = q < nb ? __ldcg(part + (size_t)(b0 + q) * n + j) : 0.0;
-    double t = 0;
-#pragma unroll
-    for (int q = 0; q < kSumGroup; ++q) t += v[q];
-    gpart[(size_t)g * n + j] = t;
-  }
-  if (threadIdx.x == 0) gcnt[g] = 0;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(top, 1u) == (unsigned)(ng - 1);
-  __syncthreads();
-  if (!s_last) return false;
-  __threadfence();
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    double t = 0;
-    for (int g0 = 0; g0 < ng; g0 += kSumGroup) {
-      double v[kSumGroup];
-#pragma unroll
-      for (int q = 0; q < kSumGroup; ++q) v[q] = g0 + q < ng ? __ldcg(gpart + (size_t)(g0 + q) * n + j) : 0.0;
-#pragma unroll
-      for (int q = 0; q < kSumGroup; ++q) t += v[q];
-    }
-    out[j] = t;
-  }
-  if (threadIdx.x == 0) *top = 0;
-  __syncthreads();
-  return true;
 }
 
 // y_c += K' p_c for the K cases. PCG (MODE MV_PCG): p_c = z_c + beta_c p_old_c
@@ -152,22 +112,49 @@ __global__ void __launch_bounds__(kHfanThreads, C <= 2 ? 3 : 2) k_matvec_multi(M
   T *fs = reinterpret_cast<T *>(smem_raw + S.fs);
   T *s_beta = reinterpret_cast<T *>(smem_raw + S.beta);
   int *s_done = reinterpret_cast<int *>(smem_raw + S.done);
-  if (MODE == MV_PCG) {  // (thread 0 reads the shared flag, see k_pcg_multi_vec)
-    if (threadIdx.x == 0) s_done[0] = P.ctl->all_done;
-    __syncthreads();
-    const bool all = s_done[0] != 0;
-    __syncthreads();
-    if (all) return;
-  }
+  const int q = P.parity;
   for (int c = threadIdx.x; c < K; c += blockDim.x) {
     s_en[c] = 0;
     s_done[c] = 0;
     s_beta[c] = 0;
-    if (MODE == MV_PCG) {
-      const MultiScalars &sc = P.sc[c];
-      s_done[c] = sc.done;
-      s_beta[c] = sc.done ? T(0) : (T)sc.beta;
+  }
+  if (MODE == MV_PCG) {
+    // every CTA: beta and the stopping tests from the update's sums (one thread
+    // per case; K is at most the block size)
+    bool stop = true;
+    if (threadIdx.x < K) {
+      const int c = threadIdx.x;
+      MultiScalars &m = P.sc[c];
+      const int it = P.ctl->iter;
+      int done = m.done[q ^ 1];
+      double b = 0;
+      if (!done && it > 0) {
+        const double g = m.sum_b[q ^ 1][0], rr = m.sum_b[q ^ 1][1];
+        const int rule = P.ctl->rule;
+        const double v = rule == 0 ? g : rr, limit = rule == 0 ? m.gamma_stop : m.rr_stop;
+        if (!finite_bits(g) || !finite_bits(m.alpha)) done = 2;
+        else if (rule == 0 ? v < limit : rule == 1 && v <= limit) done = 1;
+        else if (it >= P.ctl->maxit) done = 3;
+        b = g * m.inv_gamma;
+        if (blockIdx.x == 0) {
+          m.gamma_prev = m.gamma;
+          m.gamma = g;
+          m.rr = rr;
+          m.beta = b;
+          m.iters = it;
+        }
+      }
+      if (blockIdx.x == 0) {
+        m.done[q] = done;
+        m.sum_b[q][0] = m.sum_b[q][1] = 0;
+      }
+      s_done[c] = done;
+      s_beta[c] = done ? T(0) : (T)b;
+      stop = done != 0;
     }
+    const bool all = __syncthreads_and(stop);
+    if (blockIdx.x == 0 && threadIdx.x == 0) P.ctl->all_done = all;
+    if (all) return;
   }
   if (threadIdx.x == 0) {
     mbar_init(&bar[0], 1);
@@ -184,8 +171,8 @@ __global__ void __launch_bounds__(kHfanThreads, C <= 2 ? 3 : 2) k_matvec_multi(M
   const int64_t q0 = n_items * blockIdx.x / gridDim.x, q1 = n_items * (blockIdx.x + 1) / gridDim.x;
   int cur = -1;
   unsigned nload = 0;
-  for (int64_t q = q0; q < q1; ++q) {
-    const int patch = (int)(q / NC), c0 = (int)(q - (int64_t)patch * NC) * C;
+  for (int64_t item = q0; item < q1; ++item) {
+    const int patch = (int)(item / NC), c0 = (int)(item - (int64_t)patch * NC) * C;
     if (MODE == MV_PCG) {
       bool all = true;  // (uniform: read from shared memory)
 #pragma unroll
@@ -342,26 +329,18 @@ __global__ void __launch_bounds__(kHfanThreads, C <= 2 ? 3 : 2) k_matvec_multi(M
       if (lane < C) s_red[wid * C + lane] = (double)energy.hi + (double)energy.lo;
     }
     __syncthreads();  // sp, fs and s_red of this item are complete
-    if (MODE == MV_PCG && threadIdx.x < C) {
-      double t = 0;
+    if (MODE == MV_PCG && threadIdx.x < 8 * C) {  // (a tree of eight lanes per case)
+      double t = s_red[(threadIdx.x & 7) * C + (threadIdx.x >> 3)];
+      const unsigned mask = C < 4 ? (1u << (8 * (C & 3))) - 1u : 0xffffffffu;
 #pragma unroll
-      for (int w = 0; w < NW; ++w) t += s_red[w * C + threadIdx.x];
-      s_en[c0 + threadIdx.x] += t;
+      for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(mask, t, o);
+      if ((threadIdx.x & 7) == 0) s_en[c0 + (threadIdx.x >> 3)] += t;
     }
   }
   if (MODE != MV_PCG) return;
-  // per-case grid sums (fixed-order tree), alpha_c = gamma_c / sigma_c in the last block
   __syncthreads();
-  for (int c = threadIdx.x; c < K; c += blockDim.x) P.partials[(size_t)blockIdx.x * K + c] = s_en[c];
-  __syncthreads();
-  double *s_tot = s_en;  // (the block's own energies are in the partials now)
-  if (!tree_case_sums<1>(P.partials, P.gpart, P.gcnt_mv, &P.ctl->count_mv, K, s_tot)) return;
-  for (int c = threadIdx.x; c < K; c += blockDim.x) {
-    const double t = s_tot[c];
-    MultiScalars &s = P.sc[c];
-    s.sigma = t;
-    s.alpha = s.done ? 0.0 : s.gamma / t;
-  }
+  for (int c = threadIdx.x; c < K; c += blockDim.x)
+    if (!s_done[c]) atomicAdd(&P.sc[c].sum_a[q], s_en[c]);
 }
 
 // z_c += beta_c p_c for every (node, case) item, p_c read from pB when
@@ -381,26 +360,51 @@ static __global__ void k_multi_fold(int64_t n_items, int K, const float *beta, c
   stv<float, 4>(z, q, v);
 }
 
-// Per case: init (r = f, x = 0) or update (x += alpha p, r -= alpha u),
-// z = M^-1 r, u = 0, gamma = r.z, ||r||^2, per-case stopping tests. Items are
-// (node, case) with the case fastest; the grid stride is a multiple of K, so
+// Per case: init (r = f, x = 0; sums r.z, r.r, f.f into sum_b[0], sum_a[0]) or
+// update (x += alpha p, r -= alpha u; sums r.z, r.r), z = M^-1 r, u = 0. Items
+// are (node, case) with the case fastest; the grid stride is a multiple of K, so
 // a thread always works on the same case.
-template <typename T>
+// LOOP: the instance for the graph loop; its condition is driven like
+// k_pcg_update's.
+template <typename T, bool LOOP = false>
 __global__ void __launch_bounds__(kThreads) k_pcg_multi_vec(MultiParams<T> P, T *xv, T *r, T *z, const T *p, T *u,
                                                            const T *f, const T *dinv, int init) {
   constexpr int DIM = 3, VW = 4;
-  const int K = P.K;
+  const int K = P.K, q = P.parity;
   // the case scalars once per CTA (one thread per case), the shared flag by
   // thread 0: every thread reading the same lines would queue at one L2 slice
   __shared__ T s_alpha[kMaxCases];
   __shared__ int s_frozen[kMaxCases], s_all;
-  if (threadIdx.x == 0) s_all = init ? 0 : P.ctl->all_done;
-  for (int cc = threadIdx.x; cc < K; cc += blockDim.x) {
-    const MultiScalars &sc = P.sc[cc];
-    const int fz = !init && sc.done;
-    s_frozen[cc] = fz;
-    s_alpha[cc] = init || fz ? T(0) : (T)sc.alpha;
+  if (threadIdx.x == 0) {
+    s_all = init ? 0 : P.ctl->all_done;
+    if constexpr (LOOP)
+      if (blockIdx.x == 0) {
+        if (P.cond_role & 1) {
+          const int nl = ++P.ctl->loops;
+          P.ctl->loop_ok = nl <= P.ctl->maxit / P.cond_chunk + 16;
+          cudaGraphSetConditional(P.cond, 0u);
+        }
+        if (P.cond_role & 2) cudaGraphSetConditional(P.cond, !s_all && P.ctl->loop_ok ? 1u : 0u);
+      }
   }
+  for (int cc = threadIdx.x; cc < K; cc += blockDim.x) {
+    MultiScalars &m = P.sc[cc];
+    const int fz = !init && m.done[q];
+    double alpha = 0;
+    if (!init && !fz) {
+      const double sigma = m.sum_a[q];
+      alpha = m.gamma / sigma;
+      if (blockIdx.x == 0) {
+        m.sigma = sigma;
+        m.alpha = alpha;
+        m.inv_gamma = 1.0 / m.gamma;
+      }
+    }
+    if (!init && blockIdx.x == 0) m.sum_a[q ^ 1] = 0;
+    s_frozen[cc] = fz;
+    s_alpha[cc] = (T)alpha;
+  }
+  if (!init && blockIdx.x == 0 && threadIdx.x == 0) P.ctl->iter += 1;
   __syncthreads();
   if (s_all) return;
   const int c = threadIdx.x & (K - 1);
@@ -412,35 +416,35 @@ __global__ void __launch_bounds__(kThreads) k_pcg_multi_vec(MultiParams<T> P, T 
   // stride is a multiple of K, so every item of a thread is case c
   constexpr int U = 4;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t q0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q0 < n_items; q0 += stride * U) {
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < n_items; i0 += stride * U) {
     NodeV<T, VW> zero;
 #pragma unroll
     for (int d = 0; d < VW; ++d) zero.v[d] = 0;
     if (frozen) {
 #pragma unroll
       for (int k = 0; k < U; ++k)
-        if (q0 + k * stride < n_items) stv<T, VW>(u, q0 + k * stride, zero);
+        if (i0 + k * stride < n_items) stv<T, VW>(u, i0 + k * stride, zero);
       continue;
     }
     NodeV<T, VW> di[U], rv[U], xx[U], pp[U], uu[U];
 #pragma unroll
     for (int k = 0; k < U; ++k) {
-      const int64_t q = q0 + k * stride;
-      if (q >= n_items) continue;
-      di[k] = ldv<T, VW>(dinv, q / K);
+      const int64_t i = i0 + k * stride;
+      if (i >= n_items) continue;
+      di[k] = ldv<T, VW>(dinv, i / K);
       if (init) {
-        rv[k] = ldv<T, VW>(f, q);
+        rv[k] = ldv<T, VW>(f, i);
       } else {
-        rv[k] = ldv<T, VW>(r, q);
-        xx[k] = ldv<T, VW>(xv, q);
-        pp[k] = ldv<T, VW>(p, q);
-        uu[k] = ldv<T, VW>(u, q);
+        rv[k] = ldv<T, VW>(r, i);
+        xx[k] = ldv<T, VW>(xv, i);
+        pp[k] = ldv<T, VW>(p, i);
+        uu[k] = ldv<T, VW>(u, i);
       }
     }
 #pragma unroll
     for (int k = 0; k < U; ++k) {
-      const int64_t q = q0 + k * stride;
-      if (q >= n_items) continue;
+      const int64_t i = i0 + k * stride;
+      if (i >= n_items) continue;
       NodeV<T, VW> zz = zero;
       if (init) {
         xx[k] = zero;
@@ -461,62 +465,67 @@ __global__ void __launch_bounds__(kThreads) k_pcg_multi_vec(MultiParams<T> P, T 
       acc[0].add(rz);
       acc[1].add(rr);
       if (init) acc[2].add(rr);
-      stv<T, VW>(xv, q, xx[k]);
-      stv<T, VW>(r, q, rv[k]);
-      stv<T, VW>(z, q, zz);
-      stv<T, VW>(u, q, zero);
+      stv<T, VW>(xv, i, xx[k]);
+      stv<T, VW>(r, i, rv[k]);
+      stv<T, VW>(z, i, zz);
+      stv<T, VW>(u, i, zero);
     }
   }
-  // block partials per case: threads c, c + K, ... in order
-  __shared__ double red[3][kThreads];
+  // Totals of the block per case: lanes of the same case merge as compensated
+  // FP32, the warps' sums add up in FP64, one atomic addition per case and sum.
+  constexpr int NW = kThreads / 32;
+  __shared__ double red[3][NW * 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, KW = min(K, 32);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    if constexpr (sizeof(T) == 4) red[k][threadIdx.x] = (double)acc[k].c.hi + (double)acc[k].c.lo;
-    else red[k][threadIdx.x] = acc[k].s;
-  }
-  __syncthreads();
-  for (int cc = threadIdx.x; cc < K; cc += blockDim.x) {
-    double a = 0, b = 0, e = 0;
-    for (int t = cc; t < (int)blockDim.x; t += K) { a += red[0][t]; b += red[1][t]; e += red[2][t]; }
-    double *pt = P.partials + ((size_t)blockIdx.x * K + cc) * 3;
-    pt[0] = a; pt[1] = b; pt[2] = e;
-  }
-  __syncthreads();  // (red is reused for the totals)
-  double *s_tot = &red[0][0];  // [K][3] (K <= kThreads)
-  if (!tree_case_sums<3>(P.partials, P.gpart, P.gcnt_up, &P.ctl->count_up, K, s_tot)) return;
-  __shared__ int s_active;
-  if (threadIdx.x == 0) s_active = 0;
-  __syncthreads();
-  for (int cc = threadIdx.x; cc < K; cc += blockDim.x) {
-    const double a = s_tot[cc * 3], b = s_tot[cc * 3 + 1], e = s_tot[cc * 3 + 2];
-    MultiScalars &m = P.sc[cc];
-    if (init) {
-      m.gamma0 = m.gamma = m.gamma_prev = a;
-      m.rr = b;
-      m.ff = e;
-      m.iters = 0;
-      m.sigma = m.alpha = m.beta = 0;
-      m.done = 0;
-      if (cc >= P.ctl->k_active || a == 0.0) m.done = 1;
-      else if (P.ctl->rule == 1 && sqrt(b) <= P.ctl->tol * sqrt(e)) m.done = 1;
-      else if (!isfinite(a)) m.done = 2;
-    } else if (!m.done) {
-      m.gamma_prev = m.gamma;
-      m.gamma = a;
-      m.beta = a / m.gamma_prev;
-      m.rr = b;
-      m.iters += 1;
-      if (!isfinite(a) || !isfinite(m.alpha)) m.done = 2;
-      else if (P.ctl->rule == 0 && a < P.ctl->tol * m.gamma0) m.done = 1;
-      else if (P.ctl->rule == 1 && sqrt(b) <= P.ctl->tol * sqrt(m.ff)) m.done = 1;
-      else if (m.iters >= P.ctl->maxit) m.done = 3;
+    if (k == 2 && !init) break;
+    Comp32 a = acc[k].c;
+    for (int o = 16; o >= KW; o >>= 1) {
+      const float h2 = __shfl_xor_sync(0xffffffffu, a.hi, o), l2 = __shfl_xor_sync(0xffffffffu, a.lo, o);
+      a.merge(h2, l2);
     }
-    if (!m.done) atomicAdd(&s_active, 1);
+    if (lane < KW) red[k][wid * 32 + lane] = (double)a.hi + (double)a.lo;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    if (!init) P.ctl->iter += 1;
-    P.ctl->all_done = s_active == 0;
+  // warps w, w + K / 32, ... hold case (w mod (K / 32)) 32 + lane
+  const int groups = K / KW, n_sums = init ? 3 : 2;
+  for (int t = threadIdx.x; t < K * n_sums; t += blockDim.x) {
+    const int cc = t & (K - 1), k = t / K;
+    if (s_frozen[cc]) continue;
+    double v = 0;
+    for (int w = cc / KW; w < NW; w += groups) v += red[k][w * 32 + (cc & (KW - 1))];
+    MultiScalars &m = P.sc[cc];
+    atomicAdd(k == 2 ? &m.sum_a[0] : &m.sum_b[init ? 0 : q][k], v);
+  }
+}
+
+// After the init kernel: the scalars of every case (one block).
+static __global__ void __launch_bounds__(kMaxCases) k_multi_start(MultiScalars *sc, MultiCtl *ctl, int K) {
+  const int c = threadIdx.x;
+  bool stop = true;
+  if (c < K) {
+    MultiScalars &m = sc[c];
+    const double g = m.sum_b[0][0], rr = m.sum_b[0][1], ff = m.sum_a[0], lim = ctl->tol * sqrt(ff);
+    m.gamma0 = m.gamma = m.gamma_prev = g;
+    m.rr = rr;
+    m.ff = ff;
+    m.gamma_stop = ctl->tol * g;
+    m.rr_stop = lim < 0 ? -1.0 : lim * lim;  // (a negative tol stops nothing)
+    m.iters = 0;
+    m.sigma = m.alpha = m.beta = 0;
+    m.inv_gamma = 0;
+    m.sum_a[0] = m.sum_a[1] = 0;
+    int done = 0;
+    if (c >= ctl->k_active || g == 0.0) done = 1;
+    else if (ctl->rule == 1 && rr <= m.rr_stop) done = 1;
+    else if (!isfinite(g)) done = 2;
+    m.done[0] = m.done[1] = done;
+    stop = done != 0;
+  }
+  const bool all = __syncthreads_and(stop);
+  if (c == 0) {
+    ctl->iter = 0;
+    ctl->all_done = all;
   }
 }
 
@@ -547,19 +556,6 @@ __global__ void k_multi_to_caller(int64_t nn, int K, int k, int64_t nd, const T 
   const NodeV<T, 4> v = ldv<T, 4>(src, q);
 #pragma unroll
   for (int d = 0; d < 3; ++d) U[(size_t)c * nd + o * 3 + d] = (double)v.v[d];
-}
-
-// one case of a [node][K][4] array <-> a [node][4] array
-template <typename TA, typename TB>
-__global__ void k_case_copy(int64_t nn, int K, int c, const TA *src, TB *dst, int to_single) {
-  int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (n >= nn) return;
-  const int64_t a = to_single ? n * K + c : n, b = to_single ? n : n * K + c;
-  const NodeV<TA, 4> v = ldv<TA, 4>(src, a);
-  NodeV<TB, 4> w;
-#pragma unroll
-  for (int d = 0; d < 4; ++d) w.v[d] = (TB)v.v[d];
-  stv<TB, 4>(dst, b, w);
 }
 
 // x64 += d32 over whole multi arrays

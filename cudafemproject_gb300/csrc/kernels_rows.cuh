@@ -229,6 +229,100 @@ __global__ void __launch_bounds__(kRowsThreads) k_rows_residual(RowOp A, RowsRes
   }
 }
 
+// FP64 true residuals of K load cases at once: r_c = f_c - A x_c on
+// [node][K][4] arrays (3D), ||r_c||^2 and ||f_c||^2 added to norms[2c], [2c + 1]
+// (zero at the start). One thread per (row, case), the case fastest: a warp's
+// block loads are broadcasts and its gathers contiguous, and the FP64 pipe is
+// what bounds it (168 operations per row and case). Cases with skip[c] != 0 are
+// left out where a whole warp holds only such. Blocks of 256 threads, K a power
+// of two up to 256.
+struct RowsCases {
+  RowOp A;
+  int K;
+  const double *f, *x;
+  double *r, *norms;
+  const int *skip;
+};
+static __global__ void __launch_bounds__(kThreads) k_rows_cases_residual(RowsCases P) {
+  constexpr int DIM = 3;
+  const RowOp &A = P.A;
+  const int K = P.K, c = threadIdx.x & (K - 1);  // (the grid stride is a multiple of K)
+  const bool skip = __all_sync(0xffffffffu, P.skip[c] != 0);
+  double rr = 0, ff = 0;
+  const int64_t n_items = A.n_slices * kSliceRows * K, stride = (int64_t)gridDim.x * kThreads;
+  for (int64_t it = blockIdx.x * (int64_t)kThreads + threadIdx.x; it < n_items && !skip; it += stride) {
+    const int64_t slot = it / K, s = slot / kSliceRows;
+    const int t = (int)(slot % kSliceRows), row = A.row[slot], i = row < 0 ? 0 : row;
+    const int64_t k0 = A.off[s];
+    const int n = (int)(A.off[s + 1] - k0);
+    const bool masked = A.flag[s] != 0;
+    const unsigned b = masked ? A.bits[i] : 0u;
+    NodeV<double, 4> own = ldv<double, 4>(P.x, (int64_t)i * K + c);
+    double xi[DIM], y[DIM];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      xi[d] = (b >> d) & 1u ? 0.0 : own.v[d];
+      y[d] = 0;
+    }
+    const int32_t *col = A.col + k0 * 32 + t;
+    const double *val = A.val + k0 * (32 * DIM * DIM) + t;
+    for (int k = 0; k < n; ++k)
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int32_t j = col[k * 32 + half * 16];
+        NodeV<double, 4> v = ldv<double, 4>(P.x, (int64_t)j * K + c);
+        if (masked) {
+          const unsigned bj = A.bits[j];
+#pragma unroll
+          for (int d = 0; d < DIM; ++d)
+            if ((bj >> d) & 1u) v.v[d] = 0;
+        }
+        double M[DIM * DIM];
+#pragma unroll
+        for (int q = 0; q < DIM * DIM; ++q) M[q] = val[(k * DIM * DIM + q) * 32 + half * 16];
+#pragma unroll
+        for (int q = 0; q < DIM; ++q) {
+          const double du = v.v[q] - xi[q];
+#pragma unroll
+          for (int p = 0; p < DIM; ++p) y[p] = fma(M[p * DIM + q], du, y[p]);
+        }
+      }
+    if (masked) {
+      const double *Db = A.D + (int64_t)i * DIM * DIM;
+#pragma unroll
+      for (int p = 0; p < DIM; ++p) {
+        if ((b >> p) & 1u) {
+          y[p] = Db[p * DIM + p] * own.v[p];
+        } else {
+#pragma unroll
+          for (int q = 0; q < DIM; ++q) y[p] = fma(Db[p * DIM + q], xi[q], y[p]);
+        }
+      }
+    }
+    if (row < 0) continue;
+    const NodeV<double, 4> f = ldv<double, 4>(P.f, (int64_t)i * K + c);
+    NodeV<double, 4> r;
+#pragma unroll
+    for (int d = 0; d < 4; ++d) r.v[d] = d < DIM ? f.v[d] - y[d < DIM ? d : 0] : 0.0;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      rr += r.v[d] * r.v[d];
+      ff += f.v[d] * f.v[d];
+    }
+    stv<double, 4>(P.r, (int64_t)i * K + c, r);
+  }
+  __shared__ double red[2][kThreads];
+  red[0][threadIdx.x] = rr;
+  red[1][threadIdx.x] = ff;
+  __syncthreads();
+  for (int t = threadIdx.x; t < 2 * K; t += kThreads) {
+    const int cc = t >> 1, k = t & 1;
+    double v = 0;
+    for (int q = cc; q < kThreads; q += K) v += red[k][q];
+    if (v != 0) atomicAdd(P.norms + t, v);
+  }
+}
+
 // ------------------------------------------------------------------ Jacobi PCG
 // A whole FP64 PCG run in one cooperative kernel: the rows' products and the
 // vector updates alternate with grid-wide sums (grid_sync.cuh) instead of

@@ -201,3 +201,30 @@ def test_set_young_on_device_and_refused_values():
         p2 = meshgen.box_3d(5, 4, 11, jitter=0.2, seed=1)
         p2.elem_E = young
         assert rel(a.pcg(f, **kw)[0], O.Oracle(p2).pcg(f, tol=1e-13, rule=1)[0]) <= 1e-8
+
+
+@pytest.mark.parametrize("host_loop", [False, True])
+@pytest.mark.parametrize("k", [2, 3, 33, 130])
+def test_multi_rhs_case_counts(monkeypatch, host_loop, k):
+    """Per-case sums, stopping and FP64 residuals for case counts that fill part of
+    a warp, one, several; a case without load, one 1e6 times the others; the
+    graph loop and the host loop. Every case within 1e-8 of the oracle."""
+    from cudafemproject_gb300.solver import FemContext
+    if host_loop:
+        monkeypatch.setenv("CFEM_HOST_LOOP", "1")
+    else:
+        monkeypatch.delenv("CFEM_HOST_LOOP", raising=False)
+    p = meshgen.box_3d(4, 3, 9, jitter=0.2, seed=2)
+    o = O.Oracle(p, consistent=True).assemble()
+    rng = np.random.default_rng(k)
+    basis = rng.standard_normal((3, p.n_dof))
+    X = np.stack([o.pcg(b, tol=1e-13, rule=1)[0] for b in basis])
+    w = rng.standard_normal((k, 3))
+    w[1] = 0.0
+    w[0] *= 1e6
+    ctx = FemContext(p, semantics="consistent")
+    for tol in (0.3, 1e-4):
+        U, infos = ctx.pcg_multi(w @ basis, precision="fp32_refine", tol=tol, stop_rule="residual", outer_tol=1e-10)
+        assert all(i["status"] == 0 for i in infos)
+        assert not U[1].any()
+        assert max(rel(U[i], w[i] @ X) for i in range(k) if i != 1) <= 1e-8
