@@ -251,8 +251,11 @@ bool add_loop(cfem_ctx *c, cudaGraph_t graph, unsigned initial, const std::funct
 // FP32 Jacobi PCG on A x = V.f (V = c->v32) with A = cM*M + cK*K' (mcoef selects the mass term).
 // V.x holds the warm start when warm != 0. Returns after the device flag says
 // done and what `then` has queued behind the run is complete.
-PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
-                    const float *cont_p, double cont_gamma_prev, const std::function<void()> &then) {
+// queue_pcg_f: the run up to the loop's graph launch, nothing waited for (the
+// scalars can be read behind it); false where the loop runs on the host and
+// only its graph has been built. chunk: iterations per loop body.
+bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
+                 const float *cont_p, double cont_gamma_prev, int chunk) {
   Vecs<float> &V = c->v32;
   const PcgSite S = whole_mesh(c);
   Scalars *sc = S.sc;
@@ -281,7 +284,8 @@ PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int war
     c->launches += 1;
   }
   GraphCache &gc = c->graph32;
-  if (!gc.exec || gc.key0 != (const void *)mcoef || gc.key1 != (double)cK || gc.key2 != (double)cM) {
+  if (!gc.exec || gc.key0 != (const void *)mcoef || gc.key1 != (double)cK || gc.key2 != (double)cM ||
+      gc.chunk != chunk) {
     gc.reset();
     const int64_t launches_before_capture = c->launches;
     // Preferred: the iterations inside a CUDA-graph WHILE node, so a solve is
@@ -292,7 +296,7 @@ PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int war
       cudaGraph_t graph = nullptr;
       cudaGraphExec_t exec = nullptr;
       bool ok = cudaGraphCreate(&graph, 0) == cudaSuccess &&
-                add_loop(c, graph, 1, nullptr, [&](cudaGraphConditionalHandle cond) { capture_iterations(c, S, mv, c->chunk, cond); });
+                add_loop(c, graph, 1, nullptr, [&](cudaGraphConditionalHandle cond) { capture_iterations(c, S, mv, chunk, cond); });
       if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
       if (graph) cudaGraphDestroy(graph);
       (void)cudaGetLastError();
@@ -307,7 +311,7 @@ PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int war
       cudaGraph_t graph;
       CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
       try {
-        capture_iterations(c, S, mv, c->chunk, 0);
+        capture_iterations(c, S, mv, chunk, 0);
       } catch (...) {
         cudaGraph_t broken = nullptr;
         cudaStreamEndCapture(c->stream, &broken);
@@ -324,10 +328,29 @@ PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int war
     gc.key0 = mcoef;
     gc.key1 = cK;
     gc.key2 = cM;
+    gc.chunk = chunk;
   }
+  if (gc.device_loop) CK(cudaGraphLaunch(gc.exec, c->stream));
+  return gc.device_loop;
+}
+
+PcgResult pcg_result(const Scalars &s) {
   PcgResult res;
-  if (gc.device_loop) {
-    CK(cudaGraphLaunch(gc.exec, c->stream));
+  res.iters = s.iter;
+  res.gamma0 = s.gamma0;
+  res.gamma = s.gamma;
+  res.rr = s.rr;
+  res.ff = s.ff;
+  res.gamma_prev = s.gamma_prev;
+  res.status = s.done == 1 ? CFEM_OK : s.done == 2 ? CFEM_ERR_DIVERGED : CFEM_ERR_NOT_CONVERGED;
+  return res;
+}
+
+PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
+                    const float *cont_p, double cont_gamma_prev, const std::function<void()> &then) {
+  Scalars *sc = c->sc.p + 1;
+  const GraphCache &gc = c->graph32;
+  if (queue_pcg_f(c, cK, cM, mcoef, warm, tol, rule, maxit, cont_p, cont_gamma_prev, c->chunk)) {
     if (then) then();
     CK(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -342,7 +365,7 @@ PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int war
   } else {
     // Every replay advances the iteration count by `chunk` unless the device
     // flag is set; the cap below only guards against a stalled recurrence.
-    const int64_t max_launches = (int64_t)h.maxit / c->chunk + 16;
+    const int64_t max_launches = (int64_t)(maxit > 0 ? maxit : 1000000) / c->chunk + 16;
     int last_iter = -1, stalled = 0;
     for (int64_t launch = 0;; ++launch) {
       if (launch > max_launches || stalled > 4) {
@@ -365,15 +388,7 @@ PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int war
     }
   }
   check_copy_flag(c);
-  res.iters = c->h_sc->iter;
-  res.gamma0 = c->h_sc->gamma0;
-  res.gamma = c->h_sc->gamma;
-  res.rr = c->h_sc->rr;
-  res.ff = c->h_sc->ff;
-  res.gamma_prev = c->h_sc->gamma_prev;
-  int d = c->h_sc->done;
-  res.status = d == 1 ? CFEM_OK : d == 2 ? CFEM_ERR_DIVERGED : CFEM_ERR_NOT_CONVERGED;
-  return res;
+  return pcg_result(*c->h_sc);
 }
 
 // caller-order array (host or device) -> internal node vector of type T; a

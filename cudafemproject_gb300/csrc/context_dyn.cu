@@ -230,6 +230,13 @@ const double *young_on_device(cfem_ctx *c) {
   return c->young_d.p;
 }
 
+// Iterations per body of the PCG loop of an implicit step. A body costs about 5
+// us beyond its iterations, an iteration past the stop as much as the body's
+// share of 4; warm-started steps take 10 to 50 iterations (20 steps of 18
+// iterations on 196,608 tets: bodies of 4 and 10 6.0 ms, 6, 8 and 12 6.35, 16 7.2:
+// the fewer iterations past the 18th).
+constexpr int kStepChunk = 4;
+
 template <typename T>
 cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet *w, double *u_out, cfem_dyn_info *info) {
   single_mesh_only(c);
@@ -257,7 +264,7 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
   }();
   W.coef.ensure(coef.size());
   CK(cudaMemcpyAsync(W.coef.p, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice, c->stream));
-  S.d.ensure(2 * (size_t)c->nvec);
+  S.d.ensure(3 * (size_t)c->nvec);
   for (auto *b : {&S.v, &S.a, &S.y}) b->ensure(c->nvec);
   S.minv.ensure(2 * (size_t)c->nvec);
   for (auto *b : {&S.d, &S.v, &S.a, &S.y}) b->zero(c->stream);
@@ -437,14 +444,17 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
       }
     }
   } else {
-    for (int s = 1; s <= nsteps; ++s) {
+    const double tol = compat ? 1e-4 : (prm->pcg_tol > 0 ? prm->pcg_tol : 1e-10);
+    const int rule = compat ? CFEM_STOP_REFERENCE : prm->stop_rule;
+    const int warm = compat ? 0 : prm->warm_start;
+    auto before = [&](const T *from, T *to) {  // the predictor and the PCG's right-hand side
       if constexpr (sizeof(T) == 8) {
-        k_dyn_predict<<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, dcur, S.v.p, S.a.p, mv.c1, mv.c2, dnext);
+        k_dyn_predict<<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, from, S.v.p, S.a.p, mv.c1, mv.c2, to);
         CKL();
-        rows_apply(c, dnext, S.y.p);
+        rows_apply(c, to, S.y.p);
       } else {
-        mv.x = dcur;
-        mv.xout = dnext;
+        mv.x = from;
+        mv.xout = to;
         launch_mv_f(c, MV_DYN, mv);
       }
       dp.rhs = V.f.p;
@@ -453,17 +463,62 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
         slot_assemble_and_resort<double>(c, diag_pre.p, 0);
         set_pcg_vectors(c, diag_op.p, diag_pre.p);
       }
-      const double tol = compat ? 1e-4 : (prm->pcg_tol > 0 ? prm->pcg_tol : 1e-10);
-      const int rule = compat ? CFEM_STOP_REFERENCE : prm->stop_rule;
-      const int warm = compat ? 0 : prm->warm_start;
+    };
+    auto after = [&](T *to) {
+      dp.anew = V.x.p;
+      dp.d = to;
+      launch_dyn_correct<T>(c, dp);
+      k_dyn_end_step<T><<<1, kThreads, 0, c->stream>>>(dp, to, c->vw);
+      CKL();
+    };
+    bool pipelined = false;
+    if constexpr (sizeof(T) == 4) {
+      // The next step is queued before the PCG of this one has been looked at
+      // (a step waited 60-80 us for the host between its kernels otherwise).
+      // Three displacement buffers: a step that fails leaves the state before
+      // it alone even while one more step runs.
+      if (!W.ring) {
+        CK(cudaMallocHost(&W.ring, 2 * sizeof(Scalars)));
+        for (cudaEvent_t &e : W.done) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      }
+      const int chunk = std::getenv("CFEM_PCG_CHUNK") ? c->chunk : kStepChunk;
+      T *buf[3] = {d0, d1, S.d.p + 2 * (size_t)c->nvec};
+      pipelined = true;
+      auto look_at = [&](int s) {  // false: the run ends with the state before step s
+        CK(cudaEventSynchronize(W.done[s & 1]));
+        check_copy_flag(c);
+        const Scalars &r = W.ring[s & 1];
+        c->launches += (int64_t)2 * chunk * r.loops;
+        if (!r.done) throw Fail{CFEM_ERR_CUDA, "PCG recurrence stopped advancing on the device"};
+        const PcgResult res = pcg_result(r);
+        pcg_total += res.iters;
+        status = res.status;
+        dcur = buf[(s - (status != CFEM_OK)) % 3];
+        return status == CFEM_OK;
+      };
+      for (int s = 1; s <= nsteps; ++s) {
+        before(buf[(s - 1) % 3], buf[s % 3]);
+        if (!queue_pcg_f(c, opK, opM, opmc, warm, tol, rule, prm->max_iter, nullptr, 0, chunk)) {
+          pipelined = false;  // (s == 1: no device loop here; the step starts over below)
+          break;
+        }
+        after(buf[s % 3]);
+        CK(cudaMemcpyAsync(W.ring + (s & 1), c->sc.p + 1, sizeof(Scalars), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaEventRecord(W.done[s & 1], c->stream));
+        if (s > 1 && !look_at(s - 1)) break;
+        if (s == nsteps) look_at(s);
+      }
+      if (!pipelined) {
+        if (compat) std::swap(c->slot_src.p, c->slot_tmp.p);  // (its assembly has to be taken back)
+        S.y.zero(c->stream);
+      }
+    }
+    for (int s = 1; s <= nsteps && !pipelined; ++s) {
+      before(dcur, dnext);
       PcgResult r = run_pcg<T>(c, V, opK, opM, opmc, warm, tol, rule, prm->max_iter);
       pcg_total += r.iters;
       if (r.status != CFEM_OK) { status = r.status; break; }
-      dp.anew = V.x.p;
-      dp.d = dnext;
-      launch_dyn_correct<T>(c, dp);
-      k_dyn_end_step<T><<<1, kThreads, 0, c->stream>>>(dp, dnext, c->vw);
-      CKL();
+      after(dnext);
       std::swap(dcur, dnext);
     }
   }

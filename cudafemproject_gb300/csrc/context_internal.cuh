@@ -93,6 +93,7 @@ struct GraphCache {
   bool device_loop = false;  // exec is a WHILE node around the iterations (one launch per solve)
   const void *key0 = nullptr;
   double key1 = 0, key2 = 0;
+  int chunk = 0;  // iterations per body
   ~GraphCache() { reset(); }
   void reset() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -119,7 +120,7 @@ struct RowsData {
 // Work buffers of the time-stepping calls, kept with the context.
 template <typename T>
 struct StepVecs {
-  DBuf<T> d, v, a, y, minv;  // d: two node vectors; minv: two when re-sorted
+  DBuf<T> d, v, a, y, minv;  // d: two node vectors (three, FP32 implicit); minv: two when re-sorted
 };
 struct StepWork {
   StepVecs<double> f64;
@@ -128,6 +129,13 @@ struct StepWork {
   DBuf<int32_t> recv, rec_head, rec_next;
   DBuf<DynState> st;
   DBuf<int> stalled;
+  Scalars *ring = nullptr;        // pinned: scalars of the implicit steps in flight
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  ~StepWork() {
+    if (ring) cudaFreeHost(ring);
+    for (cudaEvent_t e : done)
+      if (e) cudaEventDestroy(e);
+  }
 };
 
 inline unsigned nblk(int64_t n, int t = kThreads) { return (unsigned)((n + t - 1) / t); }
@@ -270,6 +278,9 @@ PcgResult run_pcg_d(cfem_ctx *c, Vecs<double> &V, double cK, double cM, const do
 PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
                     const float *cont_p = nullptr, double cont_gamma_prev = 0,
                     const std::function<void()> &then = nullptr);
+bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
+                 const float *cont_p, double cont_gamma_prev, int chunk);
+PcgResult pcg_result(const Scalars &s);
 struct PcgSite {
   Scalars *sc;
   int first_patch, n_patches;

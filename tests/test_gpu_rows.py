@@ -228,3 +228,34 @@ def test_multi_rhs_case_counts(monkeypatch, host_loop, k):
         assert all(i["status"] == 0 for i in infos)
         assert not U[1].any()
         assert max(rel(U[i], w[i] @ X) for i in range(k) if i != 1) <= 1e-8
+
+
+def test_fp32_implicit_step_that_fails_keeps_the_state_before_it():
+    """Steps are queued one ahead: when a step's PCG does not converge, the result is
+    the displacement before that step, as when every step is waited for."""
+    import ctypes as C
+    from cudafemproject_gb300 import capi
+    from cudafemproject_gb300.solver import FemContext
+    p = _column(4, 3, 17)
+    ctx = FemContext(p, semantics="consistent")
+
+    def run(n, tol, cap):
+        u = np.zeros(p.n_dof)
+        prm = capi.DynParams(0.5, 0.5, 1e-3, n * 1e-3 * 1.0000001, capi.FP32, tol, capi.STOP_RESIDUAL, cap, 1, 0, None, None)
+        inf = capi.DynInfo()
+        return capi.lib().cfem_dyn(ctx._h, C.byref(prm), None, u.ctypes.data, C.byref(inf)), u, inf.pcg_iterations
+
+    need = []  # iterations of every step
+    for n in range(1, 6):
+        st, u, its = run(n, 1e-6, 1000)
+        assert st == capi.OK
+        need.append(its - sum(need))
+    cap = need[0]  # the first step just converges; find the first that does not
+    first_bad = next((i for i, k in enumerate(need) if k > cap), None)
+    if first_bad is None:
+        cap, first_bad = max(need) - 1, int(np.argmax(need))
+        first_bad = next(i for i, k in enumerate(need) if k > cap)
+    st, u, its = run(5, 1e-6, cap)
+    assert st == capi.ERR_NOT_CONVERGED
+    ref = run(first_bad, 1e-6, 1000)[1] if first_bad else np.zeros(p.n_dof)
+    assert np.linalg.norm(u - ref) <= 1e-4 * np.linalg.norm(ref)  # (FP32 sums are atomic)
