@@ -437,7 +437,6 @@ void set_diag_vectors(cfem_ctx *c) {
   if (c->diag_is_K) return;
   k_invert<double><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->diagK.p, c->v64.dinv.p);
   k_invert<float><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->diagK.p, c->v32.dinv.p);
-  CK(cudaMemcpyAsync(c->v64.diagA.p, c->diagK.p, sizeof(double) * c->nvec, cudaMemcpyDeviceToDevice, c->stream));
   k_convert<double, float><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, c->diagK.p, c->v32.diagA.p);
   CKL();
   c->diag_is_K = true;
@@ -624,6 +623,11 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
   }
   const Prep &P = c->prep;
   cudaStream_t s = c->stream;
+  CK(cudaMallocHost(&c->pinned, 64 + sizeof(Scalars)));
+  c->h_rr = static_cast<double *>(c->pinned);  // 4 doubles
+  c->h_tma_err = reinterpret_cast<int *>(c->h_rr + 4);
+  c->h_sc = reinterpret_cast<Scalars *>(static_cast<char *>(c->pinned) + 64);
+  *c->h_tma_err = 0;
   c->elem_off.upload(P.p_elem_off.data(), P.p_elem_off.size(), s);
   c->node_off.upload(P.p_node_off.data(), P.p_node_off.size(), s);
   c->nodes.upload(P.p_nodes.data(), P.p_nodes.size(), s);
@@ -747,8 +751,6 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
     c->blk32.zero(s);
     CK(cudaMemcpy2DAsync(c->blk32.p, c->L32.bytes, hb.data(), pre, pre, P.n_patches, cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));  // hb is pageable and goes out of scope
-    CK(cudaMallocHost(&c->h_tma_err, sizeof(int)));
-    *c->h_tma_err = 0;
   }
   if (c->n_inst) {
     // instance tables: patch -> instance, instance patch ranges, owned node ranges, materials
@@ -805,23 +807,17 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
   c->FB.alloc(c->nvec);
   c->FA32.alloc(c->nvec);
   c->FB32.alloc(c->nvec);
-  c->v64.f.alloc(c->nvec);
   // work vectors
-  for (auto *b : {&c->v64.x, &c->v64.r, &c->v64.z, &c->v64.pA, &c->v64.pB, &c->v64.u, &c->v64.uB, &c->v64.dinv,
-                  &c->v64.diagA}) {
-    b->alloc(c->nvec);
-    b->zero(s);
-  }
-  c->v64.f.zero(s);
-  for (auto *b : {&c->v32.x, &c->v32.r, &c->v32.z, &c->v32.pA, &c->v32.pB, &c->v32.u, &c->v32.uB, &c->v32.f,
-                  &c->v32.dinv, &c->v32.diagA}) {
-    b->alloc(c->nvec);
-    b->zero(s);
-  }
-  c->tmp64.alloc(c->nvec);
-  c->tmp64b.alloc(c->nvec);
-  c->tmp64.zero(s);
-  c->tmp64b.zero(s);
+  auto vectors = [&](auto &slab, std::initializer_list<std::remove_reference_t<decltype(slab)> *> list) {
+    slab.alloc(list.size() * c->nvec);
+    slab.zero(s);
+    size_t at = 0;
+    for (auto *b : list) b->view(slab.p + c->nvec * at++, c->nvec);
+  };
+  vectors(c->v64.slab, {&c->v64.x, &c->v64.r, &c->v64.z, &c->v64.pA, &c->v64.u, &c->v64.dinv, &c->v64.f, &c->tmp64,
+                        &c->tmp64b});
+  vectors(c->v32.slab, {&c->v32.x, &c->v32.r, &c->v32.z, &c->v32.pA, &c->v32.pB, &c->v32.u, &c->v32.uB, &c->v32.f,
+                        &c->v32.dinv, &c->v32.diagA});
   to_internal<double>(c, c->rhs.FA.data(), c->FA.p);
   to_internal<double>(c, c->rhs.FB.data(), c->FB.p);
   k_convert<double, float><<<nblk(c->nvec), kThreads, 0, s>>>(c->nvec, c->FA.p, c->FA32.p);
@@ -894,8 +890,6 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
   c->counters.zero(s);
   c->sc.alloc(3);
   c->sc.zero(s);
-  CK(cudaMallocHost(&c->h_sc, sizeof(Scalars)));
-  CK(cudaMallocHost(&c->h_rr, 4 * sizeof(double)));
   CK(cudaEventCreate(&c->ev0));
   CK(cudaEventCreate(&c->ev1));
   CK(cudaStreamSynchronize(s));

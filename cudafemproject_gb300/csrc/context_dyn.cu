@@ -132,7 +132,6 @@ void set_pcg_vectors(cfem_ctx *c, const double *diag_op, const double *diag_pre)
   c->diag_is_K = false;
   k_invert<double><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, diag_pre, c->v64.dinv.p);
   k_invert<float><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, diag_pre, c->v32.dinv.p);
-  CK(cudaMemcpyAsync(c->v64.diagA.p, diag_op, sizeof(double) * c->nvec, cudaMemcpyDeviceToDevice, c->stream));
   k_convert<double, float><<<nblk(c->nvec), kThreads, 0, c->stream>>>(c->nvec, diag_op, c->v32.diagA.p);
   CKL();
 }

@@ -50,14 +50,22 @@ template <typename T>
 struct DBuf {
   T *p = nullptr;
   size_t n = 0;
+  bool owned = true;
   DBuf() = default;
   DBuf(const DBuf &) = delete;
   DBuf &operator=(const DBuf &) = delete;
   ~DBuf() { release(); }
   void release() {
-    if (p) cudaFree(p);
+    if (p && owned) cudaFree(p);
     p = nullptr;
     n = 0;
+    owned = true;
+  }
+  void view(T *at, size_t count) {  // part of a buffer that outlives this one
+    release();
+    p = at;
+    n = count;
+    owned = false;
   }
   void alloc(size_t count) {
     release();
@@ -79,7 +87,8 @@ struct DBuf {
 
 template <typename T>
 struct Vecs {
-  DBuf<T> x, r, z, pA, pB, u, uB, f, dinv, diagA;  // u, uB: A p of even, odd PCG iterations
+  DBuf<T> slab;  // one allocation for all of them
+  DBuf<T> x, r, z, pA, pB, u, uB, f, dinv, diagA;  // u, uB: A p of even, odd PCG iterations (FP32 only, like pB, diagA)
 };
 
 inline int pcg_chunk_from_env() {
@@ -108,6 +117,7 @@ struct RowsValues {
   DBuf<uint8_t> flag;
 };
 struct RowsData {
+  DBuf<int32_t> slab;          // off, inc_off, inc, row
   DBuf<int32_t> inc_off, inc;  // elements of every node
   DBuf<int32_t> row, col;
   DBuf<int64_t> off;
@@ -206,6 +216,7 @@ struct cfem_ctx {
   DBuf<double> partials_up;  // r.z, r.r partials of the PCG update kernel [grid][2]
   DBuf<unsigned int> counters;
   DBuf<int> err;
+  void *pinned = nullptr;  // h_sc, h_rr, h_tma_err
   Scalars *h_sc = nullptr;
   double *h_rr = nullptr;
   int grid_mv = 0, grid_vec = 0;
@@ -238,9 +249,7 @@ struct cfem_ctx {
 
   ~cfem_ctx() {
     graph32.reset();
-    if (h_sc) cudaFreeHost(h_sc);
-    if (h_rr) cudaFreeHost(h_rr);
-    if (h_tma_err) cudaFreeHost(h_tma_err);
+    if (pinned) cudaFreeHost(pinned);
     if (multi) destroy_multi(multi);
     if (batch) destroy_batch(batch);
     if (ev0) cudaEventDestroy(ev0);

@@ -35,28 +35,35 @@ void build_structure(cfem_ctx *c, DBuf<int32_t> &nbr, DBuf<int32_t> &deg) {
   RowsData &R = c->rows;
   cudaStream_t s = c->stream;
   const int64_t nn = c->nn, n_inc = c->ne * NV;
-  DBuf<int32_t> cnt, steps;
-  cnt.alloc(nn);
-  cnt.zero(s);
-  k_rows_count<<<nblk(n_inc), kThreads, 0, s>>>(n_inc, c->conn.p, cnt.p);
-  R.inc_off.alloc(nn + 1);
-  k_rows_scan<int32_t><<<1, 1024, 0, s>>>(nn, cnt.p, R.inc_off.p);
-  cnt.zero(s);
-  R.inc.alloc(n_inc);
-  k_rows_fill<<<nblk(n_inc), kThreads, 0, s>>>(n_inc, NV, c->conn.p, R.inc_off.p, cnt.p, R.inc.p);
-  nbr.alloc((size_t)(NV - 1) * n_inc);
-  deg.alloc(nn);
-  k_rows_neighbours<NV><<<nblk(nn), kThreads, 0, s>>>(nn, c->conn.p, R.inc_off.p, R.inc.p, nbr.p, deg.p);
-  const int64_t windows = (nn + kRowWindow - 1) / kRowWindow;
-  R.row.alloc((size_t)windows * kRowWindow);
-  steps.alloc((size_t)windows * (kRowWindow / kSliceRows));
-  k_rows_order<<<(unsigned)windows, kRowWindow, 0, s>>>(nn, deg.p, R.row.p, steps.p);
+  const int64_t windows = (nn + kRowWindow - 1) / kRowWindow, n_steps = windows * (kRowWindow / kSliceRows);
   R.n_slices = (nn + kSliceRows - 1) / kSliceRows;  // (the padding sorts last)
-  R.off.alloc(R.n_slices + 1);
-  k_rows_scan<int64_t><<<1, 1024, 0, s>>>(R.n_slices, steps.p, R.off.p);
+  // what stays, in one allocation: inc_off, inc, row (off: 8-byte aligned first)
+  auto even = [](int64_t n) { return (n + 3) / 4 * 4; };
+  R.slab.alloc((size_t)(2 * even(R.n_slices + 1) + even(nn + 1) + even(n_inc) + even(windows * kRowWindow)));
+  int32_t *at = R.slab.p;
+  R.off.view(reinterpret_cast<int64_t *>(at), R.n_slices + 1);
+  at += 2 * even(R.n_slices + 1);
+  R.inc_off.view(at, nn + 1);
+  at += even(nn + 1);
+  R.inc.view(at, n_inc);
+  at += even(n_inc);
+  R.row.view(at, (size_t)windows * kRowWindow);
+  // what the construction needs: neighbour lists, their lengths, counts, steps per slice
+  nbr.alloc((size_t)(even((NV - 1) * n_inc) + 2 * even(nn) + n_steps));
+  int32_t *deg_p = nbr.p + even((NV - 1) * n_inc), *cnt = deg_p + even(nn), *steps = cnt + even(nn);
+  deg.view(deg_p, nn);
+  CK(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * nn, s));
+  k_rows_count<<<nblk(n_inc), kThreads, 0, s>>>(n_inc, c->conn.p, cnt);
+  k_rows_scan<int32_t><<<1, 1024, 0, s>>>(nn, cnt, R.inc_off.p);
+  CK(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * nn, s));
+  k_rows_fill<<<nblk(n_inc), kThreads, 0, s>>>(n_inc, NV, c->conn.p, R.inc_off.p, cnt, R.inc.p);
+  k_rows_neighbours<NV><<<nblk(nn), kThreads, 0, s>>>(nn, c->conn.p, R.inc_off.p, R.inc.p, nbr.p, deg.p);
+  k_rows_order<<<(unsigned)windows, kRowWindow, 0, s>>>(nn, deg.p, R.row.p, steps);
+  k_rows_scan<int64_t><<<1, 1024, 0, s>>>(R.n_slices, steps, R.off.p);
   CKL();
-  CK(cudaMemcpyAsync(&R.steps, R.off.p + R.n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));  // (cnt and steps are freed here, too)
+  CK(cudaMemcpyAsync(c->h_rr, R.off.p + R.n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  R.steps = *(volatile int64_t *)c->h_rr;
   R.col.alloc((size_t)R.steps * 32);
 }
 
@@ -65,9 +72,10 @@ void assemble_dim(cfem_ctx *c, const int32_t *nbr, const int32_t *deg, double cK
   RowsData &R = c->rows;
   cudaStream_t s = c->stream;
   if (!V.val.p) {
-    V.val.alloc((size_t)R.steps * 32 * DIM * DIM);
-    V.D.alloc((size_t)c->nn * DIM * DIM);
-    V.flag.alloc(R.n_slices);
+    const size_t n_val = (size_t)R.steps * 32 * DIM * DIM, n_D = (size_t)c->nn * DIM * DIM;
+    V.val.alloc(n_val + n_D + (R.n_slices + 7) / 8);
+    V.D.view(V.val.p + n_val, n_D);
+    V.flag.view(reinterpret_cast<uint8_t *>(V.val.p + n_val + n_D), R.n_slices);
   }
   V.flag.zero(s);
   const RowsAssembly<DIM> P = assembly<DIM>(c, cK, cM);
@@ -107,7 +115,7 @@ void build_rows(cfem_ctx *c) {
     if (c->dim == 3) build_structure<4>(c, nbr, deg);
     else build_structure<3>(c, nbr, deg);
     assemble(c, nbr.p, deg.p, 1.0, 0.0, c->rows.K);
-    CK(cudaStreamSynchronize(c->stream));  // (before nbr and deg are freed)
+    CK(cudaStreamSynchronize(c->stream));  // (before nbr is freed)
   } else {
     assemble(c, nullptr, nullptr, 1.0, 0.0, c->rows.K);
   }
