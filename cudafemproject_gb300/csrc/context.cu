@@ -80,6 +80,7 @@ void launch_mv_f(cfem_ctx *c, int mode, const MvParams<float> &P) {
       launch_pdl(k_matvec_fan_tma<float, MV_PCG, false, true>, g, b, c->smem_ft32, c->stream, P, F);
     else if (mode == MV_PLAIN) k_matvec_fan_tma<float, MV_PLAIN><<<g, b, c->smem_ft32, c->stream>>>(P, F);
     else if (mode == MV_PCG) launch_pdl(k_matvec_fan_tma<float, MV_PCG>, g, b, c->smem_ft32, c->stream, P, F);
+    else if (mode == MV_STEP) launch_pdl(k_matvec_fan_tma<float, MV_STEP>, g, b, c->smem_ft32, c->stream, P, F);
     else launch_pdl(k_matvec_fan_tma<float, MV_DYN>, g, b, c->smem_ft32, c->stream, P, F);
   CKL();
     c->launches += 1;
@@ -744,7 +745,13 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
         }
       for (int i = 0; i < c->L32.npn; ++i) {
         nd[i] = i < n ? P.p_nodes[nb + i] : P.p_nodes[nb];
-        bt[i] = i < n ? P.node_bits[P.p_nodes[nb + i]] : 0;
+        bt[i] = 0;
+        if (i < n) {
+          const int64_t o = (int64_t)P.node_new2old[nd[i]] * 3;
+          bool loaded = false;
+          for (int d = 0; d < 3; ++d) loaded |= c->rhs.FA[o + d] != 0.0 || c->rhs.FB[o + d] != 0.0;
+          bt[i] = P.node_bits[nd[i]] | (loaded ? kLoadedBit : 0u);
+        }
       }
     }
     c->blk32.alloc((size_t)c->L32.bytes * P.n_patches);
@@ -854,7 +861,7 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
   if (c->fans) {
     c->smem_ft32 = fan_tma_smem_bytes(c->L32, sizeof(float));
     for (const void *k : {(const void *)k_matvec_fan_tma<float, MV_PLAIN>, (const void *)k_matvec_fan_tma<float, MV_PCG>,
-                          (const void *)k_matvec_fan_tma<float, MV_DYN>,
+                          (const void *)k_matvec_fan_tma<float, MV_DYN>, (const void *)k_matvec_fan_tma<float, MV_STEP>,
                           (const void *)k_matvec_fan_tma<float, MV_PLAIN, false, true>,
                           (const void *)k_matvec_fan_tma<float, MV_PCG, false, true>,
                           (const void *)k_matvec_fan_tma<float, MV_PCG, false, false, true>})

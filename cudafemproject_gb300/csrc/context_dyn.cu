@@ -229,6 +229,24 @@ const double *young_on_device(cfem_ctx *c) {
   return c->young_d.p;
 }
 
+// M^-1 into the fourth lanes of d (x), v (y), a (z).
+__global__ void k_spread_lanes(int64_t nn, const float *minv, float *d, float *v, float *a) {
+  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (n >= nn) return;
+  d[4 * n + 3] = minv[4 * n];
+  v[4 * n + 3] = minv[4 * n + 1];
+  a[4 * n + 3] = minv[4 * n + 2];
+}
+template <typename T>
+__global__ void k_record(int n_recv, int dim, int vw, const int32_t *recv, const T *d, double *row) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n_recv * dim) row[i] = (double)d[(int64_t)recv[i / dim] * vw + i % dim];
+}
+
+// FP32 explicit steps per captured graph: the least common multiple of the
+// buffers' periods (2 and 3; the re-sorted masses' source alternates, too).
+constexpr int kStepCycle = 6;
+
 // Iterations per body of the PCG loop of an implicit step. A body costs about 5
 // us beyond its iterations, an iteration past the stop as much as the body's
 // share of 4; warm-started steps take 10 to 50 iterations (20 steps of 18
@@ -254,6 +272,7 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
   std::vector<double> coef(2 * (size_t)(nsteps + 1));
   sch.eval(0.f, coef[0], coef[1]);
   for (int s = 1; s <= nsteps; ++s) sch.eval((float)s * dtf, coef[2 * s], coef[2 * s + 1]);
+  coef[0] = coef[1] = 0;  // (no step reads F(0); a fused first step finds the state at rest with it)
   StepWork &W = c->steps;
   StepVecs<T> &S = [&]() -> StepVecs<T> & {
     if constexpr (sizeof(T) == 8) return W.f64; else return W.f32;
@@ -263,8 +282,12 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
   }();
   W.coef.ensure(coef.size());
   CK(cudaMemcpyAsync(W.coef.p, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice, c->stream));
+  // FP32 edge fans with stored gradients: a step is one kernel (MV_STEP)
+  const bool fused = sizeof(T) == 4 && expl && c->fans && !c->geo;
   S.d.ensure(3 * (size_t)c->nvec);
-  for (auto *b : {&S.v, &S.a, &S.y}) b->ensure(c->nvec);
+  S.v.ensure((fused ? 2 : 1) * (size_t)c->nvec);
+  S.a.ensure((fused ? 2 : 1) * (size_t)c->nvec);
+  S.y.ensure((fused ? 3 : 1) * (size_t)c->nvec);
   S.minv.ensure(2 * (size_t)c->nvec);
   for (auto *b : {&S.d, &S.v, &S.a, &S.y}) b->zero(c->stream);
   T *const d0 = S.d.p, *const d1 = S.d.p + c->nvec;
@@ -400,6 +423,74 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
       }
       launch_steps(c, P);
       dcur = (nsteps & 1) ? d1 : d0;
+    }
+  } else if (fused) {
+    if constexpr (sizeof(T) == 4) {
+      // Step n: d_n from d_{n-1} and the state before it, whose acceleration and
+      // velocity are formed on the way from y_{n-1} = K' d_{n-1}. No kernel reads
+      // what it writes: d, v, a alternate between two buffers, y between three
+      // (read, accumulated, cleared for the next).
+      bool finite = true;
+      for (double q : coef) finite &= std::isfinite(q);
+      mv.load_all = !finite;
+      mv.c_old = dp.c_old;
+      mv.c_new = dp.c_new;
+      mv.FA = FA;
+      mv.FB = FB;
+      mv.coef = W.coef.p;
+      mv.st = W.st.p;
+      mv.recv = W.recv.p;
+      mv.n_recv = nrec;
+      mv.trace = W.trace.p;
+      mv.minv = resort ? S.minv.p : nullptr;
+      if (!resort) {
+        k_spread_lanes<<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, S.minv.p, d0, S.v.p, S.a.p);
+        CKL();
+      }
+      const size_t nv = c->nvec;
+      auto one_step = [&](int n) {
+        const int q = n & 1;  // (state n - 1 in buffer q ^ 1)
+        MvParams<float> m = mv;
+        m.parity = q ^ 1;
+        m.x = q ? d0 : d1;
+        m.xout = q ? d1 : d0;
+        m.x2 = S.v.p + (q ^ 1) * nv;
+        m.v_out = S.v.p + q * nv;
+        m.x3 = S.a.p + (q ^ 1) * nv;
+        m.a_out = S.a.p + q * nv;
+        m.y_prev = S.y.p + (n + 2) % 3 * nv;
+        m.y = S.y.p + n % 3 * nv;
+        m.yzero = S.y.p + (n + 1) % 3 * nv;
+        launch_mv_f(c, MV_STEP, m);
+        if (resort) slot_assemble_and_resort<T>(c, S.minv.p, 1);
+      };
+      int n = 1;
+      if (nsteps >= 2 * kStepCycle) {
+        cudaGraph_t g;
+        cudaGraphExec_t exec = nullptr;
+        CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+        try {
+          for (int k = 1; k <= kStepCycle; ++k) one_step(k);
+        } catch (...) {
+          cudaGraph_t broken = nullptr;
+          cudaStreamEndCapture(c->stream, &broken);
+          if (broken) cudaGraphDestroy(broken);
+          (void)cudaGetLastError();
+          throw;
+        }
+        CK(cudaStreamEndCapture(c->stream, &g));
+        CK(cudaGraphInstantiate(&exec, g, 0));
+        cudaGraphDestroy(g);
+        for (; n + kStepCycle - 1 <= nsteps; n += kStepCycle) CK(cudaGraphLaunch(exec, c->stream));
+        cudaGraphExecDestroy(exec);
+      }
+      for (; n <= nsteps; ++n) one_step(n);
+      dcur = (nsteps & 1) ? d1 : d0;
+      if (nrec) {
+        k_record<<<nblk(nrec * c->dim), kThreads, 0, c->stream>>>(nrec, c->dim, c->vw, W.recv.p, dcur,
+                                                                 W.trace.p + (size_t)(nsteps - 1) * nrec * c->dim);
+        CKL();
+      }
     }
   } else if (expl) {
     if constexpr (sizeof(T) == 4) {

@@ -130,7 +130,7 @@ struct RowsData {
 // Work buffers of the time-stepping calls, kept with the context.
 template <typename T>
 struct StepVecs {
-  DBuf<T> d, v, a, y, minv;  // d: two node vectors (three, FP32 implicit); minv: two when re-sorted
+  DBuf<T> d, v, a, y, minv;  // d: two node vectors (three, FP32 implicit); v, a: two, y: three (FP32 fused steps); minv: two when re-sorted
 };
 struct StepWork {
   StepVecs<double> f64;

@@ -504,7 +504,13 @@ __device__ __forceinline__ void tet_forces_acc(const T (&d1)[3], const T (&d2)[3
 }
 
 // ------------------------------------------------------------------ matvec
-enum MvMode { MV_PLAIN = 0, MV_PCG = 1, MV_DYN = 2 };
+// MV_STEP: a whole explicit GN22 step (edge fans): the acceleration and velocity
+// of the step before are formed where the predictor is staged
+enum MvMode { MV_PLAIN = 0, MV_PCG = 1, MV_DYN = 2, MV_STEP = 3 };
+
+// Block bits of a patch node: bit d: DOF d constrained; kLoadedBit: carries a
+// load part (FA or FB).
+constexpr unsigned kBcBits = 7u, kLoadedBit = 0x80u;
 
 // Control block of a batched solve (independent meshes).
 struct BatchCtl {
@@ -535,7 +541,19 @@ struct MvParams {
   double *partials;  // [gridDim] partial sums of p.Ap
   const double *up_part;  // PCG: r.z, r.r partials of the update before it, n_up blocks
   int n_up;
-  T c1, c2;          // DYN: d_new = d + c1 v + c2 a
+  T c1, c2;          // DYN, STEP: d_new = d + c1 v + c2 a
+  // STEP: a = (F - y_prev) M^-1, v = v_old + c_old a_old + c_new a with the y of
+  // the step before; M^-1 of the x, y, z DOF in the fourth lanes of d, v, a, or
+  // in minv (re-sorted masses); F of the loaded nodes from step pstep[parity] - 1
+  const T *y_prev, *minv, *FA, *FB;
+  T *v_out, *a_out;
+  T c_old, c_new;
+  const double *coef;
+  DynState *st;
+  int parity, load_all;
+  const int32_t *recv;  // receivers of the step before (d at x) into trace
+  int n_recv;
+  double *trace;
   const uint16_t *inc, *inc_start;  // per-patch incidence lists (prep.hpp)
   int pe, np_max;    // element slots per patch, node slots per patch (multiple of 4)
   // batch of independent meshes (all nullptr for a single mesh): every patch

@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(kHfanThreads, 3) k_matvec_fan_tma(MvParams<T> 
     // 1. stage node values: each thread issues the gathers of all its nodes
     //    (up to kStageUnroll) before using any of them
     constexpr int SU = kStageUnroll;
-    NodeV<T, VW> v[SU], w[SU], a3[SU];
+    NodeV<T, VW> v[SU], w[SU], a3[SU], yp[SU], mi[SU];
     int gi[SU];
     auto stage_load = [&](int i0, bool with_w) {
 #pragma unroll
@@ -382,8 +382,12 @@ __global__ void __launch_bounds__(kHfanThreads, 3) k_matvec_fan_tma(MvParams<T> 
         gi[q] = i < nn ? nodes[i] : -1;
         if (gi[q] >= 0) {
           v[q] = ldv<T, VW>(P.x, gi[q]);
-          if (with_w || MODE == MV_DYN) w[q] = ldv<T, VW>(P.x2, gi[q]);
-          if (MODE == MV_DYN) a3[q] = ldv<T, VW>(P.x3, gi[q]);
+          if (with_w || MODE >= MV_DYN) w[q] = ldv<T, VW>(P.x2, gi[q]);
+          if (MODE >= MV_DYN) a3[q] = ldv<T, VW>(P.x3, gi[q]);
+          if (MODE == MV_STEP) {
+            yp[q] = ldv<T, VW>(P.y_prev, gi[q]);
+            if (P.minv) mi[q] = ldv<T, VW>(P.minv, gi[q]);
+          }
         }
       }
     };
@@ -421,6 +425,33 @@ __global__ void __launch_bounds__(kHfanThreads, 3) k_matvec_fan_tma(MvParams<T> 
 #pragma unroll
           for (int d = 0; d < DIM; ++d) v[q].v[d] += P.c1 * w[q].v[d] + P.c2 * a3[q].v[d];
           if (i >= own) stv<T, VW>(P.xout, gi[q], v[q]);
+        } else if (MODE == MV_STEP) {
+          T F[DIM] = {0, 0, 0};
+          if ((bits[i] & kLoadedBit) || P.load_all) {  // (few nodes: the others skip two gathers)
+            const int step = P.st->pstep[P.parity] - 1;
+            const T ca = (T)P.coef[2 * step], cb = (T)P.coef[2 * step + 1];
+            const NodeV<T, VW> fa = ldv<T, VW>(P.FA, gi[q]), fb = ldv<T, VW>(P.FB, gi[q]);
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) F[d] = ca * fa.v[d] + cb * fb.v[d];
+          }
+          if (!P.minv) {
+            mi[q].v[0] = v[q].v[3];
+            mi[q].v[1] = w[q].v[3];
+            mi[q].v[2] = a3[q].v[3];
+          }
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) {
+            const T an = (F[d] - yp[q].v[d]) * mi[q].v[d];
+            w[q].v[d] += P.c_old * a3[q].v[d] + P.c_new * an;
+            a3[q].v[d] = an;
+            v[q].v[d] += P.c1 * w[q].v[d] + P.c2 * an;
+          }
+          if (i >= own) {
+            stv<T, VW>(P.xout, gi[q], v[q]);
+            stv<T, VW>(P.v_out, gi[q], w[q]);
+            stv<T, VW>(P.a_out, gi[q], a3[q]);
+            stv_zero<T, VW>(P.yzero, gi[q]);
+          }
         }
         const unsigned bb = bits[i];
         NodeV<T, VW> m;
@@ -574,9 +605,10 @@ __global__ void __launch_bounds__(kHfanThreads, 3) k_matvec_fan_tma(MvParams<T> 
         r.v[d] = val;
         any |= val != T(0);
       }
-      if (bb && i >= own) {
-        // (I - P) diag(A) x on the constrained DOFs of an owned node
-        NodeV<T, VW> v = ldv<T, VW>(P.x, g);
+      if ((bb & kBcBits) && i >= own) {
+        // (I - P) diag(A) x on the constrained DOFs of an owned node (STEP: this
+        // thread staged the node and wrote its d)
+        NodeV<T, VW> v = ldv<T, VW>(MODE == MV_STEP ? P.xout : P.x, g);
         if (MODE == MV_PCG && beta != T(0)) {
           NodeV<T, VW> po = ldv<T, VW>(P.x2, g);
 #pragma unroll
@@ -618,6 +650,15 @@ __global__ void __launch_bounds__(kHfanThreads, 3) k_matvec_fan_tma(MvParams<T> 
         if (patch + 2 * step < P.n_patches && patch_live(patch + 2 * step)) issue_copy(patch + 2 * step, b);
       }
     }
+  }
+  if (MODE == MV_STEP && blockIdx.x == 0) {
+    const int step = P.st->pstep[P.parity];
+    if (step >= 2)
+      for (int i = threadIdx.x; i < P.n_recv * DIM; i += kHfanThreads) {
+        const int r = i / DIM, k = i - r * DIM;
+        P.trace[((int64_t)(step - 2) * P.n_recv + r) * DIM + k] = (double)P.x[(int64_t)P.recv[r] * VW + k];
+      }
+    if (threadIdx.x == 0) P.st->pstep[P.parity ^ 1] = step + 1;
   }
   if (MODE == MV_PCG && !batch) {  // p.Ap partials; the update kernel forms sigma and alpha
     // (every warp is past the last patch's compute phase: the staging area is free)

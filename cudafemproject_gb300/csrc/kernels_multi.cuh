@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kHfanThreads, C <= 2 ? 3 : 2) k_matvec_multi(M
       out.v[3] = 0;
       const int g = nodes[i];
       const int64_t idx = (int64_t)g * K + c0 + cl;
-      if (bb && i >= own) {
+      if ((bb & kBcBits) && i >= own) {
         const NodeV<T, VW> v = ldv<T, VW>(MODE == MV_PCG ? pnew : x, idx);  // this block wrote pnew[idx] while staging
         const NodeV<T, VW> dg = ldv<T, VW>(P.diagA, g);
 #pragma unroll
