@@ -45,28 +45,23 @@ void destroy_multi(MultiState *m) { delete m; }
 namespace {
 
 template <int C>
-void launch_mvm(cfem_ctx *c, MultiState &M, int mode, const MultiParams<float> &P, const float *x, const float *pold,
+void launch_mvm(cfem_ctx *c, MultiState &M, const MultiParams<float> &P, const float *z, const float *pold,
                 float *pnew, float *y) {
-  dim3 g(M.grid_mv), b(kHfanThreads);
-  if (mode == MV_PCG) k_matvec_multi<MV_PCG, C><<<g, b, M.smem, c->stream>>>(P, x, pold, pnew, y);
-  else k_matvec_multi<MV_PLAIN, C><<<g, b, M.smem, c->stream>>>(P, x, pold, pnew, y);
+  launch_pdl(k_matvec_multi<C>, dim3(M.grid_mv), dim3(multi_threads(C)), M.smem, c->stream, P, z, pold, pnew, y);
   CKL();
   c->launches += 1;
 }
 
-void launch_mvm_c(cfem_ctx *c, MultiState &M, int mode, const MultiParams<float> &P, const float *x,
-                  const float *pold, float *pnew, float *y) {
-  if (M.C == 2) launch_mvm<2>(c, M, mode, P, x, pold, pnew, y);
-  else if (M.C == 4) launch_mvm<4>(c, M, mode, P, x, pold, pnew, y);
-  else launch_mvm<8>(c, M, mode, P, x, pold, pnew, y);
+void launch_mvm_c(cfem_ctx *c, MultiState &M, const MultiParams<float> &P, const float *z, const float *pold,
+                  float *pnew, float *y) {
+  if (M.C == 2) launch_mvm<2>(c, M, P, z, pold, pnew, y);
+  else if (M.C == 4) launch_mvm<4>(c, M, P, z, pold, pnew, y);
+  else launch_mvm<8>(c, M, P, z, pold, pnew, y);
 }
 
-template <int C>
-const void *mvm_kernel_c(int mode) {
-  return mode == MV_PCG ? (const void *)k_matvec_multi<MV_PCG, C> : (const void *)k_matvec_multi<MV_PLAIN, C>;
-}
-const void *mvm_kernel(int C, int mode) {
-  return C == 2 ? mvm_kernel_c<2>(mode) : C == 4 ? mvm_kernel_c<4>(mode) : mvm_kernel_c<8>(mode);
+const void *mvm_kernel(int C) {
+  return C == 2 ? (const void *)k_matvec_multi<2>
+                : C == 4 ? (const void *)k_matvec_multi<4> : (const void *)k_matvec_multi<8>;
 }
 
 MultiParams<float> multi_params(cfem_ctx *c, MultiState &M) {
@@ -75,6 +70,7 @@ MultiParams<float> multi_params(cfem_ctx *c, MultiState &M) {
   P.node_off = c->node_off.p;
   P.own = c->own.p;
   P.diagA = c->v32.diagA.p;
+  if (M.C) P.S = multi_smem(c->L32, M.C, M.K);
   P.lam = (float)c->lam;
   P.mu = (float)c->mu;
   P.K = M.K;
@@ -98,10 +94,9 @@ bool configure_c(cfem_ctx *c, MultiState &M, int C) {
   if (smem + 1024 > (size_t)optin) return false;  // (+ the kernel's static shared memory)
   M.C = C;
   M.smem = smem;
-  for (int mode : {MV_PLAIN, MV_PCG})
-    CK(cudaFuncSetAttribute(mvm_kernel(C, mode), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(cudaFuncSetAttribute(mvm_kernel(C), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int occ = 1;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mvm_kernel(C, MV_PCG), kHfanThreads, M.smem));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mvm_kernel(C), multi_threads(C), M.smem));
   const int64_t items = (int64_t)c->prep.n_patches * (M.K / C);
   M.grid_mv = (int)std::min<int64_t>(items, (int64_t)c->n_sm * std::max(occ, 1));
   if (M.graph) {
@@ -113,23 +108,31 @@ bool configure_c(cfem_ctx *c, MultiState &M, int C) {
 }
 
 // Cases per item: the variant with the shortest matvec on this mesh and
-// batch size, timed on the context's stream (PLAIN form, current vectors; the
-// best of three runs of four launches each). CFEM_MULTI_CASES=2|4|8 fixes it
+// batch size, timed on the context's stream (beta = 1 on f and a
+// zero direction; the best of three runs of four launches each). CFEM_MULTI_CASES=2|4|8 fixes it
 // (when that width fits in shared memory).
 void autotune_c(cfem_ctx *c, MultiState &M) {
   float best = 1e30f;
   int best_c = 0, forced = 0;
   if (const char *e = std::getenv("CFEM_MULTI_CASES")) forced = std::atoi(e);
   if ((forced != 2 && forced != 4 && forced != 8) || forced > M.K || !configure_c(c, M, forced)) forced = 0;
+  std::vector<MultiScalars> sc(M.K);
+  for (auto &m : sc) m.inv_gamma = m.sum_b[1][0] = m.sum_b[1][1] = 1.0;
+  MultiCtl ctl{};
+  ctl.rule = -1;  // (no stopping test)
+  ctl.maxit = 1 << 30;
+  ctl.iter = 1;
+  CK(cudaMemcpyAsync(M.sc.p, sc.data(), sizeof(MultiScalars) * M.K, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(M.ctl.p, &ctl, sizeof(MultiCtl), cudaMemcpyHostToDevice, c->stream));
   for (int C : {2, 4, 8}) {
     if (C > M.K) break;
     if (forced && C != forced) continue;
     if (!configure_c(c, M, C)) continue;
     MultiParams<float> P = multi_params(c, M);
-    launch_mvm_c(c, M, MV_PLAIN, P, M.f.p, nullptr, nullptr, M.u.p);  // warm-up
+    launch_mvm_c(c, M, P, M.f.p, M.pA.p, M.pB.p, M.u.p);  // warm-up
     for (int rep = 0; rep < 3; ++rep) {
       CK(cudaEventRecord(c->ev0, c->stream));
-      for (int i = 0; i < 4; ++i) launch_mvm_c(c, M, MV_PLAIN, P, M.f.p, nullptr, nullptr, M.u.p);
+      for (int i = 0; i < 4; ++i) launch_mvm_c(c, M, P, M.f.p, M.pA.p, M.pB.p, M.u.p);
       CK(cudaEventRecord(c->ev1, c->stream));
       CK(cudaEventSynchronize(c->ev1));
       float ms = 0;
@@ -174,7 +177,11 @@ MultiState &multi_state(cfem_ctx *c, int K) {
 
 void launch_vec(cfem_ctx *c, MultiState &M, const MultiParams<float> &P, const float *p, int init) {
   auto go = [&](auto k) {
-    k<<<M.grid_vec, kThreads, 0, c->stream>>>(P, M.x.p, M.r.p, M.z.p, p, M.u.p, M.f.p, c->v32.dinv.p, init);
+    if (init)
+      k<<<M.grid_vec, kThreads, 0, c->stream>>>(P, M.x.p, M.r.p, M.z.p, p, M.u.p, M.f.p, c->v32.dinv.p, init);
+    else
+      launch_pdl(k, dim3(M.grid_vec), dim3(kThreads), 0, c->stream, P, M.x.p, M.r.p, M.z.p, p, M.u.p, M.f.p,
+                 (const float *)c->v32.dinv.p, init);
   };
   if (P.cond) go(k_pcg_multi_vec<float, true>);
   else go(k_pcg_multi_vec<float>);
@@ -239,7 +246,7 @@ void run_pcg_multi(cfem_ctx *c, MultiState &M, int k_active, double tol, int rul
         Q.cond = cond;
         Q.cond_role = (it == 0 ? 1 : 0) | (it == c->chunk - 1 ? 2 : 0);
         Q.cond_chunk = c->chunk;
-        launch_mvm_c(c, M, MV_PCG, Q, M.z.p, pold, pnew, M.u.p);
+        launch_mvm_c(c, M, Q, M.z.p, pold, pnew, M.u.p);
         launch_vec(c, M, Q, pnew, 0);
       }
     };

@@ -2,13 +2,13 @@
 //
 // Node vectors hold all K cases of a node contiguously: [node][K][4] (K >= k,
 // a power of two <= kMaxCases; unused cases stay zero). The matvec works on
-// items (patch, chunk of C cases): the lanes of a warp hold C cases of 32 / C
-// half-fans, so a node's values for the chunk are one contiguous C x 16-byte
-// load, every gradient read from the patch block (kernels_fan_tma.cuh) is a
-// broadcast serving C cases, and the forces go to the block's node-sorted
-// force list ([entry][3][C]), whose runs the node sums add up without atomics. Every case has
-// its own PCG scalars and stopping test; a converged case is frozen (its items
-// are skipped once all C cases of a chunk are done).
+// items (patch, chunk of C cases): a thread holds two cases of a half-fan, so a
+// node's values for the chunk are one contiguous C x 16-byte load, every
+// gradient read from the patch block (kernels_fan_tma.cuh) is a broadcast
+// serving C cases, and the forces go to the block's node-sorted force list,
+// whose runs the node sums add up without atomics. Every case has its own PCG
+// scalars and stopping test; a converged case is frozen (its items are skipped
+// once all C cases of a chunk are done).
 #pragma once
 
 #include "kernels.cuh"
@@ -44,8 +44,15 @@ struct MultiCtl {  // shared by the cases of one solve
   int loop_ok, pad;
 };
 
+// Offsets into the shared memory of k_matvec_multi (multi_smem), formed on the
+// host: the kernel has no registers to spare for them.
+struct MultiSmem {
+  int tab, sp, en, red, bar, fs, beta, done, bytes;
+};
+
 template <typename T>
 struct MultiParams {
+  MultiSmem S;
   int n_patches;
   const int32_t *node_off, *own;
   const T *diagA;       // [node][4] diagonal of the operator (constrained DOFs)
@@ -60,19 +67,73 @@ struct MultiParams {
   FanTmaParams F;       // patch blocks (layout and fan offsets)
 };
 
-// Shared memory of k_matvec_multi<MODE, C> for K cases: the patch block, the
-// staged node values [npn][C][4], per-case energies [K] and warp partials
-// [8][C] (double), the mbarrier, the force list [kFanForces x kFanThreads][3][C],
-// per-case beta and done flags [K].
-struct MultiSmem {
-  int sp, en, red, bar, fs, beta, done, bytes;
+// Two planes of shared memory for vectors of case pairs: (x0 x1 y0 y1) and (z0 z1).
+struct PairPlanes {
+  float4 *a;
+  float2 *b;
+  __device__ __forceinline__ PairPlanes(unsigned char *base, int n)
+      : a(reinterpret_cast<float4 *>(base)), b(reinterpret_cast<float2 *>(base + (size_t)n * 16)) {}
+  __device__ __forceinline__ void load(int i, float2 (&v)[3]) const {
+    const float4 q = a[i];
+    v[0] = make_float2(q.x, q.y);
+    v[1] = make_float2(q.z, q.w);
+    v[2] = b[i];
+  }
+  __device__ __forceinline__ void store(int i, const float2 (&v)[3]) const {
+    a[i] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+    b[i] = v[2];
+  }
 };
-__host__ __device__ inline MultiSmem multi_smem(const FanBlockLayout &L, int C, int K) {
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+
+// tet_forces_acc for two cases at once: the same products and sums in the same
+// order, each a packed FP32 instruction.
+__device__ __forceinline__ void tet_forces_acc2(const float2 (&d1)[3], const float2 (&d2)[3], const float2 (&d3)[3],
+                                                const float (&G)[9], float lam, float mu, float2 (&f1)[3],
+                                                float2 (&f2)[3], float2 (&f3)[3]) {
+  float2 H[3][3], g[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) g[k] = dup2(G[k]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      H[i][j] = __ffma2_rn(d3[i], g[6 + j], __ffma2_rn(d2[i], g[3 + j], __fmul2_rn(d1[i], g[j])));
+  const float2 l2 = dup2(lam), m2 = dup2(mu), mm2 = dup2(mu + mu);
+  const float2 tr = __fmul2_rn(l2, __fadd2_rn(__fadd2_rn(H[0][0], H[1][1]), H[2][2]));
+  float2 S[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) S[i][i] = __ffma2_rn(mm2, H[i][i], tr);
+  S[0][1] = S[1][0] = __fmul2_rn(m2, __fadd2_rn(H[0][1], H[1][0]));
+  S[0][2] = S[2][0] = __fmul2_rn(m2, __fadd2_rn(H[0][2], H[2][0]));
+  S[1][2] = S[2][1] = __fmul2_rn(m2, __fadd2_rn(H[1][2], H[2][1]));
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    f1[i] = __ffma2_rn(S[i][2], g[2], __ffma2_rn(S[i][1], g[1], __ffma2_rn(S[i][0], g[0], f1[i])));
+    f2[i] = __ffma2_rn(S[i][2], g[5], __ffma2_rn(S[i][1], g[4], __ffma2_rn(S[i][0], g[3], f2[i])));
+    f3[i] = __ffma2_rn(S[i][2], g[8], __ffma2_rn(S[i][1], g[7], __ffma2_rn(S[i][0], g[6], f3[i])));
+  }
+}
+
+// Threads of a CTA of k_matvec_multi<C>: 16 warps per SM in either case (the
+// shared memory of 8 cases leaves one CTA per SM, that of 2 or 4 cases two).
+// 8 cases in 256 threads: 172 us per iteration of 32 cases of 331,776 tets, in
+// 512: 151 (then the fastest width; 4 cases: 171).
+__host__ __device__ constexpr int multi_threads(int C) { return C == 8 ? 512 : 256; }
+
+// Shared memory of k_matvec_multi<C> for K cases: the patch block, a second copy
+// of its header and node tables (fstart, nodes, bits), the staged node values
+// [npn][C / 2] (planes), per-case energies [K] and warp partials [warps][C]
+// (compensated pairs), the mbarrier, the force list
+// [kFanForces x kFanThreads][C / 2] (planes), per-case beta and done flags [K].
+inline MultiSmem multi_smem(const FanBlockLayout &L, int C, int K) {
   MultiSmem m{};
   int off = L.bytes;
-  m.sp = off; off += L.npn * C * 16;
+  m.tab = off; off += 16 + L.g_off - L.fstart_off;
+  m.sp = off; off += L.npn * (C / 2) * 24;
   m.en = off; off += K * 8;
-  m.red = off; off += (kHfanThreads / 32) * C * 8;
+  m.red = off; off += (multi_threads(C) / 32) * C * 8;
   m.bar = off; off += 16;
   m.fs = off; off += kFanForces * kFanThreads * 3 * C * 4;
   m.beta = off; off += K * 4;
@@ -81,35 +142,46 @@ __host__ __device__ inline MultiSmem multi_smem(const FanBlockLayout &L, int C, 
   return m;
 }
 
-// y_c += K' p_c for the K cases. PCG (MODE MV_PCG): p_c = z_c + beta_c p_old_c
-// staged on the fly (written back by the owning patch), sigma_c = p_c.K'p_c.
-// PLAIN: y_c += K' x_c. FP32 only (the patch blocks hold FP32 gradients).
+// u_c += K' p_c for the K cases, p_c = z_c + beta_c p_old_c staged on the fly
+// (written back by the owning patch), sigma_c = p_c.K'p_c; FP32 (the patch
+// blocks hold FP32 gradients).
 //
 // Items q = patch * (K / C) + chunk; CTA b takes the contiguous items
-// [n b / G, n (b + 1) / G), so the chunks of a patch reuse its block. Lane l of
-// warp w holds case l % C of half-fan (round * 8 + w) * (32 / C) + l / C: the
-// two halves of a fan are lanes l and l ^ C. A thread's case (l % C) is the
-// same in every phase, so its energy partial needs no exchange until the end
-// of the item.
-template <int MODE, int C>
-__global__ void __launch_bounds__(kHfanThreads, C <= 2 ? 3 : 2) k_matvec_multi(MultiParams<float> P, const float *x,
-                                                                  const float *pold, float *pnew, float *y) {
+// [n b / G, n (b + 1) / G), so the chunks of a patch reuse its block. A thread
+// works on two cases with packed FP32 instructions: lane l of warp w holds
+// cases 2 (l % CL), 2 (l % CL) + 1 (CL = C / 2) of half-fan
+// (round * warps + w) * (32 / CL) + l / CL; the two halves of a fan are lanes l
+// and l ^ CL. A thread's cases are the same in every phase, so its energy
+// partials need no exchange until the end of the item.
+//
+// Bound by the phases of an item (staging, half-fans, node sums) behind one
+// another with 16 warps per SM; issue slots are 41% used, shared memory 40%.
+// Two cases per thread cut the instructions of an iteration of 32 cases from
+// 21.9 M to 14.8 M per warp. One iteration, before and after: 32 cases of 98,304
+// tets 52.0 -> 46.2 us, 8 cases 19.7 -> 16.4, 4 cases 14.4 -> 12.7; 32 cases of
+// 331,776 tets 176 -> 148, 8 cases 43.8 -> 37.3. The registers are at their
+// limit: forms that spill 50 bytes or more lost all of it (the next chunk's
+// node values prefetched into registers, z formed here from r, the step to x
+// taken here).
+template <int C>
+__global__ void __launch_bounds__(multi_threads(C), 512 / multi_threads(C))
+    k_matvec_multi(MultiParams<float> P, const float *z, const float *pold, float *pnew, float *y) {
   using T = float;
-  constexpr int DIM = 3, VW = 4, NW = kHfanThreads / 32;
-  constexpr int HPW = 32 / C;                    // half-fans per warp and round
-  constexpr int ROUNDS = kHfanThreads / (NW * HPW);
-  constexpr int SU = C <= 2 ? 2 : 4;             // staging items in flight per thread
+  constexpr int DIM = 3, VW = 4, NT = multi_threads(C), NW = NT / 32;
+  constexpr int CL = C / 2;                      // lanes per half-fan
+  constexpr int HPW = 32 / CL;                   // half-fans per warp and round
+  constexpr int ROUNDS = kHfanThreads / (NW * HPW);  // (256 half-fans of a patch)
   static_assert(C == 2 || C == 4 || C == 8, "C: 2, 4 or 8 cases per item");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const FanBlockLayout &L = P.F.L;
   const int K = P.K, NC = K / C;
-  const MultiSmem S = multi_smem(L, C, K);
+  const MultiSmem &S = P.S;
   unsigned char *B = smem_raw;
-  T *sp = reinterpret_cast<T *>(smem_raw + S.sp);
+  const PairPlanes sp(smem_raw + S.sp, L.npn * CL);
   double *s_en = reinterpret_cast<double *>(smem_raw + S.en);
-  double *s_red = reinterpret_cast<double *>(smem_raw + S.red);
+  float2 *s_red = reinterpret_cast<float2 *>(smem_raw + S.red);
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw + S.bar);
-  T *fs = reinterpret_cast<T *>(smem_raw + S.fs);
+  const PairPlanes fs(smem_raw + S.fs, kFanForces * kFanThreads * CL);
   T *s_beta = reinterpret_cast<T *>(smem_raw + S.beta);
   int *s_done = reinterpret_cast<int *>(smem_raw + S.done);
   const int q = P.parity;
@@ -118,226 +190,305 @@ __global__ void __launch_bounds__(kHfanThreads, C <= 2 ? 3 : 2) k_matvec_multi(M
     s_done[c] = 0;
     s_beta[c] = 0;
   }
-  if (MODE == MV_PCG) {
-    // every CTA: beta and the stopping tests from the update's sums (one thread
-    // per case; K is at most the block size)
-    bool stop = true;
-    if (threadIdx.x < K) {
-      const int c = threadIdx.x;
-      MultiScalars &m = P.sc[c];
-      const int it = P.ctl->iter;
-      int done = m.done[q ^ 1];
-      double b = 0;
-      if (!done && it > 0) {
-        const double g = m.sum_b[q ^ 1][0], rr = m.sum_b[q ^ 1][1];
-        const int rule = P.ctl->rule;
-        const double v = rule == 0 ? g : rr, limit = rule == 0 ? m.gamma_stop : m.rr_stop;
-        if (!finite_bits(g) || !finite_bits(m.alpha)) done = 2;
-        else if (rule == 0 ? v < limit : rule == 1 && v <= limit) done = 1;
-        else if (it >= P.ctl->maxit) done = 3;
-        b = g * m.inv_gamma;
-        if (blockIdx.x == 0) {
-          m.gamma_prev = m.gamma;
-          m.gamma = g;
-          m.rr = rr;
-          m.beta = b;
-          m.iters = it;
-        }
-      }
-      if (blockIdx.x == 0) {
-        m.done[q] = done;
-        m.sum_b[q][0] = m.sum_b[q][1] = 0;
-      }
-      s_done[c] = done;
-      s_beta[c] = done ? T(0) : (T)b;
-      stop = done != 0;
+  const int64_t n_items = (int64_t)P.n_patches * NC;  // (an int: the items of a mesh that fits the memory)
+  const int q0 = (int)(n_items * blockIdx.x / gridDim.x), q1 = (int)(n_items * (blockIdx.x + 1) / gridDim.x);
+  // the first patch's block (static operator data) is on its way before the
+  // wait for the kernel before this one
+  // Block of patch p, the header and node tables into copy t.
+  auto issue_copy = [&](int p, int t) {
+    const unsigned char *src = P.F.blocks + (size_t)p * L.bytes;
+    mbar_expect_tx(&bar[0], (unsigned)L.bytes);
+    if (t == 0) {
+      bulk_load(B, src, (unsigned)L.bytes, &bar[0]);
+    } else {
+      bulk_load(smem_raw + S.tab, src, 16u, &bar[0]);
+      bulk_load(smem_raw + S.tab + 16, src + L.fstart_off, (unsigned)(L.g_off - L.fstart_off), &bar[0]);
+      bulk_load(B + L.slot_off, src + L.slot_off, (unsigned)(L.fstart_off - L.slot_off), &bar[0]);
+      bulk_load(B + L.g_off, src + L.g_off, (unsigned)(L.bytes - L.g_off), &bar[0]);
     }
-    const bool all = __syncthreads_and(stop);
-    if (blockIdx.x == 0 && threadIdx.x == 0) P.ctl->all_done = all;
-    if (all) return;
-  }
-  if (threadIdx.x == 0) {
-    mbar_init(&bar[0], 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  const uint16_t *fstart = reinterpret_cast<const uint16_t *>(B + L.fstart_off);
-  const int32_t *nodes = reinterpret_cast<const int32_t *>(B + L.nodes_off);
-  const uint8_t *bits = B + L.bits_off;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int cl = lane & (C - 1), hs = lane / C, h = hs & 1;
-  const T lam = P.lam, mu = P.mu;
-  const int64_t n_items = (int64_t)P.n_patches * NC;
-  const int64_t q0 = n_items * blockIdx.x / gridDim.x, q1 = n_items * (blockIdx.x + 1) / gridDim.x;
-  int cur = -1;
+  };
+  int coming = -1;  // patch whose copy has been issued and not waited for
   unsigned nload = 0;
-  for (int64_t item = q0; item < q1; ++item) {
-    const int patch = (int)(item / NC), c0 = (int)(item - (int64_t)patch * NC) * C;
-    if (MODE == MV_PCG) {
-      bool all = true;  // (uniform: read from shared memory)
+  if (q0 < q1) {
+    coming = q0 / NC;
+    if (threadIdx.x == 0) {
+      mbar_init(&bar[0], 1);
+      fence_mbar_init();
+      issue_copy(coming, 0);
+    }
+  }
+  griddep_wait();
+  // every CTA: beta and the stopping tests from the update's sums (one thread
+  // per case; K is at most the block size)
+  bool stop = true;
+  if (threadIdx.x < K) {
+    const int c = threadIdx.x;
+    MultiScalars &m = P.sc[c];
+    const int it = P.ctl->iter;
+    int done = m.done[q ^ 1];
+    double b = 0;
+    if (!done && it > 0) {
+      const double g = m.sum_b[q ^ 1][0], rr = m.sum_b[q ^ 1][1];
+      const int rule = P.ctl->rule;
+      const double v = rule == 0 ? g : rr, limit = rule == 0 ? m.gamma_stop : m.rr_stop;
+      if (!finite_bits(g) || !finite_bits(m.alpha)) done = 2;
+      else if (rule == 0 ? v < limit : rule == 1 && v <= limit) done = 1;
+      else if (it >= P.ctl->maxit) done = 3;
+      b = g * m.inv_gamma;
+      if (blockIdx.x == 0) {
+        m.gamma_prev = m.gamma;
+        m.gamma = g;
+        m.rr = rr;
+        m.beta = b;
+        m.iters = it;
+      }
+    }
+    if (blockIdx.x == 0) {
+      m.done[q] = done;
+      m.sum_b[q][0] = m.sum_b[q][1] = 0;
+    }
+    s_done[c] = done;
+    s_beta[c] = done ? T(0) : (T)b;
+    stop = done != 0;
+  }
+  const bool all = __syncthreads_and(stop);
+  if (blockIdx.x == 0 && threadIdx.x == 0) P.ctl->all_done = all;
+  if (all) {
+    if (threadIdx.x == 0 && coming >= 0) mbar_wait_bounded(&bar[0], 0u);  // (the copy lands before the CTA exits)
+    return;
+  }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int cl = lane & (CL - 1), hs = lane / CL, h = hs & 1;
+  const T lam = P.lam, mu = P.mu;
+  // next item from i on with a case still running (uniform: from shared memory)
+  auto next_live = [&](int i) {
+    for (; i < q1; ++i) {
+      const int c0 = i % NC * C;
+      bool all = true;
 #pragma unroll
       for (int r = 0; r < C; ++r) all &= s_done[c0 + r] != 0;
-      if (all) continue;
+      if (!all) break;
     }
+    return i;
+  };
+  int cur = -1, tab = 1;
+  // node tables of the current patch, in copy `tab`
+  auto table = [&](int off) { return smem_raw + (tab ? S.tab + 16 - L.fstart_off : 0) + off; };
+  auto node = [&](int i) { return reinterpret_cast<const int32_t *>(table(L.nodes_off))[i]; };
+  for (int item = next_live(q0), next; item < q1; item = next) {
+    next = next_live(item + 1);
+    if (next >= q1) griddep_launch_dependents();
+    const int patch = item / NC, c0 = (item - patch * NC) * C;
     if (patch != cur) {
-      fence_proxy_async();  // earlier reads of the block precede the copy that overwrites it
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        mbar_expect_tx(&bar[0], (unsigned)L.bytes);
-        bulk_load(B, P.F.blocks + (size_t)patch * L.bytes, (unsigned)L.bytes, &bar[0]);
+      bool ok = true;
+      tab ^= 1;
+      if (coming != patch) {
+        // (the first patch, all of its items skipped: a copy that nothing waited for)
+        if (coming >= 0) ok = mbar_wait_bounded(&bar[0], nload++ & 1u);
+        if (__syncthreads_or(!ok)) {
+          if (threadIdx.x == 0) *(volatile int *)P.F.err = kErrTmaTimeout;
+          return;
+        }
+        if (threadIdx.x == 0) issue_copy(patch, tab);
       }
-      const bool ok = mbar_wait_bounded(&bar[0], nload & 1u);
-      ++nload;
+      ok = mbar_wait_bounded(&bar[0], nload++ & 1u);
+      coming = -1;
       if (__syncthreads_or(!ok)) {
         if (threadIdx.x == 0) *(volatile int *)P.F.err = kErrTmaTimeout;
         return;
       }
       cur = patch;
     }
-    const int32_t *hdr = reinterpret_cast<const int32_t *>(B + L.hdr_off);
+    const int32_t *hdr = reinterpret_cast<const int32_t *>(smem_raw + (tab ? S.tab : L.hdr_off));
     const int nn = hdr[0], own = hdr[1];
-    const int n_it = nn * C;  // staging / output items (node i, case cl): it = i * C + cl
-    const T beta = MODE == MV_PCG ? s_beta[c0 + cl] : T(0);
-    const bool case_done = MODE == MV_PCG && s_done[c0 + cl] != 0;
+    const int n_it = nn * CL;  // staging / output items (node i, pair cl): it = i * CL + cl
+    const int cc = c0 + 2 * cl;  // this thread's cases: cc, cc + 1
+    T beta[2];
+    bool case_done[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      beta[j] = s_beta[cc + j];
+      case_done[j] = s_done[cc + j] != 0;
+    }
     // 1. stage the chunk's node values: C cases of a node are one contiguous load
-    for (int i0 = threadIdx.x; i0 < n_it; i0 += SU * kHfanThreads) {
-      NodeV<T, VW> v[SU], w[SU];
-      int gi[SU];
+    for (int it = threadIdx.x; it < n_it; it += NT) {
+      const int i = it / CL;
+      const int64_t idx = (int64_t)node(i) * K + cc;
+      NodeV<T, VW> v[2], w[2];
 #pragma unroll
-      for (int u = 0; u < SU; ++u) {
-        const int it = i0 + u * kHfanThreads;
-        gi[u] = it < n_it ? nodes[it / C] : -1;
-        if (gi[u] >= 0) {
-          const int64_t idx = (int64_t)gi[u] * K + c0 + cl;
-          v[u] = ldv<T, VW>(x, idx);
-          if (MODE == MV_PCG && beta != T(0)) w[u] = ldv<T, VW>(pold, idx);
-        }
+      for (int j = 0; j < 2; ++j) {
+        v[j] = ldv<T, VW>(z, idx + j);
+        if (beta[j] != T(0)) w[j] = ldv<T, VW>(pold, idx + j);
       }
 #pragma unroll
-      for (int u = 0; u < SU; ++u) {
-        if (gi[u] < 0) continue;
-        const int it = i0 + u * kHfanThreads, i = it / C;
-        if (MODE == MV_PCG) {
-          if (beta != T(0)) {
+      for (int j = 0; j < 2; ++j) {
+        if (beta[j] != T(0)) {
 #pragma unroll
-            for (int d = 0; d < DIM; ++d) v[u].v[d] += beta * w[u].v[d];
-          }
-          // a stopped case keeps its last direction (a continued refinement
-          // step starts from it); its lanes still compute, unused
-          if (i >= own && !case_done) stv<T, VW>(pnew, (int64_t)gi[u] * K + c0 + cl, v[u]);
+          for (int d = 0; d < DIM; ++d) v[j].v[d] += beta[j] * w[j].v[d];
         }
-        const unsigned bb = bits[i];
-        NodeV<T, VW> m;
-#pragma unroll
-        for (int d = 0; d < VW; ++d) m.v[d] = (d < DIM && !(bb >> d & 1u)) ? v[u].v[d] : T(0);
-        stv<T, VW>(sp, it, m);
+        // a stopped case keeps its last direction (a continued refinement
+        // step starts from it); its lanes still compute, unused
+        if (i >= own && !case_done[j]) stv<T, VW>(pnew, idx + j, v[j]);
       }
+      const unsigned bb = table(L.bits_off)[i];
+      float2 m[DIM];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d)
+        m[d] = (bb >> d & 1u) ? make_float2(0.f, 0.f) : make_float2(v[0].v[d], v[1].v[d]);
+      sp.store(it, m);
     }
     __syncthreads();
     // 2. half-fans: forces relative to P (missing tets have zero gradients),
     //    halves combined by shuffle, written to the force list
-    Comp32 energy;
+    Comp32 energy[2];
 #pragma unroll 1
     for (int rd = 0; rd < ROUNDS; ++rd) {
       const int hf = (rd * NW + wid) * HPW + hs;
       int slot[6];
       const int nk = load_half_slots(B + L.slot_off, hf, slot);
-      T du[6][DIM], fv[6][DIM];
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        NodeV<T, VW> s;
-#pragma unroll
-        for (int d = 0; d < VW; ++d) s.v[d] = 0;
-        if (k < nk) s = ldv<T, VW>(sp, slot[k] * C + cl);
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-          du[k][d] = s.v[d];
-          fv[k][d] = 0;
-        }
+      auto force_out = [&](int k, const float2 (&v)[DIM]) {
+        if (k < nk && half_writes(h, k)) fs.store(half_fpos(B + L.fpos_off, hf, k) * CL + cl, v);
+      };
+      auto xor2 = [](float2 v) {
+        return make_float2(__shfl_xor_sync(0xffffffffu, v.x, CL), __shfl_xor_sync(0xffffffffu, v.y, CL));
+      };
+      // The ring vertices go by one after another (a: R_jj, b: R_jj+1), each force
+      // written as soon as its two tets are done: 54 registers of node values
+      // and forces instead of 72.
+      float2 p0[DIM] = {}, dq[DIM] = {}, a[DIM] = {}, fq[DIM] = {}, fa[DIM] = {}, sum[DIM] = {}, r3[DIM];
+      if (nk) {
+        sp.load(slot[0] * CL + cl, p0);
+        sp.load(slot[1] * CL + cl, dq);
+        sp.load(slot[2] * CL + cl, a);
       }
-#pragma unroll
-      for (int k = 1; k < 6; ++k)
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) du[k][d] -= du[0][d];
-#pragma unroll
-      for (int jj = 0; jj < 3; ++jj) {
-        T G[9];
-        load_tet_G(B + L.g_off, hf, jj, G);
-        tet_forces_acc<T>(du[1], du[2 + jj], du[3 + jj], G, lam, mu, fv[1], fv[2 + jj], fv[3 + jj]);
-      }
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) fv[0][d] = -(fv[1][d] + fv[2][d] + fv[3][d] + fv[4][d] + fv[5][d]);
-      if (MODE == MV_PCG) {  // the forces sum to zero: sum_k u_k.f_k = sum_k>0 du_k.f_k
-        T e = 0;
-#pragma unroll
-        for (int k = 1; k < 6; ++k)
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) e += du[k][d] * fv[k][d];
-        energy.add(e);
-      }
-      combine_half_forces<T, DIM, C>(fv, h);
-#pragma unroll
-      for (int k = 0; k < 6; ++k)
-        if (k < nk && half_writes(h, k)) {
-          T *o = fs + half_fpos(B + L.fpos_off, hf, k) * (3 * C) + cl;
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) o[d * C] = fv[k][d];
-        }
-    }
-    __syncthreads();
-    // 3. node sums over contiguous force runs, constrained DOFs: (I - P) diag(A) p on owned nodes
-    for (int it = threadIdx.x; it < n_it; it += kHfanThreads) {
-      const int i = it / C;
-      const unsigned bb = bits[i];
-      T acc[DIM] = {0, 0, 0};
-      const int k1 = fstart[i + 1];
-      for (int k = fstart[i]; k < k1; ++k) {
-        const T *f = fs + k * (3 * C) + cl;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) acc[d] += f[d * C];
-      }
-      NodeV<T, VW> out;
-      bool any = false;
+      float2 e = make_float2(0.f, 0.f);
 #pragma unroll
       for (int d = 0; d < DIM; ++d) {
-        out.v[d] = (bb >> d & 1u) ? T(0) : acc[d];
-        any |= out.v[d] != T(0);
+        dq[d] = sub2(dq[d], p0[d]);
+        a[d] = sub2(a[d], p0[d]);
       }
-      out.v[3] = 0;
-      const int g = nodes[i];
-      const int64_t idx = (int64_t)g * K + c0 + cl;
-      if ((bb & kBcBits) && i >= own) {
-        const NodeV<T, VW> v = ldv<T, VW>(MODE == MV_PCG ? pnew : x, idx);  // this block wrote pnew[idx] while staging
-        const NodeV<T, VW> dg = ldv<T, VW>(P.diagA, g);
 #pragma unroll
-        for (int d = 0; d < DIM; ++d)
-          if (bb >> d & 1u) {
-            const T t = dg.v[d] * v.v[d];
-            out.v[d] = t;
-            any |= t != T(0);
-            if (MODE == MV_PCG) energy.add(t * v.v[d]);
-          }
+      for (int jj = 0; jj < 3; ++jj) {
+        float2 b[DIM] = {}, fb[DIM] = {};
+        if (3 + jj < nk) sp.load(slot[3 + jj] * CL + cl, b);
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) b[d] = sub2(b[d], p0[d]);
+        T G[9];
+        load_tet_G(B + L.g_off, hf, jj, G);
+        tet_forces_acc2(dq, a, b, G, lam, mu, fq, fa, fb);
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+          sum[d] = __fadd2_rn(sum[d], fa[d]);
+          e = __ffma2_rn(a[d], fa[d], e);
+          if (jj == 0) r3[d] = xor2(fa[d]);  // half 1's force on R_3, its first ring vertex
+        }
+        force_out(2 + jj, fa);
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+          a[d] = b[d];
+          fa[d] = fb[d];
+        }
       }
-      if (any) atomic_addv<T, VW>(y, idx, out, DIM);
+      // the forces sum to zero, and sum_k u_k.f_k = sum_k>0 du_k.f_k
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        sum[d] = __fadd2_rn(__fadd2_rn(sum[d], fa[d]), fq[d]);
+        e = __ffma2_rn(dq[d], fq[d], __ffma2_rn(a[d], fa[d], e));
+        sum[d] = make_float2(-sum[d].x, -sum[d].y);
+      }
+      energy[0].add(e.x);
+      energy[1].add(e.y);
+      // half 1's P, Q and R_3 forces go to half 0
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        const float2 p = xor2(sum[d]), q1 = xor2(fq[d]);
+        if (h == 0) {
+          sum[d] = __fadd2_rn(sum[d], p);
+          fq[d] = __fadd2_rn(fq[d], q1);
+          fa[d] = __fadd2_rn(fa[d], r3[d]);
+        }
+      }
+      force_out(0, sum);
+      force_out(1, fq);
+      force_out(5, fa);
     }
-    if (MODE == MV_PCG) {  // per-case energy of the item: lanes of one case, then warps in order
+    const bool change = next < q1 && next / NC != patch;
+    if (change) fence_proxy_async();  // reads of the block precede the copy that overwrites it
+    __syncthreads();
+    if (change) {  // slots, force positions and gradients are done with; the node tables have a second copy
+      coming = next / NC;
+      if (threadIdx.x == 0) issue_copy(coming, tab ^ 1);
+    }
+    // 3. node sums over contiguous force runs, constrained DOFs: (I - P) diag(A) p on owned nodes
+    for (int it = threadIdx.x; it < n_it; it += NT) {
+      const int i = it / CL;
+      const unsigned bb = table(L.bits_off)[i];
+      float2 acc[DIM] = {};
+      const uint16_t *fstart = reinterpret_cast<const uint16_t *>(table(L.fstart_off));
+      const int k1 = fstart[i + 1];
+#pragma unroll 4
+      for (int k = fstart[i]; k < k1; ++k) {
+        float2 f[DIM];
+        fs.load(k * CL + cl, f);
 #pragma unroll
-      for (int o = C; o < 32; o <<= 1) {
-        const float h2 = __shfl_xor_sync(0xffffffffu, energy.hi, o), l2 = __shfl_xor_sync(0xffffffffu, energy.lo, o);
-        energy.merge(h2, l2);
+        for (int d = 0; d < DIM; ++d) acc[d] = __fadd2_rn(acc[d], f[d]);
       }
-      if (lane < C) s_red[wid * C + lane] = (double)energy.hi + (double)energy.lo;
+      const int g = node(i);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        NodeV<T, VW> out;
+        bool any = false;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+          out.v[d] = (bb >> d & 1u) ? T(0) : j ? acc[d].y : acc[d].x;
+          any |= out.v[d] != T(0);
+        }
+        out.v[3] = 0;
+        const int64_t idx = (int64_t)g * K + cc + j;
+        if ((bb & kBcBits) && i >= own) {
+          const NodeV<T, VW> v = ldv<T, VW>(pnew, idx);  // this thread wrote pnew[idx] while staging
+          const NodeV<T, VW> dg = ldv<T, VW>(P.diagA, g);
+#pragma unroll
+          for (int d = 0; d < DIM; ++d)
+            if (bb >> d & 1u) {
+              const T t = dg.v[d] * v.v[d];
+              out.v[d] = t;
+              any |= t != T(0);
+              energy[j].add(t * v.v[d]);
+            }
+        }
+        if (any) atomic_addv<T, VW>(y, idx, out, DIM);
+      }
+    }
+    // per-case energy of the item: lanes of one case, then warps in order
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+#pragma unroll
+      for (int o = CL; o < 32; o <<= 1) {
+        const float h2 = __shfl_xor_sync(0xffffffffu, energy[j].hi, o);
+        const float l2 = __shfl_xor_sync(0xffffffffu, energy[j].lo, o);
+        energy[j].merge(h2, l2);
+      }
+      if (lane < CL) s_red[wid * C + 2 * lane + j] = make_float2(energy[j].hi, energy[j].lo);
     }
     __syncthreads();  // sp, fs and s_red of this item are complete
-    if (MODE == MV_PCG && threadIdx.x < 8 * C) {  // (a tree of eight lanes per case)
-      double t = s_red[(threadIdx.x & 7) * C + (threadIdx.x >> 3)];
+    // (a tree of eight lanes per case, in FP64; two warps do it while the others
+    // go on. FP64 conversions and sums in every warp before the barrier took
+    // a tenth of an item.)
+    if (threadIdx.x < 8 * C) {
+      const float2 e0 = s_red[(threadIdx.x & 7) * C + (threadIdx.x >> 3)];
+      double t = (double)e0.x + (double)e0.y;
+      if (NW > 8) {
+        const float2 e1 = s_red[((threadIdx.x & 7) + 8) * C + (threadIdx.x >> 3)];
+        t += (double)e1.x + (double)e1.y;
+      }
       const unsigned mask = C < 4 ? (1u << (8 * (C & 3))) - 1u : 0xffffffffu;
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(mask, t, o);
       if ((threadIdx.x & 7) == 0) s_en[c0 + (threadIdx.x >> 3)] += t;
     }
   }
-  if (MODE != MV_PCG) return;
+  if (threadIdx.x == 0 && coming >= 0) mbar_wait_bounded(&bar[0], nload & 1u);
   __syncthreads();
   for (int c = threadIdx.x; c < K; c += blockDim.x)
     if (!s_done[c]) atomicAdd(&P.sc[c].sum_a[q], s_en[c]);
@@ -375,6 +526,34 @@ __global__ void __launch_bounds__(kThreads) k_pcg_multi_vec(MultiParams<T> P, T 
   // thread 0: every thread reading the same lines would queue at one L2 slice
   __shared__ T s_alpha[kMaxCases];
   __shared__ int s_frozen[kMaxCases], s_all;
+  griddep_wait();
+  griddep_launch_dependents();  // the next matvec may start its first block copies
+  // U items per thread per round, all loads issued before any is used; the
+  // stride is a multiple of K, so every item of a thread is the same case. The
+  // first round's loads are issued before the scalars are formed (an FP64
+  // division in one warp takes longer than they do).
+  constexpr int U = 4;
+  const int64_t n_items = P.n_nodes * K;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  NodeV<T, VW> di[U], rv[U], xx[U], pp[U], uu[U];
+  auto load = [&]() {
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int64_t i = i0 + k * stride;
+      if (i >= n_items) continue;
+      di[k] = ldv<T, VW>(dinv, i / K);
+      if (init) {
+        rv[k] = ldv<T, VW>(f, i);
+      } else {
+        rv[k] = ldv<T, VW>(r, i);
+        xx[k] = ldv<T, VW>(xv, i);
+        pp[k] = ldv<T, VW>(p, i);
+        uu[k] = ldv<T, VW>(u, i);
+      }
+    }
+  };
+  load();
   if (threadIdx.x == 0) {
     s_all = init ? 0 : P.ctl->all_done;
     if constexpr (LOOP)
@@ -411,12 +590,7 @@ __global__ void __launch_bounds__(kThreads) k_pcg_multi_vec(MultiParams<T> P, T 
   const bool frozen = s_frozen[c] != 0;
   const T alpha = s_alpha[c];
   DotAcc<T> acc[3];  // r.z, r.r, f.f
-  const int64_t n_items = P.n_nodes * K;
-  // U items per thread per round, all loads issued before any is used; the
-  // stride is a multiple of K, so every item of a thread is case c
-  constexpr int U = 4;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < n_items; i0 += stride * U) {
+  for (bool loaded = true; i0 < n_items; i0 += stride * U, loaded = false) {
     NodeV<T, VW> zero;
 #pragma unroll
     for (int d = 0; d < VW; ++d) zero.v[d] = 0;
@@ -426,21 +600,7 @@ __global__ void __launch_bounds__(kThreads) k_pcg_multi_vec(MultiParams<T> P, T 
         if (i0 + k * stride < n_items) stv<T, VW>(u, i0 + k * stride, zero);
       continue;
     }
-    NodeV<T, VW> di[U], rv[U], xx[U], pp[U], uu[U];
-#pragma unroll
-    for (int k = 0; k < U; ++k) {
-      const int64_t i = i0 + k * stride;
-      if (i >= n_items) continue;
-      di[k] = ldv<T, VW>(dinv, i / K);
-      if (init) {
-        rv[k] = ldv<T, VW>(f, i);
-      } else {
-        rv[k] = ldv<T, VW>(r, i);
-        xx[k] = ldv<T, VW>(xv, i);
-        pp[k] = ldv<T, VW>(p, i);
-        uu[k] = ldv<T, VW>(u, i);
-      }
-    }
+    if (!loaded) load();
 #pragma unroll
     for (int k = 0; k < U; ++k) {
       const int64_t i = i0 + k * stride;

@@ -230,6 +230,35 @@ def test_multi_rhs_case_counts(monkeypatch, host_loop, k):
         assert max(rel(U[i], w[i] @ X) for i in range(k) if i != 1) <= 1e-8
 
 
+@pytest.mark.parametrize("live", [(0,), (1, 4), (-1,), (0, 3, -1)])
+@pytest.mark.parametrize("width,k", [(2, 32), (4, 64), (8, 64)])
+def test_multi_rhs_chunks_that_stop_early(monkeypatch, width, k, live):
+    """Several items per CTA (32 or more patches), load in some chunks of `width`
+    cases only: the others stop at once and their items are skipped, also where a
+    CTA starts and where its range crosses into the next patch. Every case within
+    1e-8 of the oracle, the cases without load exactly zero."""
+    from cudafemproject_gb300.solver import FemContext
+    monkeypatch.setenv("CFEM_MULTI_CASES", str(width))
+    p = meshgen.box_3d(6, 5, 17, jitter=0.2, seed=4)
+    o = O.Oracle(p, consistent=True).assemble()
+    rng = np.random.default_rng(width)
+    basis = rng.standard_normal((2, p.n_dof))
+    X = np.stack([o.pcg(b, tol=1e-13, rule=1)[0] for b in basis])
+    w = np.zeros((k, 2))
+    for chunk in live:
+        w.reshape(-1, width, 2)[chunk] = rng.standard_normal((width, 2))
+    w.reshape(-1, width, 2)[live[0]][1] = 0.0
+    ctx = FemContext(p, semantics="consistent", patch_elems=96)
+    for tol in (0.3, 1e-4):
+        U, infos = ctx.pcg_multi(w @ basis, precision="fp32_refine", tol=tol, stop_rule="residual", outer_tol=1e-10)
+        assert all(i["status"] == 0 for i in infos)
+        for i in range(k):
+            if w[i].any():
+                assert rel(U[i], w[i] @ X) <= 1e-8
+            else:
+                assert not U[i].any()
+
+
 def test_fp32_implicit_step_that_fails_keeps_the_state_before_it():
     """Steps are queued one ahead: when a step's PCG does not converge, the result is
     the displacement before that step, as when every step is waited for."""
