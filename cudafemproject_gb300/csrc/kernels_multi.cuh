@@ -17,6 +17,12 @@
 namespace cfem {
 
 constexpr int kMaxCases = 256;
+constexpr int kReached = 5;
+// A case that runs on with the others stops at this part of its (squared) limit,
+// an order below the tolerance in the norm: where the FP32 recurrence is still
+// the true residual.
+constexpr double kReachedFloor = 1e-2;
+__host__ __device__ inline bool case_stopped(int done) { return done != 0 && done != kReached; }
 
 // Scalars of a case. The two kernels of an iteration pass their per-case sums
 // on as FP64 atomic additions and every CTA of the kernel behind derives what
@@ -32,7 +38,10 @@ struct MultiScalars {
   double gamma, gamma_prev, gamma0, sigma, alpha, beta, rr, ff;
   double gamma_stop, rr_stop, inv_gamma;  // tol gamma0, (tol ||f||)^2, 1 / gamma
   double sum_a[2], sum_b[2][2];
-  int done[2], iters;  // done: 0 running, 1 converged, 2 diverged, 3 iteration cap
+  // done: 0 running, 1 converged, 2 diverged, 3 iteration cap, 4 stopped by the
+  // others, kReached: the test has been met, running on with the others (a norm
+  // may rise again: at the end of the round it counts as it is then)
+  int done[2], iters;
   int pad;
 };
 
@@ -41,7 +50,8 @@ struct MultiCtl {  // shared by the cases of one solve
   int rule, maxit, iter, all_done;
   int k_active;     // cases 0..k_active-1 are real, the rest are padding
   int loops;        // graph loop: bodies started in this run
-  int loop_ok, pad;
+  int loop_ok;
+  int quorum;       // cases that meet the test or are stopped (padding included) at which all stop, see MultiCont
 };
 
 // Offsets into the shared memory of k_matvec_multi (multi_smem), formed on the
@@ -220,19 +230,21 @@ __global__ void __launch_bounds__(multi_threads(C), 512 / multi_threads(C))
   griddep_wait();
   // every CTA: beta and the stopping tests from the update's sums (one thread
   // per case; K is at most the block size)
-  bool stop = true;
+  int done = 0;
+  bool met = false;  // the test, in this iteration
+  double b = 0;
   if (threadIdx.x < K) {
     const int c = threadIdx.x;
     MultiScalars &m = P.sc[c];
     const int it = P.ctl->iter;
-    int done = m.done[q ^ 1];
-    double b = 0;
-    if (!done && it > 0) {
+    done = m.done[q ^ 1];
+    if (!case_stopped(done) && it > 0) {
       const double g = m.sum_b[q ^ 1][0], rr = m.sum_b[q ^ 1][1];
       const int rule = P.ctl->rule;
       const double v = rule == 0 ? g : rr, limit = rule == 0 ? m.gamma_stop : m.rr_stop;
       if (!finite_bits(g) || !finite_bits(m.alpha)) done = 2;
-      else if (rule == 0 ? v < limit : rule == 1 && v <= limit) done = 1;
+      else if ((met = rule == 0 ? v < limit : rule == 1 && v <= limit))
+        done = P.ctl->quorum <= K && v > kReachedFloor * limit ? kReached : 1;
       else if (it >= P.ctl->maxit) done = 3;
       b = g * m.inv_gamma;
       if (blockIdx.x == 0) {
@@ -243,15 +255,19 @@ __global__ void __launch_bounds__(multi_threads(C), 512 / multi_threads(C))
         m.iters = it;
       }
     }
-    if (blockIdx.x == 0) {
-      m.done[q] = done;
-      m.sum_b[q][0] = m.sum_b[q][1] = 0;
-    }
-    s_done[c] = done;
-    s_beta[c] = done ? T(0) : (T)b;
-    stop = done != 0;
   }
-  const bool all = __syncthreads_and(stop);
+  const int n_done = __syncthreads_count(done != 0);
+  if (threadIdx.x < K) {
+    const int c = threadIdx.x;
+    if (n_done >= P.ctl->quorum && P.ctl->iter > 0 && !case_stopped(done)) done = met ? 1 : 4;
+    if (blockIdx.x == 0) {
+      P.sc[c].done[q] = done;
+      P.sc[c].sum_b[q][0] = P.sc[c].sum_b[q][1] = 0;
+    }
+    s_done[c] = case_stopped(done);
+    s_beta[c] = case_stopped(done) ? T(0) : (T)b;
+  }
+  const bool all = __syncthreads_and(threadIdx.x >= K || case_stopped(done));
   if (blockIdx.x == 0 && threadIdx.x == 0) P.ctl->all_done = all;
   if (all) {
     if (threadIdx.x == 0 && coming >= 0) mbar_wait_bounded(&bar[0], 0u);  // (the copy lands before the CTA exits)
@@ -568,7 +584,7 @@ __global__ void __launch_bounds__(kThreads) k_pcg_multi_vec(MultiParams<T> P, T 
   }
   for (int cc = threadIdx.x; cc < K; cc += blockDim.x) {
     MultiScalars &m = P.sc[cc];
-    const int fz = !init && m.done[q];
+    const int fz = !init && case_stopped(m.done[q]);
     double alpha = 0;
     if (!init && !fz) {
       const double sigma = m.sum_a[q];
@@ -659,17 +675,22 @@ __global__ void __launch_bounds__(kThreads) k_pcg_multi_vec(MultiParams<T> P, T 
   }
 }
 
-// After the init kernel: the scalars of every case (one block).
-static __global__ void __launch_bounds__(kMaxCases) k_multi_start(MultiScalars *sc, MultiCtl *ctl, int K) {
+// After the init kernel: the scalars of every case (one block). ref: per case
+// ||f||^2 and r.z that the stopping test refers to instead of this run's own
+// (0: its own; null: none), the start of a refinement step that goes on.
+static __global__ void __launch_bounds__(kMaxCases)
+    k_multi_start(MultiScalars *sc, MultiCtl *ctl, int K, const double *ref) {
   const int c = threadIdx.x;
   bool stop = true;
   if (c < K) {
     MultiScalars &m = sc[c];
-    const double g = m.sum_b[0][0], rr = m.sum_b[0][1], ff = m.sum_a[0], lim = ctl->tol * sqrt(ff);
+    const double g = m.sum_b[0][0], rr = m.sum_b[0][1], ff = m.sum_a[0];
+    const bool resumed = ref && ref[2 * c] > 0;
+    const double lim = ctl->tol * sqrt(resumed ? ref[2 * c] : ff);
     m.gamma0 = m.gamma = m.gamma_prev = g;
     m.rr = rr;
     m.ff = ff;
-    m.gamma_stop = ctl->tol * g;
+    m.gamma_stop = ctl->tol * (resumed ? ref[2 * c + 1] : g);
     m.rr_stop = lim < 0 ? -1.0 : lim * lim;  // (a negative tol stops nothing)
     m.iters = 0;
     m.sigma = m.alpha = m.beta = 0;

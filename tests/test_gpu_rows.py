@@ -259,6 +259,47 @@ def test_multi_rhs_chunks_that_stop_early(monkeypatch, width, k, live):
                 assert not U[i].any()
 
 
+@pytest.mark.parametrize("rule", ["residual", "reference"])
+@pytest.mark.parametrize("tol", [0.2, 0.5])
+@pytest.mark.parametrize("k", [2, 9, 33])
+def test_multi_rhs_rounds_end_together(k, tol, rule):
+    """Loose inner tolerances: cases that reach theirs run on until the round ends,
+    the others resume. With a case solved in one iteration (load on constrained
+    DOFs only), one without load, and loads of very different size; every case
+    within 1e-8 of the oracle. Too few refinement steps, and runs that end at the
+    iteration cap: no more steps than asked for, and the case says so."""
+    from cudafemproject_gb300.solver import FemContext
+    p = meshgen.box_3d(5, 4, 15, jitter=0.2, seed=6)
+    o = O.Oracle(p, consistent=True).assemble()
+    rng = np.random.default_rng(k)
+    basis = rng.standard_normal((3, p.n_dof))
+    fixed = np.zeros((p.n_nodes, 3), dtype=bool)
+    fixed[p.cons[:, 0]] = True  # (the mesh clamps whole nodes)
+    fixed = fixed.ravel()
+    assert fixed.any()
+    basis[2][~fixed] = 0.0
+    X = np.stack([o.pcg(b, tol=1e-13, rule=1)[0] for b in basis])
+    w = np.zeros((k, 3))
+    w[:, :2] = rng.standard_normal((k, 2)) * 10.0 ** rng.uniform(-3, 3, size=(k, 1))
+    w[0] = (0.0, 0.0, 1.0)
+    if k > 2:
+        w[3] = 0.0
+    F = w @ basis
+    ctx = FemContext(p, semantics="consistent")
+    kw = dict(precision="fp32_refine", tol=tol, stop_rule=rule, outer_tol=1e-10)
+    U, infos = ctx.pcg_multi(F, max_outer=400, **kw)
+    assert all(i["status"] == 0 and i["rel_residual"] <= 1e-10 for i in infos)
+    for i in range(k):
+        if w[i].any():
+            assert rel(U[i], w[i] @ X) <= 1e-8
+        else:
+            assert not U[i].any()
+    for cap in (100000, 7):
+        U, infos = ctx.pcg_multi(F, max_iter=cap, max_outer=2, allow_not_converged=True, **kw)
+        assert np.isfinite(U).all() and all(i["outer_iterations"] <= 2 for i in infos)
+        assert infos[1]["status"] != 0 and infos[0]["status"] == 0
+
+
 def test_fp32_implicit_step_that_fails_keeps_the_state_before_it():
     """Steps are queued one ahead: when a step's PCG does not converge, the result is
     the displacement before that step, as when every step is waited for."""
