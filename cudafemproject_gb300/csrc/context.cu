@@ -256,7 +256,7 @@ bool add_loop(cfem_ctx *c, cudaGraph_t graph, unsigned initial, const std::funct
 // scalars can be read behind it); false where the loop runs on the host and
 // only its graph has been built. chunk: iterations per loop body.
 bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
-                 const float *cont_p, double cont_gamma_prev, int chunk) {
+                 const PcgCont *cont, int chunk) {
   Vecs<float> &V = c->v32;
   const PcgSite S = whole_mesh(c);
   Scalars *sc = S.sc;
@@ -264,6 +264,11 @@ bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, 
   h.tol = tol;
   h.rule = rule;
   h.maxit = maxit > 0 ? maxit : 1000000;
+  if (cont) {
+    h.leg = cont->leg;
+    h.ref_gamma = cont->ref_gamma;
+    h.ref_ff = cont->ref_ff;
+  }
   CK(cudaMemcpyAsync(sc, &h, sizeof(Scalars), cudaMemcpyHostToDevice, c->stream));
   const MvParams<float> mv = site_mv(c, S, cK, cM, mcoef);
   if (warm) {
@@ -274,13 +279,16 @@ bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, 
     launch_mv_f(c, MV_PLAIN, m);
   }
   launch_init(c, vec_params(c, S, V.pA.p, V.u.p), warm);
-  if (cont_p && cont_gamma_prev > 0) {
+  if (cont && cont->p && cont->gamma_prev > 0) {
     // Continuation of an earlier run on a new residual: its last direction
     // p_last stays, and the first direction becomes the conjugate-gradient
     // step from it, z + (gamma / gamma_prev) p_last, folded into z here (the
     // first matvec takes p = z).
-    if (c->dim == 3) k_fold_direction<float, 3><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, sc, cont_gamma_prev, cont_p, V.z.p);
-    else k_fold_direction<float, 2><<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, sc, cont_gamma_prev, cont_p, V.z.p);
+    auto fold = [&](auto k) {
+      k<<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, sc, cont->gamma_prev, cont->gamma, cont->p, V.z.p);
+    };
+    if (c->dim == 3) fold(k_fold_direction<float, 3>);
+    else fold(k_fold_direction<float, 2>);
     CKL();
     c->launches += 1;
   }
@@ -348,10 +356,10 @@ PcgResult pcg_result(const Scalars &s) {
 }
 
 PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
-                    const float *cont_p, double cont_gamma_prev, const std::function<void()> &then) {
+                    const PcgCont *cont, const std::function<void()> &then) {
   Scalars *sc = c->sc.p + 1;
   const GraphCache &gc = c->graph32;
-  if (queue_pcg_f(c, cK, cM, mcoef, warm, tol, rule, maxit, cont_p, cont_gamma_prev, c->chunk)) {
+  if (queue_pcg_f(c, cK, cM, mcoef, warm, tol, rule, maxit, cont, c->chunk)) {
     if (then) then();
     CK(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -479,29 +487,42 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
     int outer = 0, total = 0;
     status = CFEM_ERR_NOT_CONVERGED;
     double rr_prev = -1;
-    int cont_iters = 0;  // iterations of the previous FP32 run (0: start the next one afresh)
-    double cont_gprev = 0;
     const double stall = refine_stall_ratio(prm->tol);
     int stalls = 0;
+    // Every FP32 run takes over the direction of the run before (the step it
+    // ended on was taken with gamma_prev; iteration i writes its direction to pB
+    // when i is even, to pA when odd) unless the recurrence had drifted off the
+    // FP64 residual (kMaxDrift): the true residual replaces the recursive one and
+    // the Krylov directions found so far keep serving.
+    // A step with a tight inner tolerance runs as several legs, each down to
+    // kLegFactor or kLegIterations long, so that the recurrence is replaced before
+    // it drifts off and loses its directions. To 1e-9 with an inner tolerance of
+    // 1e-3, one run per step started afresh, and so: 2.65 M tets 7062 -> 4800-5200
+    // iterations (319 -> 223-241 ms), 98,304 tets 2421 -> 1283 (22.3 -> 13.1),
+    // 786,432 tets 4334 -> 2650 (87 -> 56), a Delaunay mesh 2811 -> 1377-1459
+    // (30.9 -> 17.8). Longer legs than 512 lose 4% on the first of these, shorter
+    // ones (256) 13% on the last.
+    PcgCont cont;
+    const bool legs = prm->tol > 0 && ((prm->stop_rule == 0 && prm->tol < kLegFactor) ||
+                                       (prm->stop_rule == 1 && prm->tol * prm->tol < kLegFactor));
+    const int cap = prm->max_iter > 0 ? prm->max_iter : 1000000;
+    bool in_step = false, first = true;
+    int step_iters = 0;
     while (outer < max_outer) {
-      if (std::sqrt(rr) <= outer_tol * std::sqrt(ff)) { status = CFEM_OK; break; }
-      // The FP64 true residual has a floor near eps64 * ||K|| ||x||; once two
-      // refinement steps in a row no longer reduce it as a step should (halve
-      // it; a continued step reduces it by about the replacement factor tol)
-      // the iterate is converged in FP64. (One such step alone can be an FP32
-      // run that ended early, well above the floor.)
-      stalls = rr_prev >= 0 && rr > stall * rr_prev ? stalls + 1 : 0;
-      if (stalls >= 2) { status = CFEM_OK; break; }
-      rr_prev = rr;
-      // With a loose inner tolerance (a residual-replacement factor, at least
-      // kContinueTol), from the second step on the FP32 PCG continues with its
-      // last direction (the step it ended on was taken with gamma_prev;
-      // iteration i writes its direction to pB when i is even, to pA when odd)
-      // instead of restarting from z: the FP64 true residual replaces the
-      // recursive one and the Krylov directions found so far keep serving.
-      // Replaced seldom, the recursive residual drifts too far from the true
-      // one for the old direction to stay conjugate, so tighter inner
-      // tolerances restart.
+      // (within a step with some margin: one run per step ended anywhere below)
+      if (std::sqrt(rr) <= (in_step ? 0.25 : 1.0) * outer_tol * std::sqrt(ff)) { status = CFEM_OK; break; }
+      if (!in_step) {
+        // The FP64 true residual has a floor near eps64 * ||K|| ||x||; once two
+        // refinement steps in a row no longer reduce it as a step should (halve
+        // it; a continued step reduces it by about the replacement factor tol)
+        // the iterate is converged in FP64. (One such step alone can be an FP32
+        // run that ended early, well above the floor.)
+        stalls = rr_prev >= 0 && rr > stall * rr_prev ? stalls + 1 : 0;
+        if (stalls >= 2) { status = CFEM_OK; break; }
+        rr_prev = rr;
+        step_iters = 0;
+        cont.ref_gamma = cont.ref_ff = 0;
+      }
       // behind the run, without waiting for it: x64 += d and the true residual
       // (its norms arrive with the run's scalars)
       auto then = [&]() {
@@ -509,21 +530,45 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
         CKL();
         true_residual_async(c, c->v64.f.p, c->v64.x.p, c->v64.r.p, c->v32.f.p, c->h_rr);
       };
-      PcgResult r = cont_iters > 0 && prm->tol >= kContinueTol
-                        ? run_pcg_f(c, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, prm->max_iter,
-                                           ((cont_iters - 1) & 1) ? c->v32.pA.p : c->v32.pB.p, cont_gprev, then)
-                        : run_pcg_f(c, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, prm->max_iter,
-                                           nullptr, 0, then);
-      cont_iters = r.status == CFEM_OK || r.status == CFEM_ERR_NOT_CONVERGED ? r.iters : 0;
-      cont_gprev = r.gamma_prev;
+      cont.leg = legs ? kLegFactor : 0;
+      const int maxit = legs ? std::min(kLegIterations, cap - step_iters) : cap;
+      const PcgResult r = run_pcg_f(c, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, maxit, &cont, then);
+      if (r.iters > 0) {  // (none: the last direction is still that of the run before)
+        cont.p = ((r.iters - 1) & 1) ? c->v32.pA.p : c->v32.pB.p;
+        cont.gamma_prev = r.gamma_prev;
+        cont.gamma = r.gamma;
+      }
       total += r.iters;
-      if (outer == 0) inf.gamma0 = r.gamma0;
+      step_iters += r.iters;
+      if (first) inf.gamma0 = r.gamma0;
+      first = false;
       inf.gamma = r.gamma;
-      if (r.status == CFEM_ERR_DIVERGED) { status = CFEM_ERR_DIVERGED; break; }
-      ++outer;
+      if (r.status == CFEM_ERR_DIVERGED) {
+        in_step = false;
+        status = CFEM_ERR_DIVERGED;
+        break;
+      }
+      const double rr_leg = rr;
       rr = ((volatile double *)c->h_rr)[0];
       ff = ((volatile double *)c->h_rr)[1];
+      bool step_done = true;
+      if (legs) {
+        if (!in_step) {
+          cont.ref_gamma = r.gamma0;
+          cont.ref_ff = r.ff;
+        }
+        // the step ends where its one run would have: at its tolerance or at the
+        // iteration cap; or at a leg that reduced the recurrence only (for a leg of
+        // rule 1 the first part implies the second)
+        const bool met = prm->stop_rule == 1 ? r.rr <= prm->tol * prm->tol * cont.ref_ff * (1 + 1e-9)
+                                             : r.gamma <= prm->tol * cont.ref_gamma * (1 + 1e-9);
+        const bool lost = rr > kLegStall * rr_leg && rr > kLegStall / kLegFactor * r.rr;
+        step_done = r.status == CFEM_OK ? met || lost : step_iters >= cap;
+      }
+      in_step = !step_done;
+      outer += step_done;
     }
+    outer += in_step;  // (converged within a step)
     rr_end = rr;
     ff_end = ff;
     if (status != CFEM_OK && std::sqrt(rr) <= outer_tol * std::sqrt(ff)) status = CFEM_OK;

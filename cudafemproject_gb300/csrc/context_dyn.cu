@@ -588,7 +588,7 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
       };
       for (int s = 1; s <= nsteps; ++s) {
         before(buf[(s - 1) % 3], buf[s % 3]);
-        if (!queue_pcg_f(c, opK, opM, opmc, warm, tol, rule, prm->max_iter, nullptr, 0, chunk)) {
+        if (!queue_pcg_f(c, opK, opM, opmc, warm, tol, rule, prm->max_iter, nullptr, chunk)) {
           pipelined = false;  // (s == 1: no device loop here; the step starts over below)
           break;
         }

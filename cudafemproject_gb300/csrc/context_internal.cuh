@@ -267,10 +267,24 @@ namespace detail {
 // direction across the refinement steps (the tolerance is then the factor by
 // which its recursive residual drops between FP64 true-residual replacements).
 constexpr double kContinueTol = 0.2;
+// Legs of a refinement step: gamma and ||r||^2 fall by this factor (the norm by
+// kContinueTol), or this many iterations.
+constexpr double kLegFactor = kContinueTol * kContinueTol;
+constexpr int kLegIterations = 512;
+constexpr double kLegStall = 0.25;  // a leg that leaves more of the true ||r||^2 than this was at its floor
 // A refinement step whose FP64 residual norm^2 falls by less than this is at
 // the FP64 floor: a step cuts the norm by about the inner tolerance tol (at
 // least halves it for tol up to 0.25), so the test allows twice that.
 inline double refine_stall_ratio(double tol) { return std::min(0.9, std::max(0.25, 4.0 * tol * tol)); }
+
+// What a run of the FP32 PCG takes over from the one before: the last direction
+// (p, nullptr: none) with the gamma its step length was formed with and the last
+// one; and its place in a refinement step (Scalars::leg).
+struct PcgCont {
+  const float *p = nullptr;
+  double gamma_prev = 0, gamma = 0;
+  double leg = 0, ref_gamma = 0, ref_ff = 0;
+};
 
 struct PcgResult {
   int status = CFEM_OK;
@@ -285,10 +299,9 @@ void launch_mv_f(cfem_ctx *c, int mode, const MvParams<float> &P);
 PcgResult run_pcg_d(cfem_ctx *c, Vecs<double> &V, double cK, double cM, const double *mcoef, int warm, double tol,
                     int rule, int maxit);
 PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
-                    const float *cont_p = nullptr, double cont_gamma_prev = 0,
-                    const std::function<void()> &then = nullptr);
+                    const PcgCont *cont = nullptr, const std::function<void()> &then = nullptr);
 bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
-                 const float *cont_p, double cont_gamma_prev, int chunk);
+                 const PcgCont *cont, int chunk);
 PcgResult pcg_result(const Scalars &s);
 struct PcgSite {
   Scalars *sc;

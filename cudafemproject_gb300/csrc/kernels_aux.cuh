@@ -175,13 +175,20 @@ static __global__ void k_axpby64(int64_t n, double a, const double *x, double b,
   if (i < n) y[i] = a * x[i] + b * y[i];
 }
 
+// A recurrence whose gamma = r.M^-1 r is this far below that of the FP64 residual
+// no longer knows the residual (1.1 in the norm): the direction it ended with is
+// conjugate to nothing, and beta = gamma / gamma_prev would hold on to it.
+constexpr double kMaxDrift = 1.21;
+
 // Continued PCG run: z += (gamma / gamma_prev) p_last on the DOF lanes (the
 // fourth lane carries M^-1, see k_pcg_init), gamma from the init kernel's
-// scalars (nothing to do once they say done).
+// scalars (nothing to do once they say done, or where the recurrence that ended
+// with gamma_last had drifted off).
 template <typename T, int DIM>
-__global__ void k_fold_direction(int64_t nn, const Scalars *sc, double gamma_prev, const T *p_last, T *z) {
+__global__ void k_fold_direction(int64_t nn, const Scalars *sc, double gamma_prev, double gamma_last,
+                                 const T *p_last, T *z) {
   constexpr int VW = DIM == 3 ? 4 : 2;
-  if (sc->done) return;
+  if (sc->done || sc->gamma > kMaxDrift * gamma_last) return;
   const T beta = (T)(sc->gamma / gamma_prev);
   int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= nn) return;
