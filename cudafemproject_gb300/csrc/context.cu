@@ -231,13 +231,22 @@ bool add_loop(cfem_ctx *c, cudaGraph_t graph, unsigned initial, const std::funct
     v.resize(n);
     return n == 0 || cudaGraphGetNodes(graph, v.data(), &n) == cudaSuccess;
   };
-  // the prologue is one kernel: the node it adds is the loop's dependency
+  // the prologue is a chain of kernels: the last node it adds is the loop's dependency
   cudaGraphNode_t dep{};
   if (prologue) {
     std::vector<cudaGraphNode_t> before, after;
-    if (!nodes(before) || !record(graph, prologue) || !nodes(after) || after.size() != before.size() + 1) return false;
-    for (cudaGraphNode_t v : after)
-      if (std::find(before.begin(), before.end(), v) == before.end()) dep = v;
+    if (!nodes(before) || !record(graph, prologue) || !nodes(after)) return false;
+    int last = 0;
+    for (cudaGraphNode_t v : after) {
+      size_t behind = 0;
+      if (std::find(before.begin(), before.end(), v) != before.end()) continue;
+      if (cudaGraphNodeGetDependentNodes(v, nullptr, nullptr, &behind) != cudaSuccess) return false;
+      if (behind == 0) {
+        dep = v;
+        ++last;
+      }
+    }
+    if (last != 1) return false;
   }
   cudaGraphNodeParams np{};
   np.type = cudaGraphNodeTypeConditional;
@@ -503,8 +512,7 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
     // (30.9 -> 17.8). Longer legs than 512 lose 4% on the first of these, shorter
     // ones (256) 13% on the last.
     PcgCont cont;
-    const bool legs = prm->tol > 0 && ((prm->stop_rule == 0 && prm->tol < kLegFactor) ||
-                                       (prm->stop_rule == 1 && prm->tol * prm->tol < kLegFactor));
+    const bool legs = refine_in_legs(prm->tol, prm->stop_rule);
     const int cap = prm->max_iter > 0 ? prm->max_iter : 1000000;
     bool in_step = false, first = true;
     int step_iters = 0;
@@ -557,13 +565,8 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
           cont.ref_gamma = r.gamma0;
           cont.ref_ff = r.ff;
         }
-        // the step ends where its one run would have: at its tolerance or at the
-        // iteration cap; or at a leg that reduced the recurrence only (for a leg of
-        // rule 1 the first part implies the second)
-        const bool met = prm->stop_rule == 1 ? r.rr <= prm->tol * prm->tol * cont.ref_ff * (1 + 1e-9)
-                                             : r.gamma <= prm->tol * cont.ref_gamma * (1 + 1e-9);
-        const bool lost = rr > kLegStall * rr_leg && rr > kLegStall / kLegFactor * r.rr;
-        step_done = r.status == CFEM_OK ? met || lost : step_iters >= cap;
+        step_done = leg_ends_step(cont, prm->tol, prm->stop_rule, r.status == CFEM_OK, r.gamma, r.rr, rr, rr_leg,
+                                  step_iters >= cap);
       }
       in_step = !step_done;
       outer += step_done;

@@ -56,6 +56,10 @@ struct Scalars {
   // gamma or ||r||^2 has fallen by the factor `leg`, and tol refers to the start
   // of the step (ref_ff > 0; else to the run's own).
   double leg, ref_gamma, ref_ff;
+  // Continuation inside a graph (k_fold_instance): last direction in pA (1), pB
+  // (2) or none (0), and the gammas that PcgCont names.
+  double fold_gamma_prev, fold_gamma;
+  int fold;
 };
 
 struct DynState {

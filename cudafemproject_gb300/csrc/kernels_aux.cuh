@@ -185,8 +185,8 @@ constexpr double kMaxDrift = 1.21;
 // scalars (nothing to do once they say done, or where the recurrence that ended
 // with gamma_last had drifted off).
 template <typename T, int DIM>
-__global__ void k_fold_direction(int64_t nn, const Scalars *sc, double gamma_prev, double gamma_last,
-                                 const T *p_last, T *z) {
+__device__ __forceinline__ void fold_direction(int64_t nn, const Scalars *sc, double gamma_prev, double gamma_last,
+                                               const T *p_last, T *z) {
   constexpr int VW = DIM == 3 ? 4 : 2;
   if (sc->done || sc->gamma > kMaxDrift * gamma_last) return;
   const T beta = (T)(sc->gamma / gamma_prev);
@@ -197,6 +197,16 @@ __global__ void k_fold_direction(int64_t nn, const Scalars *sc, double gamma_pre
 #pragma unroll
   for (int d = 0; d < DIM; ++d) zv.v[d] += beta * pv.v[d];
   stv<T, VW>(z, n, zv);
+}
+
+template <typename T, int DIM>
+__global__ void k_fold_direction(int64_t nn, const Scalars *sc, double gamma_prev, double gamma_last,
+                                 const T *p_last, T *z) {
+  fold_direction<T, DIM>(nn, sc, gamma_prev, gamma_last, p_last, z);
+}
+// The same inside the graph of an instance of a batch, by its scalars (3D).
+static __global__ void k_fold_instance(int64_t nn, const Scalars *sc, const float *pA, const float *pB, float *z) {
+  if (sc->fold) fold_direction<float, 3>(nn, sc, sc->fold_gamma_prev, sc->fold_gamma, sc->fold == 1 ? pA : pB, z);
 }
 
 // x64 += (double) x32 on the DOF lanes (vw 4: the fourth lane of x32 carries

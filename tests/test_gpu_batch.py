@@ -71,3 +71,23 @@ def test_batch_loops_and_shared_launches(monkeypatch, side_by_side, boxes):
             xo, _ = O.Oracle(p, consistent=True).static(tol=1e-14, rule=1)
             assert infos[i]["status"] == 0
             assert rel(us[i], xo) <= 1e-8, (i, tol)
+
+
+@pytest.mark.parametrize("rule", ["residual", "reference"])
+def test_batch_steps_continue_their_directions(rule):
+    """Instances of very different iteration counts, inner tolerances where their
+    runs keep the true residual (0.5 .. 1e-2) and where they lose it (1e-6): every
+    step takes over the last direction or starts afresh, and the oracle's solution
+    is met; no more iterations than as many fresh runs needed."""
+    from cudafemproject_gb300.solver import BatchContext
+    probs = [meshgen.box_3d(3, 3, n, jitter=0.2, seed=n) for n in (6, 12, 30)]
+    xo = [O.Oracle(p, consistent=True).static(tol=1e-14, rule=1)[0] for p in probs]
+    b = BatchContext(probs)
+    one = b.static_solve("fp32", tol=1e-3, stop_rule="residual")[1]
+    for tol in (0.5, 0.2, 0.1, 1e-2, 1e-6):
+        us, infos = b.static_solve("fp32_refine", tol=tol, stop_rule=rule, outer_tol=1e-11, max_outer=200)
+        for i in range(len(probs)):
+            assert infos[i]["status"] == 0 and infos[i]["rel_residual"] <= 1e-11
+            assert rel(us[i], xo[i]) <= 1e-8, (i, tol)
+            # (11 digits at the three digits of a fresh run, twice over for restarts)
+            assert infos[i]["iterations"] <= 2 * 4 * one[i]["iterations"], (i, tol)
