@@ -506,19 +506,26 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
     // A step with a tight inner tolerance runs as several legs, each down to
     // kLegFactor or kLegIterations long, so that the recurrence is replaced before
     // it drifts off and loses its directions. To 1e-9 with an inner tolerance of
-    // 1e-3, one run per step started afresh, and so: 2.65 M tets 7062 -> 4800-5200
-    // iterations (319 -> 223-241 ms), 98,304 tets 2421 -> 1283 (22.3 -> 13.1),
-    // 786,432 tets 4334 -> 2650 (87 -> 56), a Delaunay mesh 2811 -> 1377-1459
-    // (30.9 -> 17.8). Longer legs than 512 lose 4% on the first of these, shorter
+    // 1e-3, one run per step started afresh, and so: 2.65 M tets 7062 -> 5349
+    // iterations (319 -> 249 ms), 98,304 tets 2421 -> 1606 (22.3 -> 16.1),
+    // 786,432 tets 4334 -> 3210 (87 -> 67), a Delaunay mesh 2811 -> 1825
+    // (30.9 -> 22.0). Longer legs than 512 lose 4% on the first of these, shorter
     // ones (256) 13% on the last.
     PcgCont cont;
     const bool legs = refine_in_legs(prm->tol, prm->stop_rule);
     const int cap = prm->max_iter > 0 ? prm->max_iter : 1000000;
-    bool in_step = false, first = true;
+    bool in_step = false, first = true, whole = false;
     int step_iters = 0;
     while (outer < max_outer) {
-      // (within a step with some margin: one run per step ended anywhere below)
-      if (std::sqrt(rr) <= (in_step ? 0.25 : 1.0) * outer_tol * std::sqrt(ff)) { status = CFEM_OK; break; }
+      // Legs go on to a part of the outer tolerance while they still reduce the
+      // residual: whole steps overshot it (by 3x to 500x with inner tolerances of
+      // 1e-3), and the soft modes' error with it (a random load on 41,472 tets:
+      // 3e-10 in whole steps, 5e-9 with legs that stopped at 1e-9).
+      if (std::sqrt(rr) <= outer_tol * std::sqrt(ff) &&
+          (!legs || whole || std::sqrt(rr) <= kLegMargin * outer_tol * std::sqrt(ff))) {
+        status = CFEM_OK;
+        break;
+      }
       if (!in_step) {
         // The FP64 true residual has a floor near eps64 * ||K|| ||x||; once two
         // refinement steps in a row no longer reduce it as a step should (halve
@@ -538,13 +545,20 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
         CKL();
         true_residual_async(c, c->v64.f.p, c->v64.x.p, c->v64.r.p, c->v32.f.p, c->h_rr);
       };
-      cont.leg = legs ? kLegFactor : 0;
-      const int maxit = legs ? std::min(kLegIterations, cap - step_iters) : cap;
+      const bool leg = legs && !whole;
+      cont.leg = leg ? kLegFactor : 0;
+      if (whole) {
+        cont.p = nullptr;
+        cont.ref_gamma = cont.ref_ff = 0;
+      }
+      const int maxit = legs ? std::min(leg ? kLegIterations : cap, cap - step_iters) : cap;
       const PcgResult r = run_pcg_f(c, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, maxit, &cont, then);
       if (r.iters > 0) {  // (none: the last direction is still that of the run before)
         cont.p = ((r.iters - 1) & 1) ? c->v32.pA.p : c->v32.pB.p;
         cont.gamma_prev = r.gamma_prev;
-        cont.gamma = r.gamma;
+        // (a step of one run with a loose tolerance keeps its direction whatever the
+        // drift: at the FP64 floor it still is what the soft modes converge along)
+        cont.gamma = legs || prm->tol < kContinueTol ? r.gamma : INFINITY;
       }
       total += r.iters;
       step_iters += r.iters;
@@ -560,13 +574,19 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
       rr = ((volatile double *)c->h_rr)[0];
       ff = ((volatile double *)c->h_rr)[1];
       bool step_done = true;
-      if (legs) {
+      if (leg) {
         if (!in_step) {
           cont.ref_gamma = r.gamma0;
           cont.ref_ff = r.ff;
         }
-        step_done = leg_ends_step(cont, prm->tol, prm->stop_rule, r.status == CFEM_OK, r.gamma, r.rr, rr, rr_leg,
-                                  step_iters >= cap);
+        const bool met = leg_met(cont, prm->tol, prm->stop_rule, r.gamma, r.rr);
+        step_done = (r.status == CFEM_OK && met) || step_iters >= cap;
+        // a leg that reduced the recurrence only (at the FP64 floor, mostly): the step
+        // ends with a whole run of its own, afresh, for the modes that the residual
+        // norm no longer shows
+        whole = !step_done && r.status == CFEM_OK && rr > kLegStall * rr_leg && rr > kLegStall / kLegFactor * r.rr;
+      } else {
+        whole = false;
       }
       in_step = !step_done;
       outer += step_done;

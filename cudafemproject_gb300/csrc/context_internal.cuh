@@ -271,10 +271,11 @@ constexpr double kContinueTol = 0.2;
 // kContinueTol), or this many iterations.
 constexpr double kLegFactor = kContinueTol * kContinueTol;
 constexpr int kLegIterations = 512;
+constexpr double kLegMargin = 1.0 / 16;
 inline bool refine_in_legs(double tol, int rule) {
   return tol > 0 && ((rule == 0 && tol < kLegFactor) || (rule == 1 && tol * tol < kLegFactor));
 }
-constexpr double kLegStall = 0.25;  // a leg that leaves more of the true ||r||^2 than this was at its floor
+constexpr double kLegStall = 0.25;  // a leg that leaves more of the true ||r||^2 than this may have been at its floor
 // A refinement step whose FP64 residual norm^2 falls by less than this is at
 // the FP64 floor: a step cuts the norm by about the inner tolerance tol (at
 // least halves it for tol up to 0.25), so the test allows twice that.
@@ -289,16 +290,9 @@ struct PcgCont {
   double leg = 0, ref_gamma = 0, ref_ff = 0;
 };
 
-// Whether a run that ended as a leg ends its refinement step: where the step's
-// one run would have, at its tolerance or at the iteration cap; or at a leg that
-// reduced the recurrence only (lost; for rule 1 the first part implies the
-// second). gamma, rr: of the recurrence; rr_true, rr_before: the FP64 residual
-// after and before the leg.
-inline bool leg_ends_step(const PcgCont &c, double tol, int rule, bool converged, double gamma, double rr,
-                          double rr_true, double rr_before, bool capped) {
-  const bool met = rule == 1 ? rr <= tol * tol * c.ref_ff * (1 + 1e-9) : gamma <= tol * c.ref_gamma * (1 + 1e-9);
-  const bool lost = rr_true > kLegStall * rr_before && rr_true > kLegStall / kLegFactor * rr;
-  return converged ? met || lost : capped;
+// Whether a run that ended as a leg has met the tolerance of its refinement step.
+inline bool leg_met(const PcgCont &c, double tol, int rule, double gamma, double rr) {
+  return rule == 1 ? rr <= tol * tol * c.ref_ff * (1 + 1e-9) : gamma <= tol * c.ref_gamma * (1 + 1e-9);
 }
 
 struct PcgResult {
