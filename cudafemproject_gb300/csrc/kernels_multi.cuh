@@ -165,9 +165,9 @@ inline MultiSmem multi_smem(const FanBlockLayout &L, int C, int K) {
 // partials need no exchange until the end of the item.
 //
 // Bound by the phases of an item (staging, half-fans, node sums) behind one
-// another with 16 warps per SM; issue slots are 41% used, shared memory 40%.
-// Two cases per thread cut the instructions of an iteration of 32 cases from
-// 21.9 M to 14.8 M per warp. One iteration, before and after: 32 cases of 98,304
+// another with 16 warps per SM; issue slots are 38% used, the L1 48%. Two cases
+// per thread cut the instructions of a launch for 32 cases of 98,304 tets from
+// 21.9 M to 14.0 M (of warps). One iteration, before and after: 32 cases of 98,304
 // tets 52.0 -> 46.2 us, 8 cases 19.7 -> 16.4, 4 cases 14.4 -> 12.7; 32 cases of
 // 331,776 tets 176 -> 148, 8 cases 43.8 -> 37.3. The registers are at their
 // limit: forms that spill 50 bytes or more lost all of it (the next chunk's
