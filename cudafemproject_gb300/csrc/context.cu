@@ -514,7 +514,7 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
     PcgCont cont;
     const bool legs = refine_in_legs(prm->tol, prm->stop_rule);
     const int cap = prm->max_iter > 0 ? prm->max_iter : 1000000;
-    bool in_step = false, first = true, whole = false;
+    bool in_step = false, first = true, whole = false, at_floor = false;
     int step_iters = 0;
     while (outer < max_outer) {
       // Legs go on to a part of the outer tolerance while they still reduce the
@@ -522,7 +522,7 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
       // 1e-3), and the soft modes' error with it (a random load on 41,472 tets:
       // 3e-10 in whole steps, 5e-9 with legs that stopped at 1e-9).
       if (std::sqrt(rr) <= outer_tol * std::sqrt(ff) &&
-          (!legs || whole || std::sqrt(rr) <= kLegMargin * outer_tol * std::sqrt(ff))) {
+          (!legs || whole || at_floor || std::sqrt(rr) <= kLegMargin * outer_tol * std::sqrt(ff))) {
         status = CFEM_OK;
         break;
       }
@@ -545,9 +545,9 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
         CKL();
         true_residual_async(c, c->v64.f.p, c->v64.x.p, c->v64.r.p, c->v32.f.p, c->h_rr);
       };
-      const bool leg = legs && !whole;
+      const bool leg = legs && !whole && !at_floor;
       cont.leg = leg ? kLegFactor : 0;
-      if (whole) {
+      if (whole || at_floor) {
         cont.p = nullptr;
         cont.ref_gamma = cont.ref_ff = 0;
       }
@@ -581,10 +581,14 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
         }
         const bool met = leg_met(cont, prm->tol, prm->stop_rule, r.gamma, r.rr);
         step_done = (r.status == CFEM_OK && met) || step_iters >= cap;
-        // a leg that reduced the recurrence only (at the FP64 floor, mostly): the step
-        // ends with a whole run of its own, afresh, for the modes that the residual
-        // norm no longer shows
-        whole = !step_done && r.status == CFEM_OK && rr > kLegStall * rr_leg && rr > kLegStall / kLegFactor * r.rr;
+        // A leg that reduced the recurrence only: the step goes on as a whole run,
+        // afresh, for the modes that the residual norm no longer shows. Far down it
+        // is the FP64 floor: the steps to come are whole runs from their start, and
+        // so is this one unless earlier legs have brought it here.
+        const bool lost = !step_done && r.status == CFEM_OK && rr > kLegStall * rr_leg && rr > kLegStall / kLegFactor * r.rr;
+        at_floor = at_floor || (lost && rr <= kFloorRegion * ff);
+        step_done = step_done || (lost && at_floor && in_step);
+        whole = lost && !step_done;
       } else {
         whole = false;
       }

@@ -272,6 +272,7 @@ constexpr double kContinueTol = 0.2;
 constexpr double kLegFactor = kContinueTol * kContinueTol;
 constexpr int kLegIterations = 512;
 constexpr double kLegMargin = 1.0 / 16;
+constexpr double kFloorRegion = 1e-12;  // ||r||^2 / ||f||^2 below which a lost leg is taken for the FP64 floor
 inline bool refine_in_legs(double tol, int rule) {
   return tol > 0 && ((rule == 0 && tol < kLegFactor) || (rule == 1 && tol * tol < kLegFactor));
 }
