@@ -273,11 +273,6 @@ bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, 
   h.tol = tol;
   h.rule = rule;
   h.maxit = maxit > 0 ? maxit : 1000000;
-  if (cont) {
-    h.leg = cont->leg;
-    h.ref_gamma = cont->ref_gamma;
-    h.ref_ff = cont->ref_ff;
-  }
   CK(cudaMemcpyAsync(sc, &h, sizeof(Scalars), cudaMemcpyHostToDevice, c->stream));
   const MvParams<float> mv = site_mv(c, S, cK, cM, mcoef);
   if (warm) {
@@ -294,7 +289,7 @@ bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, 
     // step from it, z + (gamma / gamma_prev) p_last, folded into z here (the
     // first matvec takes p = z).
     auto fold = [&](auto k) {
-      k<<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, sc, cont->gamma_prev, cont->gamma, cont->p, V.z.p);
+      k<<<nblk(c->nn), kThreads, 0, c->stream>>>(c->nn, sc, cont->gamma_prev, cont->p, V.z.p);
     };
     if (c->dim == 3) fold(k_fold_direction<float, 3>);
     else fold(k_fold_direction<float, 2>);
@@ -498,46 +493,17 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
     double rr_prev = -1;
     const double stall = refine_stall_ratio(prm->tol);
     int stalls = 0;
-    // Every FP32 run takes over the direction of the run before (the step it
-    // ended on was taken with gamma_prev; iteration i writes its direction to pB
-    // when i is even, to pA when odd) unless the recurrence had drifted off the
-    // FP64 residual (kMaxDrift): the true residual replaces the recursive one and
-    // the Krylov directions found so far keep serving.
-    // A step with a tight inner tolerance runs as several legs, each down to
-    // kLegFactor or kLegIterations long, so that the recurrence is replaced before
-    // it drifts off and loses its directions. To 1e-9 with an inner tolerance of
-    // 1e-3, one run per step started afresh, and so: 2.65 M tets 7062 -> 5349
-    // iterations (319 -> 249 ms), 98,304 tets 2421 -> 1606 (22.3 -> 16.1),
-    // 786,432 tets 4334 -> 3210 (87 -> 67), a Delaunay mesh 2811 -> 1825
-    // (30.9 -> 22.0). Longer legs than 512 lose 4% on the first of these, shorter
-    // ones (256) 13% on the last.
     PcgCont cont;
-    const bool legs = refine_in_legs(prm->tol, prm->stop_rule);
-    const int cap = prm->max_iter > 0 ? prm->max_iter : 1000000;
-    bool in_step = false, first = true, whole = false, at_floor = false;
-    int step_iters = 0;
     while (outer < max_outer) {
-      // Legs go on to a part of the outer tolerance while they still reduce the
-      // residual: whole steps overshot it (by 3x to 500x with inner tolerances of
-      // 1e-3), and the soft modes' error with it (a random load on 41,472 tets:
-      // 3e-10 in whole steps, 5e-9 with legs that stopped at 1e-9).
-      if (std::sqrt(rr) <= outer_tol * std::sqrt(ff) &&
-          (!legs || whole || at_floor || std::sqrt(rr) <= kLegMargin * outer_tol * std::sqrt(ff))) {
-        status = CFEM_OK;
-        break;
-      }
-      if (!in_step) {
-        // The FP64 true residual has a floor near eps64 * ||K|| ||x||; once two
-        // refinement steps in a row no longer reduce it as a step should (halve
-        // it; a continued step reduces it by about the replacement factor tol)
-        // the iterate is converged in FP64. (One such step alone can be an FP32
-        // run that ended early, well above the floor.)
-        stalls = rr_prev >= 0 && rr > stall * rr_prev ? stalls + 1 : 0;
-        if (stalls >= 2) { status = CFEM_OK; break; }
-        rr_prev = rr;
-        step_iters = 0;
-        cont.ref_gamma = cont.ref_ff = 0;
-      }
+      if (std::sqrt(rr) <= outer_tol * std::sqrt(ff)) { status = CFEM_OK; break; }
+      // The FP64 true residual has a floor near eps64 * ||K|| ||x||; once two
+      // refinement steps in a row no longer reduce it as a step should (halve
+      // it; a continued step reduces it by about the replacement factor tol)
+      // the iterate is converged in FP64. (One such step alone can be an FP32
+      // run that ended early, well above the floor.)
+      stalls = rr_prev >= 0 && rr > stall * rr_prev ? stalls + 1 : 0;
+      if (stalls >= 2) { status = CFEM_OK; break; }
+      rr_prev = rr;
       // behind the run, without waiting for it: x64 += d and the true residual
       // (its norms arrive with the run's scalars)
       auto then = [&]() {
@@ -545,57 +511,31 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
         CKL();
         true_residual_async(c, c->v64.f.p, c->v64.x.p, c->v64.r.p, c->v32.f.p, c->h_rr);
       };
-      const bool leg = legs && !whole && !at_floor;
-      cont.leg = leg ? kLegFactor : 0;
-      if (whole || at_floor) {
-        cont.p = nullptr;
-        cont.ref_gamma = cont.ref_ff = 0;
-      }
-      const int maxit = legs ? std::min(leg ? kLegIterations : cap, cap - step_iters) : cap;
-      const PcgResult r = run_pcg_f(c, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, maxit, &cont, then);
-      if (r.iters > 0) {  // (none: the last direction is still that of the run before)
-        cont.p = ((r.iters - 1) & 1) ? c->v32.pA.p : c->v32.pB.p;
-        cont.gamma_prev = r.gamma_prev;
-        // (a step of one run with a loose tolerance keeps its direction whatever the
-        // drift: at the FP64 floor it still is what the soft modes converge along)
-        cont.gamma = legs || prm->tol < kContinueTol ? r.gamma : INFINITY;
-      }
+      const PcgResult r = run_pcg_f(c, 1.f, 0.f, nullptr, 0, prm->tol, prm->stop_rule, prm->max_iter, &cont, then);
+      // With a loose inner tolerance (a residual-replacement factor, at least
+      // kContinueTol), from the second step on the FP32 PCG continues with its
+      // last direction (the step it ended on was taken with gamma_prev;
+      // iteration i writes its direction to pB when i is even, to pA when odd)
+      // instead of restarting from z: the FP64 true residual replaces the
+      // recursive one and the Krylov directions found so far keep serving.
+      // Replaced seldom, the recursive residual drifts too far from the true
+      // one for the old direction to stay conjugate, so tighter inner
+      // tolerances restart. (Steps of tight tolerances cut into legs of 512
+      // iterations that keep their direction took 13% less time on 2.65 M tets, as
+      // long on smaller meshes, and ended slender beams, 150 to 300 cells long,
+      // as converged at relative residuals of 0.07 to 15: whole runs get there
+      // because their recurrence goes on through thousands of iterations in which
+      // the residual rises.)
+      cont.p = prm->tol >= kContinueTol && r.iters > 0 ? (((r.iters - 1) & 1) ? c->v32.pA.p : c->v32.pB.p) : nullptr;
+      cont.gamma_prev = r.gamma_prev;
       total += r.iters;
-      step_iters += r.iters;
-      if (first) inf.gamma0 = r.gamma0;
-      first = false;
+      if (outer == 0) inf.gamma0 = r.gamma0;
       inf.gamma = r.gamma;
-      if (r.status == CFEM_ERR_DIVERGED) {
-        in_step = false;
-        status = CFEM_ERR_DIVERGED;
-        break;
-      }
-      const double rr_leg = rr;
+      if (r.status == CFEM_ERR_DIVERGED) { status = CFEM_ERR_DIVERGED; break; }
+      ++outer;
       rr = ((volatile double *)c->h_rr)[0];
       ff = ((volatile double *)c->h_rr)[1];
-      bool step_done = true;
-      if (leg) {
-        if (!in_step) {
-          cont.ref_gamma = r.gamma0;
-          cont.ref_ff = r.ff;
-        }
-        const bool met = leg_met(cont, prm->tol, prm->stop_rule, r.gamma, r.rr);
-        step_done = (r.status == CFEM_OK && met) || step_iters >= cap;
-        // A leg that reduced the recurrence only: the step goes on as a whole run,
-        // afresh, for the modes that the residual norm no longer shows. Far down it
-        // is the FP64 floor: the steps to come are whole runs from their start, and
-        // so is this one unless earlier legs have brought it here.
-        const bool lost = !step_done && r.status == CFEM_OK && rr > kLegStall * rr_leg && rr > kLegStall / kLegFactor * r.rr;
-        at_floor = at_floor || (lost && rr <= kFloorRegion * ff);
-        step_done = step_done || (lost && at_floor && in_step);
-        whole = lost && !step_done;
-      } else {
-        whole = false;
-      }
-      in_step = !step_done;
-      outer += step_done;
     }
-    outer += in_step;  // (converged within a step)
     rr_end = rr;
     ff_end = ff;
     if (status != CFEM_OK && std::sqrt(rr) <= outer_tol * std::sqrt(ff)) status = CFEM_OK;

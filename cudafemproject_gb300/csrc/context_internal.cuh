@@ -267,34 +267,18 @@ namespace detail {
 // direction across the refinement steps (the tolerance is then the factor by
 // which its recursive residual drops between FP64 true-residual replacements).
 constexpr double kContinueTol = 0.2;
-// Legs of a refinement step: gamma and ||r||^2 fall by this factor (the norm by
-// kContinueTol), or this many iterations.
-constexpr double kLegFactor = kContinueTol * kContinueTol;
-constexpr int kLegIterations = 512;
-constexpr double kLegMargin = 1.0 / 16;
-constexpr double kFloorRegion = 1e-12;  // ||r||^2 / ||f||^2 below which a lost leg is taken for the FP64 floor
-inline bool refine_in_legs(double tol, int rule) {
-  return tol > 0 && ((rule == 0 && tol < kLegFactor) || (rule == 1 && tol * tol < kLegFactor));
-}
-constexpr double kLegStall = 0.25;  // a leg that leaves more of the true ||r||^2 than this may have been at its floor
 // A refinement step whose FP64 residual norm^2 falls by less than this is at
 // the FP64 floor: a step cuts the norm by about the inner tolerance tol (at
 // least halves it for tol up to 0.25), so the test allows twice that.
 inline double refine_stall_ratio(double tol) { return std::min(0.9, std::max(0.25, 4.0 * tol * tol)); }
 
 // What a run of the FP32 PCG takes over from the one before: the last direction
-// (p, nullptr: none) with the gamma its step length was formed with and the last
-// one; and its place in a refinement step (Scalars::leg).
+// (p, nullptr: none) with the gamma its step length was formed with, and the last
+// gamma (batched meshes: whether the recurrence still was the true residual).
 struct PcgCont {
   const float *p = nullptr;
   double gamma_prev = 0, gamma = 0;
-  double leg = 0, ref_gamma = 0, ref_ff = 0;
 };
-
-// Whether a run that ended as a leg has met the tolerance of its refinement step.
-inline bool leg_met(const PcgCont &c, double tol, int rule, double gamma, double rr) {
-  return rule == 1 ? rr <= tol * tol * c.ref_ff * (1 + 1e-9) : gamma <= tol * c.ref_gamma * (1 + 1e-9);
-}
 
 struct PcgResult {
   int status = CFEM_OK;

@@ -52,10 +52,6 @@ struct Scalars {
   int stalled;  // one-kernel runs: a CTA did not arrive at a grid-wide sum in time
   // stopping limits (init kernel: tol gamma0; (tol ||f||)^2) and 1 / gamma_prev (update kernel)
   double gamma_stop, rr_stop, inv_gamma_prev;
-  // A run that is one leg of a refinement step (leg > 0): it also stops once
-  // gamma or ||r||^2 has fallen by the factor `leg`, and tol refers to the start
-  // of the step (ref_ff > 0; else to the run's own).
-  double leg, ref_gamma, ref_ff;
   // Continuation inside a graph (k_fold_instance): last direction in pA (1), pB
   // (2) or none (0), and the gammas that PcgCont names.
   double fold_gamma_prev, fold_gamma;
@@ -835,14 +831,9 @@ __global__ void __launch_bounds__(kThreads) k_pcg_init(VecParams<T> P, int warm)
     s->sigma = 0;
     s->alpha = 0;
     s->beta = 0;
-    const bool own = !(s->ref_ff > 0);
-    const double lim = s->tol * sqrt(own ? acc[2] : s->ref_ff);
-    s->gamma_stop = s->tol * (own ? acc[0] : s->ref_gamma);
+    const double lim = s->tol * sqrt(acc[2]);
+    s->gamma_stop = s->tol * acc[0];
     s->rr_stop = lim < 0 ? -1.0 : lim * lim;  // (a negative tol stops nothing)
-    if (s->leg > 0) {
-      s->gamma_stop = fmax(s->gamma_stop, s->leg * acc[0]);
-      s->rr_stop = fmax(s->rr_stop, s->leg * acc[2]);
-    }
     int done = 0;
     if (acc[0] == 0.0) done = 1;
     if (s->rule == 1 && acc[1] <= s->rr_stop) done = 1;

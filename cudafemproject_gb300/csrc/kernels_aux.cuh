@@ -175,38 +175,34 @@ static __global__ void k_axpby64(int64_t n, double a, const double *x, double b,
   if (i < n) y[i] = a * x[i] + b * y[i];
 }
 
-// A recurrence whose gamma = r.M^-1 r is this far below that of the FP64 residual
-// no longer knows the residual (1.1 in the norm): the direction it ended with is
-// conjugate to nothing, and beta = gamma / gamma_prev would hold on to it.
-constexpr double kMaxDrift = 1.21;
-
 // Continued PCG run: z += (gamma / gamma_prev) p_last on the DOF lanes (the
 // fourth lane carries M^-1, see k_pcg_init), gamma from the init kernel's
-// scalars (nothing to do once they say done, or where the recurrence that ended
-// with gamma_last had drifted off).
+// scalars (nothing to do once they say done).
 template <typename T, int DIM>
-__device__ __forceinline__ void fold_direction(int64_t nn, const Scalars *sc, double gamma_prev, double gamma_last,
-                                               const T *p_last, T *z) {
+__device__ __forceinline__ void fold_direction(int64_t nn, const Scalars *sc, double gamma_prev, const T *p_last, T *z) {
   constexpr int VW = DIM == 3 ? 4 : 2;
-  if (sc->done || sc->gamma > kMaxDrift * gamma_last) return;
+  if (sc->done) return;
   const T beta = (T)(sc->gamma / gamma_prev);
   int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= nn) return;
-  NodeV<T, VW> zv = ldv<T, VW>(z, n);
-  const NodeV<T, VW> pv = ldv<T, VW>(p_last, n);
+  NodeV<T, VW> p = ldv<T, VW>(p_last, n), zv = ldv<T, VW>(z, n);
 #pragma unroll
-  for (int d = 0; d < DIM; ++d) zv.v[d] += beta * pv.v[d];
+  for (int d = 0; d < DIM; ++d) zv.v[d] += beta * p.v[d];
   stv<T, VW>(z, n, zv);
 }
-
 template <typename T, int DIM>
-__global__ void k_fold_direction(int64_t nn, const Scalars *sc, double gamma_prev, double gamma_last,
-                                 const T *p_last, T *z) {
-  fold_direction<T, DIM>(nn, sc, gamma_prev, gamma_last, p_last, z);
+__global__ void k_fold_direction(int64_t nn, const Scalars *sc, double gamma_prev, const T *p_last, T *z) {
+  fold_direction<T, DIM>(nn, sc, gamma_prev, p_last, z);
 }
+
 // The same inside the graph of an instance of a batch, by its scalars (3D).
+// Afresh where gamma = r.M^-1 r of the FP64 residual is this much above that of
+// the recurrence it replaces (1.1 in the norm): the direction that the recurrence
+// ended with is conjugate to nothing, and beta would hold on to it.
+constexpr double kMaxDrift = 1.21;
 static __global__ void k_fold_instance(int64_t nn, const Scalars *sc, const float *pA, const float *pB, float *z) {
-  if (sc->fold) fold_direction<float, 3>(nn, sc, sc->fold_gamma_prev, sc->fold_gamma, sc->fold == 1 ? pA : pB, z);
+  if (sc->fold && !(sc->gamma > kMaxDrift * sc->fold_gamma))
+    fold_direction<float, 3>(nn, sc, sc->fold_gamma_prev, sc->fold == 1 ? pA : pB, z);
 }
 
 // x64 += (double) x32 on the DOF lanes (vw 4: the fourth lane of x32 carries

@@ -1,0 +1,59 @@
+"""Calls at their limits: loads that underflow in single precision, bodies that
+need thousands of iterations."""
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import rel
+from cudafemproject_gb300 import meshgen
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rule", ["residual", "reference"])
+@pytest.mark.parametrize("tol", [1e-3, 0.1, 0.4])
+def test_refinement_of_loads_below_single_precision(tol, rule):
+    """Entries of 1e-20: r.z = r^2 / diag(K) is 1e-47, zero in FP32, where r.r =
+    1e-40 is not. The FP32 runs take no step, and the solve ends at the second
+    step that reduces nothing, with tight inner tolerances (legs) as with loose
+    ones. The same load at a size that single precision holds is solved."""
+    from cudafemproject_gb300.solver import FemContext
+    p = meshgen.box_3d(3, 3, 9, jitter=0.2, seed=2)
+    f = np.random.default_rng(4).uniform(-1, 1, p.n_dof)
+    ctx = FemContext(p, semantics="consistent")
+    assert ctx.diagonal().min() > 2e5  # (r.z < 5e-46: below half the smallest FP32 number, 1.4e-45)
+    u, info = ctx.pcg(1e-20 * f, precision="fp32_refine", tol=tol, stop_rule=rule, outer_tol=1e-9)
+    assert (info["status"], info["iterations"], info["outer_iterations"]) == (0, 0, 2)
+    assert not u.any() and info["rel_residual"] == 1.0
+    u, info = ctx.pcg(f, precision="fp32_refine", tol=tol, stop_rule=rule, outer_tol=1e-11)
+    x, _ = O.Oracle(p, consistent=True).assemble().pcg(f, tol=1e-14, rule=1)
+    assert info["rel_residual"] <= 1e-11 and rel(u, x) <= 1e-7
+
+
+@pytest.mark.parametrize("load", ["end", "random"])
+def test_refinement_of_a_slender_beam(load):
+    """A beam 300 cells long: thousands of FP32 iterations per refinement step, in
+    which the residual first rises far above its start. A solve that says it has
+    converged to 1e-6 has: f - K u from the elements, in displacement differences."""
+    from cudafemproject_gb300.solver import FemContext
+    p = meshgen.box_3d(2, 2, 300, lz=150.0, jitter=0.2, seed=0)
+    f = np.random.default_rng(5).standard_normal((p.n_nodes, 3))
+    if load == "end":
+        f[p.nodes[:, 2] < 0.95 * p.nodes[:, 2].max()] = 0
+    f[p.cons[:, 0]] = 0
+    f = f.ravel()
+    u, info = FemContext(p, semantics="consistent").pcg(f, precision="fp32_refine", tol=1e-3, stop_rule="residual",
+                                                        outer_tol=1e-6, max_iter=30000)
+    assert info["rel_residual"] <= 1e-6
+    X, U = p.nodes[p.elems], u.reshape(-1, 3)[p.elems]
+    J = X[:, 1:] - X[:, :1]
+    g = np.linalg.inv(J).transpose(0, 2, 1)  # gradients of N_1 .. N_3 (U is zero at the clamped nodes)
+    H = np.einsum("eai,eaj->eij", U[:, 1:] - U[:, :1], g)
+    lam, mu = p.E * p.nu / ((1 + p.nu) * (1 - 2 * p.nu)), p.E / (2 * (1 + p.nu))
+    S = lam * np.trace(H, axis1=1, axis2=2)[:, None, None] * np.eye(3) + mu * (H + H.transpose(0, 2, 1))
+    F = np.einsum("eij,eaj->eai", S, g) * (np.abs(np.linalg.det(J)) / 6)[:, None, None]
+    r = f.copy().reshape(-1, 3)
+    np.subtract.at(r, p.elems[:, 1:], F)
+    np.add.at(r, p.elems[:, 0], F.sum(1))
+    r[p.cons[:, 0]] = 0
+    assert np.linalg.norm(r) <= 1.5e-6 * np.linalg.norm(f)
