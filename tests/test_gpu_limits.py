@@ -32,19 +32,24 @@ def test_refinement_of_loads_below_single_precision(tol, rule):
 
 @pytest.mark.parametrize("load", ["end", "random"])
 def test_refinement_of_a_slender_beam(load):
-    """A beam 300 cells long: thousands of FP32 iterations per refinement step, in
-    which the residual first rises far above its start. A solve that says it has
+    """A beam 300 cells long: ten thousand FP32 iterations per refinement step and
+    more, in which the residual first rises far above its start; whole runs need
+    0.11 to 0.13 M in all, runs cut after 512 0.5 to 1.4 M, and capped at 20000 per
+    step they end as converged at residuals of 0.3 to 2. A solve that says it has
     converged to 1e-6 has: f - K u from the elements, in displacement differences."""
     from cudafemproject_gb300.solver import FemContext
-    p = meshgen.box_3d(2, 2, 300, lz=150.0, jitter=0.2, seed=0)
+    p = meshgen.box_3d(1, 1, 300, lz=300.0, jitter=0.2, seed=0)
     f = np.random.default_rng(5).standard_normal((p.n_nodes, 3))
     if load == "end":
         f[p.nodes[:, 2] < 0.95 * p.nodes[:, 2].max()] = 0
     f[p.cons[:, 0]] = 0
     f = f.ravel()
-    u, info = FemContext(p, semantics="consistent").pcg(f, precision="fp32_refine", tol=1e-3, stop_rule="residual",
-                                                        outer_tol=1e-6, max_iter=30000)
-    assert info["rel_residual"] <= 1e-6
+    ctx = FemContext(p, semantics="consistent")
+    _, info = ctx.pcg(f, precision="fp32_refine", tol=1e-3, stop_rule="residual", outer_tol=1e-6, max_iter=20000,
+                      allow_not_converged=True)
+    assert info["status"] != 0 or info["rel_residual"] <= 1e-6
+    u, info = ctx.pcg(f, precision="fp32_refine", tol=1e-3, stop_rule="residual", outer_tol=1e-6)
+    assert info["rel_residual"] <= 1e-6 and info["iterations"] <= 300000
     X, U = p.nodes[p.elems], u.reshape(-1, 3)[p.elems]
     J = X[:, 1:] - X[:, :1]
     g = np.linalg.inv(J).transpose(0, 2, 1)  # gradients of N_1 .. N_3 (U is zero at the clamped nodes)
