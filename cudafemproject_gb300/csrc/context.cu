@@ -882,14 +882,12 @@ void setup_context(cfem_ctx *c, const cfem_mesh *m, const cfem_material *mat, co
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o32, k_matvec_fan_tma<float, MV_PCG>, kHfanThreads, c->smem_ft32));
     c->grid_ft32 = (int)std::min<int64_t>(P.n_patches, (int64_t)c->n_sm * std::max(o32, 1));
     if (c->geo) {
-      // the largest layout (with scale rows) bounds the shared memory of every later rebuild
-      const size_t smem_max = fan_tma_smem_bytes(fan_geo_block_layout(P.np_max, true), sizeof(float));
       for (const void *k : {(const void *)k_matvec_fan_tma<float, MV_PLAIN, true>,
                             (const void *)k_matvec_fan_tma<float, MV_PCG, true>,
                             (const void *)k_matvec_fan_tma<float, MV_DYN, true>,
                             (const void *)k_matvec_fan_tma<float, MV_PLAIN, true, true>,
                             (const void *)k_matvec_fan_tma<float, MV_PCG, true, true>})
-        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
+        raise_smem_limit(c, k);
     }
   }
   c->grid_vec = (int)std::min<int64_t>(std::max<int64_t>(1, nblk(c->nn)), (int64_t)c->n_sm * 4);

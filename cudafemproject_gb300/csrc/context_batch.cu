@@ -361,9 +361,7 @@ extern "C" cfem_status cfem_batch_static_solve(cfem_ctx *ctx, const cfem_solve_p
     B.pe.ensure(c->prep.n_patches);
     B.pp.ensure((size_t)c->prep.n_patches * 3);
     B.seg.ensure((size_t)flat_grid(c) * n * 3);
-    if (flat_smem(c) > 48 * 1024)
-      CK(cudaFuncSetAttribute((const void *)k_batch_vec_flat<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)flat_smem(c)));
+    if (flat_smem(c) > 48 * 1024) raise_smem_limit(c, (const void *)k_batch_vec_flat<float>);
     B.scratch.ensure((size_t)n * 3);
     B.rrff.ensure((size_t)n * 2);
     B.active.ensure(n);

@@ -168,7 +168,10 @@ void launch_rows_loop(cfem_ctx *c, P &prm, bool all_sms, size_t smem, F pick) {
   prm.sync = start_grid_sync(c, 0);
   const int grid = (int)std::min<int64_t>(c->n_sm, all_sms ? c->n_sm : (R.n_slices + 3) / 4);
   const void *k = pick(R.n_slices <= (int64_t)grid * kStepWarps);
-  CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem && !c->steps.smem_raised) {  // (re-sorted masses: the same instance in every call of the context)
+    raise_smem_limit(c, k);
+    c->steps.smem_raised = true;
+  }
   void *args[] = {&prm};
   CK(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kStepThreads), args, smem, c->stream));
   c->launches += 1;

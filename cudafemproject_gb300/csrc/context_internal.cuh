@@ -139,6 +139,7 @@ struct StepWork {
   DBuf<int32_t> recv, rec_head, rec_next;
   DBuf<DynState> st;
   DBuf<int> stalled;
+  bool smem_raised = false;       // raise_smem_limit for the context's step kernel with re-sorted masses
   Scalars *ring = nullptr;        // pinned: scalars of the implicit steps in flight
   cudaEvent_t done[2] = {nullptr, nullptr};
   ~StepWork() {
@@ -271,6 +272,19 @@ constexpr double kContinueTol = 0.2;
 // the FP64 floor: a step cuts the norm by about the inner tolerance tol (at
 // least halves it for tol up to 0.25), so the test allows twice that.
 inline double refine_stall_ratio(double tol) { return std::min(0.9, std::max(0.25, 4.0 * tol * tol)); }
+
+// Lets every launch of a kernel ask for as much dynamic shared memory as the
+// device has beside its static part. The limit belongs to the kernel function and
+// is shared by all contexts of the process, so it is only ever set to this one
+// value: one of a context's own could be lowered by another thread's call between
+// the setting and the launch.
+inline void raise_smem_limit(const cfem_ctx *c, const void *kernel) {
+  int optin = 0;
+  cudaFuncAttributes at{};
+  CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+  CK(cudaFuncGetAttributes(&at, kernel));
+  CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)at.sharedSizeBytes));
+}
 
 // What a run of the FP32 PCG takes over from the one before: the last direction
 // (p, nullptr: none) with the gamma its step length was formed with, and the last

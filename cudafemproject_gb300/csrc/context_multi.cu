@@ -95,7 +95,7 @@ bool configure_c(cfem_ctx *c, MultiState &M, int C) {
   if (smem + 1024 > (size_t)optin) return false;  // (+ the kernel's static shared memory)
   M.C = C;
   M.smem = smem;
-  CK(cudaFuncSetAttribute(mvm_kernel(C), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(c, mvm_kernel(C));
   int occ = 1;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mvm_kernel(C), multi_threads(C), M.smem));
   const int64_t items = (int64_t)c->prep.n_patches * (M.K / C);

@@ -62,3 +62,48 @@ def test_refinement_of_a_slender_beam(load):
     np.add.at(r, p.elems[:, 0], F.sum(1))
     r[p.cons[:, 0]] = 0
     assert np.linalg.norm(r) <= 1.5e-6 * np.linalg.norm(f)
+
+
+def test_fp64_steps_of_contexts_in_several_threads():
+    """Explicit FP64 steps with re-sorted masses (96 KB of dynamic shared memory) and
+    with constant ones (none) are the same kernel. Contexts of both kinds that step
+    in threads of their own get what each gets alone."""
+    import ctypes as C
+    import threading
+    from cudafemproject_gb300 import capi
+    from cudafemproject_gb300.solver import FemContext
+    p = meshgen.box_3d(2, 2, 3, jitter=0.2, seed=2, rho=2000.0, traction=None, point_load=("top_centre", (0.4, -0.3, -1.0)))
+    ctxs = [FemContext(p, semantics=k) for k in ("compat", "consistent", "consistent")]
+    alone = [c.dyn(0.5, 0.0, 1e-5, 3e-5 * 1.0000001, precision="fp64")[0].ravel() for c in ctxs]
+    wrong = []
+
+    def steps(c, want):
+        u, inf = np.zeros(p.n_dof), capi.DynInfo()
+        prm = capi.DynParams(0.5, 0.0, 1e-5, 3e-5 * 1.0000001, capi.FP64, 0.0, 0, 0, 0, 0, None, None)
+        for _ in range(6000):
+            st = capi.lib().cfem_dyn(c._h, C.byref(prm), None, u.ctypes.data, C.byref(inf))
+            if st != capi.OK:
+                wrong.append(capi.lib().cfem_last_error_string())
+            elif not np.array_equal(u, want):
+                wrong.append("another result")
+
+    threads = [threading.Thread(target=steps, args=a) for a in zip(ctxs, alone)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, (len(wrong), wrong[0])
+
+
+def test_geometry_contexts_of_several_patch_sizes():
+    """The shared memory that a geometry-form context needs does not depend on the
+    contexts created after it."""
+    from cudafemproject_gb300.solver import FemContext
+    p = meshgen.box_3d(8, 8, 16, jitter=0.2, seed=2)
+    x = np.random.default_rng(1).standard_normal(p.n_dof).astype(np.float32)
+    large = FemContext(p, semantics="consistent", matvec_form="geometry", patch_elems=768)
+    y = large.matvec(x, precision="fp32")
+    small = FemContext(p, semantics="consistent", matvec_form="geometry", patch_elems=64)
+    # (FP32 sums of up to a hundred terms in another order)
+    assert rel(small.matvec(x, precision="fp32"), y) <= 1e-5
+    assert rel(large.matvec(x, precision="fp32"), y) <= 1e-5
