@@ -391,6 +391,7 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
   CK(cudaEventRecord(c->ev0, c->stream));
   int64_t pcg_total = 0;
   int status = CFEM_OK;
+  int taken = expl ? nsteps : 0;  // steps whose state is kept
   T *dcur = d0, *dnext = d1;
   V.x.zero(c->stream);  // acceleration warm start / PCG solution
   if (expl && sizeof(T) == 8) {
@@ -586,7 +587,8 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
         const PcgResult res = pcg_result(r);
         pcg_total += res.iters;
         status = res.status;
-        dcur = buf[(s - (status != CFEM_OK)) % 3];
+        if (status == CFEM_OK) taken = s;
+        dcur = buf[taken % 3];
         return status == CFEM_OK;
       };
       for (int s = 1; s <= nsteps; ++s) {
@@ -613,6 +615,7 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
       if (r.status != CFEM_OK) { status = r.status; break; }
       after(dnext);
       std::swap(dcur, dnext);
+      taken = s;
     }
   }
   CK(cudaEventRecord(c->ev1, c->stream));
@@ -620,6 +623,10 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
   float ms = 0;
   CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   to_caller<T>(c, dcur, u_out);
+  if (nrec && taken < nsteps) {  // (the buffer is kept: nothing of the failed step, the one queued behind it or another run)
+    const size_t at = (size_t)taken * nrec * c->dim;
+    CK(cudaMemsetAsync(W.trace.p + at, 0, sizeof(double) * (n_trace - at), c->stream));
+  }
   if (nrec) CK(cudaMemcpyAsync(prm->receiver_trace, W.trace.p, sizeof(double) * n_trace, cudaMemcpyDefault, c->stream));
   if (expl && sizeof(T) == 8) check_steps(c);
   else check_copy_error(c);

@@ -158,7 +158,8 @@ typedef struct cfem_dyn_params {
   int32_t warm_start;    /* implicit: start each PCG from the previous acceleration */
   int32_t n_receivers;   /* optional trace recording: nodes and output buffer */
   const int32_t *receiver_nodes;
-  double *receiver_trace; /* [steps][n_receivers][dim] displacements, host or device */
+  double *receiver_trace; /* [steps][n_receivers][dim] displacements, host or device; zero from an implicit
+                             step on that did not converge (the run ends with the state before it) */
 } cfem_dyn_params;
 
 typedef struct cfem_dyn_info {

@@ -107,3 +107,58 @@ def test_geometry_contexts_of_several_patch_sizes():
     # (FP32 sums of up to a hundred terms in another order)
     assert rel(small.matvec(x, precision="fp32"), y) <= 1e-5
     assert rel(large.matvec(x, precision="fp32"), y) <= 1e-5
+
+
+def _column():
+    return meshgen.box_3d(4, 3, 17, lz=4.0, jitter=0.2, seed=5, rho=2000.0, traction=None,
+                          point_load=("top_centre", (0.4, -0.3, -1.0)))
+
+
+def _implicit(ctx, p, precision, n, cap, rec):
+    """Status, displacements, trace and PCG iterations of n implicit steps with at most cap iterations each."""
+    import ctypes as C
+    from cudafemproject_gb300 import capi
+    u, trace = np.full(p.n_dof, np.nan), np.full((n, len(rec), 3), np.nan)
+    prm = capi.DynParams(0.5, 0.5, 1e-3, n * 1e-3 * 1.0000001, {"fp64": capi.FP64, "fp32": capi.FP32}[precision], 1e-6,
+                         capi.STOP_RESIDUAL, cap, 1, len(rec), rec.ctypes.data, trace.ctypes.data)
+    inf = capi.DynInfo()
+    st = capi.lib().cfem_dyn(ctx._h, C.byref(prm), None, u.ctypes.data, C.byref(inf))
+    return st, u.reshape(-1, 3), trace, inf.pcg_iterations
+
+
+@pytest.mark.parametrize("host_loop", [False, True])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_implicit_trace_and_failing_step(monkeypatch, precision, host_loop):
+    """Row n of an implicit run's receiver trace is the displacement that a run of n
+    steps ends with (FP32 sums are atomic: 1e-5), on a context that has run before.
+    Where step s does not converge, the rows before it are those, u is the state
+    before it and the rows from s on are zero: not what the kept buffers held."""
+    from cudafemproject_gb300 import capi
+    from cudafemproject_gb300.solver import FemContext
+    if host_loop:
+        monkeypatch.setenv("CFEM_HOST_LOOP", "1")
+    else:
+        monkeypatch.delenv("CFEM_HOST_LOOP", raising=False)
+    p = _column()
+    ctx = FemContext(p, semantics="consistent")
+    rec = np.array([int(p.load_node[0]), p.n_nodes - 1, p.n_nodes // 2], np.int32)
+    ends, its = [np.zeros((p.n_nodes, 3))], [0]
+    for n in range(1, 7):
+        st, u, trace, k = _implicit(ctx, p, precision, n, 1000, rec)
+        assert st == capi.OK
+        ends.append(u)
+        its.append(k)
+        for i in range(n):
+            assert rel(trace[i], ends[i + 1][rec]) <= 1e-5
+        assert np.array_equal(trace[-1], u[rec])
+    need = np.diff(its)
+    for cap in sorted({int(need[0]), int(need.max()) - 1, 1}):
+        bad = next((i for i, k in enumerate(need) if k > cap), None)
+        if bad is None:
+            continue
+        st, u, trace, _ = _implicit(ctx, p, precision, 6, cap, rec)
+        assert st == capi.ERR_NOT_CONVERGED
+        assert rel(u, ends[bad]) <= 1e-5 if bad else not u.any()
+        for i in range(bad):
+            assert rel(trace[i], ends[i + 1][rec]) <= 1e-5
+        assert not trace[bad:].any()
