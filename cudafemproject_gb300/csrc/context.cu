@@ -263,9 +263,10 @@ bool add_loop(cfem_ctx *c, cudaGraph_t graph, unsigned initial, const std::funct
 // done and what `then` has queued behind the run is complete.
 // queue_pcg_f: the run up to the loop's graph launch, nothing waited for (the
 // scalars can be read behind it); false where the loop runs on the host and
-// only its graph has been built. chunk: iterations per loop body.
+// only its graph has been built. chunk: iterations per loop body. halt: a device
+// flag with which the run takes no iteration, or nullptr.
 bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
-                 const PcgCont *cont, int chunk) {
+                 const PcgCont *cont, int chunk, const int *halt) {
   Vecs<float> &V = c->v32;
   const PcgSite S = whole_mesh(c);
   Scalars *sc = S.sc;
@@ -282,7 +283,9 @@ bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, 
     V.u.zero(c->stream);
     launch_mv_f(c, MV_PLAIN, m);
   }
-  launch_init(c, vec_params(c, S, V.pA.p, V.u.p), warm);
+  VecParams<float> init = vec_params(c, S, V.pA.p, V.u.p);
+  init.halt = halt;
+  launch_init(c, init, warm);
   if (cont && cont->p && cont->gamma_prev > 0) {
     // Continuation of an earlier run on a new residual: its last direction
     // p_last stays, and the first direction becomes the conjugate-gradient

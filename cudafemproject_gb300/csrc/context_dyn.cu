@@ -562,7 +562,7 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
       dp.anew = V.x.p;
       dp.d = to;
       launch_dyn_correct<T>(c, dp);
-      k_dyn_end_step<T><<<1, kThreads, 0, c->stream>>>(dp, to, c->vw);
+      k_dyn_end_step<T><<<1, kThreads, 0, c->stream>>>(dp, to, c->vw, sizeof(T) == 4 ? c->sc.p + 1 : nullptr);
       CKL();
     };
     bool pipelined = false;
@@ -570,7 +570,7 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
       // The next step is queued before the PCG of this one has been looked at
       // (a step waited 60-80 us for the host between its kernels otherwise).
       // Three displacement buffers: a step that fails leaves the state before
-      // it alone even while one more step runs.
+      // it alone even while one more step, which takes no PCG iteration then, runs.
       if (!W.ring) {
         CK(cudaMallocHost(&W.ring, 2 * sizeof(Scalars)));
         for (cudaEvent_t &e : W.done) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -593,7 +593,7 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
       };
       for (int s = 1; s <= nsteps; ++s) {
         before(buf[(s - 1) % 3], buf[s % 3]);
-        if (!queue_pcg_f(c, opK, opM, opmc, warm, tol, rule, prm->max_iter, nullptr, chunk)) {
+        if (!queue_pcg_f(c, opK, opM, opmc, warm, tol, rule, prm->max_iter, nullptr, chunk, &W.st.p->failed)) {
           pipelined = false;  // (s == 1: no device loop here; the step starts over below)
           break;
         }

@@ -309,7 +309,7 @@ PcgResult run_pcg_d(cfem_ctx *c, Vecs<double> &V, double cK, double cM, const do
 PcgResult run_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
                     const PcgCont *cont = nullptr, const std::function<void()> &then = nullptr);
 bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, double tol, int rule, int maxit,
-                 const PcgCont *cont, int chunk);
+                 const PcgCont *cont, int chunk, const int *halt = nullptr);
 PcgResult pcg_result(const Scalars &s);
 struct PcgSite {
   Scalars *sc;

@@ -64,6 +64,7 @@ struct DynState {
   // explicit steps in a two-step graph: the step of parity q reads pstep[q]
   // and its CTA 0 writes pstep[q ^ 1] (no CTA reads what its own kernel writes)
   int pstep[2];
+  int failed;  // implicit: the PCG of a step did not converge (one queued behind it takes no iteration)
 };
 
 // ------------------------------------------------------------------ helpers
@@ -765,6 +766,7 @@ struct VecParams {
   const T *dinv;
   const T *f;        // init: right-hand side
   Scalars *sc;
+  const int *halt;   // init: the run takes no iteration if this is set, or nullptr
   double *partials;  // init: grid-sum scratch
   const double *mv_part;  // update: p.Ap partials of the matvec before it, n_mv blocks
   int n_mv;
@@ -838,6 +840,7 @@ __global__ void __launch_bounds__(kThreads) k_pcg_init(VecParams<T> P, int warm)
     if (acc[0] == 0.0) done = 1;
     if (s->rule == 1 && acc[1] <= s->rr_stop) done = 1;
     if (!isfinite(acc[0])) done = 2;
+    if (P.halt && *P.halt) done = 3;
     s->done = done;
     if constexpr (LOOP) cudaGraphSetConditional(P.cond, done == 0 ? 1u : 0u);
   }

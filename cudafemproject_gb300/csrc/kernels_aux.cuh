@@ -319,9 +319,10 @@ __global__ void k_dyn_correct(DynParams<T> P) {
   }
 }
 
-// Ends a step: records receiver displacements and advances the step counter.
+// Ends a step: records receiver displacements and advances the step counter;
+// sc: the scalars of the step's PCG (FP32) or nullptr.
 template <typename T>
-__global__ void k_dyn_end_step(DynParams<T> P, const T *d, int VW) {
+__global__ void k_dyn_end_step(DynParams<T> P, const T *d, int VW, const Scalars *sc) {
   griddep_wait();
   griddep_launch_dependents();  // the next step's matvec starts streaming its blocks
   const int step = P.st->step;
@@ -330,7 +331,10 @@ __global__ void k_dyn_end_step(DynParams<T> P, const T *d, int VW) {
     P.trace[((int64_t)(step - 1) * P.n_recv + r) * P.dim + k] = (double)d[(int64_t)P.recv[r] * VW + k];
   }
   __syncthreads();
-  if (threadIdx.x == 0) P.st->step = step + 1;
+  if (threadIdx.x == 0) {
+    P.st->step = step + 1;
+    if (sc && sc->done != 1) P.st->failed = 1;
+  }
 }
 
 // FP64 implicit predictor: d_new = d + c1 v + c2 a

@@ -162,3 +162,29 @@ def test_implicit_trace_and_failing_step(monkeypatch, precision, host_loop):
         for i in range(bad):
             assert rel(trace[i], ends[i + 1][rec]) <= 1e-5
         assert not trace[bad:].any()
+
+
+def test_implicit_step_queued_behind_a_failing_one_takes_no_iteration():
+    """FP32 implicit steps are queued one ahead. Where a step ends at its iteration
+    cap (large steps: hundreds of iterations), the one behind it takes none: a run
+    of six steps that fails in its first takes the time of that step, not of two."""
+    import ctypes as C
+    import time
+    from cudafemproject_gb300 import capi
+    from cudafemproject_gb300.solver import FemContext
+    p = meshgen.box_3d(3, 3, 60, lz=20.0, jitter=0.2, seed=5, rho=2000.0, traction=None, point_load=("top_centre", (0.4, -0.3, -1.0)))
+    ctx = FemContext(p, semantics="consistent")
+    cap = 250
+
+    def failing(n):
+        u, inf = np.zeros(p.n_dof), capi.DynInfo()
+        prm = capi.DynParams(0.5, 0.5, 10.0, n * 10.0 * 1.0000001, capi.FP32, 1e-6, capi.STOP_RESIDUAL, cap, 1, 0, None, None)
+        t = time.perf_counter()
+        st = capi.lib().cfem_dyn(ctx._h, C.byref(prm), None, u.ctypes.data, C.byref(inf))
+        t = time.perf_counter() - t
+        assert st == capi.ERR_NOT_CONVERGED and inf.pcg_iterations == cap and not u.any()
+        return t
+
+    one, six = (sorted(failing(n) for _ in range(15))[7] for n in (1, 6))
+    # (with the whole step behind it 2.0; with its other kernels and one loop body 1.1)
+    assert six <= 1.4 * one
