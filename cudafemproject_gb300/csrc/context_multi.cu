@@ -23,7 +23,7 @@ struct MultiState {
   DBuf<MultiScalars> sc;
   DBuf<MultiCtl> ctl;
   DBuf<int> active;
-  DBuf<double> step_ref;  // [K][2] see k_multi_start
+  DBuf<double> step_ref;  // [K][3] see k_multi_start
   DBuf<double> res_norms;  // [K][2] ||r_c||^2, ||f_c||^2 of the FP64 true residuals
   DBuf<float> fold_beta;  // [K] continuation of the next run: z_c += beta_c p_last_c
   DBuf<int> fold_par;     // [K] p_last_c in pA (1) or pB (0)
@@ -118,7 +118,10 @@ void autotune_c(cfem_ctx *c, MultiState &M) {
   if (const char *e = std::getenv("CFEM_MULTI_CASES")) forced = std::atoi(e);
   if ((forced != 2 && forced != 4 && forced != 8) || forced > M.K || !configure_c(c, M, forced)) forced = 0;
   std::vector<MultiScalars> sc(M.K);
-  for (auto &m : sc) m.inv_gamma = m.sum_b[1][0] = m.sum_b[1][1] = 1.0;
+  for (auto &m : sc) {
+    m.inv_gamma = m.sum_b[1][0] = m.sum_b[1][1] = 1.0;
+    m.cap = 1 << 30;
+  }
   MultiCtl ctl{};
   ctl.rule = -1;  // (no stopping test)
   ctl.maxit = 1 << 30;
@@ -166,7 +169,7 @@ MultiState &multi_state(cfem_ctx *c, int K) {
   M->ctl.alloc(1);
   M->ctl.zero(c->stream);
   M->active.alloc(K);
-  M->step_ref.alloc((size_t)2 * K);
+  M->step_ref.alloc((size_t)3 * K);
   M->res_norms.alloc((size_t)2 * K);
   M->fold_beta.alloc(K);
   M->fold_par.alloc(K);
@@ -194,10 +197,10 @@ void launch_vec(cfem_ctx *c, MultiState &M, const MultiParams<float> &P, const f
 
 // Continuation of a multi-RHS run: per case the last run's iteration count (0:
 // start afresh) and the gamma of its last step length and the last one; the start of the
-// refinement step that the case is in (k_multi_start); and the number of cases
-// that have met the test (padding and cases without load included) at which all
-// stop: one that meets it earlier runs on, one that has not reads done_of 4, as
-// at an iteration cap.
+// refinement step that the case is in and the iterations that it has taken
+// (k_multi_start); and the number of cases that have met the test (padding and
+// cases without load included) at which all stop: one that meets it earlier runs
+// on, one that has not reads done_of 4 (3: its iteration cap).
 struct MultiCont {
   std::vector<int> iters;
   std::vector<double> gamma_prev, gamma, step_ref;
@@ -221,7 +224,7 @@ void run_pcg_multi(cfem_ctx *c, MultiState &M, int k_active, double tol, int rul
   MultiParams<float> P = multi_params(c, M);
   launch_vec(c, M, P, nullptr, 1);
   if (cont)
-    CK(cudaMemcpyAsync(M.step_ref.p, cont->step_ref.data(), sizeof(double) * 2 * M.K, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(M.step_ref.p, cont->step_ref.data(), sizeof(double) * 3 * M.K, cudaMemcpyHostToDevice, c->stream));
   k_multi_start<<<1, kMaxCases, 0, c->stream>>>(M.sc.p, M.ctl.p, M.K, cont ? M.step_ref.p : nullptr);
   CKL();
   if (cont) {
@@ -400,8 +403,9 @@ cfem_status solve_batch(cfem_ctx *c, const cfem_solve_params &p, int kb, const d
     const double stall = refine_stall_ratio(p.tol);
     // loose inner tolerances: every case continues its last direction (see solve_internal)
     MultiCont cont{std::vector<int>(K, 0), std::vector<double>(K, 0.0), std::vector<double>(K, 0.0),
-                   std::vector<double>(2 * K, 0.0), kMaxCases + 1};
+                   std::vector<double>(3 * K, 0.0), kMaxCases + 1};
     const bool continued = p.tol >= kContinueTol;
+    const int cap = p.max_iter > 0 ? p.max_iter : 1000000;
     // With them no case waits for the slowest of a round (the counts of a round
     // differ by 2x and more from case to case): a case that has reached the inner
     // tolerance runs on with the others, the round ends once three quarters of
@@ -441,7 +445,8 @@ cfem_status solve_batch(cfem_ctx *c, const cfem_solve_params &p, int kb, const d
       run_pcg_multi(c, M, kb, p.tol, p.stop_rule, p.max_iter, continued ? &cont : nullptr);
       for (int cs = 0; cs < kb; ++cs) {
         if (!act[cs]) continue;
-        const int d = M.done_of(cs);
+        double *ref = &cont.step_ref[3 * cs];
+        int d = M.done_of(cs);
         if (d == 2) {
           cont.iters[cs] = 0;
         } else if (M.h_sc[cs].iters > 0) {  // (none: the last direction is still that of the run before)
@@ -450,16 +455,19 @@ cfem_status solve_batch(cfem_ctx *c, const cfem_solve_params &p, int kb, const d
           cont.gamma[cs] = M.h_sc[cs].gamma;
         }
         if (!resumed[cs]) {
-          cont.step_ref[2 * cs] = M.h_sc[cs].ff;
-          cont.step_ref[2 * cs + 1] = M.h_sc[cs].gamma0;
+          ref[0] = M.h_sc[cs].ff;
+          ref[1] = M.h_sc[cs].gamma0;
+          ref[2] = 0;
         }
         iters[cs] += M.h_sc[cs].iters;
+        ref[2] += M.h_sc[cs].iters;
+        if (d == 4 && ref[2] >= cap) d = 3;  // (the cap holds for the step, over all of its rounds)
         if (!begun[cs]) gamma0[cs] = M.h_sc[cs].gamma0;
         begun[cs] = 1;
         gamma[cs] = M.h_sc[cs].gamma;
         if (!resumed[cs]) rr_prev[cs] = rr[cs];  // at the start of the refinement step
         resumed[cs] = d == 4;
-        if (d != 4) cont.step_ref[2 * cs] = 0;
+        if (d != 4) ref[0] = 0;
         outer[cs] += d != 4;
         if (d == 2) status[cs] = CFEM_ERR_DIVERGED;
       }

@@ -42,7 +42,7 @@ struct MultiScalars {
   // others, kReached: the test has been met, running on with the others (a norm
   // may rise again: at the end of the round it counts as it is then)
   int done[2], iters;
-  int pad;
+  int cap;  // iterations of this run at most
 };
 
 struct MultiCtl {  // shared by the cases of one solve
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(multi_threads(C), 512 / multi_threads(C))
       if (!finite_bits(g) || !finite_bits(m.alpha)) done = 2;
       else if ((met = rule == 0 ? v < limit : rule == 1 && v <= limit))
         done = P.ctl->quorum <= K && v > kReachedFloor * limit ? kReached : 1;
-      else if (it >= P.ctl->maxit) done = 3;
+      else if (it >= m.cap) done = 3;
       b = g * m.inv_gamma;
       if (blockIdx.x == 0) {
         m.gamma_prev = m.gamma;
@@ -677,7 +677,8 @@ __global__ void __launch_bounds__(kThreads) k_pcg_multi_vec(MultiParams<T> P, T 
 
 // After the init kernel: the scalars of every case (one block). ref: per case
 // ||f||^2 and r.z that the stopping test refers to instead of this run's own
-// (0: its own; null: none), the start of a refinement step that goes on.
+// (0: its own; null: none), the start of a refinement step that goes on, and the
+// iterations that this step has taken.
 static __global__ void __launch_bounds__(kMaxCases)
     k_multi_start(MultiScalars *sc, MultiCtl *ctl, int K, const double *ref) {
   const int c = threadIdx.x;
@@ -685,12 +686,13 @@ static __global__ void __launch_bounds__(kMaxCases)
   if (c < K) {
     MultiScalars &m = sc[c];
     const double g = m.sum_b[0][0], rr = m.sum_b[0][1], ff = m.sum_a[0];
-    const bool resumed = ref && ref[2 * c] > 0;
-    const double lim = ctl->tol * sqrt(resumed ? ref[2 * c] : ff);
+    const bool resumed = ref && ref[3 * c] > 0;
+    const double lim = ctl->tol * sqrt(resumed ? ref[3 * c] : ff);
     m.gamma0 = m.gamma = m.gamma_prev = g;
     m.rr = rr;
     m.ff = ff;
-    m.gamma_stop = ctl->tol * (resumed ? ref[2 * c + 1] : g);
+    m.gamma_stop = ctl->tol * (resumed ? ref[3 * c + 1] : g);
+    m.cap = ctl->maxit - (resumed ? (int)ref[3 * c + 2] : 0);
     m.rr_stop = lim < 0 ? -1.0 : lim * lim;  // (a negative tol stops nothing)
     m.iters = 0;
     m.sigma = m.alpha = m.beta = 0;

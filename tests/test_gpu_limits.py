@@ -188,3 +188,23 @@ def test_implicit_step_queued_behind_a_failing_one_takes_no_iteration():
     one, six = (sorted(failing(n) for _ in range(15))[7] for n in (1, 6))
     # (with the whole step behind it 2.0; with its other kernels and one loop body 1.1)
     assert six <= 1.4 * one
+
+
+def test_multi_rhs_iteration_cap_holds_per_step():
+    """Load cases that need few and many iterations, a loose inner tolerance: the
+    steps of the slow ones go on over several rounds, and max_iter holds for a
+    step, not for each of its rounds."""
+    from cudafemproject_gb300.solver import FemContext
+    p = meshgen.box_3d(3, 3, 40, jitter=0.2, seed=2)
+    rng = np.random.default_rng(3)
+    F = rng.standard_normal((8, p.n_dof))
+    top = p.nodes[:, 2] > p.nodes[:, 2].max() - 1e-6
+    F[:2] = 0
+    F[0].reshape(-1, 3)[top] = (1.0, 0.0, 0.0)  # bending: the slow modes only
+    F[1].reshape(-1, 3)[top] = (0.0, 1.0, 0.0)
+    ctx = FemContext(p, semantics="consistent")
+    for cap in (20, 35, 50, 75, 100, 150, 200, 300):
+        _, infos = ctx.pcg_multi(F, precision="fp32_refine", tol=0.3, stop_rule="residual", outer_tol=1e-9, max_iter=cap,
+                                 max_outer=12, allow_not_converged=True)
+        for i in infos:
+            assert i["iterations"] <= cap * max(1, i["outer_iterations"]), (cap, i)
