@@ -270,11 +270,6 @@ bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, 
   Vecs<float> &V = c->v32;
   const PcgSite S = whole_mesh(c);
   Scalars *sc = S.sc;
-  Scalars h{};
-  h.tol = tol;
-  h.rule = rule;
-  h.maxit = maxit > 0 ? maxit : 1000000;
-  CK(cudaMemcpyAsync(sc, &h, sizeof(Scalars), cudaMemcpyHostToDevice, c->stream));
   const MvParams<float> mv = site_mv(c, S, cK, cM, mcoef);
   if (warm) {
     MvParams<float> m = mv;
@@ -285,6 +280,10 @@ bool queue_pcg_f(cfem_ctx *c, float cK, float cM, const float *mcoef, int warm, 
   }
   VecParams<float> init = vec_params(c, S, V.pA.p, V.u.p);
   init.halt = halt;
+  init.start = 1;
+  init.tol = tol;
+  init.rule = rule;
+  init.maxit = maxit > 0 ? maxit : 1000000;
   launch_init(c, init, warm);
   if (cont && cont->p && cont->gamma_prev > 0) {
     // Continuation of an earlier run on a new residual: its last direction

@@ -301,8 +301,8 @@ cfem_status run_dyn(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_wavelet 
   CK(cudaMemcpyAsync(W.st.p, &hs, sizeof(hs), cudaMemcpyHostToDevice, c->stream));
   const int nrec = prm->n_receivers > 0 && prm->receiver_nodes && prm->receiver_trace ? prm->n_receivers : 0;
   const size_t n_trace = (size_t)nsteps * nrec * c->dim;
+  std::vector<int32_t> rn(nrec);  // (until the call's end: its copy is only queued)
   if (nrec) {
-    std::vector<int32_t> rn(nrec);
     for (int i = 0; i < nrec; ++i) {
       int32_t o = prm->receiver_nodes[i];
       if (o < 0 || o >= c->nn) throw Fail{CFEM_ERR_INVALID_ARGUMENT, "receiver node out of range"};

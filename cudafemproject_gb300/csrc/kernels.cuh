@@ -767,6 +767,12 @@ struct VecParams {
   const T *f;        // init: right-hand side
   Scalars *sc;
   const int *halt;   // init: the run takes no iteration if this is set, or nullptr
+  // init, `start` set: what the run is asked for, by value (a copy from the
+  // caller's stack may be made when its turn in the stream comes: cudaMemcpyAsync
+  // from pageable memory is not promised to have read it on return). Else the
+  // scalars hold it (instances of a batch).
+  int start, rule, maxit;
+  double tol;
   double *partials;  // init: grid-sum scratch
   const double *mv_part;  // update: p.Ap partials of the matvec before it, n_mv blocks
   int n_mv;
@@ -833,6 +839,12 @@ __global__ void __launch_bounds__(kThreads) k_pcg_init(VecParams<T> P, int warm)
     s->sigma = 0;
     s->alpha = 0;
     s->beta = 0;
+    if (P.start) {
+      s->tol = P.tol;
+      s->rule = P.rule;
+      s->maxit = P.maxit;
+      s->loops = 0;
+    }
     const double lim = s->tol * sqrt(acc[2]);
     s->gamma_stop = s->tol * acc[0];
     s->rr_stop = lim < 0 ? -1.0 : lim * lim;  // (a negative tol stops nothing)
