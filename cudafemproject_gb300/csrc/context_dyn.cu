@@ -667,9 +667,7 @@ cfem_status run_dyn_adjoint(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_
   // step_states_bytes(), else ceil(sqrt(N)) with the states at the start of every
   // segment kept and its steps taken again (the last segment's are still there).
   const double limit = step_states_bytes();
-  const bool whole = 2.0 * (N + 1) * nv * sizeof(double) <= limit;
-  const int C = whole ? N : (int)std::ceil(std::sqrt((double)N));
-  const int n_seg = (N + C - 1) / C;
+  bool whole = 2.0 * (N + 1) * nv * sizeof(double) <= limit;
   const double h_old = (1 - beta1) * dt, h_new = beta1 * dt, c2 = 0.5 * dt * dt;
   RhsSchedule sch;
   sch.semantics = c->semantics;
@@ -707,8 +705,22 @@ cfem_status run_dyn_adjoint(cfem_ctx *c, const cfem_dyn_params *prm, const cfem_
   S.d.zero(st);
   S.minv.ensure(2 * (size_t)nv);
   k_invert<double><<<nblk(nv), kThreads, 0, st>>>(nv, c->mlump.p, S.minv.p);
-  // d of a segment [C + 1], w of a segment [C + 1], db, vb, ab, then the states at segment starts
-  W.states.ensure(((size_t)2 * (C + 1) + 3 + (whole ? 0 : (size_t)n_seg * 3)) * nv);
+  // d of a segment [C + 1], w of a segment [C + 1], db, vb, ab, then the states at
+  // segment starts. Segments, too, where the device has no room for all states.
+  int C = 0, n_seg = 0;
+  auto hold = [&]() {
+    C = whole ? N : (int)std::ceil(std::sqrt((double)N));
+    n_seg = (N + C - 1) / C;
+    W.states.ensure(((size_t)2 * (C + 1) + 3 + (whole ? 0 : (size_t)n_seg * 3)) * nv);
+  };
+  try {
+    hold();
+  } catch (const Fail &f) {
+    if (!whole || f.st != CFEM_ERR_OUT_OF_MEMORY) throw;
+    (void)cudaGetLastError();
+    whole = false;
+    hold();
+  }
   double *seg = W.states.p, *wseg = seg + (size_t)(C + 1) * nv, *adj = wseg + (size_t)(C + 1) * nv, *cps = adj + 3 * nv;
   struct Release {  // more than the limit is not kept
     DBuf<double> &b;

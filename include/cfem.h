@@ -307,8 +307,10 @@ CFEM_API cfem_status cfem_element_stress(cfem_ctx *ctx, const double *u, double 
  * L = 1/2 sum_{n=1..N} sum_r |d_n[node_r] - obs[n-1][r]|^2 and its gradient in
  * the per-element Young's moduli by the discrete adjoint of the time stepping.
  * The states of all steps are held while they fit in 1 GB (CFEM_DYN_STATES_MB in
- * the environment overrides it); beyond that the reverse sweep takes the steps
- * again, segment by segment, from checkpoints stored every ceil(sqrt(N)) steps.
+ * the environment overrides it) and in the device's free memory; beyond that the
+ * reverse sweep takes the steps again, segment by segment, from checkpoints stored
+ * every ceil(sqrt(N)) steps. The context keeps that buffer (no more than the limit)
+ * for its next call and gives it back when it is destroyed.
  * obs: [N][n_rec][dim]. */
 CFEM_API cfem_status cfem_dyn_adjoint(cfem_ctx *ctx, const cfem_dyn_params *prm, const cfem_wavelet *w, int32_t n_rec,
                                       const int32_t *rec_nodes, const double *obs, double *loss, double *dLdE,

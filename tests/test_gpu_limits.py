@@ -208,3 +208,31 @@ def test_multi_rhs_iteration_cap_holds_per_step():
                                  max_outer=12, allow_not_converged=True)
         for i in infos:
             assert i["iterations"] <= cap * max(1, i["outer_iterations"]), (cap, i)
+
+
+def test_dyn_adjoint_without_room_for_all_states():
+    """481 MB of states within the 1 GB limit, on a device with 250 MB left: the
+    reverse sweep goes by segments, with the loss and gradient of the whole sweep
+    (the steps are taken again with the same sums)."""
+    import torch
+    from cudafemproject_gb300.solver import FemContext
+    p = meshgen.box_3d(16, 16, 64, jitter=0.2, seed=5, rho=2000.0, traction=None, point_load=("top_centre", (0.4, -0.3, -1.0)))
+    ctx = FemContext(p, semantics="consistent")
+    rec = np.array([int(p.load_node[0]), p.n_nodes - 1], np.int32)
+    args = (0.5, 1e-5, 400e-5 * 1.0000001, rec, 1e-9 * np.random.default_rng(1).standard_normal((400, 2, 3)))
+    torch.cuda.empty_cache()
+    hog = []
+    try:
+        for keep in (8 << 30, 1 << 30, 250 << 20):  # (in a few pieces: the free memory need not be one)
+            free = torch.cuda.mem_get_info()[0]
+            if free > keep:
+                hog.append(torch.empty((free - keep) // (2 << 20) * (2 << 20), dtype=torch.uint8, device="cuda"))
+        left = torch.cuda.mem_get_info()[0]
+        assert left < 2 * 401 * 4 * p.n_nodes * 8
+        by_segments = ctx.dyn_adjoint(*args)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    whole = FemContext(p, semantics="consistent").dyn_adjoint(*args)
+    assert by_segments[0] == pytest.approx(whole[0], rel=1e-12)
+    assert rel(by_segments[1], whole[1]) <= 1e-12
