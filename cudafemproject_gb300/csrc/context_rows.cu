@@ -79,9 +79,9 @@ void assemble_dim(cfem_ctx *c, const int32_t *nbr, const int32_t *deg, double cK
   }
   V.flag.zero(s);
   const RowsAssembly<DIM> P = assembly<DIM>(c, cK, cM);
-  k_rows_assemble<DIM><<<nblk(R.n_slices, 4), 128, 0, s>>>(P, R.n_slices, R.off.p, R.row.p, nbr, deg, R.col.p,
+  k_rows_assemble<DIM><<<(unsigned)R.n_slices, 32 * kAssembleWarps, 0, s>>>(P, R.off.p, R.row.p, nbr, deg, R.col.p,
                                                             V.val.p);
-  k_rows_corrections<DIM><<<nblk(R.n_slices * kSliceRows), kThreads, 0, s>>>(P, R.n_slices * kSliceRows, R.off.p,
+  k_rows_corrections<DIM><<<nblk(R.n_slices * kSliceRows * kCorrLanes), kThreads, 0, s>>>(P, R.n_slices * kSliceRows, R.off.p,
                                                                              R.row.p, R.col.p, V.D.p, V.flag.p);
   CKL();
 }

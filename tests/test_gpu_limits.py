@@ -236,3 +236,60 @@ def test_dyn_adjoint_without_room_for_all_states():
     whole = FemContext(p, semantics="consistent").dyn_adjoint(*args)
     assert by_segments[0] == pytest.approx(whole[0], rel=1e-12)
     assert rel(by_segments[1], whole[1]) <= 1e-12
+
+
+def _hub(n_rim):
+    """A double cone of tetrahedra around one axis edge, which all of them share."""
+    from cudafemproject_gb300.meshio import Problem
+    t = 2 * np.pi * np.arange(n_rim) / n_rim
+    nodes = np.concatenate([[[0, 0, -1], [0, 0, 1]], np.stack([np.cos(t), np.sin(t), 0.1 * np.cos(3 * t)], axis=1)])
+    i, z = np.arange(n_rim), np.zeros((0, 3))
+    elems = np.stack([np.zeros_like(i), np.ones_like(i), 2 + i, 2 + (i + 1) % n_rim], axis=1)
+    return Problem(dim=3, nodes=nodes.astype(np.float32).astype(np.float64), elems=elems.astype(np.int32),
+                   cons=np.array([[2, 7], [5, 1], [9, 2], [1, 4]], np.int32), load_node=np.zeros(0, np.int32), load_vec=z,
+                   face_nodes=np.zeros((0, 4), np.int32), face_elem=np.zeros(0, np.int32), face_normal=z,
+                   face_pressure=np.zeros(0), E=2e7, nu=0.25, rho=2000.0, elem_E=None)
+
+
+@pytest.mark.parametrize("n_rim", [31, 64, 65, 96, 97, 98, 128, 129, 1000, 4001])
+def test_nodes_of_many_elements(n_rim):
+    """Two nodes with n_rim + 1 neighbours and an edge that n_rim elements share (and
+    the limits from which a warp works on such a row and edge): products, diagonal
+    and a solve against the oracle, after new moduli, too. (A row of n products of
+    random signs rounds by sqrt(n) units and their sum may cancel: 1e-12. Solves to
+    a residual of 1e-13 differ by the condition number times that, (n_rim / 2 pi)^2
+    and a factor of hundreds for these needles: up to 129 of them.)"""
+    from cudafemproject_gb300.solver import FemContext
+    p = _hub(n_rim)
+    ctx = FemContext(p, semantics="consistent")
+    rng = np.random.default_rng(n_rim)
+    for young in (None, 2e7 * np.exp(0.3 * rng.standard_normal(p.n_elems))):
+        if young is not None:
+            ctx.set_young(young)
+            p.elem_E = young
+        o = O.Oracle(p, consistent=True)
+        x = rng.standard_normal(p.n_dof)
+        assert rel(ctx.matvec(x, "fp64"), o.matvec(x)) <= 1e-12
+    if n_rim <= 129:
+        f = rng.standard_normal(p.n_dof)
+        xo, _ = o.pcg(f, tol=1e-13, rule=1)
+        assert rel(ctx.pcg(f, "fp64", tol=1e-13, stop_rule="residual")[0], xo) <= 1e-8
+        for u in ctx.pcg_multi(np.stack([f, 2 * f]), "fp32_refine", tol=0.3, stop_rule="residual", outer_tol=1e-11)[0]:
+            assert min(rel(u, xo), rel(u, 2 * xo)) <= 1e-7
+
+
+def test_moduli_of_nodes_of_many_elements_take_linear_time():
+    """set_young on a node of m elements: sixteen times the elements in less than
+    forty times the time (a scan of them for each neighbour: 256 times)."""
+    import time
+    from cudafemproject_gb300.solver import FemContext
+
+    def seconds(n):
+        ctx, y, ts = FemContext(_hub(n)), np.full(n, 2e7), []
+        for _ in range(9):
+            t = time.perf_counter()
+            ctx.set_young(y)
+            ts.append(time.perf_counter() - t)
+        return sorted(ts)[4]
+
+    assert seconds(8000) <= 40 * seconds(500)
