@@ -179,6 +179,8 @@ void launch_rows_loop(cfem_ctx *c, P &prm, bool all_sms, size_t smem, F pick) {
 
 void launch_steps(cfem_ctx *c, RowsSteps &P) {
   launch_rows_loop(c, P, P.resort != 0, P.resort ? sizeof(double) * kStepWarps * kResortTile : 0, [&](bool resident) {
+    if (c->rows.wide.p)
+      return c->dim == 3 ? (const void *)k_rows_steps<3, false, true> : (const void *)k_rows_steps<2, false, true>;
     return c->dim == 3 ? (resident ? (const void *)k_rows_steps<3, true> : (const void *)k_rows_steps<3, false>)
                        : (resident ? (const void *)k_rows_steps<2, true> : (const void *)k_rows_steps<2, false>);
   });
@@ -186,6 +188,8 @@ void launch_steps(cfem_ctx *c, RowsSteps &P) {
 
 void launch_reverse(cfem_ctx *c, RowsReverse &P) {
   launch_rows_loop(c, P, false, 0, [&](bool resident) {
+    if (c->rows.wide.p)
+      return c->dim == 3 ? (const void *)k_rows_reverse<3, false, true> : (const void *)k_rows_reverse<2, false, true>;
     return c->dim == 3 ? (resident ? (const void *)k_rows_reverse<3, true> : (const void *)k_rows_reverse<3, false>)
                        : (resident ? (const void *)k_rows_reverse<2, true> : (const void *)k_rows_reverse<2, false>);
   });

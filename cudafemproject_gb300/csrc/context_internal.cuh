@@ -121,6 +121,7 @@ struct RowsData {
   DBuf<int32_t> inc_off, inc;  // elements of every node
   DBuf<int32_t> row, col;
   DBuf<int64_t> off;
+  DBuf<uint8_t> wide;  // slices of one row (kWideSlice), or nothing
   int64_t n_slices = 0, steps = 0;
   RowsValues K;                 // stiffness
   RowsValues KM;                // km_cK K + km_cM M of the last implicit FP64 run

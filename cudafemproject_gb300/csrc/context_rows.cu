@@ -49,20 +49,44 @@ void build_structure(cfem_ctx *c, DBuf<int32_t> &nbr, DBuf<int32_t> &deg) {
   at += even(n_inc);
   R.row.view(at, (size_t)windows * kRowWindow);
   // what the construction needs: neighbour lists, their lengths, counts, steps per slice
-  nbr.alloc((size_t)(even((NV - 1) * n_inc) + 2 * even(nn) + n_steps));
+  nbr.alloc((size_t)(even((NV - 1) * n_inc) + 2 * even(nn) + n_steps + 1));
   int32_t *deg_p = nbr.p + even((NV - 1) * n_inc), *cnt = deg_p + even(nn), *steps = cnt + even(nn);
+  int32_t *n_wide = steps + n_steps, *h_wide = reinterpret_cast<int32_t *>(c->h_rr + 1);
+  CK(cudaMemsetAsync(n_wide, 0, sizeof(int32_t), s));
   deg.view(deg_p, nn);
   CK(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * nn, s));
   k_rows_count<<<nblk(n_inc), kThreads, 0, s>>>(n_inc, c->conn.p, cnt);
   k_rows_scan<int32_t><<<1, 1024, 0, s>>>(nn, cnt, R.inc_off.p);
   CK(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * nn, s));
   k_rows_fill<<<nblk(n_inc), kThreads, 0, s>>>(n_inc, NV, c->conn.p, R.inc_off.p, cnt, R.inc.p);
-  k_rows_neighbours<NV><<<nblk(nn), kThreads, 0, s>>>(nn, c->conn.p, R.inc_off.p, R.inc.p, nbr.p, deg.p);
+  k_rows_neighbours<NV><<<nblk(nn), kThreads, 0, s>>>(nn, c->conn.p, R.inc_off.p, R.inc.p, nbr.p, deg.p, n_wide);
   k_rows_order<<<(unsigned)windows, kRowWindow, 0, s>>>(nn, deg.p, R.row.p, steps);
   k_rows_scan<int64_t><<<1, 1024, 0, s>>>(R.n_slices, steps, R.off.p);
   CKL();
   CK(cudaMemcpyAsync(c->h_rr, R.off.p + R.n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(h_wide, n_wide, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
+  if (*(volatile int32_t *)h_wide) {  // slices of one row for the nodes of many neighbours
+    DBuf<int32_t> first;  // slices of each window, their first ones, steps of each slice
+    first.alloc((size_t)(2 * windows + 1));
+    k_rows_window_slices<<<(unsigned)windows, kRowWindow, 0, s>>>(nn, deg.p, first.p);
+    k_rows_scan<int32_t><<<1, 1024, 0, s>>>(windows, first.p, first.p + windows);
+    CKL();
+    CK(cudaMemcpyAsync(h_wide, first.p + 2 * windows, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    R.n_slices = *(volatile int32_t *)h_wide;
+    R.off.alloc(R.n_slices + 1);
+    R.row.alloc((size_t)R.n_slices * kSliceRows);
+    R.wide.alloc(R.n_slices);
+    DBuf<int32_t> steps_of;
+    steps_of.alloc(R.n_slices);
+    CK(cudaMemsetAsync(R.row.p, 0xFF, sizeof(int32_t) * R.row.n, s));
+    k_rows_order_wide<<<(unsigned)windows, kRowWindow, 0, s>>>(nn, deg.p, first.p + windows, R.row.p, steps_of.p, R.wide.p);
+    k_rows_scan<int64_t><<<1, 1024, 0, s>>>(R.n_slices, steps_of.p, R.off.p);
+    CKL();
+    CK(cudaMemcpyAsync(c->h_rr, R.off.p + R.n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+  }
   R.steps = *(volatile int64_t *)c->h_rr;
   R.col.alloc((size_t)R.steps * 32);
 }
@@ -77,10 +101,11 @@ void assemble_dim(cfem_ctx *c, const int32_t *nbr, const int32_t *deg, double cK
     V.D.view(V.val.p + n_val, n_D);
     V.flag.view(reinterpret_cast<uint8_t *>(V.val.p + n_val + n_D), R.n_slices);
   }
-  V.flag.zero(s);
+  if (R.wide.p) CK(cudaMemcpyAsync(V.flag.p, R.wide.p, R.n_slices, cudaMemcpyDeviceToDevice, s));
+  else V.flag.zero(s);
   const RowsAssembly<DIM> P = assembly<DIM>(c, cK, cM);
   k_rows_assemble<DIM><<<(unsigned)R.n_slices, 32 * kAssembleWarps, 0, s>>>(P, R.off.p, R.row.p, nbr, deg, R.col.p,
-                                                            V.val.p);
+                                                            V.val.p, V.flag.p);
   k_rows_corrections<DIM><<<nblk(R.n_slices * kSliceRows * kCorrLanes), kThreads, 0, s>>>(P, R.n_slices * kSliceRows, R.off.p,
                                                                              R.row.p, R.col.p, V.D.p, V.flag.p);
   CKL();
@@ -124,8 +149,13 @@ void build_rows(cfem_ctx *c) {
 void rows_apply(cfem_ctx *c, const double *x, double *y, bool caller_order) {
   const RowOp A = op_of(c, c->rows.K);
   auto go = [&](auto k) { k<<<rows_grid(c), kRowsThreads, 0, c->stream>>>(A, x, y, c->node_new2old.p); };
-  if (c->dim == 3) caller_order ? go(k_rows_apply<3, true>) : go(k_rows_apply<3, false>);
-  else caller_order ? go(k_rows_apply<2, true>) : go(k_rows_apply<2, false>);
+  auto pick = [&](auto wide) {
+    constexpr bool W = decltype(wide)::value;
+    if (c->dim == 3) caller_order ? go(k_rows_apply<3, true, W>) : go(k_rows_apply<3, false, W>);
+    else caller_order ? go(k_rows_apply<2, true, W>) : go(k_rows_apply<2, false, W>);
+  };
+  if (c->rows.wide.p) pick(std::true_type{});
+  else pick(std::false_type{});
   CKL();
   c->launches += 1;
 }
@@ -138,8 +168,9 @@ void true_residual_async(cfem_ctx *c, const double *f, const double *x, double *
   RowsResidual P{c->nn, f, x, r, r32, out2, c->partials.p, c->counters.p};
   // (grid-stride over the slices: the partial sums are one pair per block)
   const unsigned g = std::min<unsigned>(rows_grid(c), c->grid_rows);
-  if (c->dim == 3) k_rows_residual<3><<<g, kRowsThreads, 0, c->stream>>>(A, P);
-  else k_rows_residual<2><<<g, kRowsThreads, 0, c->stream>>>(A, P);
+  auto go = [&](auto k) { k<<<g, kRowsThreads, 0, c->stream>>>(A, P); };
+  if (c->rows.wide.p) c->dim == 3 ? go(k_rows_residual<3, true>) : go(k_rows_residual<2, true>);
+  else c->dim == 3 ? go(k_rows_residual<3, false>) : go(k_rows_residual<2, false>);
   CKL();
   c->launches += 1;
 }
@@ -181,10 +212,12 @@ PcgResult run_pcg_d(cfem_ctx *c, Vecs<double> &V, double cK, double cM, const do
   // its slices: an exchange among 76 CTAs takes 0.4 us less than among 152, and
   // a slice runs no faster alone on an SM.
   const int grid = (int)std::min<int64_t>(c->n_sm, (R.n_slices + 3) / 4);
-  const bool small = R.n_slices <= (int64_t)grid * (kRowsPcgSmall / 32);
+  const bool wide = R.wide.p;  // (one instance per dimension for every size: few meshes have such nodes)
+  const bool small = !wide && R.n_slices <= (int64_t)grid * (kRowsPcgSmall / 32);
   const bool resident = R.n_slices <= (int64_t)grid * (kRowsPcgThreads / 32);
   auto pick = [&](auto k3, auto k2) { return c->dim == 3 ? (const void *)k3 : (const void *)k2; };
-  const void *k = small      ? pick(k_rows_pcg<3, true, kRowsPcgSmall>, k_rows_pcg<2, true, kRowsPcgSmall>)
+  const void *k = wide       ? pick(k_rows_pcg<3, false, kRowsPcgThreads, true>, k_rows_pcg<2, false, kRowsPcgThreads, true>)
+                  : small    ? pick(k_rows_pcg<3, true, kRowsPcgSmall>, k_rows_pcg<2, true, kRowsPcgSmall>)
                   : resident ? pick(k_rows_pcg<3, true, kRowsPcgThreads>, k_rows_pcg<2, true, kRowsPcgThreads>)
                              : pick(k_rows_pcg<3, false, kRowsPcgThreads>, k_rows_pcg<2, false, kRowsPcgThreads>);
   void *args[] = {&P};

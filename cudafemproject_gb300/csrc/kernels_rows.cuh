@@ -21,7 +21,10 @@
 // lane = 16 * half + r holds neighbours half, half + 2, ... of row r. Step k of
 // a slice is 32 column ids and, per block component, 32 doubles: every load of
 // the operator is one contiguous 256-byte line per warp. Unused entries repeat
-// the row itself (difference zero).
+// the row itself (difference zero). A node of more than kWideDegree neighbours has
+// a slice of its own (kWideSlice), in which lane l holds neighbours l, l + 32, ..:
+// two lanes took 0.57 ms for a product with 1000 neighbours, 5.4 with 10,000
+// (element form 0.09 and 0.10), a warp 0.06 and 0.30.
 #pragma once
 
 #include "grid_sync.cuh"
@@ -31,6 +34,8 @@ namespace cfem {
 
 constexpr int kRowWindow = 512;  // nodes among which rows are sorted by neighbour count
 constexpr int kSliceRows = 16;
+constexpr int kWideDegree = 64;  // (16 rows of 64 neighbours: 32 steps; meshes of tetrahedra have 15 to 35)
+constexpr unsigned kHasD = 1, kWideSlice = 2;  // RowOp::flag
 
 struct RowOp {
   int64_t n_slices;
@@ -38,7 +43,7 @@ struct RowOp {
   const int32_t *row;   // [n_slices][16] node, or -1
   const int32_t *col;   // [steps][32]
   const double *val;    // [steps][DIM * DIM][32]
-  const uint8_t *flag;  // [n_slices] rows with a D block
+  const uint8_t *flag;  // [n_slices] kHasD: rows with a D block; kWideSlice: one row
   const double *D;      // [n_nodes][DIM * DIM]
   const uint8_t *bits;  // [n_nodes] constrained DOFs
 };
@@ -97,8 +102,10 @@ __device__ __forceinline__ void rows_sum(const RowOp &A, int64_t k0, int n, cons
 
 // y = A x for the rows of slice s, given the rows (-1: padding) and their own
 // x; both lanes of a row get the sum. x is read with plain loads: callers may
-// have other CTAs' writes made visible by a grid barrier.
-template <int DIM, typename X>
+// have other CTAs' writes made visible by a grid barrier. WIDE: the operator has
+// slices of one row (instances of their own: the test for them in every product
+// took 4% of the time steps).
+template <int DIM, bool WIDE, typename X>
 __device__ __forceinline__ void rows_product_of(const RowOp &A, int64_t s, int row, const X &x,
                                                 const double (&xi)[DIM], double (&y)[DIM]) {
   constexpr int NC = DIM * DIM;
@@ -106,21 +113,35 @@ __device__ __forceinline__ void rows_product_of(const RowOp &A, int64_t s, int r
   const int n = (int)(A.off[s + 1] - k0);
 #pragma unroll
   for (int d = 0; d < DIM; ++d) y[d] = 0;
-  if (!A.flag[s]) {
+  const unsigned flag = A.flag[s];
+  if (!flag) {
     rows_sum<DIM, false>(A, k0, n, x, xi, y);
     return;
   }
-  const int i = row < 0 ? 0 : row;
-  const unsigned b = A.bits[i];
-  double xm[DIM];
+  double xr[DIM], xm[DIM];
 #pragma unroll
-  for (int d = 0; d < DIM; ++d) xm[d] = (b >> d) & 1u ? 0.0 : xi[d];
+  for (int d = 0; d < DIM; ++d) xr[d] = xi[d];
+  int i = row < 0 ? 0 : row;
+  const bool wide = WIDE && (flag & kWideSlice);
+  if (wide) {  // every lane works for the row of lanes 0 and 16
+    i = __shfl_sync(0xffffffffu, row, 0);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) xr[d] = __shfl_sync(0xffffffffu, xi[d], 0);
+  }
+  const unsigned b = A.bits[i];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) xm[d] = (b >> d) & 1u ? 0.0 : xr[d];
   rows_sum<DIM, true>(A, k0, n, x, xm, y);
+  if (wide)
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) y[d] += __shfl_xor_sync(0xffffffffu, y[d], o);
   const double *D = A.D + (int64_t)i * NC;
 #pragma unroll
   for (int p = 0; p < DIM; ++p) {
     if ((b >> p) & 1u) {
-      y[p] = D[p * DIM + p] * xi[p];
+      y[p] = D[p * DIM + p] * xr[p];
     } else {
 #pragma unroll
       for (int q = 0; q < DIM; ++q) y[p] = fma(D[p * DIM + q], xm[q], y[p]);
@@ -128,10 +149,10 @@ __device__ __forceinline__ void rows_product_of(const RowOp &A, int64_t s, int r
   }
 }
 
-template <int DIM>
+template <int DIM, bool WIDE>
 __device__ __forceinline__ void rows_product(const RowOp &A, int64_t s, int row, const double *x,
                                              const double (&xi)[DIM], double (&y)[DIM]) {
-  rows_product_of<DIM>(A, s, row, NodeX<DIM>{x}, xi, y);
+  rows_product_of<DIM, WIDE>(A, s, row, NodeX<DIM>{x}, xi, y);
 }
 
 // row of this lane in slice s and its own x
@@ -152,7 +173,7 @@ constexpr int kRowsThreads = 128;
 
 // y = A x; CALLER: x and y are the caller's [n_nodes][DIM] arrays (not
 // overlapping), else node vectors.
-template <int DIM, bool CALLER>
+template <int DIM, bool CALLER, bool WIDE>
 __global__ void __launch_bounds__(kRowsThreads) k_rows_apply(RowOp A, const double *x, double *y, const int32_t *new2old) {
   constexpr int VW = DIM == 3 ? 4 : 2;
   const int64_t s = blockIdx.x * (int64_t)(kRowsThreads / 32) + (threadIdx.x >> 5);
@@ -163,7 +184,7 @@ __global__ void __launch_bounds__(kRowsThreads) k_rows_apply(RowOp A, const doub
     const NodeV<double, VW> own = X(row < 0 ? 0 : row);
 #pragma unroll
     for (int d = 0; d < DIM; ++d) xi[d] = own.v[d];
-    rows_product_of<DIM>(A, s, row, X, xi, v);
+    rows_product_of<DIM, WIDE>(A, s, row, X, xi, v);
   };
   if constexpr (CALLER) product(CallerX<DIM>{x, new2old});
   else product(NodeX<DIM>{x});
@@ -190,7 +211,7 @@ struct RowsResidual {
   double *out, *partials;
   unsigned int *count;
 };
-template <int DIM>
+template <int DIM, bool WIDE>
 __global__ void __launch_bounds__(kRowsThreads) k_rows_residual(RowOp A, RowsResidual P) {
   constexpr int VW = DIM == 3 ? 4 : 2;
   double acc[2] = {0, 0};
@@ -200,7 +221,7 @@ __global__ void __launch_bounds__(kRowsThreads) k_rows_residual(RowOp A, RowsRes
     int row;
     if (P.x) {
       row = rows_own<DIM>(A, s, P.x, xi);
-      rows_product<DIM>(A, s, row, P.x, xi, v);
+      rows_product<DIM, WIDE>(A, s, row, P.x, xi, v);
     } else {
       row = A.row[s * kSliceRows + (threadIdx.x & 15)];
 #pragma unroll
@@ -255,7 +276,9 @@ static __global__ void __launch_bounds__(kThreads) k_rows_cases_residual(RowsCas
     const int t = (int)(slot % kSliceRows), row = A.row[slot], i = row < 0 ? 0 : row;
     const int64_t k0 = A.off[s];
     const int n = (int)(A.off[s + 1] - k0);
-    const bool masked = A.flag[s] != 0;
+    const unsigned flag = A.flag[s];
+    const bool masked = flag != 0, wide = flag & kWideSlice;
+    if (wide && row < 0) continue;
     const unsigned b = masked ? A.bits[i] : 0u;
     NodeV<double, 4> own = ldv<double, 4>(P.x, (int64_t)i * K + c);
     double xi[DIM], y[DIM];
@@ -266,10 +289,12 @@ static __global__ void __launch_bounds__(kThreads) k_rows_cases_residual(RowsCas
     }
     const int32_t *col = A.col + k0 * 32 + t;
     const double *val = A.val + k0 * (32 * DIM * DIM) + t;
-    for (int k = 0; k < n; ++k)
+    const int n_here = wide ? 16 * n : n;  // (a slice of one row: entry by entry)
+    for (int kk = 0; kk < n_here; ++kk)
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        const int32_t j = col[k * 32 + half * 16];
+        const int k = wide ? kk >> 4 : kk, at = half * 16 + (wide ? kk & 15 : 0);
+        const int32_t j = col[k * 32 + at];
         NodeV<double, 4> v = ldv<double, 4>(P.x, (int64_t)j * K + c);
         if (masked) {
           const unsigned bj = A.bits[j];
@@ -279,7 +304,7 @@ static __global__ void __launch_bounds__(kThreads) k_rows_cases_residual(RowsCas
         }
         double M[DIM * DIM];
 #pragma unroll
-        for (int q = 0; q < DIM * DIM; ++q) M[q] = val[(k * DIM * DIM + q) * 32 + half * 16];
+        for (int q = 0; q < DIM * DIM; ++q) M[q] = val[(k * DIM * DIM + q) * 32 + at];
 #pragma unroll
         for (int q = 0; q < DIM; ++q) {
           const double du = v.v[q] - xi[q];
@@ -348,7 +373,7 @@ struct RowsPcg {
 constexpr int kRowsPcgThreads = 512, kRowsPcgSmall = 128;
 constexpr int kRowsPcgSets = 5;  // start; p.Ap and r.z of even, of odd iterations
 
-template <int DIM, bool RESIDENT, int THREADS>
+template <int DIM, bool RESIDENT, int THREADS, bool WIDE = false>
 __global__ void __launch_bounds__(THREADS, 1) k_rows_pcg(RowsPcg P) {
   constexpr int WARPS = THREADS / 32;
   constexpr int VW = DIM == 3 ? 4 : 2;
@@ -409,7 +434,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_rows_pcg(RowsPcg P) {
     for (int d = 0; d < DIM; ++d) p[d] = y[d] = 0;
     if (mine) {
       row = rows_own<DIM>(A, s, P.x, p);
-      if (P.warm) rows_product<DIM>(A, s, row, P.x, p, y);
+      if (P.warm) rows_product<DIM, WIDE>(A, s, row, P.x, p, y);
       own_of(p, x);
       own_of(y, yo);
       NodeV<double, VW> f = ldv<double, VW>(P.f, row < 0 ? 0 : row), di = ldv<double, VW>(P.dinv, row < 0 ? 0 : row);
@@ -437,7 +462,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_rows_pcg(RowsPcg P) {
       for (int64_t q = s0 + wid; q < s1; q += WARPS) {
         double xi[DIM], v[DIM];
         const int i = rows_own<DIM>(A, q, P.x, xi);
-        rows_product<DIM>(A, q, i, P.x, xi, v);
+        rows_product<DIM, WIDE>(A, q, i, P.x, xi, v);
         if (i >= 0 && !half) {
           NodeV<double, VW> o;
 #pragma unroll
@@ -484,7 +509,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_rows_pcg(RowsPcg P) {
     double e[1] = {0};
     if constexpr (RESIDENT) {
       if (mine) {
-        rows_product<DIM>(A, s, row, P.p, p, y);
+        rows_product<DIM, WIDE>(A, s, row, P.p, p, y);
         double po[OWN];
         own_of(y, yo);
         own_of(p, po);
@@ -496,7 +521,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_rows_pcg(RowsPcg P) {
       for (int64_t q = s0 + wid; q < s1; q += WARPS) {
         double pi[DIM], v[DIM];
         const int i = rows_own<DIM>(A, q, P.p, pi);
-        rows_product<DIM>(A, q, i, P.p, pi, v);
+        rows_product<DIM, WIDE>(A, q, i, P.p, pi, v);
         if (i >= 0 && !half) {
           NodeV<double, VW> o;
 #pragma unroll
@@ -698,9 +723,10 @@ __device__ __forceinline__ void sort_list(int32_t *a, int n) {
 
 // One thread per node: its elements sorted, its neighbours sorted and unique
 // in nbr[(NV - 1) * inc_off[n] ..], their number in deg.
+// n_wide: nodes of more than kWideDegree neighbours are counted.
 template <int NV>
 __global__ void k_rows_neighbours(int64_t nn, const int32_t *conn, const int32_t *inc_off, int32_t *inc, int32_t *nbr,
-                                  int32_t *deg) {
+                                  int32_t *deg, int32_t *n_wide) {
   const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= nn) return;
   const int32_t i0 = inc_off[n], m = inc_off[n + 1] - i0;
@@ -733,6 +759,7 @@ __global__ void k_rows_neighbours(int64_t nn, const int32_t *conn, const int32_t
     c = u;
   }
   deg[n] = c;
+  if (c > kWideDegree) atomicAdd(n_wide, 1);
 }
 
 // Rows of each window by descending neighbour count (ties by node), and the
@@ -749,6 +776,35 @@ static __global__ void __launch_bounds__(kRowWindow) k_rows_order(int64_t nn, co
   for (int j = 0; j < kRowWindow; ++j) rank += d[j] > mine || (d[j] == mine && j < t);
   row[base + rank] = t < n ? (int32_t)(base + t) : -1;
   if (rank % kSliceRows == 0) steps[(base + rank) / kSliceRows] = mine < 0 ? 0 : (mine + 1) / 2;
+}
+
+// The same where there are nodes of many neighbours: they come first in their
+// window's slices, one in each. First the slices of every window, then rows (-1 at
+// the start) and steps, with `first` the windows' first slices.
+static __global__ void __launch_bounds__(kRowWindow) k_rows_window_slices(int64_t nn, const int32_t *deg, int32_t *slices) {
+  const int64_t i = (int64_t)blockIdx.x * kRowWindow + threadIdx.x;
+  const int wide = __syncthreads_count(i < nn && deg[i] > kWideDegree);
+  const int n = (int)min((int64_t)kRowWindow, nn - (int64_t)blockIdx.x * kRowWindow);
+  if (threadIdx.x == 0) slices[blockIdx.x] = wide + (n - wide + kSliceRows - 1) / kSliceRows;
+}
+static __global__ void __launch_bounds__(kRowWindow)
+    k_rows_order_wide(int64_t nn, const int32_t *deg, const int32_t *first, int32_t *row, int32_t *steps, uint8_t *wide) {
+  __shared__ int32_t d[kRowWindow];
+  const int64_t base = (int64_t)blockIdx.x * kRowWindow;
+  const int t = threadIdx.x, n = (int)min((int64_t)kRowWindow, nn - base);
+  const int mine = t < n ? deg[base + t] : -1;
+  d[t] = mine;
+  const int n_wide = __syncthreads_count(mine > kWideDegree);
+  if (t >= n) return;
+  int rank = 0;
+  for (int j = 0; j < kRowWindow; ++j) rank += d[j] > mine || (d[j] == mine && j < t);
+  const bool own = rank < n_wide;
+  const int q = rank - n_wide, s = first[blockIdx.x] + (own ? rank : n_wide + q / kSliceRows), at = own ? 0 : q % kSliceRows;
+  row[(int64_t)s * kSliceRows + at] = (int32_t)(base + t);
+  if (at == 0) {
+    steps[s] = own ? (mine + 31) / 32 : (mine + 1) / 2;
+    wide[s] = own ? kWideSlice : 0;
+  }
 }
 
 // P_i K_ij P_j of the pair from the elements that hold both (in element order,
@@ -851,11 +907,12 @@ constexpr int kLongList = 64;  // elements that one lane goes through alone
 template <int DIM>
 __global__ void __launch_bounds__(32 * kAssembleWarps) k_rows_assemble(RowsAssembly<DIM> P, const int64_t *off,
                                                        const int32_t *row, const int32_t *nbr, const int32_t *deg,
-                                                       int32_t *col, double *val) {
+                                                       int32_t *col, double *val, const uint8_t *flag) {
   constexpr int NC = DIM * DIM, NV = DIM + 1;
   const int64_t s = blockIdx.x;
-  const int lane = threadIdx.x & 31, half = lane >> 4;
-  const int32_t i = row[s * kSliceRows + (lane & 15)];
+  const bool wide = flag[s] & kWideSlice;
+  const int lane = threadIdx.x & 31;
+  const int32_t i = row[s * kSliceRows + (wide ? 0 : lane & 15)];
   const int64_t k0 = off[s];
   const int n = (int)(off[s + 1] - k0);
   const unsigned bi = i < 0 ? 0u : P.bits[i];
@@ -864,7 +921,8 @@ __global__ void __launch_bounds__(32 * kAssembleWarps) k_rows_assemble(RowsAssem
     int32_t j;
     if (nbr) {  // first assembly: the columns from the neighbour lists
       j = i < 0 ? 0 : i;
-      if (i >= 0 && 2 * k + half < deg[i]) j = nbr[(int64_t)(NV - 1) * P.inc_off[i] + 2 * k + half];
+      const int at_i = wide ? 32 * k + lane : 2 * k + (lane >> 4);
+      if (i >= 0 && at_i < deg[i]) j = nbr[(int64_t)(NV - 1) * P.inc_off[i] + at_i];
       col[at] = j;
     } else {
       j = col[at];
@@ -927,9 +985,11 @@ __global__ void k_rows_corrections(RowsAssembly<DIM> P, int64_t n_rows, const in
 #pragma unroll
   for (int p = 0; p < DIM; ++p) diag[p] = 0;
   bool any = i >= 0 && (bi != 0 || P.cM != 0);
+  const bool wide = i >= 0 && (flag[s] & kWideSlice);
+  const int width = wide ? 1 : 16;  // entries q of the row are this far apart
   if (i >= 0)
-    for (int64_t q = 2 * off[s] + part; q < 2 * off[s + 1]; q += kCorrLanes) {  // (step q / 2, half q & 1)
-      const int32_t j = col[q * 16 + (t & 15)];
+    for (int64_t q = 32 / width * off[s] + part; q < 32 / width * off[s + 1]; q += kCorrLanes) {
+      const int32_t j = col[q * width + (t & 15)];
       if (j == i) continue;
       const unsigned bj = P.bits[j];
       if (bj == bi && P.cM == 0) continue;
@@ -990,7 +1050,7 @@ __global__ void k_rows_corrections(RowsAssembly<DIM> P, int64_t n_rows, const in
 #pragma unroll
   for (int c = 0; c < NC; ++c)
     if (c % kCorrLanes == part) D[(int64_t)i * NC + c] = B[c];
-  if (any) flag[s] = 1;
+  if (any) flag[s] = wide ? kWideSlice | kHasD : kHasD;  // (the same from every lane)
 }
 
 }  // namespace cfem

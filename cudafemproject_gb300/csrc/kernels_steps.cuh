@@ -105,7 +105,7 @@ struct RowsSteps {
   int *stalled;
 };
 
-template <int DIM, bool RESIDENT>
+template <int DIM, bool RESIDENT, bool WIDE = false>
 __global__ void __launch_bounds__(kStepThreads, 1) k_rows_steps(RowsSteps P) {
   constexpr int VW = DIM == 3 ? 4 : 2;
   constexpr int OWN = DIM == 3 ? 2 : 1;
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) k_rows_steps(RowsSteps P) {
       }
     auto step = [&](int64_t s) {
       double y[DIM];
-      rows_product<DIM>(A, s, row, cur, d, y);
+      rows_product<DIM, WIDE>(A, s, row, cur, d, y);
 #pragma unroll
       for (int k = 0; k < OWN; ++k) {
         const double yk = half ? (OWN + k < DIM ? y[OWN + k < DIM ? OWN + k : 0] : 0.0) : y[k];
@@ -260,7 +260,7 @@ struct RowsReverse {
   int *stalled;
 };
 
-template <int DIM, bool RESIDENT>
+template <int DIM, bool RESIDENT, bool WIDE = false>
 __global__ void __launch_bounds__(kStepThreads, 1) k_rows_reverse(RowsReverse P) {
   constexpr int VW = DIM == 3 ? 4 : 2;
   constexpr int OWN = DIM == 3 ? 2 : 1;
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) k_rows_reverse(RowsReverse P)
   };
   auto after = [&](int64_t s, int n) {
     double y[DIM];
-    rows_product<DIM>(A, s, row, P.w + (int64_t)(n - P.n0) * P.stride, w, y);
+    rows_product<DIM, WIDE>(A, s, row, P.w + (int64_t)(n - P.n0) * P.stride, w, y);
 #pragma unroll
     for (int k = 0; k < OWN; ++k) {
       const double yk = half ? (OWN + k < DIM ? y[OWN + k < DIM ? OWN + k : 0] : 0.0) : y[k];

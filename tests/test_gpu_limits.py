@@ -293,3 +293,32 @@ def test_moduli_of_nodes_of_many_elements_take_linear_time():
         return sorted(ts)[4]
 
     assert seconds(8000) <= 40 * seconds(500)
+
+
+@pytest.mark.parametrize("semantics", ["consistent", "compat"])
+@pytest.mark.parametrize("n_rim", [63, 64, 65, 300])
+def test_steps_with_nodes_of_many_elements(n_rim, semantics):
+    """Explicit and implicit FP64 steps and the steps' adjoint on rows of their own
+    slices (n_rim + 1 neighbours each, the limit is 64), against the oracle and a
+    central difference of the loss."""
+    from cudafemproject_gb300.solver import FemContext
+    p = _hub(n_rim)
+    p.load_node, p.load_vec = np.array([0, 40], np.int32), np.array([[0.1, 0.2, -1.0], [1.0, 0.0, 0.5]])
+    dt, rec = 1e-6, np.array([0, 1, 50], np.int32)
+    ctx, o = FemContext(p, semantics=semantics), O.Oracle(p, consistent=semantics == "consistent")
+    for steps in (1, 5):
+        ug, st, _ = o.dyn(0.5, 0.0, dt, steps * dt * 1.0000001)
+        u, _, trace = ctx.dyn(0.5, 0.0, dt, steps * dt * 1.0000001, precision="fp64", receivers=rec)
+        # (a few steps with other summation orders, rows of n_rim products)
+        assert rel(u, ug) <= 1e-10 and np.array_equal(trace[-1], u[rec])
+    if semantics == "consistent":
+        obs = np.zeros((4, 3, 3))
+        young = np.full(p.n_elems, p.E)
+        loss, g, _ = ctx.dyn_adjoint(0.5, dt, 4 * dt * 1.0000001, rec, obs)
+        d = young * np.random.default_rng(1).standard_normal(p.n_elems) * 1e-4
+        ends = []
+        for s in (1, -1):
+            ctx.set_young(young + s * d)
+            ends.append(ctx.dyn_adjoint(0.5, dt, 4 * dt * 1.0000001, rec, obs)[0])
+        # (the loss is smooth in the moduli: the difference's error is of order 1e-8)
+        assert (ends[0] - ends[1]) / 2 == pytest.approx(float(g @ d), rel=1e-5, abs=1e-9 * abs(loss))
