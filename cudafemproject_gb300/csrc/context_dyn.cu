@@ -865,6 +865,45 @@ cfem_status cfem_dyn(cfem_ctx *ctx, const cfem_dyn_params *prm, const cfem_wavel
   });
 }
 
+cfem_status cfem_selftest_grid_timeout(cfem_ctx *ctx) {
+  return run_guarded([&]() -> cfem_status {
+    check_ctx(ctx);
+    single_mesh_only(ctx);
+    if (ctx->rows.n_slices <= 4 || ctx->semantics != CFEM_CONSISTENT)
+      throw Fail{CFEM_ERR_UNSUPPORTED, "the self-test needs consistent semantics and more than one CTA of node rows"};
+    enter(ctx);
+    // which: the cooperative launch of the call that runs without its CTA 0
+    auto reported = [&](const char *what, int which, const std::function<void()> &call) {
+      ctx->selftest_absent = which;
+      bool seen = false;
+      try {
+        call();
+      } catch (const Fail &f) {
+        ctx->selftest_absent = 0;
+        if (f.st != CFEM_ERR_CUDA || f.msg.find("did not arrive") == std::string::npos) throw;
+        seen = true;
+      }
+      ctx->selftest_absent = 0;
+      if (!seen) throw Fail{CFEM_ERR_CUDA, std::string("a missing CTA of ") + what + " was not reported"};
+    };
+    ctx->v64.f.zero(ctx->stream);
+    set_diag_vectors(ctx);
+    reported("the FP64 PCG", 1, [&]() { run_pcg_d(ctx, ctx->v64, 1.0, 0.0, nullptr, 0, 1e-8, CFEM_STOP_RESIDUAL, 10); });
+    std::vector<double> u(ctx->nd), obs(3 * (size_t)ctx->dim, 0.0);
+    const int32_t node = 0;
+    cfem_dyn_params prm{};
+    prm.beta1 = 0.5;
+    prm.dt = 1e-9;
+    prm.endtime = 3.0000003e-9;
+    prm.precision = CFEM_FP64;
+    reported("the time steps", 1, [&]() { run_dyn<double>(ctx, &prm, nullptr, u.data(), nullptr); });
+    reported("the steps' adjoint", 2, [&]() {
+      run_dyn_adjoint(ctx, &prm, nullptr, 1, &node, obs.data(), nullptr, nullptr, nullptr);
+    });
+    return CFEM_OK;
+  });
+}
+
 cfem_status cfem_adjoint(cfem_ctx *ctx, const cfem_solve_params *prm, const double *u, const double *dLdu, double *dLdE,
                          double *dLdf, cfem_solve_info *info) {
   return run_guarded([&]() -> cfem_status {

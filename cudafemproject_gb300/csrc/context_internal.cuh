@@ -187,6 +187,7 @@ struct cfem_ctx {
   int *h_tma_err = nullptr;  // pinned; written by a kernel whose copy wait ran out
   int selftest_skip_plus1 = 0;       // FanTmaParams::skip_patch_plus1 (cfem_selftest_copy_timeout only)
   long long selftest_wait_limit = 0;  // FanTmaParams::wait_limit (likewise)
+  int selftest_absent = 0;            // the n-th cooperative launch from here runs without its CTA 0 (cfem_selftest_grid_timeout only)
   size_t smem_ft32 = 0;
   int grid_ft32 = 0;
   // geometry blocks (FP32 single-RHS matvec of CFEM_FORM_GEOMETRY_FAN): the

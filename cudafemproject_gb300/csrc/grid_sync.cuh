@@ -34,6 +34,7 @@ struct GridSync {
   unsigned long long *slots;  // [sets][kMaxGridSums][copies][grid], all kSlotEmpty at launch
   unsigned *arrived;          // CTAs arrived at barriers, zero at launch
   long long limit;            // clock64 cycles a CTA waits for the others
+  int absent_plus1;           // self-test: CTA that leaves the kernel at its start, plus one; else 0
 };
 
 __host__ __device__ inline int grid_copies(int grid) { return (grid + kGridReaders - 1) / kGridReaders; }

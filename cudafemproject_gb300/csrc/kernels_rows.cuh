@@ -380,6 +380,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_rows_pcg(RowsPcg P) {
   constexpr int OWN = DIM == 3 ? 2 : 1;
   __shared__ GridShared<THREADS> sh;
   const GridSync &G = P.sync;
+  if (G.absent_plus1 == (int)blockIdx.x + 1) return;  // (self-test of the waits for it)
   const RowOp &A = P.A;
   const int wid = threadIdx.x >> 5, half = (threadIdx.x >> 4) & 1;
   // the CTA's slices, neighbours in node order

@@ -344,6 +344,13 @@ CFEM_API cfem_status cfem_matvec_energy_noalloc(cfem_ctx *ctx, const double *x, 
  * block. Has no counterpart in the reference (its GPU path has no bulk
  * copies). */
 CFEM_API cfem_status cfem_selftest_copy_timeout(cfem_ctx *ctx);
+/* The same for the grid-wide exchanges of the cooperative FP64 kernels
+ * (single-mesh contexts with consistent semantics and more than 64 nodes): the
+ * PCG, the explicit time steps and their adjoint are each launched without one
+ * of their CTAs, whose others give up waiting for it after ~1 ms. Returns CFEM_OK when each
+ * kernel has returned and reported it as CFEM_ERR_CUDA ("... did not arrive
+ * ..."); the context stays usable. */
+CFEM_API cfem_status cfem_selftest_grid_timeout(cfem_ctx *ctx);
 /* Per-element Young's modulus update (keeps geometry; rebuilds operator scale). */
 CFEM_API cfem_status cfem_set_young(cfem_ctx *ctx, const double *elem_young);
 

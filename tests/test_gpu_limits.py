@@ -322,3 +322,27 @@ def test_steps_with_nodes_of_many_elements(n_rim, semantics):
             ends.append(ctx.dyn_adjoint(0.5, dt, 4 * dt * 1.0000001, rec, obs)[0])
         # (the loss is smooth in the moduli: the difference's error is of order 1e-8)
         assert (ends[0] - ends[1]) / 2 == pytest.approx(float(g @ d), rel=1e-5, abs=1e-9 * abs(loss))
+
+
+@pytest.mark.parametrize("mesh", ["box", "large", "plate", "hub"])
+def test_missing_cta_is_reported_and_context_recovers(mesh):
+    """The failure path of the cooperative FP64 kernels' exchanges, without a fault:
+    each is launched without its CTA 0, with waits bounded at ~1 ms. The others
+    give up and return, the host reports it, and the context then works: rows in
+    registers, in memory (more slices than warps), 2D, rows of a warp."""
+    from cudafemproject_gb300 import capi
+    from cudafemproject_gb300.solver import FemContext
+    p = {"box": lambda: meshgen.box_3d(6, 6, 18, jitter=0.2, seed=2), "large": lambda: meshgen.box_3d(24, 24, 72, jitter=0.2, seed=2),
+         "plate": lambda: meshgen.square_2d(30), "hub": lambda: _hub(120)}[mesh]()
+    ctx = FemContext(p, semantics="consistent")
+    L = capi.lib()
+    for _ in range(2):
+        assert L.cfem_selftest_grid_timeout(ctx._h) == capi.OK, L.cfem_last_error_string()
+    x = np.random.default_rng(1).standard_normal(p.n_dof)
+    f = ctx.matvec(x, "fp64")
+    u, info = ctx.pcg(f, "fp64", tol=1e-10, stop_rule="residual")
+    # (the residual's floor, and the condition number in front of the difference)
+    assert info["status"] == 0 and info["rel_residual"] <= 1e-9
+    ud, info = ctx.dyn(0.5, 0.0, 1e-9, 3.0000003e-9, precision="fp64")
+    assert info["steps"] == 3 and np.isfinite(ud).all()
+    assert L.cfem_selftest_grid_timeout(FemContext(meshgen.square_2d(4), semantics="consistent")._h) == capi.ERR_UNSUPPORTED
