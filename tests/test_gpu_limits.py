@@ -346,3 +346,59 @@ def test_missing_cta_is_reported_and_context_recovers(mesh):
     ud, info = ctx.dyn(0.5, 0.0, 1e-9, 3.0000003e-9, precision="fp64")
     assert info["steps"] == 3 and np.isfinite(ud).all()
     assert L.cfem_selftest_grid_timeout(FemContext(meshgen.square_2d(4), semantics="consistent")._h) == capi.ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("form", ["auto", "geometry", "gradient"])
+@pytest.mark.parametrize("semantics", ["consistent", "compat"])
+@pytest.mark.parametrize("beta2", [0.0, 0.5])
+def test_fp32_traces_row_by_row(beta2, semantics, form):
+    """FP32 steps on a mesh of one patch, where no sum depends on the order of atomic
+    additions: row n of the receiver trace is the displacement that n steps end
+    with, bit by bit, on a fresh context as on one that has run before with another
+    context's run in between."""
+    from cudafemproject_gb300.meshio import WaveletParams
+    from cudafemproject_gb300.solver import FemContext
+    p = meshgen.box_3d(3, 3, 8, jitter=0.2, seed=5, rho=2000.0, traction=None, point_load=("top_centre", (0.4, -0.3, -1.0)))
+    dt = 2e-5 if beta2 == 0 else 1e-3
+    rec = np.array([int(p.load_node[0]), p.n_nodes - 1, p.n_nodes // 2], np.int32)
+    w = WaveletParams("ricker", 40.0, 0.0, 1.0)
+
+    def run(ctx, n):
+        return ctx.dyn(0.5, beta2, dt, n * dt * 1.0000001, precision="fp32", wavelet=w, pcg_tol=1e-6, receivers=rec)
+
+    ctx, other = (FemContext(p, semantics=semantics, matvec_form=form) for _ in range(2))
+    assert ctx.counts()["n_patches"] == 1
+    N = 15
+    u, _, trace = run(ctx, N)
+    assert np.array_equal(trace[-1], u[rec]) and trace.any()
+    for n in range(1, N + 1):
+        un, _, tn = run(ctx, n)
+        assert np.array_equal(un[rec], trace[n - 1]) and np.array_equal(tn, trace[:n]), n
+        run(other, 4)
+    assert np.array_equal(run(ctx, N)[0], u)
+
+
+@pytest.mark.parametrize("side", ["largest", "smallest"])
+@pytest.mark.parametrize("limit", [4, 16])
+def test_fp64_pcg_shapes_on_either_side_of_their_limits(limit, side):
+    """The one-kernel PCG has at most four slices of 16 rows per CTA (128 threads), at
+    most sixteen (512), or more: plates with the most nodes on one side of a limit
+    on this GPU and the fewest on the other, and some tens of CTAs of the first
+    kind. Iterates 1 and 2 (two recurrences that differ in the order of their sums:
+    1e-12) and a converged solve (1e-10, the bar of every FP64 solve)."""
+    import torch
+    from cudafemproject_gb300.solver import FemContext
+    slices = limit * torch.cuda.get_device_properties(0).multi_processor_count
+    n = max(n for n in range(2, 400) if -(-(n + 1) ** 2 // 16) <= slices) + (side == "smallest")
+    for m in {n, 40 if (limit, side) == (4, "largest") else n}:
+        p = meshgen.square_2d(m)
+        f = np.zeros((p.n_nodes, 2))
+        f[p.nodes[:, 0] > 1 - 1e-9] = (0.7, -0.2)
+        f = f.ravel()
+        ctx, o = FemContext(p, semantics="consistent"), O.Oracle(p, consistent=True)
+        for iters in (1, 2):
+            x, it = o.pcg(f, tol=1e-30, rule=1, maxit=iters, allow_maxit=True)
+            u, info = ctx.pcg(f, "fp64", tol=1e-30, stop_rule="residual", max_iter=iters, allow_not_converged=True)
+            assert info["iterations"] == it == iters and rel(u, x) <= 1e-12
+        u, _ = ctx.pcg(f, "fp64", tol=1e-13, stop_rule="residual")
+        assert rel(u, o.pcg(f, tol=1e-13, rule=1)[0]) <= 1e-10
