@@ -411,8 +411,8 @@ extern "C" cfem_status cfem_batch_static_solve(cfem_ctx *ctx, const cfem_solve_p
       // the recurrence still is the true residual (k_fold_instance). 12 boxes, 6 to
       // 20 cells across, to 1e-9, fresh starts and so: inner tolerance 0.3
       // 118 -> 58 ms, 0.1 86.5 -> 63.6, 0.01 69.7 -> 55.7, 1e-4 and below as
-      // before. (Legs as in solve_internal: 16 small boxes at 1e-4 25.6 -> 32.9, a
-      // round waits for its slowest instance.)
+      // before. (Steps cut into runs of 512 iterations: 16 small boxes at 1e-4
+      // 25.6 -> 32.9, a round waits for its slowest instance.)
       std::vector<PcgCont> cont(n);
       for (int round = 0; round <= max_outer; ++round) {
         int n_act = 0;

@@ -256,9 +256,11 @@ constexpr int kStepCycle = 6;
 
 // Iterations per body of the PCG loop of an implicit step. A body costs about 5
 // us beyond its iterations, an iteration past the stop as much as the body's
-// share of 4; warm-started steps take 10 to 50 iterations (20 steps of 18
-// iterations on 196,608 tets: bodies of 4 and 10 6.0 ms, 6, 8 and 12 6.35, 16 7.2:
-// the fewer iterations past the 18th).
+// share of 4: what is best depends on where a step's count lies between multiples
+// of the body (20 steps on 24,576 to 1.5 M tets, bodies of 4 / 8 / 16: 12 and 13
+// iterations per step 4.0 / 3.85 / 3.7 and 12.5 / 12.3 / 12.2 ms, 18 6.2 / 6.55 /
+// 7.3, 27 9.0 / 9.1 / 8.9, 42 34.9 / 35.1 / 34.8; long steps, 129 to 520
+// iterations, 2 to 9% longer than with 16).
 constexpr int kStepChunk = 4;
 
 template <typename T>

@@ -365,13 +365,13 @@ struct RowsPcg {
   const double *f, *dinv;
   double *x, *r, *z, *p, *u;  // RESIDENT: x and p only
   Scalars *sc;                // tol, rule, maxit in; the run's scalars out
-  GridSync sync;              // two sets of slots for the loop, one for the start
+  GridSync sync;              // kRowsPcgSets sets of slots
   int warm;                   // start from x
 };
 // Threads: 512 fill the FP64 pipe and hide the loads; 128, where no CTA has
 // more than four slices, shorten every sum by three FP64 additions.
 constexpr int kRowsPcgThreads = 512, kRowsPcgSmall = 128;
-constexpr int kRowsPcgSets = 5;  // start; p.Ap and r.z of even, of odd iterations
+constexpr int kRowsPcgSets = 5;  // one for the start; of even and of odd iterations, p.Ap and r.z with r.r
 
 template <int DIM, bool RESIDENT, int THREADS, bool WIDE = false>
 __global__ void __launch_bounds__(THREADS, 1) k_rows_pcg(RowsPcg P) {

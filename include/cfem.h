@@ -17,8 +17,9 @@
  *  - Vectors (displacements, right-hand sides) are in the caller's node order,
  *    DIM values per node, like dataKeeper::get_displacements()
  *    (datakeeper.cpp:64-66). Unless stated otherwise an array argument may be
- *    host memory or device memory of the context's GPU (copied with
- *    cudaMemcpyDefault on the context's stream).
+ *    host memory or device memory of the context's GPU. Vectors in device memory
+ *    aligned to their elements are read and written in place by kernels on the
+ *    context's stream; everything else is copied there with cudaMemcpyDefault.
  *  - One context per stream; no global mutable state besides the per-thread
  *    error string (replaces the reference's static cuBLAS handle,
  *    cuda_matrix.cpp:3-8) and the one device scratch array shared by all
