@@ -523,11 +523,11 @@ cfem_status solve_internal(cfem_ctx *c, const cfem_solve_params *prm, cfem_solve
       // Replaced seldom, the recursive residual drifts too far from the true
       // one for the old direction to stay conjugate, so tighter inner
       // tolerances restart. (Steps of tight tolerances cut into legs of 512
-      // iterations that keep their direction took 13% less time on 2.65 M tets, as
-      // long on smaller meshes, and ended slender beams, 150 to 300 cells long,
-      // as converged at relative residuals of 0.07 to 15: whole runs get there
-      // because their recurrence goes on through thousands of iterations in which
-      // the residual rises.)
+      // iterations that keep their direction took up to a third less time on
+      // well-conditioned meshes and up to ten times as long on slender beams, 100
+      // to 300 cells, which they ended as converged at relative residuals of 0.07
+      // to 15: whole runs get there because their recurrence goes on through
+      // thousands of iterations in which the residual rises.)
       cont.p = prm->tol >= kContinueTol && r.iters > 0 ? (((r.iters - 1) & 1) ? c->v32.pA.p : c->v32.pB.p) : nullptr;
       cont.gamma_prev = r.gamma_prev;
       total += r.iters;
