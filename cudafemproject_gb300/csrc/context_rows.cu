@@ -59,7 +59,7 @@ void build_structure(cfem_ctx *c, DBuf<int32_t> &nbr, DBuf<int32_t> &deg) {
   k_rows_scan<int32_t><<<1, 1024, 0, s>>>(nn, cnt, R.inc_off.p);
   CK(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * nn, s));
   k_rows_fill<<<nblk(n_inc), kThreads, 0, s>>>(n_inc, NV, c->conn.p, R.inc_off.p, cnt, R.inc.p);
-  k_rows_neighbours<NV><<<nblk(nn), kThreads, 0, s>>>(nn, c->conn.p, R.inc_off.p, R.inc.p, nbr.p, deg.p, n_wide);
+  k_rows_neighbours<NV><<<nblk(nn, 32), 32, 0, s>>>(nn, c->conn.p, R.inc_off.p, R.inc.p, nbr.p, deg.p, n_wide);
   k_rows_order<<<(unsigned)windows, kRowWindow, 0, s>>>(nn, deg.p, R.row.p, steps);
   k_rows_scan<int64_t><<<1, 1024, 0, s>>>(R.n_slices, steps, R.off.p);
   CKL();

@@ -722,7 +722,8 @@ __device__ __forceinline__ void sort_list(int32_t *a, int n) {
   }
 }
 
-// One thread per node: its elements sorted, its neighbours sorted and unique
+// One thread per node (blocks of one warp: the lists of 256 nodes do not stay in an
+// L1): its elements sorted, its neighbours sorted and unique
 // in nbr[(NV - 1) * inc_off[n] ..], their number in deg.
 // n_wide: nodes of more than kWideDegree neighbours are counted.
 template <int NV>
@@ -898,12 +899,13 @@ __device__ __forceinline__ void pair_block(const RowsAssembly<DIM> &P, int32_t i
   }
 }
 
-// Columns (first assembly) and blocks, four warps per slice: a step is a chain of
+// Columns (first assembly) and blocks, eight warps per slice: a step is a chain of
 // dependent loads (lists, elements, gradients), so the steps of a slice side by
 // side are what a small mesh has to fill the GPU with. Whole cfem_set_young, one
-// warp per slice and so: 12,288 tets 0.42 -> 0.20 ms, 98,304 0.54 -> 0.38,
-// 2.65 M 5.73 -> 5.55, 130,000 Delaunay tets 1.50 -> 0.64.
-constexpr int kAssembleWarps = 4;
+// warp per slice and so: 12,288 tets 0.42 -> 0.18 ms, 98,304 0.54 -> 0.36,
+// 2.65 M 5.73 -> 5.6, 130,000 Delaunay tets 1.50 -> 0.59. (Four warps, and eight
+// lanes per row of the corrections below: 0.20, 0.38, 5.55, 0.64.)
+constexpr int kAssembleWarps = 8;
 constexpr int kLongList = 64;  // elements that one lane goes through alone
 template <int DIM>
 __global__ void __launch_bounds__(32 * kAssembleWarps) k_rows_assemble(RowsAssembly<DIM> P, const int64_t *off,
@@ -967,10 +969,10 @@ __global__ void __launch_bounds__(32 * kAssembleWarps) k_rows_assemble(RowsAssem
   }
 }
 
-// D blocks: what the difference form misses (see the head of this file), eight
+// D blocks: what the difference form misses (see the head of this file), sixteen
 // lanes per row, which share its neighbours and elements; a slice with any is
 // flagged.
-constexpr int kCorrLanes = 8;
+constexpr int kCorrLanes = 16;
 template <int DIM>
 __global__ void k_rows_corrections(RowsAssembly<DIM> P, int64_t n_rows, const int64_t *off, const int32_t *row,
                                    const int32_t *col, double *D, uint8_t *flag) {
