@@ -1,5 +1,7 @@
 """Calls at their limits: loads that underflow in single precision, bodies that
-need thousands of iterations."""
+need thousands of iterations, contexts that step in several threads, time steps
+that do not converge, iteration caps, little free memory, nodes of many elements,
+kernels whose CTAs do not all arrive, traces row by row."""
 import numpy as np
 import pytest
 
@@ -15,8 +17,7 @@ pytestmark = pytest.mark.gpu
 def test_refinement_of_loads_below_single_precision(tol, rule):
     """Entries of 1e-20: r.z = r^2 / diag(K) is 1e-47, zero in FP32, where r.r =
     1e-40 is not. The FP32 runs take no step, and the solve ends at the second
-    step that reduces nothing, with tight inner tolerances (legs) as with loose
-    ones. The same load at a size that single precision holds is solved."""
+    step that reduces nothing, with tight inner tolerances as with loose ones. The same load at a size that single precision holds is solved."""
     from cudafemproject_gb300.solver import FemContext
     p = meshgen.box_3d(3, 3, 9, jitter=0.2, seed=2)
     f = np.random.default_rng(4).uniform(-1, 1, p.n_dof)
@@ -402,3 +403,41 @@ def test_fp64_pcg_shapes_on_either_side_of_their_limits(limit, side):
             assert info["iterations"] == it == iters and rel(u, x) <= 1e-12
         u, _ = ctx.pcg(f, "fp64", tol=1e-13, stop_rule="residual")
         assert rel(u, o.pcg(f, tol=1e-13, rule=1)[0]) <= 1e-10
+
+
+def _fan(n):
+    """A fan of n triangles around one node."""
+    from cudafemproject_gb300.meshio import Problem
+    t = 2 * np.pi * np.arange(n) / n
+    nodes = np.concatenate([[[0.0, 0.0]], np.stack([np.cos(t), np.sin(t)], axis=1)])
+    i, z = np.arange(n), np.zeros((0, 2))
+    return Problem(dim=2, nodes=nodes.astype(np.float32).astype(np.float64),
+                   elems=np.stack([np.zeros_like(i), 1 + i, 1 + (i + 1) % n], axis=1).astype(np.int32),
+                   cons=np.array([[1, 3], [4, 1], [7, 2]], np.int32), load_node=np.array([0, n // 2], np.int32),
+                   load_vec=np.array([[0.3, -1.0], [0.5, 0.2]]), face_nodes=np.zeros((0, 3), np.int32),
+                   face_elem=np.zeros(0, np.int32), face_normal=z, face_pressure=np.zeros(0), E=2e7, nu=0.25, rho=2000.0,
+                   elem_E=None)
+
+
+@pytest.mark.parametrize("body", ["fan64", "fan65", "fan300", "hub64", "hub120"])
+def test_rows_of_a_warp_in_every_fp64_call(body):
+    """Nodes of 64, 65 and more neighbours in 2D and 3D: products, a solve, explicit
+    steps and implicit ones (stiffness and mass in the same blocks) against the
+    oracle. (Products and a few explicit steps: rows of up to 300 terms, 1e-12 and
+    1e-10; a solve to 1e-13 and implicit steps whose PCG stops at 1e-12: the
+    condition number of the needles in front, up to 1e4, and two solvers: 1e-8.)"""
+    from cudafemproject_gb300.solver import FemContext
+    n = int(body[3:])
+    p = _fan(n) if body.startswith("fan") else _hub(n)
+    if body.startswith("hub"):
+        p.load_node, p.load_vec = np.array([0, 40], np.int32), np.array([[0.1, 0.2, -1.0], [1.0, 0.0, 0.5]])
+    ctx, o = FemContext(p, semantics="consistent"), O.Oracle(p, consistent=True)
+    x = np.random.default_rng(n).standard_normal(p.n_dof)
+    assert rel(ctx.matvec(x, "fp64"), o.matvec(x)) <= 1e-12
+    f = o.matvec(x)
+    assert rel(ctx.pcg(f, "fp64", tol=1e-13, stop_rule="residual")[0], o.pcg(f, tol=1e-13, rule=1)[0]) <= 1e-8
+    for beta2, dt in ((0.0, 1e-7), (0.5, 1e-5)):
+        ug, st, _ = o.dyn(0.5, beta2, dt, 3 * dt * 1.0000001, **({} if beta2 == 0 else dict(pcg_tol=1e-12)))
+        u, info = ctx.dyn(0.5, beta2, dt, 3 * dt * 1.0000001, precision="fp64", pcg_tol=1e-12)
+        assert info["steps"] == st == 3
+        assert rel(u, ug) <= (1e-10 if beta2 == 0 else 1e-8)
